@@ -238,6 +238,28 @@ def _manager(case):
     return kv
 
 
+def _stream_sets(case, src, u):
+    """Two chunks' queries, keys and values per layer (behind the projection: its raw output), taken in turn."""
+    L, H, chunk, tpf = case["layers"], case["heads"], case["chunk"], _tokens(case)
+    T, sets = chunk * tpf, []
+    for _ in range(2):
+        q = _queries(src, u, T, L, 1)                                    # [L, 1, T, H, D]
+        k = _keys(src, u, tpf, chunk, L, 1)                              # [L, 1, H, T, D]
+        v = (src.normal(L, 1, H, T, D) / 2).to(torch.bfloat16)
+        if case["kind"] == "h2o":
+            kt, vt = (t.transpose(2, 3) for t in (k, v))
+            sets.append(torch.stack([q, kt, vt], 3).reshape(L, 1, T, 3 * H * D))
+        else:
+            sets.append((q, k, v))
+    return sets
+
+
+def _chunks_seen(case):
+    """Chunks that a stream has behind it when the timed steps begin."""
+    live = 1 + case["window"] + case.get("hh", 0) + case["chunk"]
+    return max(96 if case["kind"] == "stac" else 0, live + 2 * case["chunk"]) // case["chunk"]
+
+
 def _retrieval_due(case, step):
     """The streaming loop's schedule in the steady state: once per window's worth of chunks."""
     return step % max(1, case["window"] // case["chunk"]) == 0
@@ -250,7 +272,7 @@ def _prepare_stream(case, src):
     their heavy-hitter scores along instead of computing them."""
     kind, L, H, chunk, tpf = case["kind"], case["layers"], case["heads"], case["chunk"], _tokens(case)
     kv = _manager(case)
-    T, hot = chunk * tpf, (1 + case["window"] + case.get("hh", 0)) * tpf
+    T = chunk * tpf
     u = _direction(src, H)
     st = dict(case=case, kv=kv, step=0)
     if kind == "h2o":
@@ -259,18 +281,9 @@ def _prepare_stream(case, src):
         yx = torch.stack(torch.meshgrid(torch.arange(case["rows"], device=DEV), torch.arange(case["cols"], device=DEV),
                                         indexing="ij"), -1).reshape(-1, 2) + 1
         st["pos"] = torch.cat([torch.zeros(SPECIAL, 2, dtype=torch.int64, device=DEV), yx]).repeat(chunk, 1)[None]
-    sets = []
-    for _ in range(2):
-        q = _queries(src, u, T, L, 1)                                    # [L, 1, T, H, D]
-        k = _keys(src, u, tpf, chunk, L, 1)                              # [L, 1, H, T, D]
-        v = (src.normal(L, 1, H, T, D) / 2).to(torch.bfloat16)
-        if kind == "h2o":
-            kt, vt = (t.transpose(2, 3) for t in (k, v))
-            sets.append(torch.stack([q, kt, vt], 3).reshape(L, 1, T, 3 * H * D))
-        else:
-            sets.append((q, k, v))
+    sets = _stream_sets(case, src, u)
     st["sets"] = sets
-    seen = max(96 if kind == "stac" else 0, (hot + T) // tpf + 2 * chunk) // chunk
+    seen = _chunks_seen(case)
     if kind == "stac":
         pts, mask = _camera_points(src, (seen + CYCLE) * chunk, case["rows"], case["cols"])
         pts, mask = pts.reshape(-1, T, 3), mask.reshape(-1, T)
@@ -434,3 +447,53 @@ def tolerance(case):
     # scores that differ in the last bits may swap two tokens of a row at the cut of the selection,
     # which moves the ids between them by one place
     return {"rel": 1e-2, "differ": 5e-3}
+
+
+# ------------------------------------------------------------------------------------ exact
+def _attention64(q, k, v, bias, rows, correction):
+    """One head in 64 bits: q [M, D], k and v [N, D], bias [N] or None -> output, log-sum-exp, column sums over ``rows``."""
+    s = q.double() @ k.double().T / math.sqrt(D)
+    if bias is not None:
+        s += bias.double()
+    lse = torch.logsumexp(s, 1)
+    p = torch.exp(s - lse[:, None])
+    return p @ v.double(), lse, p[rows].sum(0) * correction
+
+
+@torch.no_grad()
+def exact(case, seed):
+    """What the first pass returns, in 64 bits: the attention calls, and the sliding-window stream, whose cache
+    holds the first frame and the last ``window`` ones whatever the scores are.  The other kinds build on
+    the selections of all their earlier steps (``None``); the point maps are compared bit by bit."""
+    src = _Source(seed)
+    if case["kind"] == "attn":
+        st = _prepare_attn(case, src)
+        M, H = case["m"], case["heads"]
+        r = _scored_rows(M, case["subsample"])
+        rows = torch.arange(r, device=DEV) * (M // r)
+        q = st["q"][0] if case["drop_in"] else st["q"]
+        per_head = []
+        for h in range(H):
+            if case["drop_in"]:
+                k, v, b = st["k"][0, :, h], st["v"][0, :, h], st["bias"][0, h]
+            else:
+                k, v, b = st["k"][h], st["v"][h], None
+                if case["pivots"]:
+                    k, v = torch.cat([k, st["kr"][h]]), torch.cat([v, st["vr"][h]])
+                    b = torch.cat([torch.zeros(st["hot"], device=DEV), st["br"][h]])
+            per_head.append(_attention64(q[:, h], k, v, b, rows, M / r))
+        out, lse, colsum = (torch.stack([x[i] for x in per_head], 1 if i == 0 else 0) for i in range(3))
+        return (out[None], lse[None], colsum[None]) if case["drop_in"] else (out, lse, colsum)
+    if case["kind"] == "window":
+        tpf, chunk, seen = _tokens(case), case["chunk"], _chunks_seen(case)
+        sets = _stream_sets(case, src, _direction(src, case["heads"]))
+        frames = [0] + list(range(seen * chunk - case["window"], (seen + 1) * chunk))
+        where = [((f // chunk if f < seen * chunk else 0) % 2, f % chunk * tpf) for f in frames]
+        layers = []
+        for l in range(case["layers"]):
+            k, v = (torch.cat([sets[i][j][l, 0, :, a:a + tpf] for i, a in where], 1) for j in (1, 2))
+            q = sets[0][0][l, 0]
+            layers.append(torch.stack([_attention64(q[:, h], k[h], v[h], None, slice(0, 0), 1.0)[0]
+                                       for h in range(case["heads"])], 1)[None])
+        return {"layers": layers, "tokens": None}
+    return None
