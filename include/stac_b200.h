@@ -84,6 +84,20 @@ int stac_attn_colsum(const void* q, int64_t q_row_stride,
                      void* workspace, size_t workspace_bytes,
                      int* dev_status, stac_stream_t stream);
 
+/* The same call for a caller that keeps its workspace: the first 2048 bytes of `workspace` were
+ * zeroed (in stream order) before its first use, and since then only calls of this entry point have
+ * written to it, one after the other, with any M and H that it is large enough for.  Every call leaves
+ * those bytes zero, so nothing has to be cleared in front of the kernels. */
+int stac_attn_colsum_kept(const void* q, int64_t q_row_stride,
+                          const void* k_hot, const void* v_hot, int64_t hot_row_stride, int64_t hot_head_stride, int T_hot,
+                          const void* k_ret, const void* v_ret, int64_t ret_row_stride, int64_t ret_head_stride, int T_ret,
+                          const float* bias_ret, int64_t bias_head_stride,
+                          void* out, int64_t out_row_stride,
+                          float* lse, float* colsum, int64_t colsum_head_stride,
+                          int M, int H, int D, float scale, float subsample_ratio,
+                          void* workspace, size_t workspace_bytes,
+                          int* dev_status, stac_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------
  * Voxel table: packed 63-bit key -> stable voxel id (append-only; id = insertion rank).
  *

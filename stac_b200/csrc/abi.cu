@@ -58,12 +58,16 @@ int stac_abi_version(void) { return 2; }
 
 size_t stac_attn_workspace_bytes(int M, int H) {
   if (M <= 0 || H <= 0) return 0;
-  // row log-sum-exps (rounded up to 256 bytes), then the partial results of the split forward kernel
-  const size_t lse_bytes = (stac::attn_lse2_elems_split(M, H) * sizeof(float) + 255) & ~static_cast<size_t>(255);
+  // control words and row log-sum-exps (rounded up to 256 bytes), then the partial results
+  const size_t lse_bytes = (stac::attn_lse2_elems(M, H) * sizeof(float) + 255) & ~static_cast<size_t>(255);
   return lse_bytes + stac::attn_part_elems() * sizeof(float);
 }
 
-int stac_attn_colsum(const void* q, int64_t q_row_stride, const void* k_hot, const void* v_hot,
+}  // extern "C"
+
+namespace {
+
+int attn_colsum_in_workspace(bool zeroed, const void* q, int64_t q_row_stride, const void* k_hot, const void* v_hot,
                      int64_t hot_row_stride, int64_t hot_head_stride, int T_hot, const void* k_ret, const void* v_ret,
                      int64_t ret_row_stride, int64_t ret_head_stride, int T_ret, const float* bias_ret, int64_t bias_head_stride, void* out,
                      int64_t out_row_stride, float* lse, float* colsum, int64_t colsum_head_stride, int M, int H,
@@ -84,10 +88,39 @@ int stac_attn_colsum(const void* q, int64_t q_row_stride, const void* k_hot, con
   a.out = out; a.out_row_stride = out_row_stride;
   a.lse = lse; a.colsum = colsum; a.colsum_head_stride = colsum_head_stride;
   a.M = M; a.H = H; a.D = D; a.scale = scale; a.subsample_ratio = subsample_ratio;
-  const size_t lse_bytes = (stac::attn_lse2_elems_split(M, H) * sizeof(float) + 255) & ~static_cast<size_t>(255);
+  const size_t lse_bytes = (stac::attn_lse2_elems(M, H) * sizeof(float) + 255) & ~static_cast<size_t>(255);
   float* part = reinterpret_cast<float*>(static_cast<char*>(workspace) + lse_bytes);
-  return stac::attn_colsum_launch(a, static_cast<float*>(workspace), part, dev_status,
+  return stac::attn_colsum_launch(a, static_cast<int*>(workspace), zeroed,
+                                  static_cast<float*>(workspace) + stac::kAttnCtlWords, part, dev_status,
                                   reinterpret_cast<cudaStream_t>(stream));
+}
+
+}  // namespace
+
+extern "C" {
+
+int stac_attn_colsum(const void* q, int64_t q_row_stride, const void* k_hot, const void* v_hot,
+                     int64_t hot_row_stride, int64_t hot_head_stride, int T_hot, const void* k_ret, const void* v_ret,
+                     int64_t ret_row_stride, int64_t ret_head_stride, int T_ret, const float* bias_ret, int64_t bias_head_stride, void* out,
+                     int64_t out_row_stride, float* lse, float* colsum, int64_t colsum_head_stride, int M, int H,
+                     int D, float scale, float subsample_ratio, void* workspace, size_t workspace_bytes,
+                     int* dev_status, stac_stream_t stream) {
+  return attn_colsum_in_workspace(false, q, q_row_stride, k_hot, v_hot, hot_row_stride, hot_head_stride, T_hot, k_ret, v_ret,
+      ret_row_stride, ret_head_stride, T_ret, bias_ret, bias_head_stride, out, out_row_stride,
+      lse, colsum, colsum_head_stride, M, H, D, scale, subsample_ratio, workspace,
+      workspace_bytes, dev_status, stream);
+}
+
+int stac_attn_colsum_kept(const void* q, int64_t q_row_stride, const void* k_hot, const void* v_hot,
+                     int64_t hot_row_stride, int64_t hot_head_stride, int T_hot, const void* k_ret, const void* v_ret,
+                     int64_t ret_row_stride, int64_t ret_head_stride, int T_ret, const float* bias_ret, int64_t bias_head_stride, void* out,
+                     int64_t out_row_stride, float* lse, float* colsum, int64_t colsum_head_stride, int M, int H,
+                     int D, float scale, float subsample_ratio, void* workspace, size_t workspace_bytes,
+                     int* dev_status, stac_stream_t stream) {
+  return attn_colsum_in_workspace(true, q, q_row_stride, k_hot, v_hot, hot_row_stride, hot_head_stride, T_hot, k_ret, v_ret,
+      ret_row_stride, ret_head_stride, T_ret, bias_ret, bias_head_stride, out, out_row_stride,
+      lse, colsum, colsum_head_stride, M, H, D, scale, subsample_ratio, workspace,
+      workspace_bytes, dev_status, stream);
 }
 
 int stac_selftest_bounded_wait(int max_polls, int* dev_status, stac_stream_t stream) {

@@ -40,11 +40,13 @@ int current_device(int* dev);
 int device_sm_count(int dev, int* n_sm);
 
 void attn_subsample_plan(int M, float ratio, int* m_sub, int* stride, float* correction);
+constexpr int kAttnCtlWords = 512;   // control words in front of the row log-sum-exps of a workspace
 size_t attn_lse2_elems(int M, int H);
-size_t attn_lse2_elems_split(int M, int H);
 size_t attn_part_elems();
 // `part`: attn_part_elems() floats for the split forward kernel, or nullptr (one CTA per item then)
-int attn_colsum_launch(const AttnArgs& a, float* lse2, float* part, int* err, cudaStream_t stream);
+// `ctl`: the control words; ctl_zeroed: they are zero (else the call clears the ones it uses)
+int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2, float* part, int* err,
+                       cudaStream_t stream);
 
 // Launch with programmatic stream serialization: the kernel may become resident while the
 // kernel before it in the stream drains; it calls grid_dep_wait() before it touches anything

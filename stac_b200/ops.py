@@ -63,18 +63,23 @@ class LaggedInts:
 
 
 _workspaces = {}
+ATTN_CTL_WORDS = 512      # leading words of an attention workspace that have to be zero
 
 
 def _attn_workspace(device, M, H):
-    """Scratch of stac_attn_colsum (row log-sum-exps, split partials, arrival counters).  One per
-    (device, stream): calls on one stream are ordered and may share it, calls issued on different
-    streams may overlap on the GPU and must not."""
+    """Scratch of stac_attn_colsum_kept (arrival counters, row log-sum-exps, split partials), zeroed when
+    it is made; every call leaves the counters zero.  One per (device, stream): calls on one stream
+    are ordered and may share it, calls issued on different streams may overlap on the GPU and must
+    not.  One made during a graph capture belongs to that call alone: its zeroing is part of the graph
+    and has not happened for anyone else."""
     need = _lib.lib().stac_attn_workspace_bytes(M, H)
     key = (device, torch.cuda.current_stream(device).cuda_stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() * 4 < need:
         ws = torch.empty(max(need // 4, 1), dtype=torch.float32, device=device)
-        _workspaces[key] = ws
+        ws[:ATTN_CTL_WORDS].zero_()
+        if not torch.cuda.is_current_stream_capturing():
+            _workspaces[key] = ws
     return ws
 
 
@@ -115,7 +120,7 @@ def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T
         assert bias_ret.dtype == torch.float32 and bias_ret.stride(1) == 1
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    st = _lib.lib().stac_attn_colsum(
+    st = _lib.lib().stac_attn_colsum_kept(
         ptr(q), q.stride(0),
         ptr(k_hot) if T_hot > 0 else None, ptr(v_hot) if T_hot > 0 else None, hr, hh, T_hot,
         ptr(k_ret) if T_ret > 0 else None, ptr(v_ret) if T_ret > 0 else None, rr, rh, T_ret,
@@ -123,7 +128,7 @@ def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T
         ptr(out), out.stride(0), ptr(lse), ptr(colsum), colsum.stride(0) if colsum is not None else 0,
         M, H, D, float(scale), float(subsample_ratio), ptr(ws), ws.numel() * 4,
         ptr(status.word) if status is not None else None, stream_ptr())
-    check(st, "stac_attn_colsum")
+    check(st, "stac_attn_colsum_kept")
     return out, lse, colsum
 
 

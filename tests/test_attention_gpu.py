@@ -316,3 +316,35 @@ def test_full_size_against_torch_fp32(M, Lk, pivots):
         torch.testing.assert_close(cs[h0:h0 + 4], p.sum(1), rtol=1e-3, atol=1e-6)
         torch.testing.assert_close(lse[h0:h0 + 4], torch.logsumexp(s, -1), rtol=1e-3, atol=1e-3)
         del s, p
+
+
+def test_kept_workspace_between_calls_of_all_kinds():
+    """The kept workspace is zeroed once: every call, of any size and on either forward kernel (a call
+    that raises the fallback flag included, with and without column sums), has to leave its control
+    words zero, and gives the bits of the entry that clears a workspace full of rubbish."""
+    from stac_b200 import _lib, ops
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(3)
+    p = _lib.ptr
+    #        M, H, T_hot, scale of the keys behind the first tile, column sums
+    calls = [(300, 2, 700, 1.0, True), (1100, 16, 1000, 20.0, True), (300, 16, 3400, 1.0, True), (64, 1, 5, 1.0, False),
+             (300, 2, 700, 20.0, False), (700, 2, 2500, 20.0, True), (2600, 3, 6000, 1.0, True), (300, 2, 700, 1.0, True)]
+    for M, H, T, far, want in calls:
+        q = torch.randn(M, H, 64, generator=g).to(torch.bfloat16).to(dev)
+        k = torch.randn(H, T, 64, generator=g)
+        k[:, 128:] *= far
+        k = k.to(torch.bfloat16).to(dev)
+        v = torch.randn(H, T, 64, generator=g).to(torch.bfloat16).to(dev)
+        out, lse, cs = ops.attn_colsum(q, k, v, T, want_lse=True, want_colsum=want)
+        ws = ops._attn_workspace(dev, M, H)
+        assert int(ws[:ops.ATTN_CTL_WORDS].view(torch.int32).abs().sum().item()) == 0
+        out2, lse2 = torch.empty_like(out), torch.empty_like(lse)
+        cs2 = torch.empty_like(cs) if want else None
+        rubbish = torch.full((_lib.lib().stac_attn_workspace_bytes(M, H) // 4,), 3.0, device=dev)
+        rc = _lib.lib().stac_attn_colsum(
+            p(q), q.stride(0), p(k), p(v), k.stride(1), k.stride(0), T, None, None, 64, 64, 0, None, 0, p(out2),
+            out2.stride(0), p(lse2), p(cs2), T, M, H, 64, 0.125, 1.0, p(rubbish), rubbish.numel() * 4, None,
+            _lib.stream_ptr())
+        assert rc == 0
+        assert torch.equal(out, out2) and torch.equal(lse, lse2)
+        assert not want or torch.equal(cs, cs2)
