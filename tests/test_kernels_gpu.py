@@ -279,6 +279,42 @@ def test_merge_and_retrieve_match_oracle(name):
         np.testing.assert_allclose(Bg.cpu().numpy()[fin], Bo[fin], rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("pivot_cap,tokens,voxels,dtype", [
+    (4, 1, 1, "f32"),          # one token
+    (4, 255, 9, "f32"),        # one short of a CTA's tokens; rows of about 28: several batches of eight
+    (4, 257, 300, "bf16"),     # one more; most rows hold a single token
+    (3, 700, 12, "f32"),       # rows above 32 tokens; pivot rows that are not a 16-byte vector
+    (2, 512, 40, "f32"),
+    (1, 256, 20, "bf16"),
+])
+def test_merge_at_block_and_batch_edges(pivot_cap, tokens, voxels, dtype):
+    """Token counts around the 256 tokens of a CTA, rows with more merging tokens than one batch of
+    eight, all pivot capacities: slot maps and pool contents as in the oracle after every call."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    rs = np.random.RandomState(tokens + pivot_cap)
+    H, D = 3, 64
+    rtol, atol = (1e-3, 1e-5) if dtype == "f32" else (8e-3, 4e-3)     # as in test_merge_and_retrieve_match_oracle
+    g = VoxelKVMerger(H, D, init_voxels=voxels, pivot_cap=pivot_cap, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8,
+                      score_thresh=0.1, dtype=torch.float32 if dtype == "f32" else torch.bfloat16, device=DEV,
+                      allocator="segment", seg_size=1, slab_cap=16)
+    m = VoxelMerger(H, D, voxels, pivot_cap, 8, 0.8, 0.8, 0.1, dtype)
+    dirs = rs.randn(voxels, D).astype(np.float32)
+    for step in range(6 if tokens > 1 else 20):
+        VX = rs.randint(0, voxels, size=(H, tokens)).astype(np.int32)
+        VX[rs.rand(H, tokens) < 0.05] = -1
+        near = rs.rand(H, tokens, 1) < 0.6
+        noise = rs.randn(H, tokens, D).astype(np.float32)
+        K = m.rnd(np.where(near, dirs[np.maximum(VX, 0)] + 0.2 * noise, noise).astype(np.float32))
+        V = m.rnd(rs.randn(H, tokens, D).astype(np.float32))
+        S = np.exp(rs.randn(H, tokens)).astype(np.float32)
+        m.insert_and_merge(K, V, S, VX, voxels)
+        g.insert_and_merge(torch.from_numpy(K).to(DEV), torch.from_numpy(V).to(DEV), torch.from_numpy(S).to(DEV), None,
+                           torch.from_numpy(VX).to(DEV), voxels)
+        if m.piv.used() > 0:      # (a snapshot of a memory without pivots reads an unwritten pool)
+            _compare_pool(g.snapshot(), m, f"step {step}", rtol, atol)
+    assert m.piv.used() > 0
+
+
 def _full_size_run(steps, seed):
     """384 pool heads x 8328 evicted tokens per call (the pool-stress shape), bf16: tokens fall on
     1500 voxels, half of their keys cluster around a per-voxel direction so that similarity
