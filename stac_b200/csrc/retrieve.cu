@@ -7,9 +7,10 @@
 //
 // retrieve_select_kernel  one CTA per head: radix select of the weight threshold over the
 //                         (voxel, slot) candidates of the queried voxels, the candidates at or
-//                         above it collected in shared memory and sorted (64-bit keys = weight
-//                         bits | inverted candidate index, so equal weights resolve to the
-//                         earlier candidate); writes their order.
+//                         above it collected in shared memory, thinned out there to the power
+//                         of two above R and sorted in registers (64-bit keys = weight bits |
+//                         inverted candidate index, so equal weights resolve to the earlier
+//                         candidate); writes their order.
 // retrieve_gather_kernel  copies K/V of the selected pivots with 16-byte vectors, writes mask
 //                         and bias, zero-fills the padding.
 #include "common.cuh"
@@ -19,9 +20,13 @@ namespace stac {
 namespace {
 
 constexpr int kSelCap = 8192;     // shared-memory candidate buffer (64-bit keys)
-constexpr int kSelThreads = 512;
 constexpr int kSelBins = 8192;    // counters of one radix digit (13 + 11 + 8 bits, most significant first)
-constexpr int kSelUnroll = 2;     // queried voxels per thread in flight
+// Threads of the selection kernel and queried voxels per thread in flight.  With more heads than SMs
+// three CTAs of 512 share an SM and hide each other's loads; a launch of one CTA per SM or fewer (one
+// layer's memory, a stream whose heads are shared by several GPUs) has only its own threads for that.
+template <bool kFew> struct SelShape {
+  static constexpr int kThreads = kFew ? 1024 : 512, kUnroll = kFew ? 4 : 2, kCtas = kFew ? 1 : 3;
+};
 
 __device__ __forceinline__ unsigned int wkey(float f) {
   const unsigned int u = __float_as_uint(f);
@@ -47,8 +52,66 @@ __device__ __forceinline__ void bitonic_desc(unsigned long long* a, int n) {
   }
 }
 
+// Descending sort of kE * kT keys in shared memory by kT threads: thread t holds keys t * kE ... of the
+// bitonic network in registers, partners nearer than that are its own registers, partners inside the
+// warp come by shuffle, and only the stages that cross warps (10 of 78 at 4096 keys and 512 threads)
+// go through shared memory, one value per bank.
+template <int kE, int kT>
+__device__ __forceinline__ void sort_desc(unsigned long long* a) {
+  const int t = threadIdx.x;
+  unsigned long long v[kE];
+#pragma unroll
+  for (int e = 0; e < kE; ++e) v[e] = a[e * kT + t];        // any assignment will do: the input has no order
+#pragma unroll 1
+  for (int k = 2; k <= kE * kT; k <<= 1) {
+#pragma unroll 1
+    for (int j = k >> 1; j >= kE; j >>= 1) {
+      const int x = j / kE;                                 // partner thread: t ^ x, same register
+      const bool take_max = ((t & x) == 0) == (((t * kE) & k) == 0);
+      if (x >= 32) {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < kE; ++e) a[e * kT + t] = v[e];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < kE; ++e) {
+          const unsigned long long o = a[e * kT + (t ^ x)];
+          if ((o > v[e]) == take_max) v[e] = o;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < kE; ++e) {
+          const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[e], x);
+          if ((o > v[e]) == take_max) v[e] = o;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = kE / 2; j > 0; j >>= 1) {
+      if (j < k) {
+#pragma unroll
+        for (int e = 0; e < kE; ++e) {
+          if ((e & j) == 0) {
+            const bool desc = ((t * kE + e) & k) == 0;
+            const unsigned long long lo = v[e], hi = v[e + j];
+            if ((lo < hi) == desc) {
+              v[e] = hi;
+              v[e + j] = lo;
+            }
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < kE; ++e) a[t * kE + e] = v[e];
+  __syncthreads();
+}
+
 struct RetrieveParams {
   int heads, D, P, voxel_cap, voxel_used, R;
+  int seg_vec;             // 1: the pivot segments of a row are one aligned 16-byte vector
   const int* query_ids;    // ascending voxel ids
   const int* query_count;  // device scalar
   const int* piv_row_seg;
@@ -66,38 +129,52 @@ struct RetrieveParams {
 };
 
 // Calls f(weight key, candidate index) for every pivot of the queried voxels of head h: one
-// pass over the candidates, kSelUnroll voxels per thread in flight.  Every thread of the CTA
-// must call it (no barrier inside).
-template <typename F>
+// pass over the candidates, kUnroll voxels per thread in flight.  Every thread of the CTA
+// must call it (no barrier inside).  A voxel's segments are requested together with its count: the
+// chain id -> (count, segments) -> weights is what a pass waits for.
+template <int kThreads, int kUnroll, typename F>
 __device__ __forceinline__ void for_each_candidate(const RetrieveParams& p, int h, int Q, F f) {
-  for (int base = 0; base < Q; base += kSelThreads * kSelUnroll) {
-    int n[kSelUnroll];
-    long long r[kSelUnroll];
+  const long long hrow = static_cast<long long>(h) * p.voxel_cap;
+  for (int base = 0; base < Q; base += kThreads * kUnroll) {
+    int v[kUnroll], n[kUnroll];
+    int4 seg[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kSelUnroll; ++u) {
-      const int q = base + u * kSelThreads + threadIdx.x;
+    for (int u = 0; u < kUnroll; ++u) {
+      const int q = base + u * kThreads + threadIdx.x;
+      v[u] = q < Q ? p.query_ids[q] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
       n[u] = 0;
-      r[u] = 0;
-      if (q < Q) {
-        const int v = p.query_ids[q];
-        if (v >= 0 && v < p.voxel_used) {
-          r[u] = static_cast<long long>(h) * p.voxel_cap + v;
-          n[u] = min(p.piv_row_cnt[r[u]], 4);
+      seg[u] = make_int4(0, 0, 0, 0);
+      if (v[u] >= 0 && v[u] < p.voxel_used) {
+        const long long r = hrow + v[u];
+        n[u] = min(p.piv_row_cnt[r], 4);
+        const int* sr = p.piv_row_seg + r * p.P;
+        if (p.seg_vec) {
+          seg[u] = *reinterpret_cast<const int4*>(sr);
+        } else {
+          seg[u].x = sr[0];
+          if (p.P > 1) seg[u].y = sr[1];
+          if (p.P > 2) seg[u].z = sr[2];
+          if (p.P > 3) seg[u].w = sr[3];
         }
       }
     }
+    float w[kUnroll][4];
 #pragma unroll
-    for (int u = 0; u < kSelUnroll; ++u) {
-      const int q = base + u * kSelThreads + threadIdx.x;
-      int seg[4];
+    for (int u = 0; u < kUnroll; ++u) {
+      w[u][0] = n[u] > 0 ? p.piv_W[seg[u].x] : 0.f;
+      w[u][1] = n[u] > 1 ? p.piv_W[seg[u].y] : 0.f;
+      w[u][2] = n[u] > 2 ? p.piv_W[seg[u].z] : 0.f;
+      w[u][3] = n[u] > 3 ? p.piv_W[seg[u].w] : 0.f;
+    }
 #pragma unroll
-      for (int s = 0; s < 4; ++s) seg[s] = s < n[u] ? p.piv_row_seg[r[u] * p.P + s] : 0;
-      float w[4];
-#pragma unroll
-      for (int s = 0; s < 4; ++s) w[s] = s < n[u] ? p.piv_W[seg[s]] : 0.f;
+    for (int u = 0; u < kUnroll; ++u) {
+      const int q = base + u * kThreads + threadIdx.x;
 #pragma unroll
       for (int s = 0; s < 4; ++s)
-        if (s < n[u]) f(wkey(w[s]), static_cast<unsigned int>(q * p.P + s));
+        if (s < n[u]) f(wkey(w[u][s]), static_cast<unsigned int>(q * p.P + s));
     }
   }
 }
@@ -128,7 +205,16 @@ __device__ __forceinline__ int list_push(int* counter) {
 // shared-memory buffer, which is then sorted; with the usual spread of weights that is after the
 // first digit, i.e. two passes.  Only when more than kSelCap - R candidates share one exact
 // weight is the last group taken in candidate order by an ordered pass.
-__global__ void __launch_bounds__(kSelThreads, 3) retrieve_select_kernel(const RetrieveParams p) {
+//
+// The digit at which the collection stops leaves up to kSelCap keys of which R are wanted, and the
+// sort costs more than the passes: the select goes on over the collected keys in shared memory,
+// eight bits at a time, until at most the power of two above R are left.
+// (One layer's memory, 16 heads, R = 2048: insert and retrieval 338 -> 285 us with the 1024-thread shape
+// and the register sort; 384 heads, R = 2048: 1170 -> 1139 us.)
+template <bool kFew>
+__global__ void __launch_bounds__(SelShape<kFew>::kThreads, SelShape<kFew>::kCtas)
+retrieve_select_kernel(const RetrieveParams p) {
+  constexpr int kSelThreads = SelShape<kFew>::kThreads, kSelUnroll = SelShape<kFew>::kUnroll;
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel in the stream
   // kSelCap keys; the digit counters live in the same 64 KB (they are dead once the threshold is
   // known and the keys are collected), so three CTAs fit one SM and 384 heads run in one wave
@@ -137,6 +223,7 @@ __global__ void __launch_bounds__(kSelThreads, 3) retrieve_select_kernel(const R
   static_assert(kSelBins * 4 <= kSelCap * 8, "digit counters must fit the candidate buffer");
   __shared__ int warp_sums[kSelThreads / 32];
   __shared__ int sh_count, sh_bin, sh_above, sh_ties;
+  __shared__ int fine[256];         // counters of the select over the collected keys
   const int h = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int Q = *p.query_count;
@@ -154,7 +241,7 @@ __global__ void __launch_bounds__(kSelThreads, 3) retrieve_select_kernel(const R
     __syncthreads();
     const unsigned int pf = prefix;
     const int sh_old = shift;
-    for_each_candidate(p, h, Q, [&](unsigned int wk, unsigned int) {
+    for_each_candidate<kSelThreads, kSelUnroll>(p, h, Q, [&](unsigned int wk, unsigned int) {
       if (sh_old == 32 || (wk >> sh_old) == pf) hist_add(hist, (wk >> new_shift) & ((1u << width) - 1u));
     });
     __syncthreads();
@@ -206,7 +293,7 @@ __global__ void __launch_bounds__(kSelThreads, 3) retrieve_select_kernel(const R
   if (!ordered_ties) {
     const unsigned int pf = prefix;
     const int sh = shift;
-    for_each_candidate(p, h, Q, [&](unsigned int wk, unsigned int idx) {
+    for_each_candidate<kSelThreads, kSelUnroll>(p, h, Q, [&](unsigned int wk, unsigned int idx) {
       if (take_all || sh == 32 || (wk >> sh) >= pf) {
         const int pos = list_push(&sh_count);
         if (pos < kSelCap) cand[pos] = (static_cast<unsigned long long>(wk) << 32) | (0xFFFFFFFFu - idx);
@@ -216,7 +303,7 @@ __global__ void __launch_bounds__(kSelThreads, 3) retrieve_select_kernel(const R
     // weights above the threshold in any order, then the first `need` candidates that carry the
     // threshold weight itself, in candidate order (batches of one voxel per thread, block scan)
     const unsigned int T = prefix;
-    for_each_candidate(p, h, Q, [&](unsigned int wk, unsigned int idx) {
+    for_each_candidate<kSelThreads, kSelUnroll>(p, h, Q, [&](unsigned int wk, unsigned int idx) {
       if (wk > T) {
         const int pos = list_push(&sh_count);
         cand[pos] = (static_cast<unsigned long long>(wk) << 32) | (0xFFFFFFFFu - idx);
@@ -267,19 +354,86 @@ __global__ void __launch_bounds__(kSelThreads, 3) retrieve_select_kernel(const R
     }
   }
   __syncthreads();
-  {
-    const int cnt = min(sh_count, kSelCap);
-    int np2 = 1;
-    while (np2 < cnt) np2 <<= 1;
-    for (int i = cnt + threadIdx.x; i < np2; i += blockDim.x) cand[i] = 0ull;
-    __syncthreads();
-    if (cnt > 1) bitonic_desc(cand, np2);
-    const int keep = min(cnt, R);
-    for (int i = threadIdx.x; i < R; i += blockDim.x) {
-      int c = -1;
-      if (i < keep) c = static_cast<int>(0xFFFFFFFFu - static_cast<unsigned int>(cand[i] & 0xFFFFFFFFull));
-      p.sel[static_cast<long long>(h) * R + i] = c;
+  int cnt = min(sh_count, kSelCap);
+  int np2 = kSelThreads;
+  while (np2 < R) np2 <<= 1;
+  if (cnt > np2) {
+    // the R-th largest key, eight bits at a time (keys are distinct, so this ends with R of them at
+    // the latest); R <= np2 < cnt, so there is one
+    unsigned long long pre = 0;       // leading bits of that key found so far
+    int sh = 64, want = R;            // want: its rank among the keys that share them
+    for (;;) {
+      sh -= 8;
+      for (int i = threadIdx.x; i < 256; i += kSelThreads) fine[i] = 0;
+      __syncthreads();
+      for (int i = threadIdx.x; i < cnt; i += kSelThreads) {
+        const unsigned long long x = cand[i];
+        if (sh == 56 || (x >> (sh + 8)) == pre) hist_add(fine, static_cast<unsigned>(x >> sh) & 255u);
+      }
+      __syncthreads();
+      if (warp == 0) {
+        // lane l counts bins 8 l' .. 8 l' + 7 with l' = 31 - l: lane 0 holds the highest
+        int c[8], sum = 0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          c[e] = fine[(31 - lane) * 8 + 7 - e];
+          sum += c[e];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
+        }
+        int above = incl - sum;
+        if (above < want && incl >= want) {       // exactly one lane
+          bool found = false;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (!found) {
+              if (above + c[e] >= want) {
+                found = true;
+                sh_bin = (31 - lane) * 8 + 7 - e;
+                sh_above = above;
+                sh_ties = c[e];
+              }
+              above += found ? 0 : c[e];
+            }
+          }
+        }
+      }
+      __syncthreads();
+      pre = (pre << 8) | static_cast<unsigned>(sh_bin);
+      want -= sh_above;
+      const int left = (R - want) + sh_ties;      // keys at or above the new prefix
+      __syncthreads();
+      if (left <= np2 || sh == 0) break;
     }
+    // keep the keys at or above the prefix, in place: a batch is read before any of it is written,
+    // and what is written never lies past the batches that have been read
+    if (threadIdx.x == 0) sh_count = 0;
+    __syncthreads();
+    for (int base = 0; base < cnt; base += kSelThreads) {
+      const int i = base + threadIdx.x;
+      const unsigned long long x = i < cnt ? cand[i] : 0ull;
+      __syncthreads();
+      if (i < cnt && (x >> sh) >= pre) cand[list_push(&sh_count)] = x;
+    }
+    __syncthreads();
+    cnt = sh_count;
+  }
+  for (int i = cnt + threadIdx.x; i < np2; i += kSelThreads) cand[i] = 0ull;
+  __syncthreads();
+  if (np2 == kSelThreads) sort_desc<1, kSelThreads>(cand);
+  else if (np2 == 2 * kSelThreads) sort_desc<2, kSelThreads>(cand);
+  else if (np2 == 4 * kSelThreads) sort_desc<4, kSelThreads>(cand);
+  else if (np2 == 8 * kSelThreads) sort_desc<8, kSelThreads>(cand);
+  else bitonic_desc(cand, np2);       // 16 keys per thread would not fit three CTAs' registers
+  const int keep = min(cnt, R);
+  for (int i = threadIdx.x; i < R; i += kSelThreads) {
+    int c = -1;
+    if (i < keep) c = static_cast<int>(0xFFFFFFFFu - static_cast<unsigned int>(cand[i] & 0xFFFFFFFFull));
+    p.sel[static_cast<long long>(h) * R + i] = c;
   }
 }
 
@@ -331,21 +485,29 @@ int stac_retrieve(const stac_pool* pool, const int* query_ids, const int* query_
   rp.voxel_used = pool->voxel_used; rp.R = retrieve_size;
   rp.query_ids = query_ids; rp.query_count = query_count;
   rp.piv_row_seg = pool->piv_row_seg; rp.piv_row_cnt = pool->piv_row_cnt;
+  rp.seg_vec = rp.P == 4 && (reinterpret_cast<uintptr_t>(rp.piv_row_seg) & 15) == 0 ? 1 : 0;
   rp.piv_K = pool->piv_K; rp.piv_V = pool->piv_V; rp.piv_W = pool->piv_W; rp.piv_C = pool->piv_C;
   rp.sel = sel; rp.out_K = out_K; rp.out_V = out_V; rp.out_mask = out_mask; rp.out_bias = out_bias;
   rp.out_idx = out_idx;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int dev = 0;
   if (stac::current_device(&dev) != STAC_OK) return STAC_ERR_CUDA;
+  int n_sm = 0;
+  if (stac::device_sm_count(dev, &n_sm) != STAC_OK) return STAC_ERR_CUDA;
   static stac::PerDeviceFlag attr_done;   // the shared-memory opt-in is made once per device
   const int smem = stac::kSelCap * 8;
   if (attr_done.needs_setup(dev)) {
-    if (cudaFuncSetAttribute(stac::retrieve_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(stac::retrieve_select_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(stac::retrieve_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess)
       return STAC_ERR_CUDA;
     attr_done.mark(dev);
   }
-  if (stac::launch_behind(stac::retrieve_select_kernel, dim3(pool->heads), dim3(stac::kSelThreads), smem, st, rp) != cudaSuccess)
+  const bool few = pool->heads <= n_sm;
+  if (stac::launch_behind(few ? stac::retrieve_select_kernel<true> : stac::retrieve_select_kernel<false>,
+                          dim3(pool->heads), dim3(few ? stac::SelShape<true>::kThreads : stac::SelShape<false>::kThreads),
+                          smem, st, rp) != cudaSuccess)
     return STAC_ERR_CUDA;
   const int vpt = token_bytes / 16;
   const long long total = static_cast<long long>(retrieve_size) * vpt;

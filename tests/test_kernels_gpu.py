@@ -315,6 +315,50 @@ def test_merge_at_block_and_batch_edges(pivot_cap, tokens, voxels, dtype):
     assert m.piv.used() > 0
 
 
+@pytest.mark.parametrize("heads,voxels,pivot_cap,R,equal", [
+    (2, 600, 4, 1, False),           # R below the smallest sort
+    (2, 3000, 4, 1023, False), (2, 3000, 4, 1025, False),      # around one key per thread of the few-heads shape
+    (2, 3000, 4, 2048, False), (2, 4000, 3, 2049, False),      # exact power of two, and one more; rows of three segments
+    (2, 3000, 4, 8192, False),
+    (160, 3000, 4, 511, False), (160, 3000, 4, 513, False), (160, 2500, 4, 2048, False),   # more heads than SMs
+    (160, 3000, 4, 4097, False),     # largest sort of that shape
+    (2, 3000, 4, 1500, True), (160, 3000, 4, 1500, True),      # one weight for all: candidate order decides
+])
+def test_retrieval_order_at_the_edges_of_the_sort(heads, voxels, pivot_cap, R, equal):
+    """Top-R by (weight descending, candidate ascending) against a stable argsort on the host, for pools
+    written directly: weights in a narrow band, so that the first digits do not separate them."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    rs = np.random.RandomState(R + heads)
+    g = VoxelKVMerger(heads, 64, init_voxels=voxels, pivot_cap=pivot_cap, budget_cap=8, dtype=torch.bfloat16, device=DEV,
+                      allocator="segment", seg_size=1)
+    g._voxel_offset = voxels
+    n = heads * voxels * pivot_cap
+    g._grow_piv(n)
+    cnt = rs.randint(0, pivot_cap + 1, size=(heads, voxels)).astype(np.int32)
+    seg = rs.permutation(n).astype(np.int32).reshape(heads, voxels, pivot_cap)
+    w = (np.full(n, 18.0) if equal else 18.0 + 0.5 * rs.rand(n)).astype(np.float32)
+    w[rs.rand(n) < 0.2] = 18.25                         # ties
+    g._piv_row_cnt.copy_(torch.from_numpy(cnt))
+    g._piv_row_seg.copy_(torch.from_numpy(seg))
+    g._piv_W[:n].copy_(torch.from_numpy(w))
+    g._piv_C[:n].fill_(1.0)
+    g._piv_K[:n].copy_((torch.arange(n, device=DEV) % 251).view(-1, 1).expand(-1, 64))
+    g._piv_V[:n].zero_()
+    q = np.sort(rs.choice(voxels, size=voxels - 7, replace=False)).astype(np.int32)
+    K, _, mask, _, idx = g.retrieve_device(torch.from_numpy(q).to(DEV), torch.tensor([q.size], dtype=torch.int32, device=DEV),
+                                           R, want_idx=True)
+    K, mask, idx = K[:, :, 0].float().cpu().numpy(), mask.cpu().numpy(), idx.cpu().numpy()
+    for h in range(0, heads, max(1, heads // 4)):
+        live = np.arange(pivot_cap)[None] < cnt[h, q][:, None]
+        vox, slot = np.broadcast_to(q[:, None], live.shape)[live], np.broadcast_to(np.arange(pivot_cap), live.shape)[live]
+        segs = seg[h, vox, slot]
+        order = np.argsort(-w[segs], kind="stable")[:R]
+        k = order.size
+        assert mask[h].sum() == k and mask[h, :k].all()
+        assert np.array_equal(idx[h, :k], np.stack([vox[order], slot[order]], 1))
+        assert np.array_equal(K[h, :k], segs[order] % 251) and (idx[h, k:] == -1).all() and (K[h, k:] == 0).all()
+
+
 def _full_size_run(steps, seed):
     """384 pool heads x 8328 evicted tokens per call (the pool-stress shape), bf16: tokens fall on
     1500 voxels, half of their keys cluster around a per-voxel direction so that similarity
