@@ -1082,6 +1082,11 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 // (TMEM lane) per thread, so a thread's column sum never leaves its registers.  Three exponent
 // warps per scheduler keep the exp2 unit busier than two did (85 % against 75 % of the active
 // cycles); a fourth (kColGroup = 4, 104 registers per thread) measured the same as three.
+// The last query tile is ragged unless M_sub is a multiple of 128 (one frame of 1041 tokens fills 17
+// of its rows): its second half is not scored when no row lies in it, and of the half that holds
+// the last row only the 16-row pieces up to that row are exponentiated.
+// (M = 1041, 16 heads: N = 33312 338.7 -> 331.3 us per call with the forward pass, N = 2082 38.5 -> 37.5 us;
+// M = 4164 has its last row in the second half: 0.2 %.)
 // lse2 holds the row log-sum-exp in the log2 domain; rows past M_sub read as +inf so that
 // padded query columns contribute exp2(-inf) = 0.
 // ---------------------------------------------------------------------------------------
@@ -1192,10 +1197,10 @@ __device__ __forceinline__ void col_exp_chunk16(const uint32_t (&s)[32], const f
 // kFast: the key's bias was taken out of the exponent (every lane of the warp agrees).
 // A 64-row half is read from TMEM in four pieces of 16 rows, the next piece always in flight
 // (the first piece of the next half included: its buffer does not depend on this warpgroup
-// finishing the current one).
+// finishing the current one).  `tail` > 0: the last half has only that many pieces with rows (1 to 3).
 template <bool kFast>
 __device__ __forceinline__ float col_item_sum(ColSmem& sm, const ColParams& p, uint32_t t_base, const float* nl_item,
-                                              int n_half, int& ui, float c2, float b2_in) {
+                                              int n_half, int tail, int& ui, float c2, float b2_in) {
   uint32_t ra[32], rb[32];   // 16 registers of each are used
   float a0 = 0.f;
   uint64_t a01 = 0ull, a23 = 0ull;
@@ -1215,7 +1220,8 @@ __device__ __forceinline__ float col_item_sum(ColSmem& sm, const ColParams& p, u
     tc_fence_after();
     tmem_ld16(t_base + g * kColHalf, ra);
   }
-  for (int hu = 0; hu < n_half; ++hu, ++ui) {
+  const int n_whole = tail > 0 ? n_half - 1 : n_half;
+  for (int hu = 0; hu < n_whole; ++hu, ++ui) {
     const int g = ui & 1;
     const uint32_t s_addr = t_base + g * kColHalf;
     const float* nl = nl_item + hu * kColHalf;
@@ -1238,6 +1244,22 @@ __device__ __forceinline__ float col_item_sum(ColSmem& sm, const ColParams& p, u
     consume(rb, nl + 48);
     tc_fence_before();
     mbar_arrive(&sm.s_free[g]);
+  }
+  if (tail > 0) {
+    const int g = ui & 1;
+    const uint32_t s_addr = t_base + g * kColHalf;
+    const float* nl = nl_item + n_whole * kColHalf;
+    tmem_ld_wait();
+#pragma unroll 1
+    for (int piece = 0;;) {
+      consume(ra, nl + piece * 16);
+      if (++piece == tail) break;
+      tmem_ld16(s_addr + piece * 16, ra);
+      tmem_ld_wait();
+    }
+    tc_fence_before();
+    mbar_arrive(&sm.s_free[g]);
+    ++ui;
   }
   float b0, b1, b2, b3;
   unpack_f32x2(a01, b0, b1);
@@ -1372,8 +1394,10 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int i = i0; i < i1; ++i) {
           mbar_wait(&sm.q_full[s], s_round & 1, p.err, DEV_TIMEOUT_TMA);
           if (kColFoldLse) mbar_wait(&sm.x_full[s], s_round & 1, p.err, DEV_TIMEOUT_CONSUMER);
+          const int last_half = i * kBM + kColHalf < p.M_sub ? 1 : 0;   // no row in the second half: not scored
 #pragma unroll
-          for (int half = 0; half < 2; ++half, ++ui) {
+          for (int half = 0; half < 2; ++half) {
+            if (half > last_half) break;
             const int g = ui & 1, it = ui >> 1;
             // query rows 64*half.. of the tile: 8192 bytes further in the K-major tile
             const uint64_t q_desc = q_desc0 + static_cast<uint64_t>(s * (kTileBytes >> 4) + half * (8192 >> 4));
@@ -1394,12 +1418,13 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                           idesc, 1u);
               }
               umma_commit(&sm.s_full[g]);
-              if (half == 1) {
+              if (half == last_half) {
                 umma_commit(&sm.q_empty[s]);
                 if (i == i1 - 1) umma_commit(&sm.k_empty[kb]);
               }
             }
             __syncwarp();
+            ++ui;
           }
           if (++s == kColStages) { s = 0; ++s_round; }
         }
@@ -1448,12 +1473,15 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const bool b2_small = fabsf(b2) <= 32.f;
       const float b2_in = b2_small ? 0.f : b2;
       const bool warp_fast = __all_sync(0xffffffffu, b2_small);
-      const int n_half = 2 * (i1 - i0);
+      // halves with rows, and the 16-row pieces with rows of the last one when it is not full
+      const int rows_here = min(i1 * kBM, p.M_sub) - i0 * kBM;
+      const int n_half = (rows_here + kColHalf - 1) / kColHalf;
+      const int tail = (((rows_here - 1) % kColHalf) / 16 + 1) & 3;    // 4 pieces: a whole half, 0
       const float* nl_item = nl_s + i0 * kBM;
       // (warps whose 32 keys are all masked still run the sums: letting them only follow the
       // score buffers was measured slower in the stream, their polling disturbs the others)
-      float sum = warp_fast ? col_item_sum<true>(sm, p, t_base, nl_item, n_half, ui, c2, 0.f)
-                            : col_item_sum<false>(sm, p, t_base, nl_item, n_half, ui, c2, b2_in);
+      float sum = warp_fast ? col_item_sum<true>(sm, p, t_base, nl_item, n_half, tail, ui, c2, 0.f)
+                            : col_item_sum<false>(sm, p, t_base, nl_item, n_half, tail, ui, c2, b2_in);
       if (key < valid) {
         sum *= p.correction;
         if (b2_small) sum *= exp2f(b2);

@@ -348,3 +348,13 @@ def test_kept_workspace_between_calls_of_all_kinds():
         assert rc == 0
         assert torch.equal(out, out2) and torch.equal(lse, lse2)
         assert not want or torch.equal(cs, cs2)
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 48, 49, 63, 64, 65, 80, 112, 127, 128 + 1, 128 + 64, 128 + 65, 1041])
+@pytest.mark.parametrize("H,T_hot,T_ret", [(2, 300, 90), (16, 3400, 140)])     # one CTA per item; units cut over the SMs
+def test_ragged_last_query_tile(M, H, T_hot, T_ret):
+    """Column sums score only the halves of the last query tile that hold rows, and of the last half only
+    the 16-row pieces up to the last row; a bias out of the usual range takes the other exponent path."""
+    for shift in (0.0, -40.0):
+        got, ref = _run_two_segment(M, H, T_hot, T_ret, seed=M, bias_shift=shift)
+        _assert_close(got, ref)
