@@ -41,13 +41,15 @@ class LaggedInts:
     def __init__(self, n):
         self.pin = torch.zeros(n, dtype=torch.int32).pin_memory()
         self.event = None
+        self.parts = {}      # sizes of the pushed tensors -> the slices of `pin` that they go to
 
     def push(self, *tensors):
-        off = 0
-        for t in tensors:
-            n = t.numel()
-            self.pin[off:off + n].copy_(t.reshape(-1), non_blocking=True)
-            off += n
+        sizes = tuple(t.numel() for t in tensors)
+        parts = self.parts.get(sizes)
+        if parts is None:
+            parts = self.parts[sizes] = self.pin[:sum(sizes)].split(sizes)
+        for part, t in zip(parts, tensors):
+            part.copy_(t.reshape(-1), non_blocking=True)
         self.event = torch.cuda.Event()
         self.event.record()
 
@@ -73,7 +75,7 @@ def _attn_workspace(device, M, H):
     not.  One made during a graph capture belongs to that call alone: its zeroing is part of the graph
     and has not happened for anyone else."""
     need = _lib.lib().stac_attn_workspace_bytes(M, H)
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
+    key = (device, stream_ptr(device=device))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() * 4 < need:
         ws = torch.empty(max(need // 4, 1), dtype=torch.float32, device=device)

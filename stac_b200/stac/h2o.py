@@ -10,7 +10,7 @@ from typing import Optional
 import torch
 
 from .. import _lib
-from .._lib import check, ptr, stream_ptr
+from .._lib import check, no_grad, ptr, stream_ptr
 from .kv_manager import KVManager
 
 logger = logging.getLogger(__name__)
@@ -85,7 +85,7 @@ class HeavyHittersKV(KVManager):
         self._last_query_offset = None
         super().free()
 
-    @torch.no_grad()
+    @no_grad
     def decode_sparse_attn(self, query_states: torch.Tensor, layer_idx: int) -> torch.Tensor:
         """query_states [B, Tq, H, D] -> [B, Tq, H, D]; updates the hot scores (stac/h2o.py:139-174)."""
         slot = self._to_slot(layer_idx)
@@ -118,7 +118,7 @@ class HeavyHittersKV(KVManager):
     def prune_kv(self):
         self._parallel_prune_kv()
 
-    @torch.no_grad()
+    @no_grad
     def _parallel_prune_kv(self):
         """stac/h2o.py:244-354: keep = sort(pinned U recent U per-(layer, head) top-k of the rest)."""
         L, H = self._L_eff, self.num_heads
@@ -144,7 +144,7 @@ class HeavyHittersKV(KVManager):
             keep, drop = self._select(self._scores_hot, Tb, L * H, T, n_base + k)
         self._apply_keep_and_compact_parallel(keep, drop)
 
-    @torch.no_grad()
+    @no_grad
     def _apply_keep_and_compact_parallel(self, keep_idx_lh: torch.Tensor, drop_idx_lh: torch.Tensor = None):
         """keep_idx_lh int32 [L*H, T'] ascending kept positions (stac/h2o.py:356-436)."""
         self._compact(keep_idx_lh)

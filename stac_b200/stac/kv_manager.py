@@ -20,7 +20,7 @@ import numpy as np
 import torch
 
 from .. import _lib, ops
-from .._lib import check, ptr, stream_ptr
+from .._lib import check, no_grad, ptr, stream_ptr
 
 logger = logging.getLogger(__name__)
 
@@ -272,7 +272,7 @@ class KVManager:
               "stac_append_kv")
         self._offset_hot[slot] = old_T + new_T
 
-    @torch.no_grad()
+    @no_grad
     def append_qkv(self, qkv, layer_idx: int, *, q_norm=None, k_norm=None, rope=None, pos=None):
         """The attention layer's projection epilogue and append_kv in one kernel
         (causalvggt/layers/attention.py:119-128, :141): `qkv` is the output of the layer's QKV
@@ -333,7 +333,7 @@ class KVManager:
         self._offset_hot[slot] = old_T + T_new
         return q_out if out_dtype == torch.bfloat16 else q_out.to(out_dtype)
 
-    @torch.no_grad()
+    @no_grad
     def prefill(self, query_states, key_states, value_states, layer_idx: int):
         """query/key/value [B, T, H, D] (stac/kv_manager.py:195-224)."""
         B, T, H, D = query_states.shape
@@ -371,7 +371,7 @@ class KVManager:
         out = out.unsqueeze(0)
         return (out if out_dtype == torch.bfloat16 else out.to(out_dtype)), colsum
 
-    @torch.no_grad()
+    @no_grad
     def decode_sparse_attn(self, query_states: torch.Tensor, layer_idx: int) -> torch.Tensor:
         """Plain attention over the hot cache and, once tokens were spilled, the host part as well
         (stac/kv_manager.py:311-360); query_states [B, Tq, H, D] -> [B, Tq, H, D]."""
@@ -416,7 +416,7 @@ class KVManager:
                                          ptr(keep), ptr(drop), stream_ptr()), "stac_h2o_select")
         return keep, drop
 
-    @torch.no_grad()
+    @no_grad
     def prune_kv(self):
         """Keep pinned + recent tokens, compact (stac/kv_manager.py:362-441), all layers at once."""
         L, H = self._L_eff, self.num_heads
@@ -453,11 +453,11 @@ class KVManager:
         self._bind()
         self._offset_hot = [n_keep] * L
 
-    @torch.no_grad()
+    @no_grad
     def retrieve_kv(self, layer_idx: int, **kwargs) -> Tuple[int, int]:
         raise NotImplementedError("retrieve_kv() is not implemented for HeavyHittersKV.")
 
-    @torch.no_grad()
+    @no_grad
     def append_positions(self, new_positions: torch.Tensor, new_pos_mask: torch.Tensor):
         raise NotImplementedError("append_positions() is not implemented for HeavyHittersKV.")
 

@@ -14,7 +14,7 @@ import torch
 
 from .. import _lib
 from .._lib import META_BUF_FREE_LEN, META_BUF_TOP, META_BUF_USED, META_OVER_COUNT, META_PIV_TOP, META_PIV_USED
-from .._lib import StacEvicted, StacPool, check, ptr, stream_ptr
+from .._lib import StacEvicted, StacPool, check, no_grad, ptr, stream_ptr
 from ..ops import DeviceStatus, LaggedInts
 
 MAX_LIST = 1 << 22        # STAC_MERGE_MAX_LIST
@@ -252,7 +252,7 @@ class VoxelKVMerger:
             raise _lib.StacError(f"voxel merge: device error {code} ({DeviceStatus.NAMES.get(code, 'unknown')})")
 
     # ------------------------------------------------------------------ insert
-    @torch.no_grad()
+    @no_grad
     def insert_evicted(self, k_cache, v_cache, scores, voxel_ids, positions, tokens_per_head, num_voxels,
                        voxel_count_dev=None):
         """Evicted tokens read in place: token j of pool head h sits at position
@@ -324,7 +324,7 @@ class VoxelKVMerger:
         self._over_cur = 1 - self._over_cur
         self._push_meta()
 
-    @torch.no_grad()
+    @no_grad
     def insert_and_merge(self, K_new, V_new, S_new, I_new, VX_new, num_voxels: int, mode: str = "default"):
         """Reference signature (stac/merger.py:1157-1255): K_new/V_new [H,Tn,D], S_new [H,Tn]
         fp32, I_new ignored, VX_new [H,Tn] voxel ids."""
@@ -339,7 +339,7 @@ class VoxelKVMerger:
         return {"init_time": 0.0, "append_time": 0.0, "merge_all2one_time": 0.0, "merge_one2one_time": 0.0}
 
     # ------------------------------------------------------------------ retrieve
-    @torch.no_grad()
+    @no_grad
     def retrieve_device(self, query_ids, query_count, retrieve_size, want_idx=False):
         """query_ids int32 ascending (device), query_count int32 [1] (device).  Returns
         K, V [H,R,D], mask bool [H,R], bias fp32 [H,R] (and idx int32 [H,R,2])."""
@@ -362,7 +362,7 @@ class VoxelKVMerger:
         out = (K, V, M.bool(), Bz)
         return out + (idx,) if want_idx else out
 
-    @torch.no_grad()
+    @no_grad
     def retrieve(self, voxel_ids=None, return_buf: bool = False, retrieve_size=None, want_idx=False):
         """Reference signature (stac/merger.py:1377-1543) for retrieve_size > 0: fixed-size
         output, pivots ordered by W descending, bias log C, padding -inf.  With a positive
@@ -381,7 +381,7 @@ class VoxelKVMerger:
             ids = torch.zeros(1, dtype=torch.int32, device=dev)
         return self.retrieve_device(ids, cnt, req, want_idx)
 
-    @torch.no_grad()
+    @no_grad
     def _retrieve_unbounded(self, voxel_ids, return_buf, want_idx=False):
         """retrieve_size <= 0 (stac/merger.py:1424-1543): output width = (#queried voxels) * P,
         plus, with return_buf, the buffered tokens of those voxels ((voxel, column) order, bias 0)

@@ -12,10 +12,10 @@ from typing import Tuple
 import torch
 
 from .. import _lib
-from .._lib import check, ptr, stream_ptr
+from .._lib import check, no_grad, ptr, stream_ptr
 
 
-@torch.no_grad()
+@no_grad
 def pointmap_to_positions(world_points: torch.Tensor, world_points_conf: torch.Tensor, patch_size: int,
                           conf_threshold: float = 1.0, special_tokens_size: int = 0) -> Tuple[torch.Tensor, torch.Tensor]:
     """world_points [B,S,H,W,3] or [S,H,W,3], world_points_conf [B,S,H,W] or [S,H,W] (B == 1), CUDA.

@@ -18,6 +18,7 @@ from typing import Dict, List, Optional, Tuple
 
 import torch
 
+from .._lib import no_grad
 from .h2o import HeavyHittersKV
 from .merger import VoxelKVMerger
 from .voxel import BinaryVoxel
@@ -143,7 +144,7 @@ class STACVoxelKV(HeavyHittersKV):
         self._scores_retrieval = [t.to(dev) for t in sd["scores_retrieval"]]
 
     # ------------------------------------------------------------------ attention
-    @torch.no_grad()
+    @no_grad
     def decode_sparse_attn(self, query_states: torch.Tensor, layer_idx: int) -> torch.Tensor:
         """Attention over [hot | retrieved pivots]; only the hot columns update the scores
         (stac/stac_voxel.py:208-267)."""
@@ -179,7 +180,7 @@ class STACVoxelKV(HeavyHittersKV):
         cells = max(1, int(math.ceil(dist_thres / self._voxel_size_f)))
         self._recent_voxel_ids = self._vm.neighbor_ids(tokens, cells)
 
-    @torch.no_grad()
+    @no_grad
     def append_positions(self, new_positions: torch.Tensor, new_pos_mask: torch.Tensor):
         """new_positions [T_new,3] fp32 world points, new_pos_mask [T_new] bool.  After append_kv
         of every layer, before prune_kv (stac/stac_voxel.py:326-365)."""
@@ -199,7 +200,7 @@ class STACVoxelKV(HeavyHittersKV):
         with self._stage("voxel_neighbors"):
             self._search_recent_neighbors(slot_idx=self._L_eff - 1, dist_thres=2 * self._voxel_size_f)
 
-    @torch.no_grad()
+    @no_grad
     def append_pointmap(self, world_points: torch.Tensor, world_points_conf: torch.Tensor, patch_size: int,
                         conf_threshold: float = 1.0, special_tokens_size: int = 0):
         """get_pointmap + append_positions of the reference's streaming loop in one call
@@ -222,7 +223,7 @@ class STACVoxelKV(HeavyHittersKV):
                                                            dtype=self.dtype)
 
     # ------------------------------------------------------------------ prune + eviction
-    @torch.no_grad()
+    @no_grad
     def _apply_keep_and_compact_parallel(self, keep_idx_lh: torch.Tensor, drop_idx_lh: torch.Tensor = None):
         """Evicted tokens go to the voxel memory, then the cache is compacted
         (stac/stac_voxel.py:409-419)."""
@@ -256,7 +257,7 @@ class STACVoxelKV(HeavyHittersKV):
             return self.retrieve_kv_parallel(**kwargs)
         return 0, 0
 
-    @torch.no_grad()
+    @no_grad
     def retrieve_kv_parallel(self, **kwargs) -> Tuple[int, int]:
         """stac/stac_voxel.py:665-762: one retrieval for all layers; layer l then sees rows
         [l*H, (l+1)*H) of the result as views."""

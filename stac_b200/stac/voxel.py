@@ -10,7 +10,7 @@ reference's CUDA segment allocator and influence no output).
 import torch
 
 from .. import _lib
-from .._lib import check, ptr, stream_ptr
+from .._lib import check, no_grad, ptr, stream_ptr
 from ..ops import LaggedInts
 
 
@@ -123,7 +123,7 @@ class BinaryVoxel:
         self._mirror.push(self._n_dev)
         return ids
 
-    @torch.no_grad()
+    @no_grad
     def upsert(self, ijk_valid: torch.Tensor) -> torch.Tensor:
         """ijk_valid [N,3] int32 -> stable voxel ids [N] int32 (stac/voxel.py:195-324)."""
         if ijk_valid.numel() == 0:
@@ -132,7 +132,7 @@ class BinaryVoxel:
         ijk = ijk_valid.to(device=self.device, dtype=torch.int32).contiguous()
         return self._upsert(None, ijk, None, ijk.shape[0])
 
-    @torch.no_grad()
+    @no_grad
     def upsert_points(self, points: torch.Tensor, mask: torch.Tensor = None) -> torch.Tensor:
         """Fused quantise + upsert of world points [N,3] fp32; masked-out points get id -1
         (stac/stac_voxel.py:339-347)."""
@@ -141,7 +141,7 @@ class BinaryVoxel:
         return self._upsert(pts, None, m, pts.shape[0])
 
     # ------------------------------------------------------------------ neighbours
-    @torch.no_grad()
+    @no_grad
     def neighbor_ids(self, token_voxel_ids: torch.Tensor = None, radius_cells: int = 2, all_ids: bool = False):
         """Ascending unique ids of existing voxels within `radius_cells` (Chebyshev) of the given
         voxel ids.  Returns (ids int32 [capacity] view, count int32 [1]) on the device; only the
@@ -156,7 +156,7 @@ class BinaryVoxel:
         check(st, "stac_voxel_neighbors")
         return self._nbr_ids, self._nbr_count
 
-    @torch.no_grad()
+    @no_grad
     def neighbors(self, voxel_ids: torch.Tensor, radius_m: float, include_self: bool = True):
         """Sorted unique neighbour ids (the only part of the reference's (ids, dist2, found)
         result that the managers consume, stac/stac_voxel.py:316-323).  Self is always included."""

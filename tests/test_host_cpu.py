@@ -236,3 +236,23 @@ def test_checkpoint_file_loads_without_pickle(tmp_path):
     assert torch.equal(b.loaded["key"], want["key"]) and b.loaded["key"].dtype == torch.bfloat16
     assert torch.equal(b.loaded["memory"]["meta"], want["memory"]["meta"])
     assert b.loaded["retrieved"][1].dtype == torch.bool
+
+
+def test_no_grad_wrapper_restores_the_mode():
+    """Gradients are off inside, whatever they were before is restored, also when the function raises."""
+    import torch
+    from stac_b200._lib import no_grad
+
+    @no_grad
+    def inside(fail=False):
+        if fail:
+            raise KeyError("x")
+        return torch.is_grad_enabled()
+    for before in (True, False):
+        with torch.set_grad_enabled(before):
+            assert inside() is False and torch.is_grad_enabled() is before
+            try:
+                inside(fail=True)
+            except KeyError:
+                pass
+            assert torch.is_grad_enabled() is before
