@@ -185,6 +185,13 @@ int stac_qkv_epilogue_append(const void* qkv, int64_t qkv_token_stride, const fl
                              int64_t q_out_row_stride, void* k_cache, void* v_cache, int64_t cache_head_stride,
                              int64_t* token_idx, int64_t idx_head_stride, int H, int T_new, int old_T,
                              int64_t first_token_id, stac_stream_t stream);
+/* The same with the rows of the cos / sin tables `table_row_stride` (>= 16) values apart. */
+int stac_qkv_epilogue_append_tables(const void* qkv, int64_t qkv_token_stride, const float* q_norm_w, const float* q_norm_b,
+                             const float* k_norm_w, const float* k_norm_b, float eps, const int64_t* pos,
+                             const float* cos_table, const float* sin_table, int64_t table_row_stride, int n_pos, void* q_out,
+                             int64_t q_out_row_stride, void* k_cache, void* v_cache, int64_t cache_head_stride,
+                             int64_t* token_idx, int64_t idx_head_stride, int H, int T_new, int old_T,
+                             int64_t first_token_id, stac_stream_t stream);
 
 /* HeavyHittersKV._update_scores (stac/h2o.py:177-216) for one layer: s = colsum * T_live / Tq;
  * positions >= old_T take s, older ones score * temperature + s; counts += 1. */

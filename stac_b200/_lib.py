@@ -82,6 +82,9 @@ SIGNATURES = {
     "stac_qkv_epilogue_append": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_void_p, c_void_p, c_f32, c_void_p,
                                          c_void_p, c_void_p, c_int, c_void_p, c_i64, c_void_p, c_void_p, c_i64,
                                          c_void_p, c_i64, c_int, c_int, c_int, c_i64, c_void_p]),
+    "stac_qkv_epilogue_append_tables": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_void_p, c_void_p, c_f32, c_void_p,
+                                                c_void_p, c_void_p, c_i64, c_int, c_void_p, c_i64, c_void_p, c_void_p,
+                                                c_i64, c_void_p, c_i64, c_int, c_int, c_int, c_i64, c_void_p]),
     "stac_scores_update": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_int, c_int, c_int, c_int, c_f32,
                                    c_void_p]),
     "stac_h2o_select": (c_int, [c_void_p, c_i64, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
@@ -101,7 +104,7 @@ SIGNATURES = {
 KERNELS_PER_CALL = {
     "stac_attn_colsum": 3, "stac_attn_colsum_kept": 3, "stac_attn_colsum_noalloc": 3, "stac_selftest_bounded_wait": 1,
     "stac_voxel_hash_clear": 1, "stac_voxel_rehash": 2, "stac_voxel_upsert": 3, "stac_voxel_neighbors": 2, "stac_pointmap_to_positions": 1,
-    "stac_append_kv": 1, "stac_qkv_epilogue_append": 1, "stac_scores_update": 1, "stac_h2o_select": 1, "stac_compact": 2, "stac_merge_insert": 16, "stac_retrieve": 2,
+    "stac_append_kv": 1, "stac_qkv_epilogue_append": 1, "stac_qkv_epilogue_append_tables": 1, "stac_scores_update": 1, "stac_h2o_select": 1, "stac_compact": 2, "stac_merge_insert": 16, "stac_retrieve": 2,
 }
 CALLS = {}
 

@@ -320,14 +320,18 @@ class KVManager:
                 n_pos = int(p64.max().item()) + 1
                 self._rope_rows[T_new] = n_pos
             c32, s32 = rope._compute_frequency_components(D // 2, n_pos, self.device, torch.float32)
-            cos, sin = c32[:, : D // 4].contiguous(), s32[:, : D // 4].contiguous()
+            # the kernel reads the first D // 4 values of every table row, wherever the rows lie
+            cos, sin = c32[:, : D // 4], s32[:, : D // 4]
+            if cos.stride(1) != 1 or sin.stride(1) != 1 or cos.stride(0) != sin.stride(0) or cos.stride(0) < D // 4:
+                cos, sin = cos.contiguous(), sin.contiguous()
         q_out = torch.empty((1, T_new, H, D), dtype=torch.bfloat16, device=self.device)
         kc, vc, ti = self.key_cache_hot[slot], self.value_cache_hot[slot], self._token_indices_hot[slot]
         first_id = self._processed_frames * self.token_per_f
-        check(_lib.lib().stac_qkv_epilogue_append(
-            ptr(x), x.stride(0), ptr(qw), ptr(qb), ptr(kw), ptr(kb), eps, ptr(p64), ptr(cos), ptr(sin), n_pos,
+        check(_lib.lib().stac_qkv_epilogue_append_tables(
+            ptr(x), x.stride(0), ptr(qw), ptr(qb), ptr(kw), ptr(kb), eps, ptr(p64), ptr(cos), ptr(sin),
+            cos.stride(0) if cos is not None else D // 4, n_pos,
             ptr(q_out), q_out.stride(1), ptr(kc), ptr(vc), kc.stride(0), ptr(ti), ti.stride(0), H, T_new, old_T,
-            first_id, stream_ptr()), "stac_qkv_epilogue_append")
+            first_id, stream_ptr()), "stac_qkv_epilogue_append_tables")
         if slot == self._L_eff - 1:
             self._processed_frames += T_new // self.token_per_f
         self._offset_hot[slot] = old_T + T_new

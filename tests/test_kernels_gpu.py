@@ -185,6 +185,50 @@ def test_scores_update_and_compact():
     assert bool((S2[:, n_keep:] == 0).all()) and bool((C2[:, n_keep:] == 0).all())
 
 
+@pytest.mark.parametrize("norm,rope", [(True, True), (True, False), (False, True), (False, False)])
+@pytest.mark.parametrize("pad,tokens,heads,table", [(0, 21, 3, 16), (0, 64, 16, 32), (2, 21, 3, 32), (1, 40, 2, 16), (8, 7, 1, 40)])
+def test_projection_epilogue(pad, tokens, heads, table, norm, rope):
+    """LayerNorm + 2-D rotary embedding + append against fp32 torch, rounded once to bf16 (so at most one
+    unit in the last place apart: 2^-7 relative).  `pad` widens the rows of the projection's output, so
+    that they start on 16-, 4- and 2-byte boundaries; `table` is the distance of table rows."""
+    from stac_b200 import _lib
+    p = _lib.ptr
+    g = torch.Generator().manual_seed(tokens + pad)
+    T, H, D, n_pos, old = tokens, heads, 64, 9, 5
+    qkv = torch.randn(T, 3 * H * D + pad, generator=g).to(torch.bfloat16).to(DEV)
+    w = [torch.randn(D, generator=g).to(DEV) for _ in range(4)]
+    pos = torch.randint(0, n_pos, (T, 2), generator=g).to(DEV)
+    ang = torch.randn(n_pos, table, generator=g).to(DEV)
+    cos, sin = ang.cos(), ang.sin()
+    q = torch.empty(T, H, D, dtype=torch.bfloat16, device=DEV)
+    kc, vc = (torch.zeros(H, T + old + 3, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ti = torch.full((H, T + old + 3), -1, dtype=torch.int64, device=DEV)
+    nw = [p(t) if norm else None for t in w]
+    rc = _lib.lib().stac_qkv_epilogue_append_tables(
+        p(qkv), qkv.stride(0), *nw, 1e-5, p(pos) if rope else None, p(cos) if rope else None, p(sin) if rope else None,
+        table, n_pos if rope else 0, p(q), q.stride(0), p(kc), p(vc), kc.stride(0), p(ti), ti.stride(0), H, T, old, 100,
+        _lib.stream_ptr())
+    assert rc == 0
+    x = qkv[:, :3 * H * D].float().reshape(T, 3, H, D)
+
+    def restate(y, weight, bias):
+        if norm:
+            y = torch.nn.functional.layer_norm(y, (D,), weight, bias, 1e-5)
+        if rope:
+            halves = []
+            for half, at in zip(y.split(32, -1), (pos[:, 0], pos[:, 1])):
+                c, s = (torch.cat([t[at, :16]] * 2, -1).unsqueeze(1) for t in (cos, sin))
+                halves.append(half * c + torch.cat([-half[..., 16:], half[..., :16]], -1) * s)
+            y = torch.cat(halves, -1)
+        return y
+    torch.testing.assert_close(q.float(), restate(x[:, 0], w[0], w[1]), rtol=2 ** -7, atol=1e-4)
+    torch.testing.assert_close(kc[:, old:old + T].float(), restate(x[:, 1], w[2], w[3]).transpose(0, 1), rtol=2 ** -7, atol=1e-4)
+    assert torch.equal(vc[:, old:old + T], x[:, 2].transpose(0, 1).to(torch.bfloat16))
+    assert torch.equal(ti[:, old:old + T], (100 + torch.arange(T, device=DEV)).expand(H, -1))
+    for t in (kc, vc):
+        assert bool((t[:, :old] == 0).all()) and bool((t[:, old + T:] == 0).all())
+
+
 def _compare_pool(snap, m, tag, rtol, atol):
     sm = m.slot_map()
     for key in ("buf_offset", "buf_seg", "piv_offset", "piv_seg"):
