@@ -216,6 +216,11 @@ int stac_compact(const int* keep_idx, int n_rows, int n_keep, int T_buf, int hea
                  const int64_t* ti_src, int64_t* ti_dst, const float* s_src, float* s_dst,
                  const float* c_src, float* c_dst, const int* vx_src, int* vx_dst, stac_stream_t stream);
 
+/* The same for a cache without scores whose rows all keep the same positions: keep_idx [n_keep]. */
+int stac_compact_window(const int* keep_idx, int n_rows, int n_keep, int T_buf, int head_dim, int elem_bytes,
+                        const void* k_src, const void* v_src, void* k_dst, void* v_dst, const int64_t* ti_src,
+                        int64_t* ti_dst, stac_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------
  * Voxel memory: per (pool head, voxel) row up to budget_cap buffered tokens and pivot_cap
  * pivots, one token per pool segment.  Same observable state as the reference's

@@ -185,8 +185,9 @@ h2o_select_kernel(const float* __restrict__ scores, long long row_stride, const 
 
 // Gather-compaction into a second set of buffers: dst[row, j] = src[row, keep[row, j]].
 // K and V move as 16-byte vectors, eight threads per 128-byte (bf16) or sixteen per 256-byte
-// (fp32) row.
-__global__ void compact_kv_kernel(const int* __restrict__ keep_idx, int n_keep, const uint4* __restrict__ k_src,
+// (fp32) row.  `keep_stride` is 0 where all rows keep the same positions.
+__global__ void compact_kv_kernel(const int* __restrict__ keep_idx, long long keep_stride, int n_keep,
+                                  const uint4* __restrict__ k_src,
                                   const uint4* __restrict__ v_src, uint4* __restrict__ k_dst,
                                   uint4* __restrict__ v_dst, long long row_stride_vec, int vec_per_token) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel in the stream
@@ -195,14 +196,15 @@ __global__ void compact_kv_kernel(const int* __restrict__ keep_idx, int n_keep, 
   const long long tok = gid / vec_per_token;
   const int part = static_cast<int>(gid % vec_per_token);
   if (tok >= n_keep) return;
-  const int src = keep_idx[static_cast<long long>(row) * n_keep + tok];
+  const int src = keep_idx[row * keep_stride + tok];
   const long long so = row * row_stride_vec + static_cast<long long>(src) * vec_per_token + part;
   const long long dof = row * row_stride_vec + tok * vec_per_token + part;
   k_dst[dof] = k_src[so];
   v_dst[dof] = v_src[so];
 }
 
-__global__ void compact_meta_kernel(const int* __restrict__ keep_idx, int n_keep, int T_buf,
+// (a cache without scores passes no score and count arrays)
+__global__ void compact_meta_kernel(const int* __restrict__ keep_idx, long long keep_stride, int n_keep, int T_buf,
                                     const long long* __restrict__ ti_src, long long* __restrict__ ti_dst,
                                     const float* __restrict__ s_src, float* __restrict__ s_dst,
                                     const float* __restrict__ c_src, float* __restrict__ c_dst,
@@ -213,15 +215,19 @@ __global__ void compact_meta_kernel(const int* __restrict__ keep_idx, int n_keep
   if (j >= T_buf) return;
   const long long o = static_cast<long long>(row) * T_buf + j;
   if (j < n_keep) {
-    const long long s = static_cast<long long>(row) * T_buf + keep_idx[static_cast<long long>(row) * n_keep + j];
+    const long long s = static_cast<long long>(row) * T_buf + keep_idx[row * keep_stride + j];
     ti_dst[o] = ti_src[s];
-    s_dst[o] = s_src[s];
-    c_dst[o] = c_src[s];
+    if (s_src != nullptr) {
+      s_dst[o] = s_src[s];
+      c_dst[o] = c_src[s];
+    }
     if (vx_src != nullptr) vx_dst[o] = vx_src[s];
   } else {
     ti_dst[o] = -1;
-    s_dst[o] = 0.f;
-    c_dst[o] = 0.f;
+    if (s_dst != nullptr) {
+      s_dst[o] = 0.f;
+      c_dst[o] = 0.f;
+    }
     if (vx_dst != nullptr) vx_dst[o] = -1;
   }
 }
@@ -502,14 +508,14 @@ int stac_h2o_select(const float* scores, int64_t row_stride, int n_rows, const u
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
-int stac_compact(const int* keep_idx, int n_rows, int n_keep, int T_buf, int head_dim, int elem_bytes,
+}  // extern "C"
+
+namespace {
+
+int compact_launch(const int* keep_idx, long long keep_stride, int n_rows, int n_keep, int T_buf, int head_dim, int elem_bytes,
                  const void* k_src, const void* v_src, void* k_dst, void* v_dst, const int64_t* ti_src,
                  int64_t* ti_dst, const float* s_src, float* s_dst, const float* c_src, float* c_dst,
                  const int* vx_src, int* vx_dst, stac_stream_t stream) {
-  if (keep_idx == nullptr || k_src == nullptr || v_src == nullptr || k_dst == nullptr || v_dst == nullptr ||
-      ti_src == nullptr || ti_dst == nullptr || s_src == nullptr || s_dst == nullptr || c_src == nullptr ||
-      c_dst == nullptr || n_rows <= 0 || n_keep < 0 || n_keep > T_buf)
-    return STAC_ERR_BAD_ARG;
   if ((vx_src == nullptr) != (vx_dst == nullptr)) return STAC_ERR_BAD_ARG;
   const int token_bytes = head_dim * elem_bytes;
   if (token_bytes % 16 != 0 || (elem_bytes != 2 && elem_bytes != 4)) return STAC_ERR_BAD_ARG;
@@ -518,18 +524,44 @@ int stac_compact(const int* keep_idx, int n_rows, int n_keep, int T_buf, int hea
   if (n_keep > 0) {
     const long long total = static_cast<long long>(n_keep) * vpt;
     dim3 grid(static_cast<unsigned>((total + 255) / 256), n_rows);
-    if (stac::launch_behind(stac::compact_kv_kernel, grid, dim3(256), 0, st, keep_idx, n_keep,
+    if (stac::launch_behind(stac::compact_kv_kernel, grid, dim3(256), 0, st, keep_idx, keep_stride, n_keep,
                             static_cast<const uint4*>(k_src), static_cast<const uint4*>(v_src),
                             static_cast<uint4*>(k_dst), static_cast<uint4*>(v_dst),
                             static_cast<long long>(T_buf) * vpt, vpt) != cudaSuccess)
       return STAC_ERR_CUDA;
   }
   dim3 grid_m((T_buf + 255) / 256, n_rows);
-  if (stac::launch_behind(stac::compact_meta_kernel, grid_m, dim3(256), 0, st, keep_idx, n_keep, T_buf,
+  if (stac::launch_behind(stac::compact_meta_kernel, grid_m, dim3(256), 0, st, keep_idx, keep_stride, n_keep, T_buf,
                           reinterpret_cast<const long long*>(ti_src), reinterpret_cast<long long*>(ti_dst), s_src,
                           s_dst, c_src, c_dst, vx_src, vx_dst) != cudaSuccess)
     return STAC_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
+}
+
+}  // namespace
+
+extern "C" {
+
+int stac_compact(const int* keep_idx, int n_rows, int n_keep, int T_buf, int head_dim, int elem_bytes,
+                 const void* k_src, const void* v_src, void* k_dst, void* v_dst, const int64_t* ti_src,
+                 int64_t* ti_dst, const float* s_src, float* s_dst, const float* c_src, float* c_dst,
+                 const int* vx_src, int* vx_dst, stac_stream_t stream) {
+  if (keep_idx == nullptr || k_src == nullptr || v_src == nullptr || k_dst == nullptr || v_dst == nullptr ||
+      ti_src == nullptr || ti_dst == nullptr || s_src == nullptr || s_dst == nullptr || c_src == nullptr ||
+      c_dst == nullptr || n_rows <= 0 || n_keep < 0 || n_keep > T_buf)
+    return STAC_ERR_BAD_ARG;
+  return compact_launch(keep_idx, n_keep, n_rows, n_keep, T_buf, head_dim, elem_bytes, k_src, v_src, k_dst, v_dst, ti_src,
+                        ti_dst, s_src, s_dst, c_src, c_dst, vx_src, vx_dst, stream);
+}
+
+int stac_compact_window(const int* keep_idx, int n_rows, int n_keep, int T_buf, int head_dim, int elem_bytes,
+                        const void* k_src, const void* v_src, void* k_dst, void* v_dst, const int64_t* ti_src,
+                        int64_t* ti_dst, stac_stream_t stream) {
+  if (keep_idx == nullptr || k_src == nullptr || v_src == nullptr || k_dst == nullptr || v_dst == nullptr ||
+      ti_src == nullptr || ti_dst == nullptr || n_rows <= 0 || n_keep < 0 || n_keep > T_buf)
+    return STAC_ERR_BAD_ARG;
+  return compact_launch(keep_idx, 0, n_rows, n_keep, T_buf, head_dim, elem_bytes, k_src, v_src, k_dst, v_dst, ti_src,
+                        ti_dst, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, stream);
 }
 
 }  // extern "C"

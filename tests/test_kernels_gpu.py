@@ -229,6 +229,33 @@ def test_projection_epilogue(pad, tokens, heads, table, norm, rope):
         assert bool((t[:, :old] == 0).all()) and bool((t[:, old + T:] == 0).all())
 
 
+@pytest.mark.parametrize("rows,T_buf,n_keep", [(1, 1, 1), (3, 300, 257), (5, 256, 256), (2, 40, 0), (4, 1030, 33)])
+def test_window_compaction_is_compaction_with_one_row_of_positions(rows, T_buf, n_keep):
+    from stac_b200 import _lib
+    p = _lib.ptr
+    g = torch.Generator().manual_seed(T_buf)
+    keep = torch.sort(torch.randperm(T_buf, generator=g)[:max(n_keep, 1)])[0].to(torch.int32).to(DEV)
+    k, v = (torch.randn(rows, T_buf, 64, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    ti = torch.randint(0, 10 ** 6, (rows, T_buf), generator=g).to(DEV)
+    sc = torch.zeros(rows, T_buf, device=DEV)
+    outs = []
+    for shared in (True, False):
+        kd, vd, td = torch.zeros_like(k), torch.zeros_like(v), torch.zeros_like(ti)
+        if shared:
+            rc = _lib.lib().stac_compact_window(p(keep), rows, n_keep, T_buf, 64, 2, p(k), p(v), p(kd), p(vd), p(ti), p(td),
+                                                _lib.stream_ptr())
+        else:
+            every = keep[:n_keep].expand(rows, -1).contiguous() if n_keep else keep
+            s2 = torch.empty_like(sc)
+            rc = _lib.lib().stac_compact(p(every), rows, n_keep, T_buf, 64, 2, p(k), p(v), p(kd), p(vd), p(ti), p(td),
+                                         p(sc), p(s2), p(sc), p(s2), None, None, _lib.stream_ptr())
+        assert rc == 0
+        outs.append((kd, vd, td))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    assert bool((outs[0][2][:, n_keep:] == -1).all())
+
+
 def _compare_pool(snap, m, tag, rtol, atol):
     sm = m.slot_map()
     for key in ("buf_offset", "buf_seg", "piv_offset", "piv_seg"):
