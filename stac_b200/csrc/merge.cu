@@ -26,9 +26,12 @@
 //   rows_rank_kernel     one thread per row: score gate of the row's pivots, selection, ranking of
 //                        the buffered tokens + selected tokens by (score desc, arrival order),
 //                        counts of new segments / overflow / full; rows with many tokens are
-//                        queued for rows_rank_long_kernel (one warp per row, same result).
-//   scan_heads_kernel /  exclusive scans of those counts, allocation plan (k ids from the top
-//   scan_plan_kernel     of the free list, the rest fresh), capacity checks.
+//                        left to the CTA's warps (one per row, same result).
+//   scan_rows_kernel     exclusive scans of those counts inside every head; the CTA that finishes
+//                        last scans the heads and makes the allocation plan (k ids from the top of
+//                        the free list, the rest fresh) and the capacity checks.  Launched twice:
+//                        the second launch does something only if bounded pools were too small,
+//                        and then skips the rows that do not fit before it scans again.
 //   rows_phase_b1a_kernel one thread per row: hand out segment ids, publish occupancy, queue rows
 //                        whose buffered tokens change column / whose buffer filled up.
 //   rows_phase_b1m_kernel one warp per queued row: move buffered tokens to their new column
@@ -38,7 +41,11 @@
 //   rows_phase_b2_kernel eight lanes per full row: turn the buffer into a pivot, insert it (folding
 //                        the lowest-weight pivot into its nearest neighbour when the row is
 //                        saturated), stage the freed segment ids.
-//   finalize_kernel      append staged ids to the free list, publish counters.
+//   finalize_kernel      append staged ids to the free list (or carry the overflow list over when the
+//                        call had no valid token).
+// (Eleven launches and one memset; with the long rows, the plan, the skipping and the carried list in launches
+// of their own they were sixteen and two: bounded memory of 384 heads 1381 -> 1282 us per insert and
+// retrieval, a two-layer stream 437 -> 422 us per step.)
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -128,12 +135,11 @@ struct MergeParams {
   int4* head_base;     // [heads]
   int* plan;           // device ints, see kPlan*
   int* free_stage;     // [buf_cap]
-  int2* defer_list;    // [heads*ncap] rows (head, row index) that need the warp-per-row phase A
   int2* full_list;     // [heads*ncap] rows whose buffer filled up in this call
   int2* move_list;     // [heads*ncap] rows in which buffered tokens change column
   int* tok_row;        // [heads][ncap] row index of each sorted token
   int* tok_best;       // [heads][ncap] index of the most similar pivot of the token's row
-  int* row_flag;       // [heads][ncap] zero on entry: set once a token of the row merges into a pivot
+  int* row_flag;       // [heads][ncap] cleared with the row list: set once a token of the row merges into a pivot
   int2* merge_list;    // [heads*ncap] rows (head, row index) with at least one merging token
   int passes;          // radix passes (8 bits each)
   int seg_vec;         // 1: the pivot segments of a row are one aligned 16-byte vector
@@ -141,8 +147,8 @@ struct MergeParams {
 };
 
 enum { kPlanK = 0, kPlanFreeLen, kPlanBufTop, kPlanPivTop, kPlanTotalAdd, kPlanTotalFull, kPlanTotalOver,
-       kPlanAnyValid, kPlanAbort, kPlanDeferCount, kPlanFullCount, kPlanMoveCount, kPlanShort, kPlanAvailBuf, kPlanAvailPiv,
-       kPlanMergeCount, kPlanSize = 16 };
+       kPlanAnyValid, kPlanAbort, kPlanFullCount, kPlanMoveCount, kPlanShort, kPlanAvailBuf, kPlanAvailPiv,
+       kPlanMergeCount, kPlanTicket, kPlanTicket2, kPlanSize = 32 };
 
 // Block-wide exclusive scan, 1024 threads.
 __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
@@ -169,6 +175,38 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
   if (threadIdx.x == 0) *total = warp_sums[31];
   __syncthreads();
   return excl;
+}
+
+__device__ __forceinline__ int4 add4(int4 a, int4 b) { return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ int4 shfl_up4(int4 v, int o) {
+  return make_int4(__shfl_up_sync(kFull, v.x, o), __shfl_up_sync(kFull, v.y, o), __shfl_up_sync(kFull, v.z, o),
+                   __shfl_up_sync(kFull, v.w, o));
+}
+// Block-wide exclusive scan of four values at once, 1024 threads; every thread gets the total.
+__device__ __forceinline__ int4 block_scan4(int4 v, int4* warp_sums, int4* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int4 incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int4 t = shfl_up4(incl, o);
+    if (lane >= o) incl = add4(incl, t);
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int4 w = warp_sums[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int4 t = shfl_up4(w, o);
+      if (lane >= o) w = add4(w, t);
+    }
+    warp_sums[lane] = w;
+  }
+  __syncthreads();
+  const int4 before = warp > 0 ? warp_sums[warp - 1] : make_int4(0, 0, 0, 0);
+  *total = warp_sums[31];
+  __syncthreads();
+  return make_int4(before.x + incl.x - v.x, before.y + incl.y - v.y, before.z + incl.z - v.z, before.w + incl.w - v.w);
 }
 
 // ------------------------------------------------------------------------------------ sort
@@ -354,6 +392,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
         if (hf[t]) {
           rvx[r] = static_cast<int>(key[t]);
           rst[r] = i;
+          p.row_flag[static_cast<long long>(h) * p.ncap + r] = 0;
         }
         p.tok_row[static_cast<long long>(h) * p.ncap + i] = r + hf[t] - 1;
         r += hf[t];
@@ -764,22 +803,10 @@ __device__ __forceinline__ void rank_row_warp(const MergeParams& p, const int h,
   }
 }
 
-// The same for short rows, one thread per row; rows with more than 32 tokens are queued for the
-// warp-per-row kernel.
-__global__ void __launch_bounds__(256) rows_rank_kernel(const MergeParams p) {
-  grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  const int h = blockIdx.y;
-  const int ri = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p.plan[kPlanAnyValid] == 0) return;
-  if (ri >= p.n_rows[h]) return;
+// The same for a short row, by one thread.
+__device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int h, const int ri, const int vx,
+                                                const int s0, const int s1) {
   const long long hb = static_cast<long long>(h) * p.ncap;
-  const int vx = p.row_vx[hb + ri];
-  const int* rst = p.row_start + static_cast<long long>(h) * (p.ncap + 1);
-  const int s0 = rst[ri], s1 = rst[ri + 1];
-  if (s1 - s0 > 32) {
-    p.defer_list[list_push(&p.plan[kPlanDeferCount])] = make_int2(h, ri);
-    return;
-  }
   const long long r = static_cast<long long>(h) * p.voxel_cap + vx;
   const int npiv = p.piv_row_cnt[r];
   const int nbuf = p.buf_row_cnt[r];
@@ -833,89 +860,64 @@ __global__ void __launch_bounds__(256) rows_rank_kernel(const MergeParams p) {
   p.row_info[hb + ri] = info;
 }
 
-__global__ void __launch_bounds__(256) rows_rank_long_kernel(const MergeParams p) {
+// One thread per row; a row with more than 32 tokens is ranked by a warp of its CTA afterwards.
+__global__ void __launch_bounds__(256) rows_rank_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  const int lane = threadIdx.x & 31;
-  const int warps_per_block = blockDim.x >> 5;
-  const int n = p.plan[kPlanDeferCount];
-  for (int w = blockIdx.x * warps_per_block + (threadIdx.x >> 5); w < n; w += gridDim.x * warps_per_block) {
-    const int2 hr = p.defer_list[w];
-    rank_row_warp(p, hr.x, hr.y, lane);
+  __shared__ int long_rows[256];
+  __shared__ int n_long;
+  const int h = blockIdx.y;
+  const int r0 = blockIdx.x * 256;
+  if (p.plan[kPlanAnyValid] == 0) return;
+  const int n_rows = p.n_rows[h];
+  if (r0 >= n_rows) return;
+  if (threadIdx.x == 0) n_long = 0;
+  __syncthreads();
+  const int ri = r0 + threadIdx.x;
+  if (ri < n_rows) {
+    const int* rst = p.row_start + static_cast<long long>(h) * (p.ncap + 1);
+    const int s0 = rst[ri], s1 = rst[ri + 1];
+    const int vx = p.row_vx[static_cast<long long>(h) * p.ncap + ri];
+    if (s1 - s0 > 32) long_rows[list_push(&n_long)] = ri;
+    else rank_row_thread(p, h, ri, vx, s0, s1);
   }
+  __syncthreads();
+  for (int w = threadIdx.x >> 5; w < n_long; w += 8) rank_row_warp(p, h, long_rows[w], threadIdx.x & 31);
 }
 
 // ------------------------------------------------------------------------------------ scans
-// pass 0 always runs; pass 1 only when pass 0 found the pools too small and rows were trimmed
-__global__ void __launch_bounds__(1024, 1) scan_heads_kernel(const MergeParams p, const int pass) {
-  grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  __shared__ int warp_sums[32];
-  __shared__ int sh_total;
-  __shared__ int carry[4];
-  if (pass == 1 && p.plan[kPlanShort] == 0) return;
-  const int h = blockIdx.x;
-  const long long hb = static_cast<long long>(h) * p.ncap;
-  const int n = p.plan[kPlanAnyValid] ? p.n_rows[h] : 0;
-  if (threadIdx.x < 4) carry[threadIdx.x] = 0;
-  __syncthreads();
-  for (int base = 0; base < n; base += 1024) {
-    const int i = base + threadIdx.x;
-    int4 info = make_int4(0, 0, 0, 0);
-    if (i < n) info = p.row_info[hb + i];
-    int4 pref;
-    const int v0 = info.x, v1 = info.y, v2 = info.z & 1, v3 = (info.z >> 1) & 1;
-    pref.x = carry[0] + block_scan(v0, warp_sums, &sh_total);
-    const int t0 = sh_total;
-    pref.y = carry[1] + block_scan(v1, warp_sums, &sh_total);
-    const int t1 = sh_total;
-    pref.z = carry[2] + block_scan(v2, warp_sums, &sh_total);
-    const int t2 = sh_total;
-    pref.w = carry[3] + block_scan(v3, warp_sums, &sh_total);
-    const int t3 = sh_total;
-    if (i < n) p.row_pref[hb + i] = pref;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      carry[0] += t0; carry[1] += t1; carry[2] += t2; carry[3] += t3;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) p.head_tot[h] = make_int4(carry[0], carry[1], carry[2], carry[3]);
+// Bounded pools: a row that would open new buffer columns, or need a new pivot segment, beyond
+// what is left is skipped as a whole (its selected tokens are dropped, the row stays as it
+// was).  The cut follows the allocation order, i.e. (head, voxel) ascending, so it is
+// deterministic; merges into existing pivots done before stay.  A skipped row is left with no
+// selected token (info.w = 0): tokens_place_kernel looks at that.  Returns the tokens dropped.
+__device__ __forceinline__ int skip_row_that_does_not_fit(const MergeParams& p, int4& info, int4 pref, int4 hbase) {
+  if (info.w == 0) return 0;
+  const bool no_buf = info.x > 0 && hbase.x + pref.x + info.x > p.plan[kPlanAvailBuf];
+  const bool no_piv = (info.z & 2) && hbase.w + pref.w + 1 > p.plan[kPlanAvailPiv];
+  if (!no_buf && !no_piv) return 0;
+  const int dropped = info.w;
+  info = make_int4(0, 0, info.z & ~3, 0);
+  return dropped;
 }
 
-__global__ void __launch_bounds__(1024, 1) scan_plan_kernel(const MergeParams p, const int pass) {
-  grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  __shared__ int warp_sums[32];
-  __shared__ int sh_total;
-  __shared__ int carry[4];
-  if (pass == 1 && p.plan[kPlanShort] == 0) return;
-  if (threadIdx.x < 4) carry[threadIdx.x] = 0;
-  __syncthreads();
+// Scan over the heads and allocation plan, by one CTA of 1024 threads.
+__device__ __forceinline__ void make_plan(const MergeParams& p, const int pass, int4* warp_sums) {
+  int4 carry = make_int4(0, 0, 0, 0);
   for (int base = 0; base < p.heads; base += 1024) {
     const int h = base + threadIdx.x;
-    int4 t = make_int4(0, 0, 0, 0);
-    if (h < p.heads) t = p.head_tot[h];
-    int4 b;
-    b.x = carry[0] + block_scan(t.x, warp_sums, &sh_total);
-    const int t0 = sh_total;
-    b.y = carry[1] + block_scan(t.y, warp_sums, &sh_total);
-    const int t1 = sh_total;
-    b.z = carry[2] + block_scan(t.z, warp_sums, &sh_total);
-    const int t2 = sh_total;
-    b.w = carry[3] + block_scan(t.w, warp_sums, &sh_total);
-    const int t3 = sh_total;
+    int4 t = make_int4(0, 0, 0, 0), total;
+    if (h < p.heads) t = __ldcg(&p.head_tot[h]);
+    const int4 b = add4(carry, block_scan4(t, warp_sums, &total));
     if (h < p.heads) {
       p.head_base[h] = b;
       p.over_start_out[h] = b.y;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      carry[0] += t0; carry[1] += t1; carry[2] += t2; carry[3] += t3;
-    }
-    __syncthreads();
+    carry = add4(carry, total);
   }
   if (threadIdx.x == 0) {
     if (pass == 0 && p.voxel_count != nullptr) p.meta[STAC_META_VOXELS] = max(p.meta[STAC_META_VOXELS], *p.voxel_count);
     const int any = p.plan[kPlanAnyValid];
-    const int total_add = carry[0], total_over = carry[1], total_full = carry[2], total_piv = carry[3];
+    const int total_add = carry.x, total_over = carry.y, total_full = carry.z, total_piv = carry.w;
     const int free_len = p.meta[STAC_META_BUF_FREE_LEN];
     const int buf_top = p.meta[STAC_META_BUF_TOP];
     const int piv_top = p.meta[STAC_META_PIV_TOP];
@@ -932,8 +934,8 @@ __global__ void __launch_bounds__(1024, 1) scan_plan_kernel(const MergeParams p,
       const int avail_buf = free_len + (p.buf_cap - buf_top);
       const int avail_piv = p.piv_cap - piv_top;
       if (pass == 0 && (total_add > avail_buf || total_piv > avail_piv)) {
-        // The pools are bounded and this call does not fit: rows are trimmed in (head, voxel)
-        // order by trim_rows_kernel and the plan is recomputed by pass 1.
+        // The pools are bounded and this call does not fit: rows are skipped in (head, voxel)
+        // order by the second launch, which makes the plan again.
         p.plan[kPlanShort] = 1;
         p.plan[kPlanAvailBuf] = avail_buf;
         p.plan[kPlanAvailPiv] = avail_piv;
@@ -957,37 +959,51 @@ __global__ void __launch_bounds__(1024, 1) scan_plan_kernel(const MergeParams p,
   }
 }
 
-// ------------------------------------------------------------------------------------ phase B
-// Bounded pools: a row that would open new buffer columns, or need a new pivot segment, beyond
-// what is left is skipped as a whole (its selected tokens are dropped, the row stays as it
-// was).  The cut follows the allocation order, i.e. (head, voxel) ascending, so it is
-// deterministic; merges into existing pivots done in phase A stay.
-__global__ void __launch_bounds__(256) trim_rows_kernel(const MergeParams p) {
+// pass 0 always runs; pass 1 only when pass 0 found the pools too small
+__global__ void __launch_bounds__(1024, 2) scan_rows_kernel(const MergeParams p, const int pass) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  const int h = blockIdx.y;
-  const int ri = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p.plan[kPlanAnyValid] == 0 || p.plan[kPlanShort] == 0) return;
-  if (ri >= p.n_rows[h]) return;
+  __shared__ int4 warp_sums[32];
+  __shared__ int sh_last;
+  if (pass == 1 && p.plan[kPlanShort] == 0) return;
+  const int h = blockIdx.x;
   const long long hb = static_cast<long long>(h) * p.ncap;
-  const int4 info = p.row_info[hb + ri];
-  if (info.w == 0) return;
-  const int4 pref = p.row_pref[hb + ri];
-  const int4 hbase = p.head_base[h];
-  const bool no_buf = info.x > 0 && hbase.x + pref.x + info.x > p.plan[kPlanAvailBuf];
-  const bool no_piv = (info.z & 2) && hbase.w + pref.w + 1 > p.plan[kPlanAvailPiv];
-  if (!no_buf && !no_piv) return;
-  const int* rst = p.row_start + static_cast<long long>(h) * (p.ncap + 1);
+  const int n = p.plan[kPlanAnyValid] ? p.n_rows[h] : 0;
+  int4 hbase = make_int4(0, 0, 0, 0), carry = make_int4(0, 0, 0, 0);
+  if (pass == 1) hbase = p.head_base[h];
   int dropped = 0;
-  for (int i = rst[ri]; i < rst[ri + 1]; ++i) {
-    if (p.tok_dest[hb + i] >= 0) {
-      p.tok_dest[hb + i] = -1;
-      ++dropped;
+  for (int base = 0; base < n; base += 1024) {
+    const int i = base + threadIdx.x;
+    int4 info = make_int4(0, 0, 0, 0), total;
+    if (i < n) {
+      info = p.row_info[hb + i];
+      if (pass == 1) {
+        const int d = skip_row_that_does_not_fit(p, info, p.row_pref[hb + i], hbase);
+        if (d > 0) p.row_info[hb + i] = info;
+        dropped += d;
+      }
     }
+    const int4 v = make_int4(info.x, info.y, info.z & 1, (info.z >> 1) & 1);
+    const int4 pref = add4(carry, block_scan4(v, warp_sums, &total));
+    if (i < n) p.row_pref[hb + i] = pref;
+    carry = add4(carry, total);
   }
-  p.row_info[hb + ri] = make_int4(0, 0, info.z & ~3, 0);
-  atomicAdd(&p.meta[STAC_META_DROPPED], dropped);
+  if (pass == 1) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dropped += __shfl_xor_sync(kFull, dropped, o);
+    if ((threadIdx.x & 31) == 0 && dropped > 0) atomicAdd(&p.meta[STAC_META_DROPPED], dropped);
+  }
+  // the CTA that arrives last sees every head's total
+  if (threadIdx.x == 0) {
+    p.head_tot[h] = carry;
+    __threadfence();
+    sh_last = atomicAdd(&p.plan[pass == 0 ? kPlanTicket : kPlanTicket2], 1) == p.heads - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (sh_last) make_plan(p, pass, warp_sums);
 }
 
+// ------------------------------------------------------------------------------------ phase B
 // Phase B, step 1 (one thread per row): hand out the segment ids of the new columns in
 // (row, column) order from the allocation plan, publish the new occupancy, and queue the rows
 // whose buffered tokens change column or whose buffer filled up.
@@ -1107,9 +1123,10 @@ __global__ void __launch_bounds__(kTokBlock) tokens_place_kernel(const MergePara
   __syncthreads();
   const long long hb = static_cast<long long>(h) * p.ncap;
   const int i = i0 + threadIdx.x;
+  const bool short_of_room = p.plan[kPlanShort] != 0;     // rows may have been skipped since their tokens were ranked
   if (i < n_tok) {
     const int d = p.tok_dest[hb + i];
-    if (d >= 0) {
+    if (d >= 0 && (!short_of_room || p.row_info[hb + p.tok_row[hb + i]].w != 0)) {
       const int code = (((p.passes & 1) ? p.vals_b : p.vals_a) + hb)[i];
       const int vx = static_cast<int>((((p.passes & 1) ? p.keys_b : p.keys_a) + hb)[i]);
       const float sc = p.tok_score[hb + i];
@@ -1367,43 +1384,39 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
   }
 }
 
-// Freed ids are appended after the part of the free list that was not handed out.
+// Freed ids are appended after the part of the free list that was not handed out.  Without a valid
+// evicted token in the whole call the reference returns before touching the carried overflow
+// (stac/merger.py:1203-1208), so the list is carried over unchanged.
+template <typename T>
 __global__ void finalize_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  if (p.plan[kPlanAnyValid] == 0 || p.plan[kPlanAbort] != 0) return;
-  const int n_freed = p.plan[kPlanTotalFull] * p.B;
-  const int base = p.plan[kPlanFreeLen] - p.plan[kPlanK];
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_freed; i += stride) p.buf_free[base + i] = p.free_stage[i];
-}
-
-// No valid evicted token in the whole call: the reference returns before touching the
-// carried overflow (stac/merger.py:1203-1208), so the list is carried over unchanged.
-template <typename T>
-__global__ void carry_overflow_kernel(const MergeParams p) {
-  grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  if (p.plan[kPlanAnyValid] != 0 && p.plan[kPlanAbort] == 0) return;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (p.plan[kPlanAnyValid] != 0 && p.plan[kPlanAbort] == 0) {
+    const int n_freed = p.plan[kPlanTotalFull] * p.B;
+    const int base = p.plan[kPlanFreeLen] - p.plan[kPlanK];
+    for (long long i = first; i < n_freed; i += stride) p.buf_free[base + i] = p.free_stage[i];
+    return;
+  }
   const int n = p.over_start_in[p.heads];
   const long long total = static_cast<long long>(n) * p.D;
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
+  for (long long i = first; i < total; i += stride) {
     static_cast<T*>(p.over_K_out)[i] = static_cast<const T*>(p.over_K_in)[i];
     static_cast<T*>(p.over_V_out)[i] = static_cast<const T*>(p.over_V_in)[i];
   }
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+  for (long long i = first; i < n; i += stride) {
     p.over_S_out[i] = p.over_S_in[i];
     p.over_hv_out[2 * i] = p.over_hv_in[2 * i];
     p.over_hv_out[2 * i + 1] = p.over_hv_in[2 * i + 1];
   }
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i <= p.heads; i += stride)
-    p.over_start_out[i] = p.over_start_in[i];
+  for (long long i = first; i <= p.heads; i += stride) p.over_start_out[i] = p.over_start_in[i];
 }
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct ScratchLayout {
   size_t keys_a, keys_b, vals_a, vals_b, n_tok, n_rows, row_vx, row_start, row_info, row_pref, old_dest, tok_dest,
-      tok_sim, tok_score, head_tot, head_base, plan, free_stage, defer_list, full_list, move_list, tok_row, tok_best, row_flag, merge_list, total;
+      tok_sim, tok_score, head_tot, head_base, plan, free_stage, full_list, move_list, tok_row, tok_best, row_flag, merge_list, total;
 };
 
 ScratchLayout scratch_layout(int heads, int ncap, int buf_cap) {
@@ -1422,7 +1435,7 @@ ScratchLayout scratch_layout(int heads, int ncap, int buf_cap) {
   L.tok_dest = take(hn * 4); L.tok_sim = take(hn * 4); L.tok_score = take(hn * 4);
   L.head_tot = take(static_cast<size_t>(heads) * 16); L.head_base = take(static_cast<size_t>(heads) * 16);
   L.plan = take(kPlanSize * 4); L.free_stage = take(static_cast<size_t>(buf_cap) * 4);
-  L.defer_list = take(hn * 8); L.full_list = take(hn * 8);
+  L.full_list = take(hn * 8);
   L.move_list = take(hn * 8); L.tok_row = take(hn * 4);
   L.tok_best = take(hn * 4); L.row_flag = take(hn * 4); L.merge_list = take(hn * 8);
   L.total = off;
@@ -1432,25 +1445,19 @@ ScratchLayout scratch_layout(int heads, int ncap, int buf_cap) {
 template <typename T>
 int launch_merge(MergeParams& mp, cudaStream_t st) {
   if (cudaMemsetAsync(mp.plan, 0, kPlanSize * 4, st) != cudaSuccess) return STAC_ERR_CUDA;
-  if (cudaMemsetAsync(mp.row_flag, 0, static_cast<size_t>(mp.heads) * mp.ncap * 4, st) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(sort_tokens_kernel, dim3(mp.heads), dim3(1024), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   dim3 grid_a1((mp.ncap + 255) / 256, mp.heads);
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
   if (launch_behind(tokens_sim_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_merge_kernel<T>, dim3(148 * 5), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_rank_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(rows_rank_long_kernel, dim3(148 * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(scan_heads_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 0) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(scan_plan_kernel, dim3(1), dim3(1024), 0, st, mp, 0) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(trim_rows_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(scan_heads_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 1) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(scan_plan_kernel, dim3(1), dim3(1024), 0, st, mp, 1) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(scan_rows_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 0) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(scan_rows_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 1) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_phase_b1a_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_phase_b1m_kernel<T, 2>, dim3(148 * 6), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(tokens_place_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_phase_b2_kernel<T>, dim3(148 * 16), dim3(128), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(finalize_kernel, dim3(148 * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;   // grid-stride over the freed ids (known on the device only)
-  if (launch_behind(carry_overflow_kernel<T>, dim3(148), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(finalize_kernel<T>, dim3(148 * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;   // grid-stride over the freed ids (known on the device only)
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
@@ -1516,7 +1523,6 @@ int stac_merge_insert(const stac_pool* pool, const stac_evicted* ev, void* scrat
   mp.head_base = reinterpret_cast<int4*>(base + L.head_base);
   mp.plan = reinterpret_cast<int*>(base + L.plan);
   mp.free_stage = reinterpret_cast<int*>(base + L.free_stage);
-  mp.defer_list = reinterpret_cast<int2*>(base + L.defer_list);
   mp.full_list = reinterpret_cast<int2*>(base + L.full_list);
   mp.move_list = reinterpret_cast<int2*>(base + L.move_list);
   mp.tok_row = reinterpret_cast<int*>(base + L.tok_row);

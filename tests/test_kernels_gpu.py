@@ -357,6 +357,7 @@ def test_merge_and_retrieve_match_oracle(name):
     (3, 700, 12, "f32"),       # rows above 32 tokens; pivot rows that are not a 16-byte vector
     (2, 512, 40, "f32"),
     (1, 256, 20, "bf16"),
+    (4, 2500, 2400, "f32"),    # more than 1024 rows in a head: two rounds of the row scan
 ])
 def test_merge_at_block_and_batch_edges(pivot_cap, tokens, voxels, dtype):
     """Token counts around the 256 tokens of a CTA, rows with more merging tokens than one batch of
@@ -384,6 +385,28 @@ def test_merge_at_block_and_batch_edges(pivot_cap, tokens, voxels, dtype):
         if m.piv.used() > 0:      # (a snapshot of a memory without pivots reads an unwritten pool)
             _compare_pool(g.snapshot(), m, f"step {step}", rtol, atol)
     assert m.piv.used() > 0
+
+
+@pytest.mark.parametrize("bound", [None, 9000])
+def test_merge_with_more_heads_than_one_round_of_the_plan(bound):
+    """1100 pool heads (the plan scans 1024 at a time), unbounded and with pools that fill up."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    rs = np.random.RandomState(4)
+    H, D, Tn, NV = 1100, 64, 6, 3
+    g = VoxelKVMerger(H, D, init_voxels=NV, pivot_cap=4, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8,
+                      score_thresh=0.1, dtype=torch.float32, device=DEV, slab_cap=16, max_buffer_slots=bound,
+                      max_pivot_slots=bound)
+    kw = {} if bound is None else dict(max_buf_slots=bound, max_piv_slots=bound)
+    m = VoxelMerger(H, D, NV, 4, 8, 0.8, 0.8, 0.1, "f32", **kw)
+    for step in range(6):
+        VX = rs.randint(0, NV, size=(H, Tn)).astype(np.int32)
+        K, V = (rs.randn(H, Tn, D).astype(np.float32) for _ in range(2))
+        S = np.exp(rs.randn(H, Tn)).astype(np.float32)
+        m.insert_and_merge(K, V, S, VX, NV)
+        g.insert_and_merge(*(torch.from_numpy(x).to(DEV) for x in (K, V, S)), None, torch.from_numpy(VX).to(DEV), NV)
+        if m.piv.used() > 0:
+            _compare_pool(g.snapshot(), m, f"step {step}", 1e-3, 1e-5)
+    assert m.piv.used() > 0 and g.info()["dropped_tokens"] == (m.dropped if bound else 0)
 
 
 @pytest.mark.parametrize("heads,voxels,pivot_cap,R,equal", [
