@@ -212,7 +212,12 @@ __device__ __forceinline__ int4 block_scan4(int4 v, int4* warp_sums, int4* total
 // ------------------------------------------------------------------------------------ sort
 __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  __shared__ int hist[256 * 32];  // [digit][warp]
+  // Digit counters, [warp][digit]: a warp's lanes count different digits of the same warp, so neighbouring
+  // digits lie in neighbouring banks; rows of 257 words let the scan, which walks them digit by
+  // digit, read without conflicts too.  ([digit][warp] put all of a warp's counters in one bank.)
+  // (384 heads, 8328 tokens each: insert + retrieval 1112 -> 1068 us; 16 heads, fp32: 278 -> 263 us.)
+  constexpr int kHistRow = 257;
+  __shared__ int hist[kHistRow * 32];
   __shared__ int warp_sums[32];
   __shared__ int sh_total;
   __shared__ int sh_carry;
@@ -278,60 +283,49 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
   const int c0 = warp * chunk;
   const int c1 = min(n, c0 + chunk);
   unsigned int* kin = ka; int* vin = va; unsigned int* kout = kb; int* vout = vb;
-  // A warp's chunk is read into registers once per pass when it is at most kRegIt * 32 items
-  // (lists of up to 8192 tokens): one round trip to L2 per pass instead of one per 32 items in
-  // each of the two loops.
+  // The first kRegIt * 32 items of a warp's chunk (all of it in lists of up to 8192 tokens) are read into
+  // registers once per pass: one round trip to L2 instead of one per 32 items in each of the two
+  // loops.
   constexpr int kRegIt = 8;
-  const bool in_regs = chunk <= 32 * kRegIt;
+  int* my_hist = hist + warp * kHistRow;
   for (int pass = 0; pass < p.passes; ++pass) {
     const int shift = pass * 8;
-    for (int i = threadIdx.x; i < 256 * 32; i += 1024) hist[i] = 0;
+    for (int i = threadIdx.x; i < kHistRow * 32; i += 1024) hist[i] = 0;
     unsigned int kreg[kRegIt];
     int vreg[kRegIt];
-    if (in_regs) {
 #pragma unroll
-      for (int t = 0; t < kRegIt; ++t) {
-        const int i = c0 + t * 32 + lane;
-        kreg[t] = i < c1 ? kin[i] : 0u;
-        vreg[t] = i < c1 ? vin[i] : 0;
-      }
+    for (int t = 0; t < kRegIt; ++t) {
+      const int i = c0 + t * 32 + lane;
+      kreg[t] = i < c1 ? kin[i] : 0u;
+      vreg[t] = i < c1 ? vin[i] : 0;
     }
     __syncthreads();
-    if (in_regs) {
+    auto count = [&](bool in, unsigned int key) {
+      const unsigned int d = in ? ((key >> shift) & 255u) : (256u + lane);
+      const unsigned int peers = __match_any_sync(kFull, d);
+      if (in && (peers & ((1u << lane) - 1)) == 0) my_hist[d] += __popc(peers);
+      __syncwarp();
+    };
 #pragma unroll
-      for (int t = 0; t < kRegIt; ++t) {
-        const int base = c0 + t * 32;
-        if (base < c1) {                                   // warp-uniform
-          const bool in = base + lane < c1;
-          const unsigned int d = in ? ((kreg[t] >> shift) & 255u) : (256u + lane);
-          const unsigned int peers = __match_any_sync(kFull, d);
-          if (in && (peers & ((1u << lane) - 1)) == 0) hist[d * 32 + warp] += __popc(peers);
-          __syncwarp();
-        }
-      }
-    } else {
-      for (int base = c0; base < c1; base += 32) {
-        const int i = base + lane;
-        const bool in = i < c1;
-        const unsigned int d = in ? ((kin[i] >> shift) & 255u) : (256u + lane);
-        const unsigned int peers = __match_any_sync(kFull, d);
-        if (in && (peers & ((1u << lane) - 1)) == 0) hist[d * 32 + warp] += __popc(peers);
-        __syncwarp();
-      }
+    for (int t = 0; t < kRegIt; ++t) {
+      const int base = c0 + t * 32;
+      if (base < c1) count(base + lane < c1, kreg[t]);       // warp-uniform
     }
+    for (int base = c0 + kRegIt * 32; base < c1; base += 32) count(base + lane < c1, base + lane < c1 ? kin[base + lane] : 0u);
     __syncthreads();
-    // exclusive scan of hist in (digit, warp) order: 8 consecutive entries per thread
+    // exclusive scan of the counters in (digit, warp) order: 8 consecutive entries per thread
     int loc[8];
     int sum = 0;
+    int* of_thread = hist + (threadIdx.x & 3) * 8 * kHistRow + (threadIdx.x >> 2);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      loc[e] = hist[threadIdx.x * 8 + e];
+      loc[e] = of_thread[e * kHistRow];
       sum += loc[e];
     }
     int run = block_scan(sum, warp_sums, &sh_total);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      hist[threadIdx.x * 8 + e] = run;
+      of_thread[e * kHistRow] = run;
       run += loc[e];
     }
     __syncthreads();
@@ -340,26 +334,22 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
       const unsigned int peers = __match_any_sync(kFull, d);
       const unsigned int before = peers & ((1u << lane) - 1);
       if (in) {
-        const int dst = hist[d * 32 + warp] + __popc(before);
+        const int dst = my_hist[d] + __popc(before);
         kout[dst] = key;
         vout[dst] = val;
       }
       __syncwarp();
-      if (in && before == 0) hist[d * 32 + warp] += __popc(peers);
+      if (in && before == 0) my_hist[d] += __popc(peers);
       __syncwarp();
     };
-    if (in_regs) {
 #pragma unroll
-      for (int t = 0; t < kRegIt; ++t) {
-        const int base = c0 + t * 32;
-        if (base < c1) scatter(base + lane < c1, kreg[t], vreg[t]);
-      }
-    } else {
-      for (int base = c0; base < c1; base += 32) {
-        const int i = base + lane;
-        const bool in = i < c1;
-        scatter(in, in ? kin[i] : 0u, in ? vin[i] : 0);
-      }
+    for (int t = 0; t < kRegIt; ++t) {
+      const int base = c0 + t * 32;
+      if (base < c1) scatter(base + lane < c1, kreg[t], vreg[t]);
+    }
+    for (int base = c0 + kRegIt * 32; base < c1; base += 32) {
+      const int i = base + lane;
+      scatter(i < c1, i < c1 ? kin[i] : 0u, i < c1 ? vin[i] : 0);
     }
     __syncthreads();
     unsigned int* tk = kin; kin = kout; kout = tk;
