@@ -80,6 +80,7 @@ class VoxelKVMerger:
         self._voxel_count_dev = None     # device scalar with the table's voxel count (set by the manager)
         # counters, overflow offsets and the status word of the last insert, read one call late
         self._mirror = LaggedInts(_lib.META_SIZE + self.H + 1 + 1)
+        self._no_status = torch.zeros(1, dtype=torch.int32, device=dev)    # stands in for a missing status word
         self._scratch = None
         self._ret_sel = None
 
@@ -233,7 +234,7 @@ class VoxelKVMerger:
     def _push_meta(self):
         """Enqueue the copy of the pool counters, the per-head overflow offsets and the status word
         to pinned host memory behind the insert that produced them; nothing waits here."""
-        word = self._status.word if self._status is not None else torch.zeros(1, dtype=torch.int32, device=self.device)
+        word = self._status.word if self._status is not None else self._no_status
         self._mirror.push(self._meta, self._over[self._over_cur]["start"], word)
 
     def _pull_meta(self):
@@ -349,7 +350,7 @@ class VoxelKVMerger:
         dev = self.device
         K = torch.empty((self.H, R, self.D), dtype=self.dtype, device=dev)
         V = torch.empty((self.H, R, self.D), dtype=self.dtype, device=dev)
-        M = torch.empty((self.H, R), dtype=torch.uint8, device=dev)
+        M = torch.empty((self.H, R), dtype=torch.bool, device=dev)     # the kernel writes bytes 0 and 1
         Bz = torch.empty((self.H, R), dtype=torch.float32, device=dev)
         idx = torch.empty((self.H, R, 2), dtype=torch.int32, device=dev) if want_idx else None
         if self._ret_sel is None or self._ret_sel.numel() < self.H * R:
@@ -359,7 +360,7 @@ class VoxelKVMerger:
                                       ptr(self._ret_sel), ptr(K), ptr(V), ptr(M), ptr(Bz), ptr(idx),
                                       stream_ptr())
         check(st, "stac_retrieve")
-        out = (K, V, M.bool(), Bz)
+        out = (K, V, M, Bz)
         return out + (idx,) if want_idx else out
 
     @no_grad

@@ -137,7 +137,12 @@ class BinaryVoxel:
         """Fused quantise + upsert of world points [N,3] fp32; masked-out points get id -1
         (stac/stac_voxel.py:339-347)."""
         pts = points.to(device=self.device, dtype=torch.float32).contiguous()
-        m = None if mask is None else mask.to(device=self.device, dtype=torch.uint8).contiguous()
+        m = mask
+        if m is not None:
+            if m.dtype == torch.bool:      # the same bytes: no conversion launch
+                m = m.to(device=self.device).contiguous().view(torch.uint8)
+            else:
+                m = m.to(device=self.device, dtype=torch.uint8).contiguous()
         return self._upsert(pts, None, m, pts.shape[0])
 
     # ------------------------------------------------------------------ neighbours
