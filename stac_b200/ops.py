@@ -1,5 +1,6 @@
 """Thin torch-tensor wrappers over the C ABI (one function per entry point)."""
 
+import functools
 import math
 
 import torch
@@ -68,19 +69,26 @@ _workspaces = {}
 ATTN_CTL_WORDS = 512      # leading words of an attention workspace that have to be zero
 
 
+@functools.lru_cache(maxsize=256)      # asking for a capture added 1.0 us to a call of 23 us on the host; this takes it off again
+def _attn_workspace_bytes(M, H):
+    return _lib.lib().stac_attn_workspace_bytes(M, H)
+
+
 def _attn_workspace(device, M, H):
     """Scratch of stac_attn_colsum_kept (arrival counters, row log-sum-exps, split partials), zeroed when
     it is made; every call leaves the counters zero.  One per (device, stream): calls on one stream
     are ordered and may share it, calls issued on different streams may overlap on the GPU and must
-    not.  One made during a graph capture belongs to that call alone: its zeroing is part of the graph
-    and has not happened for anyone else."""
-    need = _lib.lib().stac_attn_workspace_bytes(M, H)
+    not.  A call under graph capture takes one of its own: it comes from the graph's memory, is zeroed by
+    the graph, and is used by that graph alone.  (One kept for eager calls may be gone when the graph is
+    replayed, or in use by an eager call on the stream that the graph was captured on.)"""
+    need = _attn_workspace_bytes(M, H)
+    capturing = torch.cuda.is_current_stream_capturing()
     key = (device, stream_ptr(device=device))
-    ws = _workspaces.get(key)
+    ws = None if capturing else _workspaces.get(key)
     if ws is None or ws.numel() * 4 < need:
         ws = torch.empty(max(need // 4, 1), dtype=torch.float32, device=device)
         ws[:ATTN_CTL_WORDS].zero_()
-        if not torch.cuda.is_current_stream_capturing():
+        if not capturing:
             _workspaces[key] = ws
     return ws
 

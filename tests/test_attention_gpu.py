@@ -267,6 +267,45 @@ def test_calls_replay_from_a_cuda_graph():
         assert torch.equal(a, b) and torch.equal(a, c)
 
 
+@pytest.mark.parametrize("warm", [True, False])     # eager calls made before on the stream of the capture, or not
+@pytest.mark.parametrize("M,H,T_hot", [(700, 4, 2000), (2600, 16, 700)])   # parts joined at cuts: column sums; forward
+def test_replay_after_the_eager_workspace_was_replaced(M, H, T_hot, warm):
+    """A larger eager call on the stream of the capture replaces the workspace kept for that stream, other
+    tensors take its memory: a replay still gives the eager bits, and writes to none of them."""
+    from stac_b200 import ops
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(21)
+
+    def inputs(M, H, T):
+        return [torch.randn(*s, generator=g).to(torch.bfloat16).to(dev) for s in ((M, H, 64), (H, T, 64), (H, T, 64))]
+    q, k, v = inputs(M, H, T_hot)
+    big = inputs(2 * M, 2 * H, T_hot)
+    status = ops.DeviceStatus(dev)
+    eager = ops.attn_colsum(q, k, v, T_hot, want_lse=True, status=status)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream(device=dev)
+    with torch.cuda.stream(side):
+        if warm:
+            ops.attn_colsum(q, k, v, T_hot, want_lse=True, status=status)
+            torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            captured = ops.attn_colsum(q, k, v, T_hot, want_lse=True, status=status)
+        size = ops._attn_workspace(dev, M, H).numel()
+        ops.attn_colsum(big[0], big[1], big[2], T_hot, status=status)
+        others = [torch.full((size,), 3.0, device=dev) for _ in range(4)]
+        for _ in range(2):
+            for t in captured:
+                t.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            for a, b in zip(eager, captured):
+                assert torch.equal(a, b)
+        assert all(bool((t == 3.0).all()) for t in others)
+    status.raise_if_set("graph replay")
+    torch.cuda.synchronize()
+
+
 def test_bounded_wait_reports_and_returns():
     """A wait on a barrier nothing completes runs out, sets the status word and the kernel
     returns; the context stays usable."""

@@ -256,3 +256,24 @@ def test_no_grad_wrapper_restores_the_mode():
             except KeyError:
                 pass
             assert torch.is_grad_enabled() is before
+
+
+def test_captured_calls_have_a_workspace_of_their_own(monkeypatch):
+    """The workspace kept for eager calls of a stream is not handed to a call that is captured on it (the
+    graph would outlive it, and would run beside eager calls), nor one of a capture to an eager call."""
+    import torch
+    from stac_b200 import ops
+
+    dev = torch.device("cpu")
+    capturing = [False]
+    monkeypatch.setattr(ops, "stream_ptr", lambda device=None: 7)
+    monkeypatch.setattr(ops, "_workspaces", {})
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    eager = ops._attn_workspace(dev, 8, 2)
+    assert ops._attn_workspace(dev, 8, 2) is eager
+    capturing[0] = True
+    a, b = ops._attn_workspace(dev, 8, 2), ops._attn_workspace(dev, 8, 2)
+    assert a is not eager and b is not eager and a is not b
+    assert all(int(t[:ops.ATTN_CTL_WORDS].count_nonzero()) == 0 for t in (a, b))
+    capturing[0] = False
+    assert ops._attn_workspace(dev, 8, 2) is eager
