@@ -5,8 +5,6 @@ import ctypes
 import functools
 import os
 
-import torch
-
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libstac_b200.so")
 
@@ -168,8 +166,18 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-_raw_stream = torch._C._cuda_getCurrentRawStream
-_current_device = torch._C._cuda_getDevice
+_stream_calls = None
+
+
+def _torch_stream_calls():
+    """torch's functions for the raw handle of a stream and for the current device, looked up at the first
+    use: this module is also imported without torch, and with a torch that has no CUDA."""
+    global _stream_calls
+    import torch
+    if not hasattr(torch._C, "_cuda_getCurrentRawStream"):
+        raise StacError("this torch has no CUDA: there is no stream to launch on")
+    _stream_calls = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+    return _stream_calls
 
 
 def stream_ptr(stream=None, device=None):
@@ -179,20 +187,24 @@ def stream_ptr(stream=None, device=None):
     host time: 537 -> 440 us with the lighter calls of this file; points to voxel ids 82 -> 71 us)."""
     if stream is not None:
         return stream.cuda_stream
+    raw_stream, current_device = _stream_calls or _torch_stream_calls()
     index = device.index if device is not None else None
-    return _raw_stream(_current_device() if index is None else index)
+    return raw_stream(current_device() if index is None else index)
 
 
 def no_grad(fn):
     """torch.no_grad() around a plain function, for functions called several times per layer: nothing is
     done where gradients are off already (they call one another), and no context object is made."""
+    import torch
+    is_enabled, set_enabled = torch.is_grad_enabled, torch._C._set_grad_enabled
+
     @functools.wraps(fn)
     def wrapped(*args, **kwargs):
-        if not torch.is_grad_enabled():
+        if not is_enabled():
             return fn(*args, **kwargs)
-        torch._C._set_grad_enabled(False)
+        set_enabled(False)
         try:
             return fn(*args, **kwargs)
         finally:
-            torch._C._set_grad_enabled(True)
+            set_enabled(True)
     return wrapped

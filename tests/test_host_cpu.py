@@ -277,3 +277,25 @@ def test_captured_calls_have_a_workspace_of_their_own(monkeypatch):
     assert all(int(t[:ops.ATTN_CTL_WORDS].count_nonzero()) == 0 for t in (a, b))
     capturing[0] = False
     assert ops._attn_workspace(dev, 8, 2) is eager
+
+
+@pytest.mark.parametrize("without,code", [
+    ("import sys; sys.modules['torch'] = None", "import stac_b200._lib as l; assert l.lib().stac_abi_version() == 2"),
+    ("import torch; del torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice",
+     """
+import stac_b200._lib as l, stac_b200.ops, stac_b200.stac as s
+for use in (l.stream_ptr, lambda: s.KVManager(num_layers=1, num_heads=2, head_dim=64, token_per_frame=8, buffer_size=4,
+                                              device="cpu", dtype=torch.bfloat16)):
+    try:
+        use()
+    except l.StacError:
+        continue
+    raise SystemExit("no StacError")
+"""),
+], ids=["no torch", "torch without CUDA"])
+def test_import_needs_no_cuda_build_of_torch(without, code):
+    """The ctypes binding loads without torch; with a torch that was built without CUDA the package imports
+    and says so at the first use."""
+    import subprocess
+    res = subprocess.run([sys.executable, "-c", without + "\n" + code], cwd=ROOT, capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
