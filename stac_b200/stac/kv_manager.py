@@ -122,6 +122,7 @@ class KVManager:
         self._status = None
         self._base_cache = {}
         self._base_pos_cache = {}
+        self._graph_tables = []      # tables of the two caches above that a captured prune reads
         self._rope_rows = {}         # query length -> rows of the rotary tables (largest position + 1)
         self.stage_trace = None      # set to a list to collect (stage, start event, end event)
 
@@ -414,7 +415,15 @@ class KVManager:
             m = self._base_mask_host(T)
             hit = (torch.from_numpy(m).to(self.device), int(m.sum()))
             self._base_cache = {T: hit}
+        self._keep_for_graph(hit[0])
         return hit
+
+    def _keep_for_graph(self, table):
+        """A graph that captures a prune reads `table` whenever it is replayed, also after an eager prune of
+        another length has put its own table into the cache: it has to stay (positions that another
+        tensor has overwritten would send the gather out of the cache)."""
+        if torch.cuda.is_current_stream_capturing() and all(t is not table for t in self._graph_tables):
+            self._graph_tables.append(table)
 
     def _select(self, scores_rows, row_stride, n_rows, T, n_keep):
         base, _ = self._base_mask(T)
@@ -450,7 +459,9 @@ class KVManager:
         if T not in self._base_pos_cache:
             pos = np.flatnonzero(self._base_mask_host(T)).astype(np.int32)
             self._base_pos_cache = {T: torch.from_numpy(pos).to(self.device)}
-        return self._base_pos_cache[T]
+        table = self._base_pos_cache[T]
+        self._keep_for_graph(table)
+        return table
 
     def _compact(self, keep):
         """Gather-compaction into the idle buffers (the same positions `keep` of every row), then swap."""

@@ -299,3 +299,28 @@ def test_import_needs_no_cuda_build_of_torch(without, code):
     import subprocess
     res = subprocess.run([sys.executable, "-c", without + "\n" + code], cwd=ROOT, capture_output=True, text=True)
     assert res.returncode == 0, res.stderr
+
+
+def test_tables_of_a_captured_prune_stay(monkeypatch):
+    """The positions and the mask that a captured prune reads outlive their place in the manager's cache;
+    those of eager prunes do not."""
+    import weakref
+    import torch
+    from stac_b200.stac import KVManager
+    capturing = [False]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    kv = KVManager(num_layers=1, num_heads=2, head_dim=64, token_per_frame=8, buffer_size=6, chunk_size=1, recent_size=2,
+                   pinned_idx=[0], device=torch.device("cuda"), dtype=torch.bfloat16)
+    kv.device = torch.device("cpu")
+
+    def tables(T, captured):
+        capturing[0] = captured
+        return weakref.ref(kv._base_mask(T)[0]), weakref.ref(kv._base_positions(T))
+    eager, graph = tables(32, False), tables(40, True)
+    assert all(t() is None for t in eager)
+    again = tables(40, True)                      # a second capture finds them in the cache
+    tables(48, False)
+    assert all(a() is not None and a() is b() for a, b in zip(graph, again))
+    assert graph[1]().tolist() == list(range(8)) + list(range(24, 40))
+    assert len(kv._graph_tables) == 2
