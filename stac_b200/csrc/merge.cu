@@ -25,8 +25,8 @@
 //                        order (exp(sim) weights), publish the new pivot weights.
 //   rows_rank_kernel     one thread per row: score gate of the row's pivots, selection, ranking of
 //                        the buffered tokens + selected tokens by (score desc, arrival order),
-//                        counts of new segments / overflow / full; rows with many tokens are
-//                        left to the CTA's warps (one per row, same result).
+//                        counts of new segments / overflow / full; rows with many tokens, which
+//                        sort_tokens_kernel has listed, by a warp each (same result).
 //   scan_rows_kernel     exclusive scans of those counts inside every head; the CTA that finishes
 //                        last scans the heads and makes the allocation plan (k ids from the top of
 //                        the free list, the rest fresh) and the capacity checks.  Launched twice:
@@ -56,6 +56,7 @@ namespace {
 
 constexpr int kMaxB = 8;
 constexpr int kMaxP = 4;
+constexpr int kLongRow = 32;   // rows with more tokens are ranked by a warp each
 constexpr unsigned kFull = 0xffffffffu;
 
 // ------------------------------------------------------------------------------------ helpers
@@ -136,6 +137,7 @@ struct MergeParams {
   int* plan;           // device ints, see kPlan*
   int* free_stage;     // [buf_cap]
   int2* full_list;     // [heads*ncap] rows whose buffer filled up in this call
+  int2* long_list;     // rows with more than kLongRow tokens: the memory of full_list, which is filled later
   int2* move_list;     // [heads*ncap] rows in which buffered tokens change column
   int* tok_row;        // [heads][ncap] row index of each sorted token
   int* tok_best;       // [heads][ncap] index of the most similar pivot of the token's row
@@ -148,7 +150,7 @@ struct MergeParams {
 
 enum { kPlanK = 0, kPlanFreeLen, kPlanBufTop, kPlanPivTop, kPlanTotalAdd, kPlanTotalFull, kPlanTotalOver,
        kPlanAnyValid, kPlanAbort, kPlanFullCount, kPlanMoveCount, kPlanShort, kPlanAvailBuf, kPlanAvailPiv,
-       kPlanMergeCount, kPlanTicket, kPlanTicket2, kPlanSize = 32 };
+       kPlanMergeCount, kPlanTicket, kPlanTicket2, kPlanLongCount, kPlanSize = 32 };
 
 // Block-wide exclusive scan, 1024 threads.
 __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
@@ -366,6 +368,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
     int hf[4];
     int sum = 0;
     const unsigned int prev = (i0 > 0 && i0 - 1 < n) ? kin[i0 - 1] : 0u;
+    const unsigned int back = i0 >= kLongRow - 3 && i0 < n ? kin[i0 - (kLongRow - 3)] : ~0u;   // (no voxel has this id)
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const int i = i0 + t;
@@ -375,6 +378,14 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
       sum += hf[t];
     }
     int r = sh_carry + block_scan(sum, warp_sums, &sh_total);    // rows that begin before this thread's tokens
+    if (back == key[0]) {      // the first token's row reaches far back: the token behind kLongRow others lists it
+      for (int t = 0; t < 4; ++t) {
+        const int s0 = i0 + t - kLongRow;
+        if (s0 >= 0 && s0 + kLongRow < n && kin[s0 + kLongRow] == key[0] && kin[s0] == key[0] &&
+            (s0 == 0 || kin[s0 - 1] != key[0]))
+          p.long_list[list_push(&p.plan[kPlanLongCount])] = make_int2(h, r - 1);
+      }
+    }
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const int i = i0 + t;
@@ -763,17 +774,26 @@ __device__ __forceinline__ void rank_row_warp(const MergeParams& p, const int h,
   for (int base = s0; base < s1; base += 32) {
     const int i = base + lane;
     const bool sel = i < s1 && tdest[i] >= 0;
+    if (!__any_sync(kFull, sel)) continue;
     const float mine = sel ? tscore[i] : 0.f;
     int rank = 0;
     for (int c = 0; c < nbuf; ++c) {
       const float sc = __shfl_sync(kFull, ex_s, c);
       if (sc >= mine) ++rank;  // existing entries win ties
     }
-    if (sel) {
-      for (int i2 = s0; i2 < s1; ++i2) {
-        if (tdest[i2] >= 0) {
-          const float s2 = tscore[i2];
-          if (s2 > mine || (s2 == mine && i2 < i)) ++rank;
+    for (int base2 = s0; base2 < s1; base2 += 32) {
+      const int i2 = base2 + lane;
+      const bool sel2 = i2 < s1 && tdest[i2] >= 0;
+      if (!__any_sync(kFull, sel2)) continue;
+      const float sc = sel2 ? tscore[i2] : __int_as_float(0x7fffffff);      // NaN: not counted
+      if (base2 < base) {                    // earlier tokens win ties
+#pragma unroll
+        for (int t = 0; t < 32; ++t) rank += __shfl_sync(kFull, sc, t) >= mine ? 1 : 0;
+      } else {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) {
+          const float s2 = __shfl_sync(kFull, sc, t);
+          rank += (s2 > mine || (s2 == mine && base2 + t < i)) ? 1 : 0;
         }
       }
     }
@@ -850,28 +870,34 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
   p.row_info[hb + ri] = info;
 }
 
-// One thread per row; a row with more than 32 tokens is ranked by a warp of its CTA afterwards.
+// One thread per row; the rows with more than kLongRow tokens are listed and ranked by a warp each, which
+// may be any warp of the grid: their ranking is quadratic in their tokens, and with few, large voxels
+// there are few CTAs with rows.  The list is dealt out one row per CTA first, CTAs without rows of their
+// own in front.  (8328 tokens a head, fourth to seventh call: 16 heads on 60
+// voxels 1490 us per insert when the warps of the CTA that held a long row had to rank it, 767 us with
+// the list, 572 us with the scores passed between lanes instead of read one by one; 48 heads on 20 voxels 4966,
+// 2910 and 1938 us; 384 heads on 200 voxels 2816, 2378 and 2240 us.)
 __global__ void __launch_bounds__(256) rows_rank_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  __shared__ int long_rows[256];
-  __shared__ int n_long;
   const int h = blockIdx.y;
   const int r0 = blockIdx.x * 256;
+  const int n_long = p.plan[kPlanLongCount];
   if (p.plan[kPlanAnyValid] == 0) return;
   const int n_rows = p.n_rows[h];
-  if (r0 >= n_rows) return;
-  if (threadIdx.x == 0) n_long = 0;
-  __syncthreads();
+  if (r0 >= n_rows && n_long == 0) return;
   const int ri = r0 + threadIdx.x;
   if (ri < n_rows) {
     const int* rst = p.row_start + static_cast<long long>(h) * (p.ncap + 1);
     const int s0 = rst[ri], s1 = rst[ri + 1];
     const int vx = p.row_vx[static_cast<long long>(h) * p.ncap + ri];
-    if (s1 - s0 > 32) long_rows[list_push(&n_long)] = ri;
-    else rank_row_thread(p, h, ri, vx, s0, s1);
+    if (s1 - s0 <= kLongRow) rank_row_thread(p, h, ri, vx, s0, s1);
   }
-  __syncthreads();
-  for (int w = threadIdx.x >> 5; w < n_long; w += 8) rank_row_warp(p, h, long_rows[w], threadIdx.x & 31);
+  __syncwarp();
+  const int cta = (gridDim.x - 1 - blockIdx.x) * gridDim.y + h, n_cta = gridDim.x * gridDim.y;
+  for (int w = cta + (threadIdx.x >> 5) * n_cta; w < n_long; w += 8 * n_cta) {
+    const int2 hr = p.long_list[w];
+    rank_row_warp(p, hr.x, hr.y, threadIdx.x & 31);
+  }
 }
 
 // ------------------------------------------------------------------------------------ scans
@@ -1514,6 +1540,7 @@ int stac_merge_insert(const stac_pool* pool, const stac_evicted* ev, void* scrat
   mp.plan = reinterpret_cast<int*>(base + L.plan);
   mp.free_stage = reinterpret_cast<int*>(base + L.free_stage);
   mp.full_list = reinterpret_cast<int2*>(base + L.full_list);
+  mp.long_list = mp.full_list;
   mp.move_list = reinterpret_cast<int2*>(base + L.move_list);
   mp.tok_row = reinterpret_cast<int*>(base + L.tok_row);
   mp.tok_best = reinterpret_cast<int*>(base + L.tok_best);

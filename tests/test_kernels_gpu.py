@@ -387,6 +387,36 @@ def test_merge_at_block_and_batch_edges(pivot_cap, tokens, voxels, dtype):
     assert m.piv.used() > 0
 
 
+@pytest.mark.parametrize("lengths,heads", [
+    ([1, 31, 32, 33, 34, 63, 64, 65, 66, 97, 300], 2),      # around the rows that a warp takes, and around its batches
+    ([33] * 40, 3),                                         # more long rows than CTAs
+    ([700, 2], 5),
+])
+@pytest.mark.parametrize("levels", [0, 3])                  # scores all different, or three values: ties by arrival
+def test_merge_of_rows_with_many_tokens(lengths, heads, levels):
+    """Rows above 32 tokens are listed and ranked by a warp wherever there is one: slot maps and pool contents
+    as in the oracle after every call, every head with its rows in another order."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    rs = np.random.RandomState(len(lengths))
+    D, NV, Tn = 64, len(lengths), sum(lengths)
+    g = VoxelKVMerger(heads, D, init_voxels=NV, pivot_cap=4, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8,
+                      score_thresh=0.2, dtype=torch.float32, device=DEV, allocator="segment", seg_size=1, slab_cap=16)
+    m = VoxelMerger(heads, D, NV, 4, 8, 0.8, 0.8, 0.2, "f32")
+    dirs = rs.randn(NV, D).astype(np.float32)
+    for step in range(4):
+        VX = np.stack([rs.permutation(np.repeat(rs.permutation(NV), lengths)) for _ in range(heads)]).astype(np.int32)
+        near = rs.rand(heads, Tn, 1) < 0.5
+        noise = rs.randn(heads, Tn, D).astype(np.float32)
+        K = np.where(near, dirs[VX] + 0.2 * noise, noise).astype(np.float32)
+        V = rs.randn(heads, Tn, D).astype(np.float32)
+        S = np.exp(rs.randint(0, levels, (heads, Tn)) if levels else rs.randn(heads, Tn)).astype(np.float32)
+        m.insert_and_merge(K, V, S, VX, NV)
+        g.insert_and_merge(*(torch.from_numpy(x).to(DEV) for x in (K, V, S)), None, torch.from_numpy(VX).to(DEV), NV)
+        if m.piv.used() > 0:
+            _compare_pool(g.snapshot(), m, f"step {step}", 1e-3, 1e-5)
+    assert m.piv.used() > 0
+
+
 @pytest.mark.parametrize("bound", [None, 9000])
 def test_merge_with_more_heads_than_one_round_of_the_plan(bound):
     """1100 pool heads (the plan scans 1024 at a time), unbounded and with pools that fill up."""
