@@ -21,11 +21,14 @@ namespace {
 
 constexpr int kSelCap = 8192;     // shared-memory candidate buffer (64-bit keys)
 constexpr int kSelBins = 8192;    // counters of one radix digit (13 + 11 + 8 bits, most significant first)
-// Threads of the selection kernel and queried voxels per thread in flight.  With more heads than SMs
-// three CTAs of 512 share an SM and hide each other's loads; a launch of one CTA per SM or fewer (one
-// layer's memory, a stream whose heads are shared by several GPUs) has only its own threads for that.
+constexpr int kSelUnroll = 2;     // queried voxels per thread in flight
+// Threads of the selection kernel.  With more heads than SMs three CTAs of 512 share an SM and hide each
+// other's loads; a launch of one CTA per SM or fewer (one layer's memory, a stream whose heads are shared
+// by several GPUs) has only its own threads for that.  (Four voxels per thread in flight there made the code
+// that every call walks through longer and were slower at all sizes: 16 heads, 300 voxels, R = 64 22.9 us
+// against 21.2 us with two; 5000 voxels, R = 2048 55.8 against 53.8 us.)
 template <bool kFew> struct SelShape {
-  static constexpr int kThreads = kFew ? 1024 : 512, kUnroll = kFew ? 4 : 2, kCtas = kFew ? 1 : 3;
+  static constexpr int kThreads = kFew ? 1024 : 512, kCtas = kFew ? 1 : 3;
 };
 
 __device__ __forceinline__ unsigned int wkey(float f) {
@@ -129,22 +132,22 @@ struct RetrieveParams {
 };
 
 // Calls f(weight key, candidate index) for every pivot of the queried voxels of head h: one
-// pass over the candidates, kUnroll voxels per thread in flight.  Every thread of the CTA
+// pass over the candidates, kSelUnroll voxels per thread in flight.  Every thread of the CTA
 // must call it (no barrier inside).  A voxel's segments are requested together with its count: the
 // chain id -> (count, segments) -> weights is what a pass waits for.
-template <int kThreads, int kUnroll, typename F>
+template <int kThreads, typename F>
 __device__ __forceinline__ void for_each_candidate(const RetrieveParams& p, int h, int Q, F f) {
   const long long hrow = static_cast<long long>(h) * p.voxel_cap;
-  for (int base = 0; base < Q; base += kThreads * kUnroll) {
-    int v[kUnroll], n[kUnroll];
-    int4 seg[kUnroll];
+  for (int base = 0; base < Q; base += kThreads * kSelUnroll) {
+    int v[kSelUnroll], n[kSelUnroll];
+    int4 seg[kSelUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kSelUnroll; ++u) {
       const int q = base + u * kThreads + threadIdx.x;
       v[u] = q < Q ? p.query_ids[q] : -1;
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kSelUnroll; ++u) {
       n[u] = 0;
       seg[u] = make_int4(0, 0, 0, 0);
       if (v[u] >= 0 && v[u] < p.voxel_used) {
@@ -161,16 +164,17 @@ __device__ __forceinline__ void for_each_candidate(const RetrieveParams& p, int 
         }
       }
     }
-    float w[kUnroll][4];
+    float w[kSelUnroll][4];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kSelUnroll; ++u) {
       w[u][0] = n[u] > 0 ? p.piv_W[seg[u].x] : 0.f;
       w[u][1] = n[u] > 1 ? p.piv_W[seg[u].y] : 0.f;
       w[u][2] = n[u] > 2 ? p.piv_W[seg[u].z] : 0.f;
       w[u][3] = n[u] > 3 ? p.piv_W[seg[u].w] : 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kSelUnroll; ++u) {
+      if (base + u * kThreads >= Q) break;      // the same for the whole CTA
       const int q = base + u * kThreads + threadIdx.x;
 #pragma unroll
       for (int s = 0; s < 4; ++s)
@@ -208,13 +212,15 @@ __device__ __forceinline__ int list_push(int* counter) {
 //
 // The digit at which the collection stops leaves up to kSelCap keys of which R are wanted, and the
 // sort costs more than the passes: the select goes on over the collected keys in shared memory,
-// eight bits at a time, until at most the power of two above R are left.
+// eight bits at a time, until at most the power of two above R are left.  The sort is as wide as what
+// was collected, which may be much less than R (16 heads, one voxel queried, R = 4000: 67 us with a sort of
+// 4096 keys, 48 us).
 // (One layer's memory, 16 heads, R = 2048: insert and retrieval 338 -> 285 us with the 1024-thread shape
 // and the register sort; 384 heads, R = 2048: 1170 -> 1139 us.)
 template <bool kFew>
 __global__ void __launch_bounds__(SelShape<kFew>::kThreads, SelShape<kFew>::kCtas)
 retrieve_select_kernel(const RetrieveParams p) {
-  constexpr int kSelThreads = SelShape<kFew>::kThreads, kSelUnroll = SelShape<kFew>::kUnroll;
+  constexpr int kSelThreads = SelShape<kFew>::kThreads;
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel in the stream
   // kSelCap keys; the digit counters live in the same 64 KB (they are dead once the threshold is
   // known and the keys are collected), so three CTAs fit one SM and 384 heads run in one wave
@@ -241,7 +247,7 @@ retrieve_select_kernel(const RetrieveParams p) {
     __syncthreads();
     const unsigned int pf = prefix;
     const int sh_old = shift;
-    for_each_candidate<kSelThreads, kSelUnroll>(p, h, Q, [&](unsigned int wk, unsigned int) {
+    for_each_candidate<kSelThreads>(p, h, Q, [&](unsigned int wk, unsigned int) {
       if (sh_old == 32 || (wk >> sh_old) == pf) hist_add(hist, (wk >> new_shift) & ((1u << width) - 1u));
     });
     __syncthreads();
@@ -293,7 +299,7 @@ retrieve_select_kernel(const RetrieveParams p) {
   if (!ordered_ties) {
     const unsigned int pf = prefix;
     const int sh = shift;
-    for_each_candidate<kSelThreads, kSelUnroll>(p, h, Q, [&](unsigned int wk, unsigned int idx) {
+    for_each_candidate<kSelThreads>(p, h, Q, [&](unsigned int wk, unsigned int idx) {
       if (take_all || sh == 32 || (wk >> sh) >= pf) {
         const int pos = list_push(&sh_count);
         if (pos < kSelCap) cand[pos] = (static_cast<unsigned long long>(wk) << 32) | (0xFFFFFFFFu - idx);
@@ -303,7 +309,7 @@ retrieve_select_kernel(const RetrieveParams p) {
     // weights above the threshold in any order, then the first `need` candidates that carry the
     // threshold weight itself, in candidate order (batches of one voxel per thread, block scan)
     const unsigned int T = prefix;
-    for_each_candidate<kSelThreads, kSelUnroll>(p, h, Q, [&](unsigned int wk, unsigned int idx) {
+    for_each_candidate<kSelThreads>(p, h, Q, [&](unsigned int wk, unsigned int idx) {
       if (wk > T) {
         const int pos = list_push(&sh_count);
         cand[pos] = (static_cast<unsigned long long>(wk) << 32) | (0xFFFFFFFFu - idx);
@@ -355,11 +361,11 @@ retrieve_select_kernel(const RetrieveParams p) {
   }
   __syncthreads();
   int cnt = min(sh_count, kSelCap);
-  int np2 = kSelThreads;
-  while (np2 < R) np2 <<= 1;
-  if (cnt > np2) {
+  int limit = kSelThreads;
+  while (limit < R) limit <<= 1;
+  if (cnt > limit) {
     // the R-th largest key, eight bits at a time (keys are distinct, so this ends with R of them at
-    // the latest); R <= np2 < cnt, so there is one
+    // the latest); R <= limit < cnt, so there is one
     unsigned long long pre = 0;       // leading bits of that key found so far
     int sh = 64, want = R;            // want: its rank among the keys that share them
     for (;;) {
@@ -407,7 +413,7 @@ retrieve_select_kernel(const RetrieveParams p) {
       want -= sh_above;
       const int left = (R - want) + sh_ties;      // keys at or above the new prefix
       __syncthreads();
-      if (left <= np2 || sh == 0) break;
+      if (left <= limit || sh == 0) break;
     }
     // keep the keys at or above the prefix, in place: a batch is read before any of it is written,
     // and what is written never lies past the batches that have been read
@@ -422,13 +428,15 @@ retrieve_select_kernel(const RetrieveParams p) {
     __syncthreads();
     cnt = sh_count;
   }
+  int np2 = 1;
+  while (np2 < cnt) np2 <<= 1;
   for (int i = cnt + threadIdx.x; i < np2; i += kSelThreads) cand[i] = 0ull;
   __syncthreads();
   if (np2 == kSelThreads) sort_desc<1, kSelThreads>(cand);
   else if (np2 == 2 * kSelThreads) sort_desc<2, kSelThreads>(cand);
   else if (np2 == 4 * kSelThreads) sort_desc<4, kSelThreads>(cand);
   else if (np2 == 8 * kSelThreads) sort_desc<8, kSelThreads>(cand);
-  else bitonic_desc(cand, np2);       // 16 keys per thread would not fit three CTAs' registers
+  else if (np2 > 1) bitonic_desc(cand, np2);       // (16 keys per thread would not fit three CTAs' registers)
   const int keep = min(cnt, R);
   for (int i = threadIdx.x; i < R; i += kSelThreads) {
     int c = -1;

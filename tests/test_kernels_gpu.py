@@ -439,16 +439,7 @@ def test_merge_with_more_heads_than_one_round_of_the_plan(bound):
     assert m.piv.used() > 0 and g.info()["dropped_tokens"] == (m.dropped if bound else 0)
 
 
-@pytest.mark.parametrize("heads,voxels,pivot_cap,R,equal", [
-    (2, 600, 4, 1, False),           # R below the smallest sort
-    (2, 3000, 4, 1023, False), (2, 3000, 4, 1025, False),      # around one key per thread of the few-heads shape
-    (2, 3000, 4, 2048, False), (2, 4000, 3, 2049, False),      # exact power of two, and one more; rows of three segments
-    (2, 3000, 4, 8192, False),
-    (160, 3000, 4, 511, False), (160, 3000, 4, 513, False), (160, 2500, 4, 2048, False),   # more heads than SMs
-    (160, 3000, 4, 4097, False),     # largest sort of that shape
-    (2, 3000, 4, 1500, True), (160, 3000, 4, 1500, True),      # one weight for all: candidate order decides
-])
-def test_retrieval_order_at_the_edges_of_the_sort(heads, voxels, pivot_cap, R, equal):
+def _check_retrieval_order(heads, voxels, pivot_cap, R, equal=False, full=False):
     """Top-R by (weight descending, candidate ascending) against a stable argsort on the host, for pools
     written directly: weights in a narrow band, so that the first digits do not separate them."""
     from stac_b200.stac.merger import VoxelKVMerger
@@ -458,7 +449,7 @@ def test_retrieval_order_at_the_edges_of_the_sort(heads, voxels, pivot_cap, R, e
     g._voxel_offset = voxels
     n = heads * voxels * pivot_cap
     g._grow_piv(n)
-    cnt = rs.randint(0, pivot_cap + 1, size=(heads, voxels)).astype(np.int32)
+    cnt = rs.randint(pivot_cap if full else 0, pivot_cap + 1, size=(heads, voxels)).astype(np.int32)
     seg = rs.permutation(n).astype(np.int32).reshape(heads, voxels, pivot_cap)
     w = (np.full(n, 18.0) if equal else 18.0 + 0.5 * rs.rand(n)).astype(np.float32)
     w[rs.rand(n) < 0.2] = 18.25                         # ties
@@ -481,6 +472,29 @@ def test_retrieval_order_at_the_edges_of_the_sort(heads, voxels, pivot_cap, R, e
         assert mask[h].sum() == k and mask[h, :k].all()
         assert np.array_equal(idx[h, :k], np.stack([vox[order], slot[order]], 1))
         assert np.array_equal(K[h, :k], segs[order] % 251) and (idx[h, k:] == -1).all() and (K[h, k:] == 0).all()
+
+
+@pytest.mark.parametrize("heads,voxels,pivot_cap,R,equal", [
+    (2, 600, 4, 1, False),           # R below the smallest sort
+    (2, 3000, 4, 1023, False), (2, 3000, 4, 1025, False),      # around one key per thread of the few-heads shape
+    (2, 3000, 4, 2048, False), (2, 4000, 3, 2049, False),      # exact power of two, and one more; rows of three segments
+    (2, 3000, 4, 8192, False),
+    (160, 3000, 4, 511, False), (160, 3000, 4, 513, False), (160, 2500, 4, 2048, False),   # more heads than SMs
+    (160, 3000, 4, 4097, False),     # largest sort of that shape
+    (2, 3000, 4, 1500, True), (160, 3000, 4, 1500, True),      # one weight for all: candidate order decides
+])
+def test_retrieval_order_at_the_edges_of_the_sort(heads, voxels, pivot_cap, R, equal):
+    _check_retrieval_order(heads, voxels, pivot_cap, R, equal)
+
+
+@pytest.mark.parametrize("heads,voxels,pivot_cap,R", [
+    (2, 8, 4, 1), (160, 8, 4, 4000),                    # one voxel queried
+    (2, 24, 4, 8192), (2, 300, 4, 64), (2, 519, 1, 2048), (160, 135, 4, 300),      # fewer and more than R, below a key per thread
+    (160, 520, 2, 4000), (2, 1031, 3, 4000),            # above it
+])
+def test_retrieval_order_of_few_candidates(heads, voxels, pivot_cap, R):
+    """The sort is as wide as what was collected, from nothing to several keys per thread."""
+    _check_retrieval_order(heads, voxels, pivot_cap, R)
 
 
 def _full_size_run(steps, seed):
