@@ -497,6 +497,14 @@ def test_retrieval_order_of_few_candidates(heads, voxels, pivot_cap, R):
     _check_retrieval_order(heads, voxels, pivot_cap, R)
 
 
+@pytest.mark.parametrize("heads", [2, 160])
+@pytest.mark.parametrize("voxels,R", [(2016, 16), (2017, 16), (2017, 2048), (2048, 1), (2048, 8192), (2049, 100)])
+def test_retrieval_order_around_a_full_buffer(heads, voxels, R):
+    """8064 candidates leave room for the counters of the second select in their buffer, 8068 do not, 8192
+    fill it and 8196 need a finer digit."""
+    _check_retrieval_order(heads, voxels + 7, 4, R, full=True)
+
+
 def _full_size_run(steps, seed):
     """384 pool heads x 8328 evicted tokens per call (the pool-stress shape), bf16: tokens fall on
     1500 voxels, half of their keys cluster around a per-voxel direction so that similarity
