@@ -499,7 +499,8 @@ class VoxelKVMerger:
             idx = seg.clamp(min=0).long()
             out = pool.float().cpu()[idx]
             mask = (seg >= 0)
-            return out * mask.reshape(mask.shape + (1,) * (out.dim() - mask.dim())).float()
+            # (selected, not multiplied: an empty place may point at memory that was never written)
+            return torch.where(mask.reshape(mask.shape + (1,) * (out.dim() - mask.dim())), out, out.new_zeros(()))
 
         return {
             "buf_offset": self._buf_row_cnt[:, :V].cpu().numpy(), "buf_seg": brs.numpy(),

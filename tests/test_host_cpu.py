@@ -324,3 +324,26 @@ def test_tables_of_a_captured_prune_stay(monkeypatch):
     assert all(a() is not None and a() is b() for a, b in zip(graph, again))
     assert graph[1]().tolist() == list(range(8)) + list(range(24, 40))
     assert len(kv._graph_tables) == 2
+
+
+def test_snapshot_of_empty_places_reads_as_zero():
+    """A snapshot of the voxel memory is zero where a row has no segment, whatever the unwritten memory
+    that an empty place may point at holds."""
+    import types
+    import torch
+    from stac_b200.stac.merger import VoxelKVMerger
+    H, V, B, P, D = 2, 3, 8, 4, 64
+    nan = lambda *s: torch.full(s, float("nan"))
+    seg = lambda n: torch.where(torch.arange(n) < 1, 0, -1).to(torch.int32).expand(H, V, n).clone()
+    seg_b, seg_p = seg(B), torch.full((H, V, P), -1, dtype=torch.int32)
+    over = dict(hv=torch.zeros(1, 2, dtype=torch.int32), K=nan(1, D), V=nan(1, D), S=nan(1))
+    buf = [torch.cat([torch.ones(1, *s), nan(4, *s)]) for s in ((D,), (D,), ())]
+    fake = types.SimpleNamespace(
+        _pull_meta=lambda: None, used_voxels=lambda: V, _meta=torch.zeros(8, dtype=torch.int32), _over=[over], _over_cur=0,
+        _buf_row_seg=seg_b, _piv_row_seg=seg_p, _buf_row_cnt=torch.zeros(H, V, dtype=torch.int32),
+        _piv_row_cnt=torch.zeros(H, V, dtype=torch.int32), _buf_free=torch.zeros(0, dtype=torch.int32),
+        _buf_K=buf[0], _buf_V=buf[1], _buf_S=buf[2], _piv_K=nan(5, D), _piv_V=nan(5, D), _piv_W=nan(5), _piv_S=nan(5), _piv_C=nan(5))
+    s = VoxelKVMerger.snapshot(fake)
+    for k in ("buf_K", "buf_V", "buf_S"):
+        assert (s[k][:, :, 0] == 1).all() and (s[k][:, :, 1:] == 0).all(), k
+    assert all((s[k] == 0).all() for k in ("piv_K", "piv_V", "piv_W", "piv_S", "piv_C"))
