@@ -87,7 +87,8 @@ int stac_attn_colsum(const void* q, int64_t q_row_stride,
 /* The same call for a caller that keeps its workspace: the first 2048 bytes of `workspace` were
  * zeroed (in stream order) before its first use, and since then only calls of this entry point have
  * written to it, one after the other, with any M and H that it is large enough for.  Every call leaves
- * those bytes zero, so nothing has to be cleared in front of the kernels. */
+ * those bytes zero, so nothing has to be cleared in front of the kernels.  A call that is captured into a
+ * graph needs a workspace that only that graph uses, zeroed by it, and that lives as long as it. */
 int stac_attn_colsum_kept(const void* q, int64_t q_row_stride,
                           const void* k_hot, const void* v_hot, int64_t hot_row_stride, int64_t hot_head_stride, int T_hot,
                           const void* k_ret, const void* v_ret, int64_t ret_row_stride, int64_t ret_head_stride, int T_ret,

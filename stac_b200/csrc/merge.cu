@@ -8,10 +8,10 @@
 // (stac/allocator.py:559-723, :2237-2345, :2306-2319), and the merger-cuda pipeline that the
 // reference uses on the GPU (merger-cuda/csrc/kernels/merger_kernels.cu).
 //
-// Every output is a pure function of the inputs: per-(head, voxel) work is done by one warp
-// in token order, and everything that depends on an order across rows (which segment id a
-// row gets, where its overflow lands, where freed ids go) is computed from exclusive scans
-// over the rows in (head, voxel) order.  No floating-point atomics and no slot pops by
+// Every output is a pure function of the inputs: per-(head, voxel) work is done in token order by one
+// thread, eight lanes or a warp, and everything that depends on an order across rows (which
+// segment id a row gets, where its overflow lands, where freed ids go) is computed from
+// exclusive scans over the rows in (head, voxel) order.  No floating-point atomics and no slot pops by
 // atomics, so keys, slot maps and merged values repeat bit for bit from run to run.
 //
 // Kernels, in launch order:
@@ -45,7 +45,7 @@
 //                        call had no valid token).
 // (Eleven launches and one memset; with the long rows, the plan, the skipping and the carried list in launches
 // of their own they were sixteen and two: bounded memory of 384 heads 1381 -> 1282 us per insert and
-// retrieval, a two-layer stream 437 -> 422 us per step.)
+// retrieval.)
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -63,17 +63,12 @@ constexpr unsigned kFull = 0xffffffffu;
 template <typename T> struct Elem;
 template <> struct Elem<float> {
   static __device__ __forceinline__ float load(const float* p) { return *p; }
-  static __device__ __forceinline__ float load_cg(const float* p) { return __ldcg(p); }
   static __device__ __forceinline__ void store(float* p, float v) { *p = v; }
   static __device__ __forceinline__ float round(float v) { return v; }
   static constexpr bool kIsBf16 = false;
 };
 template <> struct Elem<__nv_bfloat16> {
   static __device__ __forceinline__ float load(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-  static __device__ __forceinline__ float load_cg(const __nv_bfloat16* p) {
-    const unsigned short u = __ldcg(reinterpret_cast<const unsigned short*>(p));
-    return __uint_as_float(static_cast<unsigned int>(u) << 16);
-  }
   static __device__ __forceinline__ void store(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
   static __device__ __forceinline__ float round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
   static constexpr bool kIsBf16 = true;

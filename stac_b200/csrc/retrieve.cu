@@ -25,7 +25,10 @@ constexpr int kSelBins = 8192;    // counters of one radix digit (13 + 11 + 8 bi
 constexpr int kSelUnroll = 2;     // queried voxels per thread in flight
 // Threads of the selection kernel.  With more heads than SMs three CTAs of 512 share an SM and hide each
 // other's loads; a launch of one CTA per SM or fewer (one layer's memory, a stream whose heads are shared
-// by several GPUs) has only its own threads for that.  (Four voxels per thread in flight there made the code
+// by several GPUs) has only its own threads for that.  (5000 voxels, R = 2048, 512 and 1024 threads: 16 heads 57 and 54 us, 148
+// heads 94 and 88 us, 149 heads 114 and 131 us, 384 heads 194 and 245 us.  With a few hundred voxels the smaller
+// shape is ahead by up to 3 us at any number of heads, but how many there are is known on the device only.
+// Four voxels per thread in flight there made the code
 // that every call walks through longer and were slower at all sizes: 16 heads, 300 voxels, R = 64 22.9 us
 // against 21.2 us with two; 5000 voxels, R = 2048 55.8 against 53.8 us.)
 template <bool kFew> struct SelShape {

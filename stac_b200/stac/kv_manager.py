@@ -454,8 +454,8 @@ class KVManager:
     def _base_positions(self, T):
         """int32 device positions of the always-kept tokens (ascending): with a plain window every
         (layer, head) row keeps these and nothing else, so there is nothing to select (24 layers of 16
-        heads, ten frames of 1041 tokens: 1934 -> 1885 us per step without the selection over zero
-        scores and the compaction of scores that do not exist)."""
+        heads, ten frames of 1041 tokens: 43 us of selection over zero scores per step are gone, and the
+        compaction without scores that do not exist takes 281 us instead of 303)."""
         if T not in self._base_pos_cache:
             pos = np.flatnonzero(self._base_mask_host(T)).astype(np.int32)
             self._base_pos_cache = {T: torch.from_numpy(pos).to(self.device)}
