@@ -16,6 +16,8 @@
 //   attn_colsum_kernel  one CTA per (128 keys, head): S^T = K Q^T into TMEM so that each thread
 //                       owns one key (TMEM lane) and sums exp2(S^T - lse[m]) over the query
 //                       columns in registers: no shuffles, no atomics, deterministic.
+#include <type_traits>
+
 #include "common.cuh"
 #include "stac_internal.h"
 
@@ -434,15 +436,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // Shared memory carries only the operands TMA brings in.  Key tiles are 112 keys wide so that
 // FOUR score buffers fit beside the output accumulator in the 512 TMEM columns (4 x 112 + 64):
 // with four softmax warpgroups each has a buffer of its own and the other three keep the
-// exponential unit busy while one waits for its buffer to go through P V and the next Q K^T
-// (with three, the fourth buffer is scored ahead, so a warpgroup finds its next tile ready;
-// measured 3.4 % slower at 4164 x 17697 keys than four).  The probabilities go back into
-// the columns their scores came from (bf16, two per column) and feed the P V MMA as its A
-// operand straight from tensor memory.  The tensor pipe has a floor of about 48 clocks per
-// MMA instruction whatever its width and idles while its issuing thread does anything else,
-// so scores use one wide instruction per K step, the two MMA streams (scores, P V) have a
-// warp each, and the instructions of a group are issued back to back with operands prepared
-// beforehand.
+// exponential unit busy while one waits for its buffer to go through P V and the next Q K^T.
+// The probabilities go back into the columns their scores came from (bf16, two per column) and feed
+// the P V MMA as its A operand straight from tensor memory.
+//
+// What bounds the kernel beside the exponentials: a tile costs 361 + 7.3 x keys cycles per SM whatever the
+// exponentials cost (96 and 112 keys, 16 384-score loops alone take the 7.3), and the 361 are the warps that
+// issue and load, which share their schedulers with the softmax warps: an instruction takes them 6 to 8
+// cycles, a wait on a barrier that is already complete 75 to 110.  So ONE warp issues both MMA streams: P V
+// of a tile and, right behind it, Q K^T of the tile that takes over its buffer (the tensor pipe keeps the
+// order of a thread's MMAs, so there is no barrier between them), with the operands of both behind one
+// barrier, one commit per tile, and a loop without bookkeeping.  (Two warps, one per stream, with rings of
+// their own: 583 against 569 thousand cycles at 4164 x 17697 keys, 93.0 against 90.0 at 1041 x 9369; the card runs
+// these loops at its power limit, 1.6 to 1.8 GHz, so 1 to 3 % of the time.  Measured and not taken: three
+// softmax warpgroups with probabilities in columns of their own, 96-key tiles, 10 % slower; two issuing warps, one
+// per accumulator for even and odd tiles, 96-key tiles, 1 to 3 % slower; larger FMA shares of the
+// exponentials, fewer cycles but no less time.)
 //
 // Work = items (head, 128-row query tile) x key tiles.  With enough items the kernel runs one
 // CTA per SM and cuts that unit sequence into equal contiguous ranges (no partly filled last
@@ -452,72 +461,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // CTA counts its arrival at the cut and the one that arrives second joins the two parts (plain
 // split-softmax algebra, operands in a fixed order: same bits whichever CTA does it).  With at
 // most half as many items as SMs every item is cut in exactly two halves instead.  Barrier
-// phases, the score ring and the K/V rings run on across segments; the query tile, the row references and the partial row sums are double
-// buffered by segment parity, and so are the barriers that several warpgroups arrive on per
-// segment: a warpgroup without a tile in a short first or last segment runs one segment ahead,
-// never two (a CTA's middle segments are whole items of at least kFastMinSplitTiles tiles, far
-// longer than the few tiles the score ring lets the warpgroups be apart).
+// phases, the stages and the score buffers run on across segments; the query tile, the row references and the
+// partial row sums are double buffered by segment parity, and so are the barriers that several warpgroups
+// arrive on per segment: a warpgroup without a tile in a short first or last segment runs one segment ahead,
+// never two (a CTA's middle segments are whole items of at least kFastMinSplitTiles tiles: the scores of a
+// warpgroup's last tile there are issued behind a P V of that segment, whose first one waits until the
+// accumulator of the segment before has been read out).
 // ---------------------------------------------------------------------------------------
-#ifndef STAC_FAST_WGS
-#define STAC_FAST_WGS 4
-#endif
-constexpr int kFastWgs = STAC_FAST_WGS;            // softmax warpgroups (3 or 4); key tile c goes to warpgroup c % kFastWgs
-static_assert(kFastWgs == 3 || kFastWgs == 4, "three or four softmax warpgroups");
-// With three warpgroups a thread double-buffers its tensor-memory loads (64 score registers) and
-// prefetches its next tile; with four the launch leaves 96 registers per thread, so loads are
-// single-buffered and the fourth warp per scheduler hides their latency instead.  The hand-over
-// rules between segments hold for both: a warpgroup's last tile of a middle segment (at least
-// kFastMinSplitTiles >= 2 * kFastWgs tiles) lies kFastRing or more tiles into it, so its score
-// buffer is a reused one and cannot be scored before the previous segment's accumulator has
-// been read out.
-constexpr bool kFastDouble = kFastWgs == 3;
-constexpr int kFastThreads = 128 + 128 * kFastWgs;   // warpgroup 0 control (warps 0, 3 TMA, warps 1-2 MMA issue), then softmax
-#ifndef STAC_FAST_STAGES
-#define STAC_FAST_STAGES 5
-#endif
-constexpr int kFastKStages = STAC_FAST_STAGES;
-constexpr int kFastVStages = STAC_FAST_STAGES;
-#ifndef STAC_FAST_KEYS
-#define STAC_FAST_KEYS 112
-#endif
-constexpr int kFT = STAC_FAST_KEYS;             // keys per tile: 112 (four score buffers); 80 (five buffers, one scored ahead) measured 2 % slower
-static_assert(kFT % 32 == 16 && kFT <= kBN, "a tile is a number of 32-key chunks and one of 16");
-static_assert(kFT == 112 || !kFastDouble, "the double-buffered path is written for 112-key tiles");
+constexpr int kFastWgs = 4;                     // softmax warpgroups; key tile c goes to warpgroup and score buffer c % kFastWgs
+constexpr int kFastThreads = 128 + 128 * kFastWgs;   // warpgroup 0 control (warp 0 TMA, warp 1 MMA issue), then softmax
+constexpr int kFT = 112;                        // keys per tile: three chunks of 32 and one of 16
+static_assert(kFT % 32 == 16 && kFT <= kBN && kFastWgs * kFT + kD <= 512, "tensor memory");
 constexpr int kFastTileBytes = kFT * 128;       // kFT rows x 64 bf16
-constexpr int kFastRing = (512 - kD) / kFT;     // score buffers beside the 64 accumulator columns
 constexpr float kFastRowSumLimit = 1.152921504606846976e18f;  // 2^60
 constexpr int kPartFloats = kBM * kD + 2 * kBM; // one partial result: O[128][64], row sums, row references
 constexpr int kFastMaxCtas = 160;               // partial-result slots are provided for this many CTAs
-// shorter key ranges run one CTA per item; every warpgroup has a tile at least kFastRing tiles into a
+// shorter key ranges run one CTA per item; every warpgroup has a tile at least kFastWgs tiles into a
 // middle segment, i.e. one whose score buffer was last used inside the same segment
-constexpr int kFastMinSplitTiles = kFastRing + kFastWgs;
-static_assert(kFastMinSplitTiles >= 2 * kFastWgs, "segment hand-over rule");
+constexpr int kFastMinSplitTiles = 2 * kFastWgs;
 #ifndef STAC_FAST_PAIR_MASK
 #define STAC_FAST_PAIR_MASK 0x8080u
 #endif
 constexpr unsigned kFastPairMask = STAC_FAST_PAIR_MASK;   // which of 16 consecutive PAIRS of exponentials run on the FMA pipes
 // setmaxnreg targets; must fit the launch allocation
-constexpr int kFastCtlRegs = kFastWgs == 3 ? 56 : 40, kFastSoftmaxRegs = kFastWgs == 3 ? 152 : 104;
+constexpr int kFastCtlRegs = 64, kFastSoftmaxRegs = 104;
 static_assert(128 * kFastCtlRegs + 128 * kFastWgs * kFastSoftmaxRegs <= kFastThreads * ((65536 / kFastThreads) / 8 * 8),
               "fast forward kernel: setmaxnreg targets exceed the CTA's register allocation");
 
 struct FastSmem {
   uint8_t q[2][kTileBytes];                     // query tile of the segment (parity)
-  uint8_t k[kFastKStages][kFastTileBytes];
-  uint8_t v[kFastVStages][kFastTileBytes];
+  uint8_t k[kFastWgs][kFastTileBytes];          // stage of tile c: the keys of tile c ...
+  uint8_t v[kFastWgs][kFastTileBytes];          // ... and the values of tile c - kFastWgs
   float bias2[kFastWgs][kBN];
   float m_ref[2][kBM];                          // row references of the segment (parity)
   float lpart[2][kFastWgs - 1][kBM];            // row sums of warpgroups 1.. (segment parity)
   int live[2][kFastWgs - 1];                    // did warpgroup 1.. see a key that is not masked (segment parity)
   uint64_t q_full[2];
   uint64_t q_empty[2];
-  uint64_t k_full[kFastKStages];
-  uint64_t k_empty[kFastKStages];
-  uint64_t v_full[kFastVStages];
-  uint64_t v_empty[kFastVStages];
-  uint64_t s_full[kFastRing];    // scores of a tile are in TMEM
-  uint64_t p_full[kFastRing];    // its probabilities are in TMEM
-  uint64_t buf_free[kFastRing];  // the P V MMAs that read them are done
+  uint64_t kv_full[kFastWgs];
+  uint64_t s_full[kFastWgs];     // scores of a tile are in TMEM; the stage that its keys came from is free again
+  uint64_t p_full[kFastWgs];     // its probabilities are in TMEM
   uint64_t ref_ready[2];
   uint64_t l_ready[2];           // warpgroups 1.. have published their row sums of the segment (parity)
   uint64_t o_done;               // all P V MMAs of the segment are complete
@@ -531,26 +514,29 @@ struct FastSmem {
 // contiguous ranges, one per CTA (an item on a cut is then finished by two CTAs); without it
 // CTA i owns item i.  Every role of the CTA walks the same sequence.
 struct FwdWalk {
-  long long u, u_end;
-  int nt;
+  int item, t0, left, nt;     // next item, its first tile, tiles of the CTA that are left, tiles per item
   __device__ FwdWalk(const FwdParams& p, int n_tiles) {
     nt = n_tiles;
     if (p.split) {
       const long long total = static_cast<long long>(p.n_items) * nt;
-      u = total * blockIdx.x / gridDim.x;
-      u_end = total * (blockIdx.x + 1) / gridDim.x;
+      const long long u = total * blockIdx.x / gridDim.x;
+      left = static_cast<int>(total * (blockIdx.x + 1) / gridDim.x - u);
+      item = static_cast<int>(u / nt);
+      t0 = static_cast<int>(u - static_cast<long long>(item) * nt);
     } else {
-      u = static_cast<long long>(blockIdx.x) * nt;
-      u_end = u + nt;
+      left = nt;
+      item = blockIdx.x;
+      t0 = 0;
     }
   }
-  __device__ bool next(int& item, int& t0, int& t1) {
-    if (u >= u_end) return false;
-    item = static_cast<int>(u / nt);
-    t0 = static_cast<int>(u - static_cast<long long>(item) * nt);
-    const long long e = static_cast<long long>(item + 1) * nt;
-    t1 = static_cast<int>((e < u_end ? e : u_end) - static_cast<long long>(item) * nt);
-    u = static_cast<long long>(item) * nt + t1;
+  __device__ bool next(int& item_, int& t0_, int& t1_) {
+    if (left <= 0) return false;
+    item_ = item;
+    t0_ = t0;
+    t1_ = min(nt, t0 + left);
+    left -= t1_ - t0_;
+    ++item;
+    t0 = 0;
     return true;
   }
 };
@@ -624,20 +610,12 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       mbar_init(&sm.ref_ready[i], 128);
       mbar_init(&sm.l_ready[i], 128 * (kFastWgs - 1));
     }
-    for (int s = 0; s < kFastKStages; ++s) {
-      mbar_init(&sm.k_full[s], 1);
-      mbar_init(&sm.k_empty[s], 1);
-    }
-    for (int s = 0; s < kFastVStages; ++s) {
-      mbar_init(&sm.v_full[s], 1);
-      mbar_init(&sm.v_empty[s], 1);
-    }
-    for (int b = 0; b < kFastRing; ++b) {
+    mbar_init(&sm.o_done, 1);
+    for (int b = 0; b < kFastWgs; ++b) {
+      mbar_init(&sm.kv_full[b], 1);
       mbar_init(&sm.s_full[b], 1);
       mbar_init(&sm.p_full[b], 128);
-      mbar_init(&sm.buf_free[b], 1);
     }
-    mbar_init(&sm.o_done, 1);
     mbar_init(&sm.o_free, 128);
     mbar_fence_init();
   }
@@ -649,7 +627,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-  const uint32_t o_tmem = tmem + kFastRing * kFT;   // 64 columns behind the score buffers
+  const uint32_t o_tmem = tmem + kFastWgs * kFT;   // 64 columns behind the score buffers
   // Launched with programmatic serialization behind whatever wrote the queries and the cache: barriers
   // and tensor memory are set up while that drains, nothing in global memory is touched before this.
   grid_dep_wait();
@@ -670,13 +648,27 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (warp < 4) {
     setmaxnreg_dec<kFastCtlRegs>();
     if (warp == 0 && lane == 0) {
-      // ---------------------------------------------------------------- TMA producer: Q and K
+      // ---------------------------------------------------------------- TMA producer
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k_hot);
-      FwdWalk walk(p, n_tiles);
-      int seg = 0, item, t0, t1;
-      int ks = 0, kr = 0;   // stage and round of the K ring
-      for (; walk.next(item, t0, t1); ++seg) {
+      tma_prefetch_desc(&tm_v_hot);
+      FwdWalk walk(p, n_tiles), walk_v(p, n_tiles);
+      int item, t0, t1, item_v, j_v = 0, t1_v = 0, h_v = 0;
+      int c = 0, b = 0, par = 1;         // stage b = c % kFastWgs; par: phase of the stage's previous use
+      auto load_v = [&]() {
+        if (j_v == t1_v) {
+          walk_v.next(item_v, j_v, t1_v);
+          h_v = item_v / p.n_q_tiles;
+        }
+        const bool hot = j_v < n_hot;
+        tma_load_3d(sm.v[b], hot ? &tm_v_hot : &tm_v_ret, &sm.kv_full[b], 0, (hot ? j_v : j_v - n_hot) * kFT, h_v);
+        ++j_v;
+      };
+      auto next_stage = [&]() {
+        ++c;
+        if (++b == kFastWgs) { b = 0; par ^= 1; }
+      };
+      for (int seg = 0; walk.next(item, t0, t1); ++seg) {
         const int h = item / p.n_q_tiles, m_tile = item - h * p.n_q_tiles;
         const int qb = seg & 1;
         if (seg >= 2) mbar_wait(&sm.q_empty[qb], ((seg >> 1) - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
@@ -684,99 +676,123 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tma_load_3d(sm.q[qb], &tm_q, &sm.q_full[qb], 0, h, m_tile * kBM);
         for (int j = t0; j < t1; ++j) {
           const bool hot = j < n_hot;
-          const int n0 = (hot ? j : j - n_hot) * kFT;
-          if (kr > 0) mbar_wait(&sm.k_empty[ks], (kr - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-          mbar_arrive_expect_tx(&sm.k_full[ks], kFastTileBytes);
-          tma_load_3d(sm.k[ks], hot ? &tm_k_hot : &tm_k_ret, &sm.k_full[ks], 0, n0, h);
-          if (++ks == kFastKStages) { ks = 0; ++kr; }
+          const bool with_v = c >= kFastWgs;
+          if (with_v) mbar_wait(&sm.s_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
+          mbar_arrive_expect_tx(&sm.kv_full[b], with_v ? 2 * kFastTileBytes : kFastTileBytes);
+          tma_load_3d(sm.k[b], hot ? &tm_k_hot : &tm_k_ret, &sm.kv_full[b], 0, (hot ? j : j - n_hot) * kFT, h);
+          if (with_v) load_v();
+          next_stage();
         }
       }
-    } else if (warp == 3 && lane == 0) {
-      // ---------------------------------------------------------------- TMA producer: V
-      // (its own thread: V tiles are released several tiles later than K tiles, and one
-      // thread serving both rings in order would hold K back whenever the V ring is full)
-      tma_prefetch_desc(&tm_v_hot);
-      FwdWalk walk(p, n_tiles);
-      int item, t0, t1;
-      int vs = 0, vr = 0;
-      while (walk.next(item, t0, t1)) {
-        const int h = item / p.n_q_tiles;
-        for (int j = t0; j < t1; ++j) {
-          const bool hot = j < n_hot;
-          const int n0 = (hot ? j : j - n_hot) * kFT;
-          if (vr > 0) mbar_wait(&sm.v_empty[vs], (vr - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-          mbar_arrive_expect_tx(&sm.v_full[vs], kFastTileBytes);
-          tma_load_3d(sm.v[vs], hot ? &tm_v_hot : &tm_v_ret, &sm.v_full[vs], 0, n0, h);
-          if (++vs == kFastVStages) { vs = 0; ++vr; }
+      // the values of the last tiles (a CTA with fewer than kFastWgs tiles leaves the stages in between out)
+      for (int e = 0; e < kFastWgs; ++e) {
+        if (c >= kFastWgs) {
+          mbar_wait(&sm.s_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
+          mbar_arrive_expect_tx(&sm.kv_full[b], kFastTileBytes);
+          load_v();
         }
+        next_stage();
       }
     } else if (warp == 1) {
-      // ---------------------------------------------------------------- MMA issuer: S = Q K^T
+      // ---------------------------------------------------------------- MMA issuer
+      // Step u: O += P V of tile u - kFastWgs, whose probabilities lie where tile u's scores go, and right
+      // behind it S = Q K^T of tile u.  The tensor pipe works through the MMAs of a thread in order, so
+      // nothing has to be waited for in between, one barrier per stage covers the operands of both, and one
+      // commit tells the warpgroup that its scores are there and the producer that the stage is free.
+      // This warp shares its scheduler with softmax warps and gets 6 to 8 cycles per instruction: the
+      // steps inside a segment run in a loop of their own without any bookkeeping.
       // (all lanes run the loop, one elected lane issues)
       constexpr uint32_t idesc_s = umma_idesc_bf16(kBM, kFT, 0);
+      constexpr uint32_t idesc_o = umma_idesc_bf16(kBM, kD, 1);
       const uint64_t q_desc0 = smem_desc_sw128(smem_u32(sm.q[0]));
       const uint64_t k_desc0 = smem_desc_sw128(smem_u32(sm.k[0]));
-      FwdWalk walk(p, n_tiles);
-      int seg = 0, item, t0, t1;
-      int b = 0, round = 0, ks = 0, kr = 0;
-      for (; walk.next(item, t0, t1); ++seg) {
-        const int qb = seg & 1;
-        const uint64_t q_desc = q_desc0 + static_cast<uint64_t>(qb * (kTileBytes >> 4));
-        mbar_wait(&sm.q_full[qb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_TMA);
-#pragma unroll 1
-        for (int j = t0; j < t1; ++j) {
-          const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(ks * (kFastTileBytes >> 4));
-          const uint32_t d = tmem + b * kFT;
-          mbar_wait(&sm.k_full[ks], kr & 1, p.err, DEV_TIMEOUT_TMA);
-          if (round > 0) mbar_wait(&sm.buf_free[b], (round - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-          tc_fence_after();
-          if (elect_one()) {
-            umma_ss(d, q_desc, k_desc, idesc_s, 0u);
-            umma_ss(d, q_desc + 2, k_desc + 2, idesc_s, 1u);
-            umma_ss(d, q_desc + 4, k_desc + 4, idesc_s, 1u);
-            umma_ss(d, q_desc + 6, k_desc + 6, idesc_s, 1u);
-            umma_commit(&sm.s_full[b]);
-            umma_commit(&sm.k_empty[ks]);
-            if (j == t1 - 1) umma_commit(&sm.q_empty[qb]);
-          }
-          __syncwarp();
-          if (++ks == kFastKStages) { ks = 0; ++kr; }
-          if (++b == kFastRing) { b = 0; ++round; }
-        }
-      }
-    } else if (warp == 2) {
-      // ---------------------------------------------------------------- MMA issuer: O += P V
-      constexpr uint32_t idesc_o = umma_idesc_bf16(kBM, kD, 1);
       const uint64_t v_desc0 = smem_desc_sw128(smem_u32(sm.v[0]));
-      FwdWalk walk(p, n_tiles);
-      int seg = 0, item, t0, t1;
-      int b = 0, round = 0, vs = 0, vr = 0;
-      for (; walk.next(item, t0, t1); ++seg) {
-#pragma unroll 1
-        for (int j = t0; j < t1; ++j) {
-          // A: 16 keys = 8 columns of packed probabilities; B: V advances 16 rows = 2048 bytes
-          const uint32_t pa = tmem + b * kFT;
-          const uint64_t vb = v_desc0 + static_cast<uint64_t>(vs * (kFastTileBytes >> 4));
-          const uint32_t acc0 = j > t0 ? 1u : 0u;
-          mbar_wait(&sm.v_full[vs], vr & 1, p.err, DEV_TIMEOUT_TMA);
-          mbar_wait(&sm.p_full[b], round & 1, p.err, DEV_TIMEOUT_CONSUMER);
-          // a new segment overwrites the accumulator: the previous one must have been read out
-          if (j == t0 && seg > 0) mbar_wait(&sm.o_free, (seg - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
+      uint64_t q_desc = q_desc0;
+      uint32_t b = 0, par = 1;     // stage and buffer of step u, phase of their previous use
+      auto issue_pv = [&](uint32_t sc, uint64_t vd, uint32_t acc) {
+        // A: 16 keys = 8 columns of packed probabilities; B: V advances 16 rows = 2048 bytes
+        umma_ts(o_tmem, sc, vd, idesc_o, acc);
+#pragma unroll
+        for (int kk = 1; kk < kFT / 16; ++kk)
+          umma_ts(o_tmem, sc + kk * 8, vd + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_o, 1u);
+      };
+      auto issue_s = [&](uint32_t sc, uint64_t kd) {
+        umma_ss(sc, q_desc, kd, idesc_s, 0u);
+        umma_ss(sc, q_desc + 2, kd + 2, idesc_s, 1u);
+        umma_ss(sc, q_desc + 4, kd + 4, idesc_s, 1u);
+        umma_ss(sc, q_desc + 6, kd + 6, idesc_s, 1u);
+      };
+      auto next_step = [&]() {
+        if (++b == kFastWgs) { b = 0; par ^= 1; }
+      };
+      // steps at the edges of segments; the P V cursor walks the segments behind the scores
+      FwdWalk walk_v(p, n_tiles);
+      int v_seg = -1, v_left = 0, v_item, v_t0, v_t1, u = 0;
+      auto edge_step = [&](bool with_s) {
+        const uint32_t sc = tmem + b * kFT;
+        const uint64_t off = static_cast<uint64_t>(b * (kFastTileBytes >> 4));
+        const bool with_v = u >= kFastWgs;
+        bool first_o = false;
+        if (with_v && v_left == 0) {
+          walk_v.next(v_item, v_t0, v_t1);
+          v_left = v_t1 - v_t0;
+          ++v_seg;
+          first_o = true;
+        }
+        if (with_s || with_v) {
+          mbar_wait(&sm.kv_full[b], par ^ 1, p.err, DEV_TIMEOUT_TMA);
+          if (with_v) {
+            mbar_wait(&sm.p_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
+            // a new segment overwrites the accumulator: the previous one must have been read out
+            if (first_o && v_seg > 0) mbar_wait(&sm.o_free, (v_seg - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
+            --v_left;
+          }
           tc_fence_after();
           if (elect_one()) {
-            umma_ts(o_tmem, pa, vb, idesc_o, acc0);
-#pragma unroll
-            for (int kk = 1; kk < kFT / 16; ++kk)
-              umma_ts(o_tmem, pa + kk * 8, vb + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_o, 1u);
-            umma_commit(&sm.buf_free[b]);
-            umma_commit(&sm.v_empty[vs]);
-            if (j == t1 - 1) umma_commit(&sm.o_done);
+            if (with_v) {
+              issue_pv(sc, v_desc0 + off, first_o ? 0u : 1u);
+              if (v_left == 0) umma_commit(&sm.o_done);
+            }
+            if (with_s) issue_s(sc, k_desc0 + off);
+            umma_commit(&sm.s_full[b]);
           }
           __syncwarp();
-          if (++vs == kFastVStages) { vs = 0; ++vr; }
-          if (++b == kFastRing) { b = 0; ++round; }
         }
+        ++u;
+        next_step();
+      };
+      FwdWalk walk(p, n_tiles);
+      int item, t0, t1;
+      for (int seg = 0; walk.next(item, t0, t1); ++seg) {
+        const int n = t1 - t0, qb = seg & 1;
+        mbar_wait(&sm.q_full[qb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_TMA);
+        q_desc = q_desc0 + static_cast<uint64_t>(qb * (kTileBytes >> 4));
+        // scores beside the last P V of the previous segment, then the first P V of this one
+        for (int e = 0; e < min(n, kFastWgs + 1); ++e) edge_step(true);
+        const int more = n - (kFastWgs + 1);
+        if (more > 0) {
+          u += more;
+          v_left -= more;
+#pragma unroll 1
+          for (int e = 0; e < more; ++e) {
+            const uint32_t sc = tmem + b * kFT;
+            const uint64_t off = static_cast<uint64_t>(b * (kFastTileBytes >> 4));
+            mbar_wait(&sm.kv_full[b], par ^ 1, p.err, DEV_TIMEOUT_TMA);
+            mbar_wait(&sm.p_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
+            tc_fence_after();
+            if (elect_one()) {
+              issue_pv(sc, v_desc0 + off, 1u);
+              issue_s(sc, k_desc0 + off);
+              umma_commit(&sm.s_full[b]);
+            }
+            __syncwarp();
+            next_step();
+          }
+        }
+        if (elect_one()) umma_commit(&sm.q_empty[qb]);
+        __syncwarp();
       }
+      for (int e = 0; e < kFastWgs; ++e) edge_step(false);
     }
   } else {
     // ------------------------------------------------------------------ softmax warpgroups
@@ -788,11 +804,13 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const float c2 = p.scale_log2;
     const uint64_t c2c2 = pack_f32x2(c2, c2);
     const float* bias2 = sm.bias2[g];
-    uint32_t ra[32], rb[32], pk[16];   // rb: second score buffer (three warpgroups) and the read-out of O
+    uint32_t ra[32], rb[32], pk[16];   // rb: the read-out of O
+    const uint32_t s_addr = tmem + lane_base + g * kFT;
     bool overflow = false;
     FwdWalk walk(p, n_tiles);
     int seg = 0, item, t0, t1;
-    int c_base = 0;   // key tiles of earlier segments: tile c of the CTA uses ring buffer c % kFastRing, warpgroup c % kFastWgs
+    int c_base = 0;   // key tiles of earlier segments
+    int round = 0;    // tiles that this warpgroup has behind it
     for (; walk.next(item, t0, t1); ++seg) {
       const int h = item / p.n_q_tiles, m_tile = item - h * p.n_q_tiles;
       const int len = t1 - t0;
@@ -802,136 +820,95 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       uint64_t negm2 = 0ull;            // (-m_ref, -m_ref)
       bool have_ref = false;
       bool any_live = false;  // some key tile of this warpgroup in this segment had a key that is not masked
-      bool fetching = false;  // the first 32 scores of the next tile are already on their way into ra
-      for (int x = (g + kFastWgs - c_base % kFastWgs) % kFastWgs; x < len; x += kFastWgs) {
-        const int c = c_base + x;
-        const int b = c % kFastRing, round = c / kFastRing;
+      int x = (g - c_base) & (kFastWgs - 1);
+      // The reference of the segment, at the first tile of this warpgroup; the first 32 scores are in ra behind it.
+      auto reference = [&](bool need_bias) {
+        have_ref = true;
+        if (x == 0) {
+          // exact row maximum of the segment's first tile = the row's reference for the segment
+          float mx = -INFINITY;
+#pragma unroll
+          for (int ch = 0; ch < kFT / 32; ++ch) {
+            tmem_ld_wait();
+            mx = fast_max_chunk<32>(ra, bias2 + 32 * ch, need_bias, c2, mx);
+            if (ch + 1 < kFT / 32) tmem_ld32(s_addr + 32 * (ch + 1), ra);
+            else tmem_ld16(s_addr + 32 * (ch + 1), ra);
+          }
+          tmem_ld_wait();
+          mx = fast_max_chunk<16>(ra, bias2 + kFT - 16, need_bias, c2, mx);
+          tmem_ld32(s_addr, ra);
+          m_ref = (mx == -INFINITY) ? 0.f : mx;
+          sm.m_ref[sb][row] = m_ref;
+          mbar_arrive(&sm.ref_ready[sb]);
+        } else {
+          mbar_wait(&sm.ref_ready[sb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
+          m_ref = sm.m_ref[sb][row];
+        }
+        negm2 = pack_f32x2(-m_ref, -m_ref);
+      };
+      // Scores -> probabilities in place, chunk by chunk: load, wait, convert, store.
+      auto convert = [&](auto bias_tag) {
+        constexpr bool kBias = decltype(bias_tag)::value;
+#pragma unroll
+        for (int ch = 0; ch < kFT / 32; ++ch) {
+          tmem_ld_wait();
+          fast_exp_chunk<kBias, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1);
+          if (ch + 1 < kFT / 32) tmem_ld32(s_addr + 32 * (ch + 1), ra);
+          else tmem_ld16(s_addr + 32 * (ch + 1), ra);
+          tmem_st16(s_addr + 16 * ch, pk);
+        }
+        tmem_ld_wait();
+        fast_exp_chunk<kBias, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1);
+        tmem_st8(s_addr + (kFT - 16) / 2, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&sm.p_full[g]);
+      };
+      // whole tiles of the hot cache: no bias, nothing masked
+      const int n_plain = min(len, p.T_hot / kFT - t0);
+      any_live = x < n_plain;
+#pragma unroll 1
+      for (; x < n_plain; x += kFastWgs, ++round) {
+        mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
+        tc_fence_after();
+        tmem_ld32(s_addr, ra);
+        if (!have_ref) reference(false);
+        convert(std::false_type{});
+      }
+      // the ragged last tile of the hot cache, the retrieved pivots
+#pragma unroll 1
+      for (; x < len; x += kFastWgs, ++round) {
         const int j = t0 + x;
         const bool is_ret = j >= n_hot;
         const int n0 = (is_ret ? j - n_hot : j) * kFT;
         const int valid = min(kFT, (is_ret ? p.T_ret : p.T_hot) - n0);
-        const bool need_bias = is_ret || valid < kFT;
-        bool tile_live = true;   // false: every key of the tile is masked (padding behind the valid pivots)
-        if (need_bias) {
-          named_bar_sync(1 + g, 128);
-          bool live = false;
-          if (row < kFT) {
-            float bv = -INFINITY;
-            if (row < valid) bv = is_ret ? p.bias_ret[h * p.bias_head_stride + n0 + row] * kLog2e : 0.f;
-            sm.bias2[g][row] = bv;
-            live = bv != -INFINITY;
-          }
-          tile_live = named_bar_or(1 + g, 128, live);
+        named_bar_sync(1 + g, 128);
+        bool live = false;
+        if (row < kFT) {
+          float bv = -INFINITY;
+          if (row < valid) bv = is_ret ? p.bias_ret[h * p.bias_head_stride + n0 + row] * kLog2e : 0.f;
+          sm.bias2[g][row] = bv;
+          live = bv != -INFINITY;
         }
+        const bool tile_live = named_bar_or(1 + g, 128, live);   // false: every key of the tile is masked (padding behind the valid pivots)
         any_live = any_live || tile_live;
-        const uint32_t s_addr = tmem + lane_base + b * kFT;
-        if (!fetching) {
-          mbar_wait(&sm.s_full[b], round & 1, p.err, DEV_TIMEOUT_MMA);
-          tc_fence_after();
-          if (tile_live || !have_ref) tmem_ld32(s_addr, ra);
-        }
+        mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
+        tc_fence_after();
         if (!tile_live && have_ref) {
           // nothing to exponentiate: all probabilities of this tile are zero
-          if (fetching) tmem_ld_wait();      // the prefetched scores are not needed
 #pragma unroll
           for (int i = 0; i < 16; ++i) pk[i] = 0u;
 #pragma unroll
           for (int ch = 0; ch < kFT / 32; ++ch) tmem_st16(s_addr + 16 * ch, pk);
           tmem_st8(s_addr + (kFT - 16) / 2, pk);
-          const int b2n = (c + kFastWgs) % kFastRing, round2n = (c + kFastWgs) / kFastRing;
-          fetching = false;
-          if (kFastDouble && x + kFastWgs < len &&
-              __all_sync(0xffffffffu, mbar_test(&sm.s_full[b2n], round2n & 1))) {
-            tc_fence_after();
-            tmem_ld32(tmem + lane_base + b2n * kFT, ra);
-            fetching = true;
-          }
           tmem_st_wait();
           tc_fence_before();
-          mbar_arrive(&sm.p_full[b]);
+          mbar_arrive(&sm.p_full[g]);
           continue;
         }
-        if (!have_ref) {
-          have_ref = true;
-          if (x == 0) {
-            // exact row maximum of the segment's first tile = the row's reference for the segment
-            float mx = -INFINITY;
-#pragma unroll
-            for (int ch = 0; ch < kFT / 32; ++ch) {
-              tmem_ld_wait();
-              mx = fast_max_chunk<32>(ra, bias2 + 32 * ch, need_bias, c2, mx);
-              if (ch + 1 < kFT / 32) tmem_ld32(s_addr + 32 * (ch + 1), ra);
-              else tmem_ld16(s_addr + 32 * (ch + 1), ra);
-            }
-            tmem_ld_wait();
-            mx = fast_max_chunk<16>(ra, bias2 + kFT - 16, need_bias, c2, mx);
-            m_ref = (mx == -INFINITY) ? 0.f : mx;
-            sm.m_ref[sb][row] = m_ref;
-            mbar_arrive(&sm.ref_ready[sb]);
-            tmem_ld32(s_addr, ra);
-          } else {
-            mbar_wait(&sm.ref_ready[sb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-            m_ref = sm.m_ref[sb][row];
-          }
-          negm2 = pack_f32x2(-m_ref, -m_ref);
-        }
-        // keys 0..31 are on their way into ra
-        if constexpr (kFastDouble) {
-          tmem_ld_wait();
-          tmem_ld32(s_addr + 32, rb);
-          if (need_bias) fast_exp_chunk<true, 32>(ra, pk, bias2, c2c2, negm2, l0, l1);
-          else fast_exp_chunk<false, 32>(ra, pk, bias2, c2c2, negm2, l0, l1);
-          tmem_st16(s_addr, pk);
-          tmem_ld_wait();
-          tmem_ld32(s_addr + 64, ra);
-          if (need_bias) fast_exp_chunk<true, 32>(rb, pk, bias2 + 32, c2c2, negm2, l0, l1);
-          else fast_exp_chunk<false, 32>(rb, pk, bias2 + 32, c2c2, negm2, l0, l1);
-          tmem_st16(s_addr + 16, pk);
-          tmem_ld_wait();
-          tmem_ld16(s_addr + 96, rb);
-          if (need_bias) fast_exp_chunk<true, 32>(ra, pk, bias2 + 64, c2c2, negm2, l0, l1);
-          else fast_exp_chunk<false, 32>(ra, pk, bias2 + 64, c2c2, negm2, l0, l1);
-          tmem_st16(s_addr + 32, pk);
-          tmem_ld_wait();
-          // this warpgroup's next tile of the segment is normally scored by now: start fetching it
-          // (never wait for it here: its buffer is released by another warpgroup's P V, which may
-          // be behind this one)
-          const int b2 = (c + kFastWgs) % kFastRing, round2 = (c + kFastWgs) / kFastRing;
-          const bool more = x + kFastWgs < len;
-          fetching = false;
-          if (more && __all_sync(0xffffffffu, mbar_test(&sm.s_full[b2], round2 & 1))) {
-            tc_fence_after();
-            tmem_ld32(tmem + lane_base + b2 * kFT, ra);
-            fetching = true;
-          }
-          if (need_bias) fast_exp_chunk<true, 16>(rb, pk, bias2 + 96, c2c2, negm2, l0, l1);
-          else fast_exp_chunk<false, 16>(rb, pk, bias2 + 96, c2c2, negm2, l0, l1);
-          tmem_st8(s_addr + 48, pk);
-          if (more && !fetching && __all_sync(0xffffffffu, mbar_test(&sm.s_full[b2], round2 & 1))) {
-            tc_fence_after();                  // second chance, a chunk later
-            tmem_ld32(tmem + lane_base + b2 * kFT, ra);
-            fetching = true;
-          }
-        } else {
-          // one score buffer per thread: load, wait, convert, store, chunk by chunk
-#pragma unroll
-          for (int ch = 0; ch < kFT / 32; ++ch) {
-            tmem_ld_wait();
-            if (need_bias) fast_exp_chunk<true, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1);
-            else fast_exp_chunk<false, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1);
-            if (ch + 1 < kFT / 32) tmem_ld32(s_addr + 32 * (ch + 1), ra);
-            else tmem_ld16(s_addr + 32 * (ch + 1), ra);
-            tmem_st16(s_addr + 16 * ch, pk);
-          }
-          tmem_ld_wait();
-          if (need_bias) fast_exp_chunk<true, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1);
-          else fast_exp_chunk<false, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1);
-          tmem_st8(s_addr + (kFT - 16) / 2, pk);
-          fetching = false;
-        }
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(&sm.p_full[b]);
+        tmem_ld32(s_addr, ra);
+        if (!have_ref) reference(true);
+        convert(std::true_type{});
       }
       // ---- end of the segment
       float la, lb, lc, ld;
@@ -949,14 +926,12 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           m_ref = sm.m_ref[sb][row];
         }
         mbar_wait(&sm.l_ready[sb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-        float l = (lsum + sm.lpart[sb][0][row]) + sm.lpart[sb][1][row];
-        if constexpr (kFastWgs == 4) l += sm.lpart[sb][2][row];
+        const float l = ((lsum + sm.lpart[sb][0][row]) + sm.lpart[sb][1][row]) + sm.lpart[sb][2][row];
         // A segment whose keys are all masked has no reference (m_ref is a placeholder): it must not
         // take part in a join.  A segment with live keys whose probabilities all underflowed (its
         // first tile was masked, so the placeholder was used, and the live scores lie far below
         // it) cannot be represented: the exact kernel redoes the call.
-        bool seg_live = any_live || sm.live[sb][0] != 0 || sm.live[sb][1] != 0;
-        if constexpr (kFastWgs == 4) seg_live = seg_live || sm.live[sb][2] != 0;
+        const bool seg_live = any_live || sm.live[sb][0] != 0 || sm.live[sb][1] != 0 || sm.live[sb][2] != 0;
         if (seg_live && !(l > 0.f)) overflow = true;
         mbar_wait(&sm.o_done, seg & 1, p.err, DEV_TIMEOUT_MMA);
         tc_fence_after();

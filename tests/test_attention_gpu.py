@@ -70,6 +70,13 @@ def test_two_segment(M, H, T_hot, T_ret):
     _assert_close(got, ref)
 
 
+@pytest.mark.parametrize("T_hot,T_ret", [(50, 0), (112, 0), (113, 0), (225, 90), (336, 112), (449, 0), (460, 120), (896, 0)])
+@pytest.mark.parametrize("M,H", [(130, 2), (2600, 8)])      # one CTA per item; units cut over the SMs from eight tiles on
+def test_one_to_nine_key_tiles(M, H, T_hot, T_ret):
+    """Fewer key tiles than score buffers, as many, one more; P V lags four tiles behind the scores."""
+    _assert_close(*_run_two_segment(M, H, T_hot, T_ret, seed=T_hot + T_ret))
+
+
 def test_peaked_scores():
     """Large logits exercise the running-max rescale of the online softmax."""
     got, ref = _run_two_segment(300, 2, 700, 130, seed=5, spread=3.0)
