@@ -147,7 +147,8 @@ enum { kPlanK = 0, kPlanFreeLen, kPlanBufTop, kPlanPivTop, kPlanTotalAdd, kPlanT
        kPlanAnyValid, kPlanAbort, kPlanFullCount, kPlanMoveCount, kPlanShort, kPlanAvailBuf, kPlanAvailPiv,
        kPlanMergeCount, kPlanTicket, kPlanTicket2, kPlanLongCount, kPlanSize = 32 };
 
-// Block-wide exclusive scan, 1024 threads.
+// Block-wide exclusive scan over kWarps warps.
+template <int kWarps = 32>
 __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int incl = v;
@@ -159,17 +160,17 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
   if (lane == 31) warp_sums[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    int w = warp_sums[lane];
+    int w = lane < kWarps ? warp_sums[lane] : 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < kWarps; o <<= 1) {
       const int t = __shfl_up_sync(kFull, w, o);
       if (lane >= o) w += t;
     }
-    warp_sums[lane] = w;
+    if (lane < kWarps) warp_sums[lane] = w;
   }
   __syncthreads();
   const int excl = (warp > 0 ? warp_sums[warp - 1] : 0) + incl - v;
-  if (threadIdx.x == 0) *total = warp_sums[31];
+  if (threadIdx.x == 0) *total = warp_sums[kWarps - 1];
   __syncthreads();
   return excl;
 }
@@ -207,14 +208,21 @@ __device__ __forceinline__ int4 block_scan4(int4 v, int4* warp_sums, int4* total
 }
 
 // ------------------------------------------------------------------------------------ sort
-__global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams p) {
+// Threads: 1024, two CTAs per SM, as long as that is one wave of heads, else 512 and four per SM: the kernel is
+// a chain of latencies and barriers, and a second wave costs as much as the first.
+// (384 heads: 8328 tokens each 121 -> 106 us, 1041 each 31.9 -> 19.3 us.  16 heads, 8328 tokens: 44.7 -> 34.3 us since
+// the digits are counted with shared-memory adds; matching the lanes of a warp first cost more than the adds'
+// conflicts.)
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 2048 / kThreads) sort_tokens_kernel(const MergeParams p) {
+  constexpr int kWarps = kThreads / 32;
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
   // Digit counters, [warp][digit]: a warp's lanes count different digits of the same warp, so neighbouring
   // digits lie in neighbouring banks; rows of 257 words let the scan, which walks them digit by
   // digit, read without conflicts too.  ([digit][warp] put all of a warp's counters in one bank.)
   // (384 heads, 8328 tokens each: insert + retrieval 1112 -> 1068 us; 16 heads, fp32: 278 -> 263 us.)
   constexpr int kHistRow = 257;
-  __shared__ int hist[kHistRow * 32];
+  __shared__ int hist[kHistRow * kWarps];
   __shared__ int warp_sums[32];
   __shared__ int sh_total;
   __shared__ int sh_carry;
@@ -228,8 +236,8 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
   // 1. valid evicted tokens in position order
   if (threadIdx.x == 0) sh_carry = 0;
   __syncthreads();
-  // four consecutive positions per thread: one block scan per 4096 tokens, loads issued together
-  for (int base = 0; base < p.n_new; base += 4096) {
+  // four consecutive positions per thread: one block scan per 4 kThreads tokens, loads issued together
+  for (int base = 0; base < p.n_new; base += 4 * kThreads) {
     const int j0 = base + threadIdx.x * 4;
     int vxs[4];
     int sum = 0;
@@ -244,7 +252,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
       vxs[t] = (vx >= 0 && vx < p.voxel_used) ? vx : -1;
       sum += vxs[t] >= 0 ? 1 : 0;
     }
-    int off = sh_carry + block_scan(sum, warp_sums, &sh_total);
+    int off = sh_carry + block_scan<kWarps>(sum, warp_sums, &sh_total);
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       if (vxs[t] >= 0) {
@@ -266,7 +274,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
     if (threadIdx.x == 0) report_error(p.err, DEV_SORT_CAPACITY);
     n = p.ncap;
   }
-  for (int o = os + threadIdx.x; o < oe; o += 1024) {
+  for (int o = os + threadIdx.x; o < oe; o += kThreads) {
     const int dst = n_valid + (o - os);
     if (dst < n) {
       ka[dst] = static_cast<unsigned int>(p.over_hv_in[2 * o + 1]);
@@ -276,18 +284,18 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
   __syncthreads();
   // 3. stable LSD radix sort by voxel id.  Each warp owns a contiguous chunk of the list so
   //    that (warp, position in chunk) preserves the input order.
-  const int chunk = ((n + 31) / 32 + 31) / 32 * 32;  // items per warp, multiple of 32
+  const int chunk = ((n + kWarps - 1) / kWarps + 31) / 32 * 32;  // items per warp, multiple of 32
   const int c0 = warp * chunk;
   const int c1 = min(n, c0 + chunk);
   unsigned int* kin = ka; int* vin = va; unsigned int* kout = kb; int* vout = vb;
-  // The first kRegIt * 32 items of a warp's chunk (all of it in lists of up to 8192 tokens) are read into
+  // The first kRegIt * 32 items of a warp's chunk (all of it in lists of up to 8 kThreads tokens) are read into
   // registers once per pass: one round trip to L2 instead of one per 32 items in each of the two
   // loops.
   constexpr int kRegIt = 8;
   int* my_hist = hist + warp * kHistRow;
   for (int pass = 0; pass < p.passes; ++pass) {
     const int shift = pass * 8;
-    for (int i = threadIdx.x; i < kHistRow * 32; i += 1024) hist[i] = 0;
+    for (int i = threadIdx.x; i < kHistRow * kWarps; i += kThreads) hist[i] = 0;
     unsigned int kreg[kRegIt];
     int vreg[kRegIt];
 #pragma unroll
@@ -298,10 +306,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
     }
     __syncthreads();
     auto count = [&](bool in, unsigned int key) {
-      const unsigned int d = in ? ((key >> shift) & 255u) : (256u + lane);
-      const unsigned int peers = __match_any_sync(kFull, d);
-      if (in && (peers & ((1u << lane) - 1)) == 0) my_hist[d] += __popc(peers);
-      __syncwarp();
+      if (in) atomicAdd(&my_hist[(key >> shift) & 255u], 1);
     };
 #pragma unroll
     for (int t = 0; t < kRegIt; ++t) {
@@ -313,13 +318,14 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
     // exclusive scan of the counters in (digit, warp) order: 8 consecutive entries per thread
     int loc[8];
     int sum = 0;
-    int* of_thread = hist + (threadIdx.x & 3) * 8 * kHistRow + (threadIdx.x >> 2);
+    constexpr int kParts = kWarps / 8;      // threads per digit
+    int* of_thread = hist + (threadIdx.x % kParts) * 8 * kHistRow + threadIdx.x / kParts;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       loc[e] = of_thread[e * kHistRow];
       sum += loc[e];
     }
-    int run = block_scan(sum, warp_sums, &sh_total);
+    int run = block_scan<kWarps>(sum, warp_sums, &sh_total);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       of_thread[e * kHistRow] = run;
@@ -357,7 +363,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
   __syncthreads();
   int* rvx = p.row_vx + static_cast<long long>(h) * p.ncap;
   int* rst = p.row_start + static_cast<long long>(h) * (p.ncap + 1);
-  for (int base = 0; base < n; base += 4096) {
+  for (int base = 0; base < n; base += 4 * kThreads) {
     const int i0 = base + threadIdx.x * 4;
     unsigned int key[4];
     int hf[4];
@@ -372,7 +378,7 @@ __global__ void __launch_bounds__(1024, 2) sort_tokens_kernel(const MergeParams 
       if (i < n) hf[t] = (i == 0 || key[t] != (t == 0 ? prev : key[t - 1])) ? 1 : 0;
       sum += hf[t];
     }
-    int r = sh_carry + block_scan(sum, warp_sums, &sh_total);    // rows that begin before this thread's tokens
+    int r = sh_carry + block_scan<kWarps>(sum, warp_sums, &sh_total);    // rows that begin before this thread's tokens
     if (back == key[0]) {      // the first token's row reaches far back: the token behind kLongRow others lists it
       for (int t = 0; t < 4; ++t) {
         const int s0 = i0 + t - kLongRow;
@@ -1456,7 +1462,10 @@ ScratchLayout scratch_layout(int heads, int ncap, int buf_cap) {
 template <typename T>
 int launch_merge(MergeParams& mp, cudaStream_t st) {
   if (cudaMemsetAsync(mp.plan, 0, kPlanSize * 4, st) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(sort_tokens_kernel, dim3(mp.heads), dim3(1024), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  const bool one_wave = mp.heads <= 2 * 148;
+  if (launch_behind(one_wave ? sort_tokens_kernel<1024> : sort_tokens_kernel<512>, dim3(mp.heads), dim3(one_wave ? 1024 : 512), 0, st,
+                    mp) != cudaSuccess)
+    return STAC_ERR_CUDA;
   dim3 grid_a1((mp.ncap + 255) / 256, mp.heads);
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
   if (launch_behind(tokens_sim_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
