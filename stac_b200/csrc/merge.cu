@@ -18,11 +18,11 @@
 //   sort_tokens_kernel   one CTA per pool head: list the head's valid evicted tokens followed
 //                        by its carried overflow tokens, stable LSD radix sort by voxel id,
 //                        emit the unique rows (CSR).
-//   tokens_sim_kernel    token-parallel (a thread per token, then eight lanes per token whose row has
-//                        pivots, 16-byte loads): cosine of the token with the pivots of its row,
-//                        best pivot; rows in which a token reaches the merge threshold are queued for
-//   rows_merge_kernel    eight lanes per queued row: fold those tokens into their pivots in token
-//                        order (exp(sim) weights), publish the new pivot weights.
+//   tokens_sim_merge_kernel  token-parallel (a thread per token, then eight lanes per token whose row has
+//                        pivots, 16-byte loads): cosine of the token with the pivots of its row, best pivot; then
+//                        eight lanes per row of up to eight tokens: fold the tokens that reach the merge threshold
+//                        into their pivots in token order (exp(sim) weights), publish the new pivot weights.
+//   rows_merge_kernel    the same folding for longer rows, which the kernel above queues.
 //   rows_rank_kernel     one thread per row: score gate of the row's pivots, selection, ranking of
 //                        the buffered tokens + selected tokens by (score desc, arrival order),
 //                        counts of new segments / overflow / full; rows with many tokens, which
@@ -460,59 +460,160 @@ __device__ __forceinline__ const T* token_row_at(const MergeParams& p, int h, in
   return static_cast<const T*>(want_v ? p.over_V_in : p.over_K_in) + static_cast<long long>(~code) * p.D;
 }
 
-// Sums of eight values over the eight lanes of a group: lane j of the group gets the total of v[j].
-// Seven shuffles instead of three per value; the same additions as group8_sum makes, so the same bits.
-__device__ __forceinline__ float group8_sum_scatter(const float (&v)[8], int sub, unsigned gmask) {
-  float a[4], b[2];
-  const bool h4 = sub & 4, h2 = sub & 2, h1 = sub & 1;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float give = h4 ? v[j] : v[j + 4], keep = h4 ? v[j + 4] : v[j];
-    a[j] = keep + __shfl_xor_sync(gmask, give, 4);
-  }
+// Sums of four values over the eight lanes of a group: lanes 2 q and 2 q + 1 get the total of v[q] (the same
+// additions as group8_sum makes, so the same bits).
+__device__ __forceinline__ float group8_sum_scatter4(const float (&v)[4], int sub, unsigned gmask) {
+  float a[2];
+  const bool h4 = sub & 4, h2 = sub & 2;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    const float give = h2 ? a[j] : a[j + 2], keep = h2 ? a[j + 2] : a[j];
-    b[j] = keep + __shfl_xor_sync(gmask, give, 2);
+    const float give = h4 ? v[j] : v[j + 2], keep = h4 ? v[j + 2] : v[j];
+    a[j] = keep + __shfl_xor_sync(gmask, give, 4);
   }
-  const float give = h1 ? b[0] : b[1], keep = h1 ? b[1] : b[0];
-  return keep + __shfl_xor_sync(gmask, give, 1);
+  const float give = h2 ? a[0] : a[1], keep = h2 ? a[1] : a[0];
+  const float b = keep + __shfl_xor_sync(gmask, give, 2);
+  return b + __shfl_xor_sync(gmask, b, 1);
+}
+
+// Raw values of one lane's eighth of a row: loads that are in flight while others are worked on.
+template <typename T> struct Raw8;
+template <> struct Raw8<__nv_bfloat16> {
+  uint4 u;
+  __device__ __forceinline__ void load(const __nv_bfloat16* row, int sub) { u = reinterpret_cast<const uint4*>(row)[sub]; }
+  __device__ __forceinline__ void values(float (&x)[8]) const {
+    x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
+    x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
+    x[4] = __uint_as_float(u.z << 16); x[5] = __uint_as_float(u.z & 0xffff0000u);
+    x[6] = __uint_as_float(u.w << 16); x[7] = __uint_as_float(u.w & 0xffff0000u);
+  }
+};
+template <> struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* row, int sub) {
+    a = reinterpret_cast<const float4*>(row)[2 * sub];
+    b = reinterpret_cast<const float4*>(row)[2 * sub + 1];
+  }
+  __device__ __forceinline__ void values(float (&x)[8]) const {
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  }
+};
+
+// What the tokens of a row that merge into one pivot add up to, in token order, held by eight lanes.
+struct MergeSums {
+  float K[8], V[8], A, S, C;
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) K[e] = V[e] = 0.f;
+    A = S = C = 0.f;
+  }
+  __device__ __forceinline__ void add(float a, float s, const float (&k)[8], const float (&v)[8]) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      K[e] = __fadd_rn(K[e], __fmul_rn(a, k[e]));
+      V[e] = __fadd_rn(V[e], __fmul_rn(a, v[e]));
+    }
+    A = __fadd_rn(A, a);
+    S = __fadd_rn(S, s);
+    C = __fadd_rn(C, 1.f);
+  }
+};
+// K <- (W K + sum a k) / (W + sum a), same for V, W += sum a, S += sum of the scores, C += count; stored in
+// the pool dtype (stac/merger.py:660-760).
+template <typename T>
+__device__ __forceinline__ void merge_into_pivot(const MergeParams& p, int seg, float W, const MergeSums& m, int sub) {
+  T* kb = static_cast<T*>(p.piv_K) + static_cast<long long>(seg) * p.D;
+  T* vb = static_cast<T*>(p.piv_V) + static_cast<long long>(seg) * p.D;
+  const float denom = fmaxf(__fadd_rn(W, m.A), 1e-8f);
+  const float fo = __fdiv_rn(W, denom), fn = __fdiv_rn(1.0f, denom);
+  Raw8<T> k_old, v_old;
+  k_old.load(kb, sub);
+  v_old.load(vb, sub);
+  const float S = sub == 0 ? p.piv_S[seg] : 0.f, C = sub == 0 ? p.piv_C[seg] : 0.f;
+  float o[8];
+  k_old.values(o);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) o[e] = __fadd_rn(__fmul_rn(fo, o[e]), __fmul_rn(fn, m.K[e]));
+  Row8<T>::store(kb, sub, o);
+  v_old.values(o);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) o[e] = __fadd_rn(__fmul_rn(fo, o[e]), __fmul_rn(fn, m.V[e]));
+  Row8<T>::store(vb, sub, o);
+  if (sub == 0) {
+    p.piv_W[seg] = denom;
+    p.piv_S[seg] = __fadd_rn(S, m.S);
+    p.piv_C[seg] = __fadd_rn(C, m.C);
+  }
 }
 
 // Tokens against the pivots of their row (stac/merger.py:586-660): cosine with every pivot key
 // (both L2-normalised, norms clamped at 1e-6), clamped to [-1, 1]; the first largest wins.  All
 // similarities are taken against the pivots as they are BEFORE this call's merges, as the
-// reference's vectorised code does.
+// reference's vectorised code does.  Then the tokens whose best similarity reaches the threshold are folded
+// into that pivot in token order with weights exp(sim).
 //
-// A CTA takes 256 consecutive tokens of a head.  First one thread per token fetches what is known
-// about it (coalesced; the sorted key is the voxel id) and settles the tokens whose row has no
-// pivot; the others go to a list in shared memory, and groups of eight lanes (16 bytes of a bf16
-// row each) walk that list.  The walk is bound by its dependent loads and by the reductions: the
-// pivot segments come with the pivot count, and the eight sums of a token are reduced together,
-// each lane then finishing one of them.
-// (1.6 M tokens whose rows hold pivots: 318 -> 240 us against eight lanes per token throughout; 3.2 M
-// tokens of a bounded memory, few rows with pivots: 155 -> 59 us.)
+// A CTA takes 256 consecutive tokens of a head (sorted by row).  First one thread per token fetches what is
+// known about it (coalesced; the sorted key is the voxel id) and settles the tokens whose row has no pivot;
+// the others are listed in shared memory, and groups of eight lanes (16 bytes of a bf16 row each) walk that
+// list: the next token's key row is in flight while one is compared, only pivots that exist are compared, and
+// the dot products of a token are reduced together, lane pairs then finishing one pivot each.
+// Then the rows of up to eight tokens in which a token merges are folded, eight lanes per row, lane j knowing
+// token j, one pivot after the other (one set of sums live), with everything but the rows themselves in
+// shared memory.  Such a row belongs to the CTA in which it starts, which fetches eight tokens more than its
+// own; only that CTA looks at its pivots, so all of its similarities are taken before.  Longer rows are
+// queued for rows_merge_kernel.
+// (As two kernels, which read a row's tokens twice and found them again through lists in memory, similarities
+// and merges took 288 + 293 us with 384 heads of 8328 tokens in a bounded memory, 102 + 166 us with 384 heads of 1041
+// tokens, 31 + 51 us with 16 heads of 8328 fp32 tokens; now 394 + 10, 162 + 2, 67 + 2.  Eight lanes taking a whole row
+// for comparing and merging in one go were slower, 414, 200 and 95 us: the four rows of a warp diverge.)
 constexpr int kTokBlock = 256;
+constexpr int kShortRow = 8;           // one lane per token
 template <typename T>
-__global__ void __launch_bounds__(kTokBlock) tokens_sim_kernel(const MergeParams p) {
+__global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
-  __shared__ int4 list[kTokBlock];   // token, code, position, pivot count
+  constexpr int kAll = kTokBlock + kShortRow;
+  constexpr int kNoKey = -1;           // not a voxel id
+  __shared__ int key_s[kShortRow + kAll];        // voxel ids from eight tokens before to eight behind
+  __shared__ uintptr_t krow_s[kAll];             // address of the token's key row (16-byte aligned); bit 0: a carried token
+  __shared__ float score_s[kAll], sim_s[kAll];
+  __shared__ signed char best_s[kAll];           // pivot that the token merges into, -1 = none
   __shared__ int4 segs[kTokBlock];
-  __shared__ int n_list;
+  __shared__ unsigned char npiv_s[kTokBlock], len_s[kTokBlock];   // len: tokens of the short row that starts here
+  __shared__ unsigned short list[kAll];          // token, (tokens of its row before it) << 12; then rows to merge
+  __shared__ unsigned todo_mask[kTokBlock / 32]; // bit per token: a token of the row that starts there merges
+  __shared__ int n_list, n_todo;
   const int h = blockIdx.y;
   if (p.plan[kPlanAnyValid] == 0) return;
   const int n_tok = p.n_tok[h];
   const int i0 = blockIdx.x * kTokBlock;
   if (i0 >= n_tok) return;
-  if (threadIdx.x == 0) n_list = 0;
-  __syncthreads();
+  const int t = threadIdx.x, lane = t & 31, sub = t & 7, gbase = lane & 24;
+  const unsigned gmask = 0xffu << gbase;
   const long long hb = static_cast<long long>(h) * p.ncap;
-  const int i = i0 + threadIdx.x;
+  const unsigned* keys = ((p.passes & 1) ? p.keys_b : p.keys_a) + hb;
+  const int* codes = ((p.passes & 1) ? p.vals_b : p.vals_a) + hb;
+  auto fetch = [&](int t) {            // key, source and score of token t of this CTA
+    const int i = i0 + t;
+    const int code = codes[i];
+    key_s[kShortRow + t] = static_cast<int>(keys[i]);
+    int pos = 0;
+    float score;
+    if (code >= 0) {
+      pos = token_pos(p, h, code);
+      score = p.s_src[h * p.meta_head_stride + pos];
+    } else {
+      score = p.over_S_in[~code];
+    }
+    krow_s[t] = reinterpret_cast<uintptr_t>(token_row_at<T>(p, h, code, pos, false)) | (code < 0 ? 1u : 0u);
+    score_s[t] = score;
+    best_s[t] = -1;
+  };
+  if (t == 0) n_list = n_todo = 0;
+  if (t < kTokBlock / 32) todo_mask[t] = 0u;
+  const int i = i0 + t;
+  int npiv = 0;
   if (i < n_tok) {
-    const int code = (((p.passes & 1) ? p.vals_b : p.vals_a) + hb)[i];
-    const int vx = static_cast<int>((((p.passes & 1) ? p.keys_b : p.keys_a) + hb)[i]);
-    const long long r = static_cast<long long>(h) * p.voxel_cap + vx;
-    const int npiv = p.piv_row_cnt[r];
+    const long long r = static_cast<long long>(h) * p.voxel_cap + static_cast<int>(keys[i]);
+    npiv = p.piv_row_cnt[r];
     int4 sg = make_int4(0, 0, 0, 0);
     if (p.seg_vec) {
       sg = reinterpret_cast<const int4*>(p.piv_row_seg)[r];
@@ -522,67 +623,85 @@ __global__ void __launch_bounds__(kTokBlock) tokens_sim_kernel(const MergeParams
       if (npiv > 2) sg.z = p.piv_row_seg[r * p.P + 2];
       if (npiv > 3) sg.w = p.piv_row_seg[r * p.P + 3];
     }
-    int pos = 0;
-    float score;
-    if (code >= 0) {
-      pos = token_pos(p, h, code);
-      score = p.s_src[h * p.meta_head_stride + pos];
-    } else {
-      score = p.over_S_in[~code];
-    }
-    p.tok_score[hb + i] = score;
+    fetch(t);
+    p.tok_score[hb + i] = score_s[t];
     if (npiv == 0) {
       p.tok_sim[hb + i] = -INFINITY;
       p.tok_best[hb + i] = 0;
-    } else {
-      const int e = list_push(&n_list);
-      list[e] = make_int4(i, code, pos, npiv);
-      segs[e] = sg;
     }
+    segs[t] = sg;
+  } else {
+    key_s[kShortRow + t] = kNoKey;
+  }
+  npiv_s[t] = static_cast<unsigned char>(npiv);
+  if (t < kShortRow) {
+    if (i + kTokBlock < n_tok) fetch(t + kTokBlock);
+    else key_s[kShortRow + kTokBlock + t] = kNoKey;
+    key_s[t] = i0 > 0 ? static_cast<int>(keys[i0 - kShortRow + t]) : kNoKey;
   }
   __syncthreads();
+  // Lists token t: tokens of a short row with pivots where the row starts in this CTA, tokens of a longer one in the
+  // CTA that they lie in.
+  auto enlist = [&](int t) {
+    const int* k = key_s + kShortRow + t;
+    const int key = k[0];
+    if (key == kNoKey || (t < kTokBlock && npiv_s[t] == 0)) return;
+    int before = 0, behind = 1;
+    while (before < kShortRow && k[-before - 1] == key) ++before;
+    while (before + behind <= kShortRow && t + behind < kAll && k[behind] == key) ++behind;
+    const bool is_short = before + behind <= kShortRow;
+    const int first = is_short ? t - before : t;
+    if (first < 0 || first >= kTokBlock || npiv_s[first] == 0) return;
+    if (is_short && before == 0) len_s[t] = static_cast<unsigned char>(behind);
+    list[list_push(&n_list)] = static_cast<unsigned short>(t | ((is_short ? before : kShortRow) << 12));
+  };
+  enlist(t);
+  if (t < kShortRow) enlist(kTokBlock + t);
+  __syncthreads();
   const int n = n_list;
-  const int lane = threadIdx.x & 31, sub = threadIdx.x & 7;
-  const unsigned gmask = 0xffu << (lane & 24);
-  for (int e = threadIdx.x >> 3; e < n; e += kTokBlock / 8) {
-    const int4 tk = list[e];
-    const int4 sg = segs[e];
-    const int npiv = tk.w;
-    float k[8], pk[kMaxP][8];
-    Row8<T>::load(token_row_at<T>(p, h, tk.y, tk.z, false), sub, k);
+  if (n == 0) return;        // the same for the whole CTA
+  constexpr int kStep = kTokBlock / 8;
+  auto key_row = [&](int t) { return reinterpret_cast<const T*>(krow_s[t] & ~static_cast<uintptr_t>(1)); };
+  Raw8<T> next_k;
+  int e = t >> 3;
+  if (e < n) next_k.load(key_row(list[e] & 0xfff), sub);
+  for (; e < n; e += kStep) {
+    const int entry = list[e], tk = entry & 0xfff, before = entry >> 12;
+    const bool is_short = before < kShortRow;
+    const int first = is_short ? tk - before : tk;
+    const int np = npiv_s[first];
+    const int4 sg = segs[first];
     const int seg[kMaxP] = {sg.x, sg.y, sg.z, sg.w};
+    Raw8<T> rp[kMaxP];
 #pragma unroll
-    for (int q = 0; q < kMaxP; ++q) {
-      if (q < npiv) {
-        Row8<T>::load(static_cast<const T*>(p.piv_K) + static_cast<long long>(seg[q]) * p.D, sub, pk[q]);
-      } else {
-#pragma unroll
-        for (int x = 0; x < 8; ++x) pk[q][x] = 0.f;
-      }
-    }
+    for (int q = 0; q < kMaxP; ++q)
+      if (q < np) rp[q].load(static_cast<const T*>(p.piv_K) + static_cast<long long>(seg[q]) * p.D, sub);
+    float k[8];
+    next_k.values(k);
+    if (e + kStep < n) next_k.load(key_row(list[e + kStep] & 0xfff), sub);
     float kk = 0.f;
 #pragma unroll
     for (int x = 0; x < 8; ++x) kk = fmaf(k[x], k[x], kk);
-    float part[8];                     // dot and squared norm of pivot q in entries 2 q and 2 q + 1
+    float dot[kMaxP], nrm[kMaxP];
 #pragma unroll
     for (int q = 0; q < kMaxP; ++q) {
-      float d = 0.f, pp = 0.f;
+      dot[q] = nrm[q] = 0.f;
+      if (q < np) {
+        float pk[8];
+        rp[q].values(pk);
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        d = fmaf(k[x], pk[q][x], d);
-        pp = fmaf(pk[q][x], pk[q][x], pp);
+        for (int x = 0; x < 8; ++x) {
+          dot[q] = fmaf(k[x], pk[x], dot[q]);
+          nrm[q] = fmaf(pk[x], pk[x], nrm[q]);
+        }
       }
-      part[2 * q] = d;
-      part[2 * q + 1] = pp;
     }
     const float den_k = fmaxf(sqrtf(group8_sum(kk, gmask)), 1e-6f);
-    const float tot = group8_sum_scatter(part, sub, gmask);
-    const float oth = __shfl_xor_sync(gmask, tot, 1);
-    // lanes 2 q and 2 q + 1 both compute pivot q's similarity
-    const float d = (sub & 1) ? oth : tot, pp = (sub & 1) ? tot : oth;
-    const float den_p = fmaxf(sqrtf(pp), 1e-6f);
+    // lanes 2 q and 2 q + 1 both finish pivot q
+    const float d = group8_sum_scatter4(dot, sub, gmask);
+    const float den_p = fmaxf(sqrtf(group8_sum_scatter4(nrm, sub, gmask)), 1e-6f);
     int best = sub >> 1;
-    float best_sim = best < npiv ? fminf(1.f, fmaxf(-1.f, __fdiv_rn(d, __fmul_rn(den_k, den_p)))) : -INFINITY;
+    float best_sim = best < np ? fminf(1.f, fmaxf(-1.f, __fdiv_rn(d, __fmul_rn(den_k, den_p)))) : -INFINITY;
 #pragma unroll
     for (int o = 2; o <= 4; o <<= 1) {
       const float s2 = __shfl_xor_sync(gmask, best_sim, o);
@@ -593,28 +712,71 @@ __global__ void __launch_bounds__(kTokBlock) tokens_sim_kernel(const MergeParams
       }
     }
     if (sub == 0) {
-      p.tok_sim[hb + tk.x] = best_sim;
-      p.tok_best[hb + tk.x] = best;
+      const long long o = hb + i0 + tk;
+      p.tok_sim[o] = best_sim;
+      p.tok_best[o] = best;
       if (best_sim >= p.sim_thresh) {
-        const int ri = p.tok_row[hb + tk.x];
-        if (atomicExch(&p.row_flag[hb + ri], 1) == 0) p.merge_list[list_push(&p.plan[kPlanMergeCount])] = make_int2(h, ri);
+        if (is_short) {
+          best_s[tk] = static_cast<signed char>(best);
+          sim_s[tk] = best_sim;
+          atomicOr(&todo_mask[first >> 5], 1u << (first & 31));
+        } else {
+          const int ri = p.tok_row[o];
+          if (atomicExch(&p.row_flag[hb + ri], 1) == 0) p.merge_list[list_push(&p.plan[kPlanMergeCount])] = make_int2(h, ri);
+        }
       }
+    }
+  }
+  __syncthreads();
+  if ((todo_mask[t >> 5] >> lane) & 1u) list[list_push(&n_todo)] = static_cast<unsigned short>(t);
+  __syncthreads();
+  const int n_rows = n_todo;
+  const long long to_v = static_cast<const char*>(p.v_src) - static_cast<const char*>(p.k_src);
+  const long long to_v_over = static_cast<const char*>(p.over_V_in) - static_cast<const char*>(p.over_K_in);
+  for (int e = t >> 3; e < n_rows; e += kStep) {
+    const int t0 = list[e], len = len_s[t0], np = npiv_s[t0];
+    const int4 sg = segs[t0];
+    const int seg_l = sub == 0 ? sg.x : sub == 1 ? sg.y : sub == 2 ? sg.z : sg.w;
+    const float W_l = sub < np ? p.piv_W[seg_l] : 0.f;         // lane q < np: segment and weight of pivot q
+    const int best_l = sub < len ? best_s[t0 + sub] : -1;      // lane j: token j
+    const float a_l = best_l >= 0 ? expf(sim_s[t0 + sub]) : 0.f;
+    for (int q = 0; q < np; ++q) {
+      unsigned todo = __ballot_sync(gmask, best_l == q) >> gbase & 0xffu;
+      if (todo == 0u) continue;
+      MergeSums m;
+      m.clear();
+      // the next token's rows are in flight while this one's are added
+      Raw8<T> nk, nv;
+      auto load = [&](int j) {
+        const uintptr_t a = krow_s[t0 + j], kr = a & ~static_cast<uintptr_t>(1);
+        nk.load(reinterpret_cast<const T*>(kr), sub);
+        nv.load(reinterpret_cast<const T*>(kr + ((a & 1) ? to_v_over : to_v)), sub);
+      };
+      int j = __ffs(todo) - 1;
+      load(j);
+      while (todo) {
+        todo &= todo - 1;
+        float k[8], v[8];
+        nk.values(k);
+        nv.values(v);
+        const int jc = j;
+        if (todo) {
+          j = __ffs(todo) - 1;
+          load(j);
+        }
+        m.add(__shfl_sync(gmask, a_l, gbase + jc), fmaxf(score_s[t0 + jc], 1e-6f), k, v);
+      }
+      merge_into_pivot<T>(p, __shfl_sync(gmask, seg_l, gbase + q), __shfl_sync(gmask, W_l, gbase + q), m, sub);
     }
   }
 }
 
-// Rows with merging tokens: the tokens whose best similarity reaches the threshold are folded into
-// that pivot in token order with weights exp(sim): K <- (W K + sum a k) / (W + sum a), same for V,
-// W += sum a, S += sum of the (clamped) scores, C += count; the result is stored in the pool dtype
-// (stac/merger.py:660-760).
+// The same for the queued rows, those with more than kShortRow tokens.
 // What a row waits for is its chain of dependent loads, so the number of rows in flight decides:
-// eight lanes per row (16 bytes of a bf16 row each) instead of a warp, what is known about a row's
-// tokens fetched eight at a time (a lane per token), and one pivot after the other, so that only one
-// pair of accumulators is live and five CTAs of 32 rows share an SM.
-// (384 heads, 4164 tokens each: 364 -> 165 us against a warp per row; a warp per row with its tokens'
-// loads issued ahead, at 80 registers, measured 374 us.)
+// eight lanes per row (16 bytes of a bf16 row each), what is known about a row's tokens fetched eight at a
+// time (a lane per token), and one pivot after the other, so that only one pair of accumulators is live.
 template <typename T>
-__global__ void __launch_bounds__(256, 5) rows_merge_kernel(const MergeParams p) {
+__global__ void __launch_bounds__(256, 4) rows_merge_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
   const int lane = threadIdx.x & 31, sub = threadIdx.x & 7, gbase = lane & 24;
   const unsigned gmask = 0xffu << gbase;
@@ -656,9 +818,8 @@ __global__ void __launch_bounds__(256, 5) rows_merge_kernel(const MergeParams p)
     const bool one_batch = s1 - s0 <= 8;
     fetch(s0 + sub);
     for (int q = 0; q < npiv; ++q) {
-      float accK[8], accV[8], accA = 0.f, accS = 0.f, accC = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) accK[e] = accV[e] = 0.f;
+      MergeSums m;
+      m.clear();
       for (int base = s0; base < s1; base += 8) {
         if (!one_batch) fetch(base + sub);
         unsigned todo = __ballot_sync(gmask, best_l == q) >> gbase & 0xffu;
@@ -670,37 +831,11 @@ __global__ void __launch_bounds__(256, 5) rows_merge_kernel(const MergeParams p)
           float k[8], v[8];
           Row8<T>::load(token_row_at<T>(p, h, code, pos, false), sub, k);
           Row8<T>::load(token_row_at<T>(p, h, code, pos, true), sub, v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            accK[e] = __fadd_rn(accK[e], __fmul_rn(a, k[e]));
-            accV[e] = __fadd_rn(accV[e], __fmul_rn(a, v[e]));
-          }
-          accA = __fadd_rn(accA, a);
-          accS = __fadd_rn(accS, s_t);
-          accC = __fadd_rn(accC, 1.f);
+          m.add(a, s_t, k, v);
         }
       }
-      if (!(accA > 0.f)) continue;
-      const int seg = __shfl_sync(gmask, seg_l, gbase + q);
-      const float W = __shfl_sync(gmask, W_l, gbase + q);
-      T* kb = static_cast<T*>(p.piv_K) + static_cast<long long>(seg) * p.D;
-      T* vb = static_cast<T*>(p.piv_V) + static_cast<long long>(seg) * p.D;
-      const float denom = fmaxf(__fadd_rn(W, accA), 1e-8f);
-      const float fo = __fdiv_rn(W, denom), fn = __fdiv_rn(1.0f, denom);
-      float o[8];
-      Row8<T>::load(kb, sub, o);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = __fadd_rn(__fmul_rn(fo, o[e]), __fmul_rn(fn, accK[e]));
-      Row8<T>::store(kb, sub, o);
-      Row8<T>::load(vb, sub, o);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = __fadd_rn(__fmul_rn(fo, o[e]), __fmul_rn(fn, accV[e]));
-      Row8<T>::store(vb, sub, o);
-      if (sub == 0) {
-        p.piv_W[seg] = denom;
-        p.piv_S[seg] = __fadd_rn(p.piv_S[seg], accS);
-        p.piv_C[seg] = __fadd_rn(p.piv_C[seg], accC);
-      }
+      if (!(m.A > 0.f)) continue;
+      merge_into_pivot<T>(p, __shfl_sync(gmask, seg_l, gbase + q), __shfl_sync(gmask, W_l, gbase + q), m, sub);
     }
   }
 }
@@ -1468,8 +1603,8 @@ int launch_merge(MergeParams& mp, cudaStream_t st) {
     return STAC_ERR_CUDA;
   dim3 grid_a1((mp.ncap + 255) / 256, mp.heads);
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
-  if (launch_behind(tokens_sim_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(rows_merge_kernel<T>, dim3(148 * 5), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(tokens_sim_merge_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(rows_merge_kernel<T>, dim3(148 * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_rank_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(scan_rows_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 0) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(scan_rows_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 1) != cudaSuccess) return STAC_ERR_CUDA;

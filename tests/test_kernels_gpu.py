@@ -415,6 +415,39 @@ def test_merge_of_rows_with_many_tokens(lengths, heads, levels):
     assert m.piv.used() > 0
 
 
+@pytest.mark.parametrize("lengths,heads,dtype", [
+    ([7] * 80, 3, "bf16"),                                  # rows that straddle the 256 tokens of a CTA at every offset
+    ([8] * 70, 3, "f32"),                                   # the longest row that a CTA merges itself, never straddling
+    ([1] + [8] * 70, 3, "f32"),                             # one token over the edge
+    ([9] * 60, 3, "bf16"),                                  # the shortest row that is queued
+    ([248, 8, 8, 1, 9, 8, 255, 7], 2, "f32"),               # long and short rows side by side at the edges
+    ([3, 8, 9, 1], 300, "f32"),                             # many heads
+])
+def test_merge_of_rows_around_eight_tokens(lengths, heads, dtype):
+    """Rows of up to eight tokens are merged by the CTA in which they start, wherever its 256 tokens end: slot maps
+    and pool contents as in the oracle after every call."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    rs = np.random.RandomState(len(lengths) + heads)
+    rtol, atol = (1e-3, 1e-5) if dtype == "f32" else (8e-3, 4e-3)     # as in test_merge_and_retrieve_match_oracle
+    D, NV, Tn = 64, len(lengths), sum(lengths)
+    g = VoxelKVMerger(heads, D, init_voxels=NV, pivot_cap=4, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8,
+                      score_thresh=0.1, dtype=torch.float32 if dtype == "f32" else torch.bfloat16, device=DEV,
+                      allocator="segment", seg_size=1, slab_cap=16)
+    m = VoxelMerger(heads, D, NV, 4, 8, 0.8, 0.8, 0.1, dtype)
+    dirs = rs.randn(NV, D).astype(np.float32)
+    for step in range(4):
+        VX = np.stack([rs.permutation(np.repeat(np.arange(NV), lengths)) for _ in range(heads)]).astype(np.int32)
+        near = rs.rand(heads, Tn, 1) < 0.6
+        noise = rs.randn(heads, Tn, D).astype(np.float32)
+        K = m.rnd(np.where(near, dirs[VX] + 0.2 * noise, noise).astype(np.float32))
+        V = m.rnd(rs.randn(heads, Tn, D).astype(np.float32))
+        S = np.exp(rs.randn(heads, Tn)).astype(np.float32)
+        m.insert_and_merge(K, V, S, VX, NV)
+        g.insert_and_merge(*(torch.from_numpy(x).to(DEV) for x in (K, V, S)), None, torch.from_numpy(VX).to(DEV), NV)
+        _compare_pool(g.snapshot(), m, f"step {step}", rtol, atol)
+    assert m.piv.used() > 0
+
+
 @pytest.mark.parametrize("bound", [None, 9000])
 def test_merge_with_more_heads_than_one_round_of_the_plan(bound):
     """1100 pool heads (the plan scans 1024 at a time), unbounded and with pools that fill up."""
