@@ -591,30 +591,19 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
   const long long hb = static_cast<long long>(h) * p.ncap;
   const unsigned* keys = ((p.passes & 1) ? p.keys_b : p.keys_a) + hb;
   const int* codes = ((p.passes & 1) ? p.vals_b : p.vals_a) + hb;
-  auto fetch = [&](int t) {            // key, source and score of token t of this CTA
-    const int i = i0 + t;
-    const int code = codes[i];
-    key_s[kShortRow + t] = static_cast<int>(keys[i]);
-    int pos = 0;
-    float score;
-    if (code >= 0) {
-      pos = token_pos(p, h, code);
-      score = p.s_src[h * p.meta_head_stride + pos];
-    } else {
-      score = p.over_S_in[~code];
-    }
-    krow_s[t] = reinterpret_cast<uintptr_t>(token_row_at<T>(p, h, code, pos, false)) | (code < 0 ? 1u : 0u);
-    score_s[t] = score;
-    best_s[t] = -1;
-  };
   if (t == 0) n_list = n_todo = 0;
   if (t < kTokBlock / 32) todo_mask[t] = 0u;
+  // Key, source and score of token t and, by the first threads, of one of the tokens behind the CTA's: both
+  // chains of loads go out side by side.
   const int i = i0 + t;
+  const bool mine = i < n_tok, extra = t < kShortRow && i + kTokBlock < n_tok;
+  const int key = mine ? static_cast<int>(keys[i]) : kNoKey, key_x = extra ? static_cast<int>(keys[i + kTokBlock]) : kNoKey;
+  const int code = mine ? codes[i] : 0, code_x = extra ? codes[i + kTokBlock] : 0;
   int npiv = 0;
-  if (i < n_tok) {
-    const long long r = static_cast<long long>(h) * p.voxel_cap + static_cast<int>(keys[i]);
+  int4 sg = make_int4(0, 0, 0, 0);
+  if (mine) {
+    const long long r = static_cast<long long>(h) * p.voxel_cap + key;
     npiv = p.piv_row_cnt[r];
-    int4 sg = make_int4(0, 0, 0, 0);
     if (p.seg_vec) {
       sg = reinterpret_cast<const int4*>(p.piv_row_seg)[r];
     } else if (npiv > 0) {
@@ -623,23 +612,31 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
       if (npiv > 2) sg.z = p.piv_row_seg[r * p.P + 2];
       if (npiv > 3) sg.w = p.piv_row_seg[r * p.P + 3];
     }
-    fetch(t);
-    p.tok_score[hb + i] = score_s[t];
+  }
+  const int pos = mine && code >= 0 ? token_pos(p, h, code) : 0, pos_x = extra && code_x >= 0 ? token_pos(p, h, code_x) : 0;
+  auto score_of = [&](int code, int pos) { return code >= 0 ? p.s_src[h * p.meta_head_stride + pos] : p.over_S_in[~code]; };
+  const float score = mine ? score_of(code, pos) : 0.f, score_x = extra ? score_of(code_x, pos_x) : 0.f;
+  auto keep = [&](int t, int key, int code, int pos, float score) {
+    key_s[kShortRow + t] = key;
+    krow_s[t] = reinterpret_cast<uintptr_t>(token_row_at<T>(p, h, code, pos, false)) | (code < 0 ? 1u : 0u);
+    score_s[t] = score;
+    best_s[t] = -1;
+  };
+  keep(t, key, code, pos, score);
+  npiv_s[t] = static_cast<unsigned char>(npiv);
+  segs[t] = sg;
+  if (t < kShortRow) {
+    keep(t + kTokBlock, key_x, code_x, pos_x, score_x);
+    key_s[t] = i0 > 0 ? static_cast<int>(keys[i0 - kShortRow + t]) : kNoKey;
+  }
+  if (mine) {
+    p.tok_score[hb + i] = score;
     if (npiv == 0) {
       p.tok_sim[hb + i] = -INFINITY;
       p.tok_best[hb + i] = 0;
     }
-    segs[t] = sg;
-  } else {
-    key_s[kShortRow + t] = kNoKey;
   }
-  npiv_s[t] = static_cast<unsigned char>(npiv);
-  if (t < kShortRow) {
-    if (i + kTokBlock < n_tok) fetch(t + kTokBlock);
-    else key_s[kShortRow + kTokBlock + t] = kNoKey;
-    key_s[t] = i0 > 0 ? static_cast<int>(keys[i0 - kShortRow + t]) : kNoKey;
-  }
-  __syncthreads();
+  if (!__syncthreads_or(npiv > 0)) return;
   // Lists token t: tokens of a short row with pivots where the row starts in this CTA, tokens of a longer one in the
   // CTA that they lie in.
   auto enlist = [&](int t) {
@@ -659,7 +656,6 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
   if (t < kShortRow) enlist(kTokBlock + t);
   __syncthreads();
   const int n = n_list;
-  if (n == 0) return;        // the same for the whole CTA
   constexpr int kStep = kTokBlock / 8;
   auto key_row = [&](int t) { return reinterpret_cast<const T*>(krow_s[t] & ~static_cast<uintptr_t>(1)); };
   Raw8<T> next_k;
