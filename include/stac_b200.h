@@ -99,6 +99,21 @@ int stac_attn_colsum_kept(const void* q, int64_t q_row_stride,
                           void* workspace, size_t workspace_bytes,
                           int* dev_status, stac_stream_t stream);
 
+/* The same with a kept workspace, and the running scores of the hot keys updated from their column sums by the
+ * kernel that makes them, or by a launch behind it where two CTAs add up one sum: the effect of
+ * stac_scores_update(colsum, ..., T_live = T_hot, old_T, Tq, temperature) behind the call, bit for bit.  `colsum`
+ * must not be NULL. */
+int stac_attn_colsum_scored(const void* q, int64_t q_row_stride,
+                            const void* k_hot, const void* v_hot, int64_t hot_row_stride, int64_t hot_head_stride, int T_hot,
+                            const void* k_ret, const void* v_ret, int64_t ret_row_stride, int64_t ret_head_stride, int T_ret,
+                            const float* bias_ret, int64_t bias_head_stride,
+                            void* out, int64_t out_row_stride,
+                            float* lse, float* colsum, int64_t colsum_head_stride,
+                            int M, int H, int D, float scale, float subsample_ratio,
+                            float* scores, float* counts, int64_t score_row_stride, int old_T, int Tq, float temperature,
+                            void* workspace, size_t workspace_bytes,
+                            int* dev_status, stac_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------
  * Voxel table: packed 63-bit key -> stable voxel id (append-only; id = insertion rank).
  *

@@ -66,6 +66,10 @@ SIGNATURES = {
     "stac_attn_colsum_noalloc": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_i64, c_int, c_void_p,
                                          c_void_p, c_i64, c_i64, c_int, c_void_p, c_i64, c_void_p, c_i64, c_void_p,
                                          c_void_p, c_i64, c_int, c_int, c_int, c_f32, c_f32, c_void_p, c_void_p]),
+    "stac_attn_colsum_scored": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_i64, c_int, c_void_p, c_void_p,
+                                        c_i64, c_i64, c_int, c_void_p, c_i64, c_void_p, c_i64, c_void_p, c_void_p, c_i64,
+                                        c_int, c_int, c_int, c_f32, c_f32, c_void_p, c_void_p, c_i64, c_int, c_int,
+                                        c_f32, c_void_p, c_size_t, c_void_p, c_void_p]),
     "stac_selftest_bounded_wait": (c_int, [c_int, c_void_p, c_void_p]),
     "stac_voxel_scratch_bytes": (c_size_t, [c_int]),
     "stac_voxel_hash_clear": (c_int, [c_void_p, c_i64, c_void_p]),
@@ -103,7 +107,7 @@ SIGNATURES = {
 # used to report how many of this library's kernels ran in a timed region
 # (stac_attn_colsum: fast forward, exact forward, column sums)
 KERNELS_PER_CALL = {
-    "stac_attn_colsum": 3, "stac_attn_colsum_kept": 3, "stac_attn_colsum_noalloc": 3, "stac_selftest_bounded_wait": 1,
+    "stac_attn_colsum": 3, "stac_attn_colsum_kept": 3, "stac_attn_colsum_scored": 4, "stac_attn_colsum_noalloc": 3, "stac_selftest_bounded_wait": 1,
     "stac_voxel_hash_clear": 1, "stac_voxel_rehash": 2, "stac_voxel_upsert": 3, "stac_voxel_neighbors": 2, "stac_pointmap_to_positions": 1,
     "stac_append_kv": 1, "stac_qkv_epilogue_append": 1, "stac_qkv_epilogue_append_tables": 1, "stac_scores_update": 1, "stac_h2o_select": 1, "stac_compact": 2, "stac_compact_window": 2, "stac_merge_insert": 11, "stac_retrieve": 2,
 }

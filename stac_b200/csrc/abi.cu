@@ -72,7 +72,8 @@ int attn_colsum_in_workspace(bool zeroed, const void* q, int64_t q_row_stride, c
                      int64_t ret_row_stride, int64_t ret_head_stride, int T_ret, const float* bias_ret, int64_t bias_head_stride, void* out,
                      int64_t out_row_stride, float* lse, float* colsum, int64_t colsum_head_stride, int M, int H,
                      int D, float scale, float subsample_ratio, void* workspace, size_t workspace_bytes,
-                     int* dev_status, stac_stream_t stream) {
+                     int* dev_status, stac_stream_t stream, float* scores = nullptr, float* counts = nullptr,
+                     int64_t score_stride = 0, int old_T = 0, int Tq = 0, float temperature = 0.f) {
   if (q == nullptr || out == nullptr || workspace == nullptr) return STAC_ERR_BAD_ARG;
   if (!(subsample_ratio > 0.f && subsample_ratio <= 1.f)) return STAC_ERR_BAD_ARG;
   if (workspace_bytes < stac_attn_workspace_bytes(M, H)) return STAC_ERR_CAPACITY;
@@ -88,6 +89,8 @@ int attn_colsum_in_workspace(bool zeroed, const void* q, int64_t q_row_stride, c
   a.out = out; a.out_row_stride = out_row_stride;
   a.lse = lse; a.colsum = colsum; a.colsum_head_stride = colsum_head_stride;
   a.M = M; a.H = H; a.D = D; a.scale = scale; a.subsample_ratio = subsample_ratio;
+  a.scores = scores; a.counts = counts; a.score_stride = score_stride;
+  a.old_T = old_T; a.score_Tq = Tq; a.temperature = temperature;
   const size_t lse_bytes = (stac::attn_lse2_elems(M, H) * sizeof(float) + 255) & ~static_cast<size_t>(255);
   float* part = reinterpret_cast<float*>(static_cast<char*>(workspace) + lse_bytes);
   return stac::attn_colsum_launch(a, static_cast<int*>(workspace), zeroed,
@@ -127,6 +130,20 @@ int stac_selftest_bounded_wait(int max_polls, int* dev_status, stac_stream_t str
   if (max_polls <= 0 || dev_status == nullptr) return STAC_ERR_BAD_ARG;
   stac::bounded_wait_selftest_kernel<<<1, 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(max_polls, dev_status);
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
+}
+
+int stac_attn_colsum_scored(const void* q, int64_t q_row_stride, const void* k_hot, const void* v_hot,
+                            int64_t hot_row_stride, int64_t hot_head_stride, int T_hot, const void* k_ret, const void* v_ret,
+                            int64_t ret_row_stride, int64_t ret_head_stride, int T_ret, const float* bias_ret,
+                            int64_t bias_head_stride, void* out, int64_t out_row_stride, float* lse, float* colsum,
+                            int64_t colsum_head_stride, int M, int H, int D, float scale, float subsample_ratio,
+                            float* scores, float* counts, int64_t score_row_stride, int old_T, int Tq, float temperature,
+                            void* workspace, size_t workspace_bytes, int* dev_status, stac_stream_t stream) {
+  if (colsum == nullptr || scores == nullptr || counts == nullptr || old_T < 0 || Tq <= 0) return STAC_ERR_BAD_ARG;
+  return attn_colsum_in_workspace(true, q, q_row_stride, k_hot, v_hot, hot_row_stride, hot_head_stride, T_hot, k_ret, v_ret,
+                                  ret_row_stride, ret_head_stride, T_ret, bias_ret, bias_head_stride, out, out_row_stride,
+                                  lse, colsum, colsum_head_stride, M, H, D, scale, subsample_ratio, workspace,
+                                  workspace_bytes, dev_status, stream, scores, counts, score_row_stride, old_T, Tq, temperature);
 }
 
 }  // extern "C"

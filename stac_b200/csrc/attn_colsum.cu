@@ -1108,6 +1108,14 @@ struct ColParams {
   // an item has at most two parts, added onto the zeroed output with one atomic each.
   float* parts;       // [2 * gridDim.x][kColGroup * kBN]
   int* part_count;    // [n_items], zero on entry, left zero
+  // Running scores that the column sums of the hot keys go into (stac/h2o.py:177-216), or nullptr (no atomics then):
+  // s = colsum * T_hot / Tq; an old key's score decays, score * temperature + s (two roundings, as mul_ then
+  // add_), a new one's is s; counts += 1.
+  float* scores;      // [H, score_stride]
+  float* counts;
+  long long score_stride;
+  int old_T;
+  float tq, temperature;
   int* err;
 };
 
@@ -1453,6 +1461,13 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const int n_half = (rows_here + kColHalf - 1) / kColHalf;
       const int tail = (((rows_here - 1) % kColHalf) / 16 + 1) & 3;    // 4 pieces: a whole half, 0
       const float* nl_item = nl_s + i0 * kBM;
+      // the key's running score, on its way while the rows are summed up
+      const long long score_at = static_cast<long long>(h) * p.score_stride + n0 + key;
+      float old_score = 0.f, old_count = 0.f;
+      if (p.scores != nullptr && !is_ret && key < valid) {
+        old_score = p.scores[score_at];
+        old_count = p.counts[score_at];
+      }
       // (warps whose 32 keys are all masked still run the sums: letting them only follow the
       // score buffers was measured slower in the stream, their polling disturbs the others)
       float sum = warp_fast ? col_item_sum<true>(sm, p, t_base, nl_item, n_half, tail, ui, c2, 0.f)
@@ -1463,22 +1478,30 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (masked) sum = 0.f;
       }
       float* dst = p.colsum + static_cast<long long>(h) * p.colsum_stride + (is_ret ? p.T_hot : 0) + n0 + key;
+      auto finish = [&](float total) {
+        *dst = total;
+        if (p.scores != nullptr && !is_ret) {
+          const float sc = __fdiv_rn(__fmul_rn(total, static_cast<float>(p.T_hot)), p.tq);
+          p.scores[score_at] = n0 + key >= p.old_T ? sc : __fadd_rn(__fmul_rn(old_score, p.temperature), sc);
+          p.counts[score_at] = __fadd_rn(old_count, 1.0f);
+        }
+      };
+      constexpr int kSlot = kColGroup * kBN;
       if (i0 == 0 && i1 == nq) {
-        if (key < valid) *dst = sum;
+        if (key < valid) finish(sum);
       } else if (p.parts == nullptr) {
         if (key < valid) atomicAdd(dst, sum);
       } else {
-        constexpr int kSlot = kColGroup * kBN;
+        // CTA c owns the units [total * c / G, total * (c + 1) / G): owner(u) = ((u + 1) * G - 1) / total
+        const long long total = static_cast<long long>(p.n_items) * nq, G = gridDim.x;
+        const int c_first = static_cast<int>(((static_cast<long long>(item) * nq + 1) * G - 1) / total);
+        const int c_last = static_cast<int>(((static_cast<long long>(item + 1) * nq) * G - 1) / total);
         float* slot = p.parts + static_cast<size_t>(2 * blockIdx.x + (i0 > 0 ? 0 : 1)) * kSlot;
         slot[w * kBN + key] = key < valid ? sum : 0.f;
         __threadfence();                          // this thread's part is visible device-wide ...
         named_bar_sync(1, kColExpThreads);        // ... and so is every other key's
         if (tid == 0) sm.join_flag = atomicAdd(p.part_count + item, 1);
         named_bar_sync(1, kColExpThreads);
-        // CTA c owns the units [total * c / G, total * (c + 1) / G): owner(u) = ((u + 1) * G - 1) / total
-        const long long total = static_cast<long long>(p.n_items) * nq, G = gridDim.x;
-        const int c_first = static_cast<int>(((static_cast<long long>(item) * nq + 1) * G - 1) / total);
-        const int c_last = static_cast<int>(((static_cast<long long>(item + 1) * nq) * G - 1) / total);
         if (sm.join_flag == c_last - c_first) {
           // every other part was complete before its counter increment, which came earlier
           __threadfence();
@@ -1486,7 +1509,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             float acc = 0.f;
             for (int c = c_first; c <= c_last; ++c)
               acc = __fadd_rn(acc, __ldcg(p.parts + static_cast<size_t>(2 * c + (c == c_first ? 1 : 0)) * kSlot + w * kBN + key));
-            *dst = acc;
+            finish(acc);
           }
           if (tid == 0) p.part_count[item] = 0;
         }
@@ -1578,6 +1601,8 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   if (a.M <= 0 || a.H <= 0 || a.T_hot < 0 || a.T_ret < 0 || a.T_hot + a.T_ret <= 0) return STAC_ERR_BAD_ARG;
   if (a.T_ret > 0 && (a.k_ret == nullptr || a.v_ret == nullptr || a.bias_ret == nullptr)) return STAC_ERR_BAD_ARG;
   if (a.T_hot > 0 && (a.k_hot == nullptr || a.v_hot == nullptr)) return STAC_ERR_BAD_ARG;
+  if (a.scores != nullptr && (part == nullptr || a.colsum == nullptr || a.counts == nullptr || a.old_T < 0 || a.score_Tq <= 0))
+    return STAC_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_hot) | reinterpret_cast<uintptr_t>(a.v_hot) |
        reinterpret_cast<uintptr_t>(a.k_ret) | reinterpret_cast<uintptr_t>(a.v_ret) |
        reinterpret_cast<uintptr_t>(a.out)) & 15)
@@ -1677,15 +1702,15 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   const int grid_fast = fp.split ? grid_split : fp.n_items;
   // Column sums: with at least one item per SM the units are cut evenly over one CTA per SM and an
   // item on a cut gets one atomic add per key from each of its two CTAs (the forward kernel clears
-  // the output for that).  With fewer items (few heads, short key ranges) and a workspace, the
-  // units are still cut evenly; an item may then have three or more parts, which go through the
-  // workspace and are added in CTA order by the CTA that finishes last.
+  // the output for that; a join through the workspace took 1 to 2 us more per call).  With fewer items (few heads,
+  // short key ranges) and a workspace, the units are still cut evenly; an item may then have three or more parts,
+  // which go through the workspace and are added in CTA order by the CTA that finishes last.
   const int col_items = ((fp.n_hot_tiles + fp.n_ret_tiles + kColGroup - 1) / kColGroup) * a.H;
   const bool col_split = a.colsum != nullptr && col_items >= n_sm;
   // (worth it from about six units per CTA: below that the extra key-tile loads and the join of a
   // CTA that touches two items cost more than the even cut gains; measured at M = 1041, N = 2082)
   const bool col_parts = a.colsum != nullptr && !col_split && part != nullptr && n_sm <= kFastMaxCtas &&
-                         static_cast<long long>(col_items) * ((m_sub + kBM - 1) / kBM) >= 6ll * n_sm;
+                         static_cast<long long>(col_items) * nq >= 6ll * n_sm;
   // Every call leaves the control words as it found them, so a workspace that was zeroed once needs no
   // clearing: one memset less per call, and the forward kernel follows the kernel before it directly
   // (M = 1041, N = 2082, H = 16: 42.5 -> 38.2 us per call).
@@ -1716,15 +1741,19 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     cp.lse2 = lse2; cp.lse2_stride = a.M;
     cp.colsum = a.colsum; cp.colsum_stride = a.colsum_head_stride;
     cp.err = err;
-    // enough items: cut the units evenly over one CTA per SM (an item is then shared by at most
-    // two CTAs, which add their partial sums onto zeros); else one item per CTA
     cp.split = (col_split || col_parts) ? 1 : 0;      // col_split: the forward kernel has cleared a.colsum
     cp.parts = col_parts ? part + kFwdPartElems : nullptr;
+    // running scores: updated by the thread that has a key's final sum; where atomics make it, by a launch behind
+    cp.scores = col_split ? nullptr : a.scores; cp.counts = a.counts; cp.score_stride = a.score_stride;
+    cp.old_T = a.old_T; cp.tq = static_cast<float>(a.score_Tq); cp.temperature = a.temperature;
     cp.part_count = ctl + kCtlColItems;
     const int grid_c = cp.split ? n_sm : cp.n_items;
     if (launch_behind(attn_colsum_kernel, dim3(grid_c), dim3(kColThreads), col_smem, stream, tm_qs, tm_kh, tm_kr,
                       cp) != cudaSuccess)
       return STAC_ERR_CUDA;
+    if (col_split && a.scores != nullptr)
+      return stac_scores_update(a.colsum, a.colsum_head_stride, a.scores, a.counts, a.score_stride, a.H, a.T_hot, a.old_T,
+                                a.score_Tq, a.temperature, reinterpret_cast<stac_stream_t>(stream));
   }
   return STAC_OK;
 }

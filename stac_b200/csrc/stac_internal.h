@@ -33,6 +33,12 @@ struct AttnArgs {
   int M, H, D;
   float scale;
   float subsample_ratio;
+  // running scores that the column sums of the hot keys go into, or nullptr (needs `colsum` and `part`)
+  float* scores = nullptr;  // [H, score_stride]
+  float* counts = nullptr;
+  long long score_stride = 0;
+  int old_T = 0, score_Tq = 0;
+  float temperature = 0.f;
 };
 
 // Ordinal of the current device (checked against kMaxDevices) / its SM count, cached per device.

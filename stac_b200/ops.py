@@ -103,9 +103,10 @@ def _kv_strides(t, layout):
 
 def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T_ret=0, *,
                 layout="htd", scale=None, subsample_ratio=1.0, want_lse=False, want_colsum=True,
-                out=None, colsum=None, status=None):
+                out=None, colsum=None, status=None, score_update=None):
     """q [M,H,64] bf16 (row stride arbitrary); hot and retrieved keys/values in ``layout``;
-    bias_ret [H, >=T_ret] fp32.  Returns (out [M,H,64] bf16, lse [H,M] | None,
+    bias_ret [H, >=T_ret] fp32.  ``score_update``: (scores, counts, row stride, old_T, Tq, temperature), the
+    running scores of the hot keys that the column sums go into.  Returns (out [M,H,64] bf16, lse [H,M] | None,
     colsum [H, T_hot+T_ret] fp32 | None)."""
     assert q.is_cuda and q.dtype == torch.bfloat16 and q.dim() == 3 and q.stride(2) == 1
     M, H, D = q.shape
@@ -130,15 +131,19 @@ def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T
         assert bias_ret.dtype == torch.float32 and bias_ret.stride(1) == 1
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    st = _lib.lib().stac_attn_colsum_kept(
-        ptr(q), q.stride(0),
-        ptr(k_hot) if T_hot > 0 else None, ptr(v_hot) if T_hot > 0 else None, hr, hh, T_hot,
-        ptr(k_ret) if T_ret > 0 else None, ptr(v_ret) if T_ret > 0 else None, rr, rh, T_ret,
-        ptr(bias_ret) if T_ret > 0 else None, bias_ret.stride(0) if T_ret > 0 else 0,
-        ptr(out), out.stride(0), ptr(lse), ptr(colsum), colsum.stride(0) if colsum is not None else 0,
-        M, H, D, float(scale), float(subsample_ratio), ptr(ws), ws.numel() * 4,
-        ptr(status.word) if status is not None else None, stream_ptr())
-    check(st, "stac_attn_colsum_kept")
+    call = [ptr(q), q.stride(0),
+            ptr(k_hot) if T_hot > 0 else None, ptr(v_hot) if T_hot > 0 else None, hr, hh, T_hot,
+            ptr(k_ret) if T_ret > 0 else None, ptr(v_ret) if T_ret > 0 else None, rr, rh, T_ret,
+            ptr(bias_ret) if T_ret > 0 else None, bias_ret.stride(0) if T_ret > 0 else 0,
+            ptr(out), out.stride(0), ptr(lse), ptr(colsum), colsum.stride(0) if colsum is not None else 0,
+            M, H, D, float(scale), float(subsample_ratio)]
+    name = "stac_attn_colsum_kept"
+    if score_update is not None:
+        scores, counts, row_stride, old_T, Tq, temperature = score_update
+        call += [ptr(scores), ptr(counts), row_stride, old_T, Tq, float(temperature)]
+        name = "stac_attn_colsum_scored"
+    check(getattr(_lib.lib(), name)(*call, ptr(ws), ws.numel() * 4, ptr(status.word) if status is not None else None,
+                                    stream_ptr()), name)
     return out, lse, colsum
 
 

@@ -89,10 +89,21 @@ class HeavyHittersKV(KVManager):
     def decode_sparse_attn(self, query_states: torch.Tensor, layer_idx: int) -> torch.Tensor:
         """query_states [B, Tq, H, D] -> [B, Tq, H, D]; updates the hot scores (stac/h2o.py:139-174)."""
         slot = self._to_slot(layer_idx)
-        out, colsum = self._attend(query_states, slot, want_colsum=True, subsample_ratio=self.subsample_ratio)
-        self._last_query_offset[slot] = query_states.shape[1]
-        self._update_scores_dev(colsum, colsum.stride(0), self._offset_hot[slot], slot)
-        return out
+        return self._attend_and_score(query_states, slot)[0]
+
+    def _attend_and_score(self, query_states, slot, *retrieved):
+        """Attention whose column sums go into the running scores of the hot keys in the same call: in the kernel
+        that makes them where the heads are few (24 layers, 2 heads: 2911 -> 2870 us per step)."""
+        Tq, T_live = query_states.shape[1], self._offset_hot[slot]
+        update = None
+        if T_live > 0:
+            update = (self._scores_hot[slot], self._scores_hot_count[slot], self.reserved_buffer_token_size,
+                      self._last_score_offset[slot], Tq, self.temperature)
+        res = self._attend(query_states, slot, *retrieved, want_colsum=True, subsample_ratio=self.subsample_ratio,
+                           score_update=update)
+        self._last_query_offset[slot] = Tq
+        self._last_score_offset[slot] = T_live
+        return res
 
     def _update_scores_dev(self, colsum, head_stride, T_live, slot):
         old_T = self._last_score_offset[slot]

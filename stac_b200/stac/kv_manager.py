@@ -358,7 +358,7 @@ class KVManager:
 
     # ------------------------------------------------------------------ attention
     def _attend(self, query_states, slot, k_ret=None, v_ret=None, bias_ret=None, T_ret=0,
-                want_colsum=False, subsample_ratio=1.0):
+                want_colsum=False, subsample_ratio=1.0, score_update=None):
         B, Tq, H, D = query_states.shape
         assert H == self.num_heads and D == self.head_dim, "Incompatible head or head_dim."
         assert B == 1, "Batch size > 1 not supported in decode_sparse_attn()."
@@ -373,7 +373,7 @@ class KVManager:
         T_main = self._offset_hot[slot]
         out, _, colsum = ops.attn_colsum(q, self.key_cache_hot[slot], self.value_cache_hot[slot], T_main,
                                          k_ret, v_ret, bias_ret, T_ret, subsample_ratio=subsample_ratio,
-                                         want_colsum=want_colsum, status=self._status)
+                                         want_colsum=want_colsum, status=self._status, score_update=score_update)
         out = out.unsqueeze(0)
         return (out if out_dtype == torch.bfloat16 else out.to(out_dtype)), colsum
 

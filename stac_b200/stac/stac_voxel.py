@@ -156,10 +156,7 @@ class STACVoxelKV(HeavyHittersKV):
             k_ret = self.key_cache_retrieval[slot]
             v_ret = self.value_cache_retrieval[slot]
             b_ret = self._bias_retrieval[slot]
-        out, colsum = self._attend(query_states, slot, k_ret, v_ret, b_ret, T_ret, want_colsum=True,
-                                   subsample_ratio=self.subsample_ratio)
-        self._last_query_offset[slot] = query_states.shape[1]
-        self._update_scores_dev(colsum, colsum.stride(0), T_main, slot)
+        out, colsum = self._attend_and_score(query_states, slot, k_ret, v_ret, b_ret, T_ret)
         if T_ret > 0:
             self._scores_retrieval[slot] = colsum[:, T_main:T_main + T_ret]
         return out

@@ -404,3 +404,34 @@ def test_ragged_last_query_tile(M, H, T_hot, T_ret):
     for shift in (0.0, -40.0):
         got, ref = _run_two_segment(M, H, T_hot, T_ret, seed=M, bias_shift=shift)
         _assert_close(got, ref)
+
+
+@pytest.mark.parametrize("M,H,T_hot,T_ret,old_T,ratio", [
+    (130, 2, 300, 90, 170, 1.0),          # one CTA per item: updated by the kernel
+    (1041, 16, 3400, 140, 2359, 1.0),     # items shared by two CTAs: by a launch behind it
+    (2600, 3, 6000, 0, 0, 1.0),           # by three and more: by the CTA that joins them
+    (900, 5, 1500, 260, 1500, 0.25),      # rows left out; no new key
+])
+def test_scores_updated_by_the_column_sum_kernel(M, H, T_hot, T_ret, old_T, ratio):
+    """The running scores and counts get the bits that the update behind the call gives; the other outputs, the keys
+    behind the live ones and the retrieved keys are left alone."""
+    from stac_b200 import _lib, ops
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(M + H)
+    q, k, v = (torch.randn(*shape, generator=g).to(torch.bfloat16).to(dev) for shape in
+               ((M, H, 64), (H, T_hot + 37, 64), (H, T_hot + 37, 64)))
+    kr, vr = (torch.randn(H, max(T_ret, 1), 64, generator=g).to(torch.bfloat16).to(dev) for _ in range(2))
+    br = torch.log(torch.randint(1, 9, (H, max(T_ret, 1)), generator=g).float()).to(dev)
+    ret = (kr, vr, br, T_ret) if T_ret else (None, None, None, 0)
+    width = T_hot + 50
+    scores, counts = (torch.rand(H, width, generator=g).to(dev) for _ in range(2))
+    want_s, want_c = scores.clone(), counts.clone()
+    out, lse, cs = ops.attn_colsum(q, k, v, T_hot, *ret, want_lse=True, subsample_ratio=ratio)
+    rc = _lib.lib().stac_scores_update(_lib.ptr(cs), cs.stride(0), _lib.ptr(want_s), _lib.ptr(want_c), width, H, T_hot, old_T,
+                                       M, 0.9, _lib.stream_ptr())
+    assert rc == 0
+    for _ in range(2):        # the second call finds the workspace as the first one leaves it
+        s2, c2 = scores.clone(), counts.clone()
+        got = ops.attn_colsum(q, k, v, T_hot, *ret, want_lse=True, subsample_ratio=ratio, score_update=(s2, c2, width, old_T, M, 0.9))
+        assert all(torch.equal(a, b) for a, b in zip(got, (out, lse, cs)))
+        assert torch.equal(s2, want_s) and torch.equal(c2, want_c)
