@@ -440,18 +440,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // The probabilities go back into the columns their scores came from (bf16, two per column) and feed
 // the P V MMA as its A operand straight from tensor memory.
 //
-// What bounds the kernel beside the exponentials: a tile costs 361 + 7.3 x keys cycles per SM whatever the
-// exponentials cost (96 and 112 keys, 16 384-score loops alone take the 7.3), and the 361 are the warps that
-// issue and load, which share their schedulers with the softmax warps: an instruction takes them 6 to 8
-// cycles, a wait on a barrier that is already complete 75 to 110.  So ONE warp issues both MMA streams: P V
-// of a tile and, right behind it, Q K^T of the tile that takes over its buffer (the tensor pipe keeps the
-// order of a thread's MMAs, so there is no barrier between them), with the operands of both behind one
-// barrier, one commit per tile, and a loop without bookkeeping.  (Two warps, one per stream, with rings of
-// their own: 583 against 569 thousand cycles at 4164 x 17697 keys, 93.0 against 90.0 at 1041 x 9369; the card runs
-// these loops at its power limit, 1.6 to 1.8 GHz, so 1 to 3 % of the time.  Measured and not taken: three
-// softmax warpgroups with probabilities in columns of their own, 96-key tiles, 10 % slower; two issuing warps, one
-// per accumulator for even and odd tiles, 96-key tiles, 1 to 3 % slower; larger FMA shares of the
-// exponentials, fewer cycles but no less time.)
+// The scores of tile c + kFastWgs overwrite the probabilities of tile c, which P V reads.  tcgen05.mma instructions
+// are only ordered among themselves where they have the accumulator and the shape in common, and these two have neither, so
+// the warp that issues Q K^T waits for the commit of that P V: a warp each for the two streams, because a single warp that
+// waits between them leaves the tensor pipe idle (M = 1041, N = 2082 38.1 against 37.1 us per call, M = 2000, N = 900 58.4
+// against 55.8).  The warps that issue and load share their schedulers with the softmax warps, so their loops hold little
+// beside the waits.  (One warp that issues both without a wait in between gave the same bits and took 0.4 to
+// 1.5 % less of this kernel's time at 9369 keys and more, 2 % with a bias on every key, but relied on an order that is
+// observed and not documented.  Measured and not taken: three softmax warpgroups with
+// probabilities in columns of their own, 96-key tiles, 10 % slower; larger FMA shares of the exponentials, no less time.)
 //
 // Work = items (head, 128-row query tile) x key tiles.  With enough items the kernel runs one
 // CTA per SM and cuts that unit sequence into equal contiguous ranges (no partly filled last
@@ -465,11 +462,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // partial row sums are double buffered by segment parity, and so are the barriers that several warpgroups
 // arrive on per segment: a warpgroup without a tile in a short first or last segment runs one segment ahead,
 // never two (a CTA's middle segments are whole items of at least kFastMinSplitTiles tiles: the scores of a
-// warpgroup's last tile there are issued behind a P V of that segment, whose first one waits until the
+// warpgroup's last tile there wait for a P V of that segment, whose first one waits until the
 // accumulator of the segment before has been read out).
 // ---------------------------------------------------------------------------------------
 constexpr int kFastWgs = 4;                     // softmax warpgroups; key tile c goes to warpgroup and score buffer c % kFastWgs
-constexpr int kFastThreads = 128 + 128 * kFastWgs;   // warpgroup 0 control (warp 0 TMA, warp 1 MMA issue), then softmax
+constexpr int kFastThreads = 128 + 128 * kFastWgs;   // warpgroup 0 control (warp 0 TMA, warps 1 and 2 MMA issue), then softmax
 constexpr int kFT = 112;                        // keys per tile: three chunks of 32 and one of 16
 static_assert(kFT % 32 == 16 && kFT <= kBN && kFastWgs * kFT + kD <= 512, "tensor memory");
 constexpr int kFastTileBytes = kFT * 128;       // kFT rows x 64 bf16
@@ -498,9 +495,11 @@ struct FastSmem {
   int live[2][kFastWgs - 1];                    // did warpgroup 1.. see a key that is not masked (segment parity)
   uint64_t q_full[2];
   uint64_t q_empty[2];
-  uint64_t kv_full[kFastWgs];
+  uint64_t k_full[kFastWgs];
+  uint64_t v_full[kFastWgs];
   uint64_t s_full[kFastWgs];     // scores of a tile are in TMEM; the stage that its keys came from is free again
   uint64_t p_full[kFastWgs];     // its probabilities are in TMEM
+  uint64_t pv_done[kFastWgs];    // the P V MMAs that read them are done: scores may overwrite them
   uint64_t ref_ready[2];
   uint64_t l_ready[2];           // warpgroups 1.. have published their row sums of the segment (parity)
   uint64_t o_done;               // all P V MMAs of the segment are complete
@@ -612,9 +611,11 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
     mbar_init(&sm.o_done, 1);
     for (int b = 0; b < kFastWgs; ++b) {
-      mbar_init(&sm.kv_full[b], 1);
+      mbar_init(&sm.k_full[b], 1);
+      mbar_init(&sm.v_full[b], 1);
       mbar_init(&sm.s_full[b], 1);
       mbar_init(&sm.p_full[b], 128);
+      mbar_init(&sm.pv_done[b], 1);
     }
     mbar_init(&sm.o_free, 128);
     mbar_fence_init();
@@ -661,7 +662,8 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           h_v = item_v / p.n_q_tiles;
         }
         const bool hot = j_v < n_hot;
-        tma_load_3d(sm.v[b], hot ? &tm_v_hot : &tm_v_ret, &sm.kv_full[b], 0, (hot ? j_v : j_v - n_hot) * kFT, h_v);
+        mbar_arrive_expect_tx(&sm.v_full[b], kFastTileBytes);
+        tma_load_3d(sm.v[b], hot ? &tm_v_hot : &tm_v_ret, &sm.v_full[b], 0, (hot ? j_v : j_v - n_hot) * kFT, h_v);
         ++j_v;
       };
       auto next_stage = [&]() {
@@ -678,8 +680,8 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const bool hot = j < n_hot;
           const bool with_v = c >= kFastWgs;
           if (with_v) mbar_wait(&sm.s_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
-          mbar_arrive_expect_tx(&sm.kv_full[b], with_v ? 2 * kFastTileBytes : kFastTileBytes);
-          tma_load_3d(sm.k[b], hot ? &tm_k_hot : &tm_k_ret, &sm.kv_full[b], 0, (hot ? j : j - n_hot) * kFT, h);
+          mbar_arrive_expect_tx(&sm.k_full[b], kFastTileBytes);
+          tma_load_3d(sm.k[b], hot ? &tm_k_hot : &tm_k_ret, &sm.k_full[b], 0, (hot ? j : j - n_hot) * kFT, h);
           if (with_v) load_v();
           next_stage();
         }
@@ -688,111 +690,77 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       for (int e = 0; e < kFastWgs; ++e) {
         if (c >= kFastWgs) {
           mbar_wait(&sm.s_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
-          mbar_arrive_expect_tx(&sm.kv_full[b], kFastTileBytes);
           load_v();
         }
         next_stage();
       }
     } else if (warp == 1) {
-      // ---------------------------------------------------------------- MMA issuer
-      // Step u: O += P V of tile u - kFastWgs, whose probabilities lie where tile u's scores go, and right
-      // behind it S = Q K^T of tile u.  The tensor pipe works through the MMAs of a thread in order, so
-      // nothing has to be waited for in between, one barrier per stage covers the operands of both, and one
-      // commit tells the warpgroup that its scores are there and the producer that the stage is free.
-      // This warp shares its scheduler with softmax warps and gets 6 to 8 cycles per instruction: the
-      // steps inside a segment run in a loop of their own without any bookkeeping.
+      // ---------------------------------------------------------------- MMA issuer: S = Q K^T
       // (all lanes run the loop, one elected lane issues)
       constexpr uint32_t idesc_s = umma_idesc_bf16(kBM, kFT, 0);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(kBM, kD, 1);
       const uint64_t q_desc0 = smem_desc_sw128(smem_u32(sm.q[0]));
       const uint64_t k_desc0 = smem_desc_sw128(smem_u32(sm.k[0]));
-      const uint64_t v_desc0 = smem_desc_sw128(smem_u32(sm.v[0]));
-      uint64_t q_desc = q_desc0;
-      uint32_t b = 0, par = 1;     // stage and buffer of step u, phase of their previous use
-      auto issue_pv = [&](uint32_t sc, uint64_t vd, uint32_t acc) {
-        // A: 16 keys = 8 columns of packed probabilities; B: V advances 16 rows = 2048 bytes
-        umma_ts(o_tmem, sc, vd, idesc_o, acc);
-#pragma unroll
-        for (int kk = 1; kk < kFT / 16; ++kk)
-          umma_ts(o_tmem, sc + kk * 8, vd + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_o, 1u);
-      };
-      auto issue_s = [&](uint32_t sc, uint64_t kd) {
-        umma_ss(sc, q_desc, kd, idesc_s, 0u);
-        umma_ss(sc, q_desc + 2, kd + 2, idesc_s, 1u);
-        umma_ss(sc, q_desc + 4, kd + 4, idesc_s, 1u);
-        umma_ss(sc, q_desc + 6, kd + 6, idesc_s, 1u);
-      };
-      auto next_step = [&]() {
-        if (++b == kFastWgs) { b = 0; par ^= 1; }
-      };
-      // steps at the edges of segments; the P V cursor walks the segments behind the scores
-      FwdWalk walk_v(p, n_tiles);
-      int v_seg = -1, v_left = 0, v_item, v_t0, v_t1, u = 0;
-      auto edge_step = [&](bool with_s) {
-        const uint32_t sc = tmem + b * kFT;
-        const uint64_t off = static_cast<uint64_t>(b * (kFastTileBytes >> 4));
-        const bool with_v = u >= kFastWgs;
-        bool first_o = false;
-        if (with_v && v_left == 0) {
-          walk_v.next(v_item, v_t0, v_t1);
-          v_left = v_t1 - v_t0;
-          ++v_seg;
-          first_o = true;
-        }
-        if (with_s || with_v) {
-          mbar_wait(&sm.kv_full[b], par ^ 1, p.err, DEV_TIMEOUT_TMA);
-          if (with_v) {
-            mbar_wait(&sm.p_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
-            // a new segment overwrites the accumulator: the previous one must have been read out
-            if (first_o && v_seg > 0) mbar_wait(&sm.o_free, (v_seg - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-            --v_left;
-          }
+      FwdWalk walk(p, n_tiles);
+      int item, t0, t1;
+      uint32_t b = 0, par = 1;     // stage and buffer of the tile, phase of their previous use
+      bool reused = false;         // a buffer's first scores overwrite nothing
+      for (int seg = 0; walk.next(item, t0, t1); ++seg) {
+        const int qb = seg & 1;
+        const uint64_t q_desc = q_desc0 + static_cast<uint64_t>(qb * (kTileBytes >> 4));
+        mbar_wait(&sm.q_full[qb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_TMA);
+#pragma unroll 1
+        for (int j = t0; j < t1; ++j) {
+          const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(b * (kFastTileBytes >> 4));
+          const uint32_t d = tmem + b * kFT;
+          mbar_wait(&sm.k_full[b], par ^ 1, p.err, DEV_TIMEOUT_TMA);
+          if (reused) mbar_wait(&sm.pv_done[b], par, p.err, DEV_TIMEOUT_CONSUMER);
           tc_fence_after();
           if (elect_one()) {
-            if (with_v) {
-              issue_pv(sc, v_desc0 + off, first_o ? 0u : 1u);
-              if (v_left == 0) umma_commit(&sm.o_done);
-            }
-            if (with_s) issue_s(sc, k_desc0 + off);
+            umma_ss(d, q_desc, k_desc, idesc_s, 0u);
+            umma_ss(d, q_desc + 2, k_desc + 2, idesc_s, 1u);
+            umma_ss(d, q_desc + 4, k_desc + 4, idesc_s, 1u);
+            umma_ss(d, q_desc + 6, k_desc + 6, idesc_s, 1u);
             umma_commit(&sm.s_full[b]);
           }
           __syncwarp();
-        }
-        ++u;
-        next_step();
-      };
-      FwdWalk walk(p, n_tiles);
-      int item, t0, t1;
-      for (int seg = 0; walk.next(item, t0, t1); ++seg) {
-        const int n = t1 - t0, qb = seg & 1;
-        mbar_wait(&sm.q_full[qb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_TMA);
-        q_desc = q_desc0 + static_cast<uint64_t>(qb * (kTileBytes >> 4));
-        // scores beside the last P V of the previous segment, then the first P V of this one
-        for (int e = 0; e < min(n, kFastWgs + 1); ++e) edge_step(true);
-        const int more = n - (kFastWgs + 1);
-        if (more > 0) {
-          u += more;
-          v_left -= more;
-#pragma unroll 1
-          for (int e = 0; e < more; ++e) {
-            const uint32_t sc = tmem + b * kFT;
-            const uint64_t off = static_cast<uint64_t>(b * (kFastTileBytes >> 4));
-            mbar_wait(&sm.kv_full[b], par ^ 1, p.err, DEV_TIMEOUT_TMA);
-            mbar_wait(&sm.p_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
-            tc_fence_after();
-            if (elect_one()) {
-              issue_pv(sc, v_desc0 + off, 1u);
-              issue_s(sc, k_desc0 + off);
-              umma_commit(&sm.s_full[b]);
-            }
-            __syncwarp();
-            next_step();
-          }
+          if (++b == kFastWgs) { b = 0; par ^= 1; reused = true; }
         }
         if (elect_one()) umma_commit(&sm.q_empty[qb]);
         __syncwarp();
       }
-      for (int e = 0; e < kFastWgs; ++e) edge_step(false);
+    } else if (warp == 2) {
+      // ---------------------------------------------------------------- MMA issuer: O += P V
+      constexpr uint32_t idesc_o = umma_idesc_bf16(kBM, kD, 1);
+      const uint64_t v_desc0 = smem_desc_sw128(smem_u32(sm.v[0]));
+      FwdWalk walk(p, n_tiles);
+      int item, t0, t1;
+      uint32_t b = 0, par = 0;     // stage and buffer of the tile, their phase
+      for (int seg = 0; walk.next(item, t0, t1); ++seg) {
+        uint32_t acc = 0u;
+#pragma unroll 1
+        for (int j = t0; j < t1; ++j) {
+          // A: 16 keys = 8 columns of packed probabilities; B: V advances 16 rows = 2048 bytes
+          const uint32_t pa = tmem + b * kFT;
+          const uint64_t v_desc = v_desc0 + static_cast<uint64_t>(b * (kFastTileBytes >> 4));
+          mbar_wait(&sm.v_full[b], par, p.err, DEV_TIMEOUT_TMA);
+          mbar_wait(&sm.p_full[b], par, p.err, DEV_TIMEOUT_CONSUMER);
+          // a new segment overwrites the accumulator: the previous one must have been read out
+          if (acc == 0u && seg > 0) mbar_wait(&sm.o_free, (seg - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
+          tc_fence_after();
+          if (elect_one()) {
+            umma_ts(o_tmem, pa, v_desc, idesc_o, acc);
+#pragma unroll
+            for (int kk = 1; kk < kFT / 16; ++kk)
+              umma_ts(o_tmem, pa + kk * 8, v_desc + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_o, 1u);
+            umma_commit(&sm.pv_done[b]);
+          }
+          __syncwarp();
+          acc = 1u;
+          if (++b == kFastWgs) { b = 0; par ^= 1; }
+        }
+        if (elect_one()) umma_commit(&sm.o_done);
+        __syncwarp();
+      }
     }
   } else {
     // ------------------------------------------------------------------ softmax warpgroups
