@@ -140,6 +140,8 @@ int stac_attn_colsum_scored(const void* q, int64_t q_row_stride, const void* k_h
                             float* scores, float* counts, int64_t score_row_stride, int old_T, int Tq, float temperature,
                             void* workspace, size_t workspace_bytes, int* dev_status, stac_stream_t stream) {
   if (colsum == nullptr || scores == nullptr || counts == nullptr || old_T < 0 || Tq <= 0) return STAC_ERR_BAD_ARG;
+  // rows of different heads that overlap would be written by several CTAs at once
+  if (H > 1 && score_row_stride < T_hot) return STAC_ERR_BAD_ARG;
   return attn_colsum_in_workspace(true, q, q_row_stride, k_hot, v_hot, hot_row_stride, hot_head_stride, T_hot, k_ret, v_ret,
                                   ret_row_stride, ret_head_stride, T_ret, bias_ret, bias_head_stride, out, out_row_stride,
                                   lse, colsum, colsum_head_stride, M, H, D, scale, subsample_ratio, workspace,

@@ -101,12 +101,20 @@ def _kv_strides(t, layout):
     return t.stride(0), t.stride(1)
 
 
+def _check_score_update(scores, counts, row_stride, H, T_hot, device):
+    """The kernel writes [H, T_hot] fp32 scores and counts at ``row_stride`` and is given pointers only."""
+    for t in (scores, counts):
+        assert t.dtype == torch.float32 and t.device == device, "running scores and counts: fp32 on the queries' device"
+        assert t.dim() == 2 and t.shape[0] == H and t.shape[1] >= T_hot, "running scores and counts: [H, >= T_hot]"
+        assert t.stride() == (row_stride, 1) and (H == 1 or row_stride >= T_hot), "running scores and counts: strides"
+
+
 def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T_ret=0, *,
                 layout="htd", scale=None, subsample_ratio=1.0, want_lse=False, want_colsum=True,
                 out=None, colsum=None, status=None, score_update=None):
     """q [M,H,64] bf16 (row stride arbitrary); hot and retrieved keys/values in ``layout``;
     bias_ret [H, >=T_ret] fp32.  ``score_update``: (scores, counts, row stride, old_T, Tq, temperature), the
-    running scores of the hot keys that the column sums go into.  Returns (out [M,H,64] bf16, lse [H,M] | None,
+    running scores [H, >=T_hot] fp32 of the hot keys that the column sums go into.  Returns (out [M,H,64] bf16, lse [H,M] | None,
     colsum [H, T_hot+T_ret] fp32 | None)."""
     assert q.is_cuda and q.dtype == torch.bfloat16 and q.dim() == 3 and q.stride(2) == 1
     M, H, D = q.shape
@@ -140,6 +148,7 @@ def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T
     name = "stac_attn_colsum_kept"
     if score_update is not None:
         scores, counts, row_stride, old_T, Tq, temperature = score_update
+        _check_score_update(scores, counts, row_stride, H, T_hot, dev)
         call += [ptr(scores), ptr(counts), row_stride, old_T, Tq, float(temperature)]
         name = "stac_attn_colsum_scored"
     check(getattr(_lib.lib(), name)(*call, ptr(ws), ws.numel() * 4, ptr(status.word) if status is not None else None,

@@ -258,6 +258,33 @@ def test_no_grad_wrapper_restores_the_mode():
             assert torch.is_grad_enabled() is before
 
 
+def test_running_scores_are_checked_before_their_pointers_are_used():
+    """Rows that overlap are refused by the C entry, and tensors that do not hold what the kernel writes by the caller."""
+    import torch
+    from stac_b200 import _lib, ops
+    H, M, T = 2, 128, 300
+    need = _lib.lib().stac_attn_workspace_bytes(M, H)
+    p = 1 << 20                                   # aligned; nothing is read before the arguments are checked
+
+    def call(stride):
+        return _lib.lib().stac_attn_colsum_scored(p, H * 64, p, p, 64, T * 64, T, None, None, 64, 64, 0, None, 0, p, H * 64,
+                                                  None, p, T, M, H, 64, 0.125, 1.0, p, p, stride, 0, M, 0.9, p, need,
+                                                  None, None)
+    assert call(T - 1) == 1 and call(0) == 1      # STAC_ERR_BAD_ARG
+    dev = torch.device("cpu")
+    good = torch.zeros(H, T + 5)
+    ops._check_score_update(good, good.clone(), T + 5, H, T, dev)
+    ops._check_score_update(good[:, :T], good[:, :T], T + 5, H, T, dev)
+    bad = [good.double(), good.half(), good.to("meta"), good[:1], good[:, :T - 1], good.t().contiguous().t(),
+           torch.zeros(1, T + 5).expand(H, T + 5), good.flatten()]
+    for t in bad:
+        for pair in ((t, good), (good, t)):
+            with pytest.raises(AssertionError):
+                ops._check_score_update(*pair, T + 5, H, T, dev)
+    with pytest.raises(AssertionError):
+        ops._check_score_update(good, good, T, H, T, dev)
+
+
 def test_captured_calls_have_a_workspace_of_their_own(monkeypatch):
     """The workspace kept for eager calls of a stream is not handed to a call that is captured on it (the
     graph would outlive it, and would run beside eager calls), nor one of a capture to an eager call."""
