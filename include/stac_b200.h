@@ -45,6 +45,10 @@ const char* stac_status_string(int status);
 /* Library/ABI version, bumped when a signature changes. */
 int stac_abi_version(void);
 
+/* Kernels that this library has launched in this process so far (a launch into a graph capture counts once, replays
+ * don't). */
+uint64_t stac_kernel_launches(void);
+
 /* ---------------------------------------------------------------------------------------
  * Window + pivot attention with per-key softmax column sums.
  *

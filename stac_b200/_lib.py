@@ -56,6 +56,7 @@ ERR_CAPACITY = 3           # STAC_ERR_CAPACITY
 SIGNATURES = {
     "stac_status_string": (ctypes.c_char_p, [c_int]),
     "stac_abi_version": (c_int, []),
+    "stac_kernel_launches": (ctypes.c_uint64, []),
     "stac_attn_workspace_bytes": (c_size_t, [c_int, c_int]),
     "stac_attn_colsum": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_i64, c_int, c_void_p, c_void_p,
                                  c_i64, c_i64, c_int, c_void_p, c_i64, c_void_p, c_i64, c_void_p, c_void_p, c_i64,
@@ -103,38 +104,10 @@ SIGNATURES = {
                               c_void_p, c_void_p, c_void_p, c_void_p]),
 }
 
-# kernels launched by one call of each entry point (the upper figure where it depends on arguments);
-# used to report how many of this library's kernels ran in a timed region
-# (stac_attn_colsum: fast forward, exact forward, column sums)
-KERNELS_PER_CALL = {
-    "stac_attn_colsum": 3, "stac_attn_colsum_kept": 3, "stac_attn_colsum_scored": 4, "stac_attn_colsum_noalloc": 3, "stac_selftest_bounded_wait": 1,
-    "stac_voxel_hash_clear": 1, "stac_voxel_rehash": 2, "stac_voxel_upsert": 3, "stac_voxel_neighbors": 2, "stac_pointmap_to_positions": 1,
-    "stac_append_kv": 1, "stac_qkv_epilogue_append": 1, "stac_qkv_epilogue_append_tables": 1, "stac_scores_update": 1, "stac_h2o_select": 1, "stac_compact": 2, "stac_compact_window": 2, "stac_merge_insert": 11, "stac_retrieve": 2,
-}
-CALLS = {}
-
-
-class _CountingLib:
-    """Forwards to the ctypes handle and counts calls per entry point."""
-
-    def __init__(self, handle):
-        self._handle = handle
-
-    def __getattr__(self, name):
-        fn = getattr(self._handle, name)
-        if name not in KERNELS_PER_CALL:
-            return fn
-
-        def counted(*args):
-            CALLS[name] = CALLS.get(name, 0) + 1
-            return fn(*args)
-        self.__dict__[name] = counted
-        return counted
-
 
 def kernel_launches():
-    """Kernels of this library launched so far (by the entry-point calls made through lib())."""
-    return sum(KERNELS_PER_CALL[n] * c for n, c in CALLS.items())
+    """Kernels that the library has launched so far, counted where they are launched."""
+    return lib().stac_kernel_launches()
 
 
 _lib = None
@@ -155,7 +128,7 @@ def lib():
             fn = getattr(handle, name)
             fn.restype = res
             fn.argtypes = args
-        _lib = _CountingLib(handle)
+        _lib = handle
     return _lib
 
 

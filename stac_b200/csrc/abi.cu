@@ -56,6 +56,8 @@ const char* stac_status_string(int status) {
 
 int stac_abi_version(void) { return 2; }
 
+uint64_t stac_kernel_launches(void) { return stac::g_kernel_launches.load(std::memory_order_relaxed); }
+
 size_t stac_attn_workspace_bytes(int M, int H) {
   if (M <= 0 || H <= 0) return 0;
   // control words and row log-sum-exps (rounded up to 256 bytes), then the partial results
@@ -129,7 +131,7 @@ int stac_attn_colsum_kept(const void* q, int64_t q_row_stride, const void* k_hot
 int stac_selftest_bounded_wait(int max_polls, int* dev_status, stac_stream_t stream) {
   if (max_polls <= 0 || dev_status == nullptr) return STAC_ERR_BAD_ARG;
   stac::bounded_wait_selftest_kernel<<<1, 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(max_polls, dev_status);
-  return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
+  return stac::count_launch(cudaGetLastError()) == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
 int stac_attn_colsum_scored(const void* q, int64_t q_row_stride, const void* k_hot, const void* v_hot,

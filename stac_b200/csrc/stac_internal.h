@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/stac_b200.h"
 #include "per_device.h"
 
@@ -54,6 +56,14 @@ size_t attn_part_elems();
 int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2, float* part, int* err,
                        cudaStream_t stream);
 
+// Kernels that this library has launched in this process (stac_kernel_launches): `launched` is the
+// result of a launch, counted where it succeeded and handed on.
+inline std::atomic<uint64_t> g_kernel_launches{0};
+inline cudaError_t count_launch(cudaError_t launched) {
+  if (launched == cudaSuccess) g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  return launched;
+}
+
 // Launch with programmatic stream serialization: the kernel may become resident while the
 // kernel before it in the stream drains; it calls grid_dep_wait() before it touches anything
 // that kernel wrote.  STAC_PDL=0 builds fall back to plain stream order.
@@ -73,7 +83,7 @@ cudaError_t launch_behind(void (*kernel)(KArgs...), dim3 grid, dim3 block, int s
   attr[0].val.programmaticStreamSerializationAllowed = STAC_PDL;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  return count_launch(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 }  // namespace stac

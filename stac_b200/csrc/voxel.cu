@@ -369,7 +369,7 @@ int stac_voxel_hash_clear(void* hash_keys, int64_t hash_cap, stac_stream_t strea
   const long long blocks = (hash_cap + threads - 1) / threads;
   stac::fill_u64_kernel<<<static_cast<unsigned>(blocks), threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       static_cast<unsigned long long*>(hash_keys), hash_cap, stac::kEmpty);
-  return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
+  return stac::count_launch(cudaGetLastError()) == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
 int stac_voxel_rehash(const int64_t* table_keys, const int* n_voxels, int table_cap, void* hash_keys, int* hash_vals,
@@ -381,11 +381,11 @@ int stac_voxel_rehash(const int64_t* table_keys, const int* n_voxels, int table_
   if (rc != STAC_OK) return rc;
   const int threads = 256;
   const int blocks = (table_cap + threads - 1) / threads;
-  if (blocks > 0)
-    stac::rehash_kernel<<<blocks, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const long long*>(table_keys), n_voxels, static_cast<unsigned long long*>(hash_keys),
-        hash_vals, static_cast<int>(hash_cap));
-  return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
+  if (blocks <= 0) return STAC_OK;
+  stac::rehash_kernel<<<blocks, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const long long*>(table_keys), n_voxels, static_cast<unsigned long long*>(hash_keys),
+      hash_vals, static_cast<int>(hash_cap));
+  return stac::count_launch(cudaGetLastError()) == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
 int stac_voxel_upsert(const float* points, const int32_t* ijk, const uint8_t* mask, int n_points, float voxel_size,
@@ -475,7 +475,7 @@ int stac_pointmap_to_positions(const float* world_points, const float* conf, int
   if (blocks > 0x7fffffffLL) return STAC_ERR_BAD_ARG;
   stac::pointmap_kernel<<<static_cast<unsigned>(blocks), threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       world_points, conf, S, H, W, oh, ow, special, conf_threshold, points_out, mask_out);
-  return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
+  return stac::count_launch(cudaGetLastError()) == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
 }  // extern "C"

@@ -664,3 +664,14 @@ def test_bounded_pools_match_oracle(max_buf, max_piv):
         if max_piv is not None:
             assert g.snapshot()["piv_top"] <= max_piv
     assert m.dropped > 0
+
+
+def test_launches_are_counted_where_they_are_made():
+    """The attention call with running scores takes three kernels where its column-sum kernel updates them, else four."""
+    from stac_b200 import _lib, ops
+    for M, H, T, want in ((130, 2, 300, 3), (1041, 16, 3800, 4)):
+        q, k, v = (torch.randn(*s, device=DEV).to(torch.bfloat16) for s in ((M, H, 64), (H, T, 64), (H, T, 64)))
+        scores, counts = torch.zeros(H, T, device=DEV), torch.zeros(H, T, device=DEV)
+        before = _lib.kernel_launches()
+        ops.attn_colsum(q, k, v, T, score_update=(scores, counts, T, 0, M, 0.9))
+        assert _lib.kernel_launches() - before == want
