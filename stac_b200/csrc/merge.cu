@@ -135,9 +135,9 @@ struct MergeParams {
   int2* long_list;     // rows with more than kLongRow tokens: the memory of full_list, which is filled later
   int2* move_list;     // [heads*ncap] rows in which buffered tokens change column
   int* tok_row;        // [heads][ncap] row index of each sorted token
-  int* tok_best;       // [heads][ncap] index of the most similar pivot of the token's row
-  int* row_flag;       // [heads][ncap] cleared with the row list: set once a token of the row merges into a pivot
-  int2* merge_list;    // [heads*ncap] rows (head, row index) with at least one merging token
+  int* tok_best;       // [heads][ncap] index of the most similar pivot of the token's row (rows of more than kShortRow tokens)
+  int* row_flag;       // [heads][ncap] cleared with the row list: set once the row is in merge_list
+  int2* merge_list;    // [heads*ncap] rows (head, row index) of more than kShortRow tokens with at least one merging token
   int passes;          // radix passes (8 bits each)
   int seg_vec;         // 1: the pivot segments of a row are one aligned 16-byte vector
   int* err;
@@ -633,7 +633,6 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
     p.tok_score[hb + i] = score;
     if (npiv == 0) {
       p.tok_sim[hb + i] = -INFINITY;
-      p.tok_best[hb + i] = 0;
     }
   }
   if (!__syncthreads_or(npiv > 0)) return;
@@ -710,7 +709,7 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
     if (sub == 0) {
       const long long o = hb + i0 + tk;
       p.tok_sim[o] = best_sim;
-      p.tok_best[o] = best;
+      if (!is_short) p.tok_best[o] = best;
       if (best_sim >= p.sim_thresh) {
         if (is_short) {
           best_s[tk] = static_cast<signed char>(best);
@@ -811,13 +810,11 @@ __global__ void __launch_bounds__(256, 4) rows_merge_kernel(const MergeParams p)
         }
       }
     };
-    const bool one_batch = s1 - s0 <= 8;
-    fetch(s0 + sub);
     for (int q = 0; q < npiv; ++q) {
       MergeSums m;
       m.clear();
       for (int base = s0; base < s1; base += 8) {
-        if (!one_batch) fetch(base + sub);
+        fetch(base + sub);
         unsigned todo = __ballot_sync(gmask, best_l == q) >> gbase & 0xffu;
         while (todo) {
           const int src = gbase + __ffs(todo) - 1;
