@@ -413,33 +413,44 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) sort_tokens_kernel(
 
 // ------------------------------------------------------------------------------------ phase A
 // Eight consecutive lanes work on one token: each holds eight of its 64 values (16 bytes of a
-// bf16 row, 32 of an fp32 row).
-template <typename T> struct Row8;
-template <> struct Row8<__nv_bfloat16> {
-  static __device__ __forceinline__ void load(const __nv_bfloat16* row, int sub, float (&x)[8]) {
-    const uint4 u = reinterpret_cast<const uint4*>(row)[sub];
+// bf16 row, 32 of an fp32 row).  Raw8: those values as they were loaded, in flight while others are worked on.
+template <typename T> struct Raw8;
+template <> struct Raw8<__nv_bfloat16> {
+  uint4 u;
+  __device__ __forceinline__ void load(const __nv_bfloat16* row, int sub) { u = reinterpret_cast<const uint4*>(row)[sub]; }
+  __device__ __forceinline__ void values(float (&x)[8]) const {
     x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
     x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
     x[4] = __uint_as_float(u.z << 16); x[5] = __uint_as_float(u.z & 0xffff0000u);
     x[6] = __uint_as_float(u.w << 16); x[7] = __uint_as_float(u.w & 0xffff0000u);
   }
-  static __device__ __forceinline__ void store(__nv_bfloat16* row, int sub, const float (&x)[8]) {
-    uint4 u;
-    u.x = pack_bf16x2(x[0], x[1]); u.y = pack_bf16x2(x[2], x[3]);
-    u.z = pack_bf16x2(x[4], x[5]); u.w = pack_bf16x2(x[6], x[7]);
-    reinterpret_cast<uint4*>(row)[sub] = u;
-  }
 };
-template <> struct Row8<float> {
-  static __device__ __forceinline__ void load(const float* row, int sub, float (&x)[8]) {
-    const float4 a = reinterpret_cast<const float4*>(row)[2 * sub], b = reinterpret_cast<const float4*>(row)[2 * sub + 1];
+template <> struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* row, int sub) {
+    a = reinterpret_cast<const float4*>(row)[2 * sub];
+    b = reinterpret_cast<const float4*>(row)[2 * sub + 1];
+  }
+  __device__ __forceinline__ void values(float (&x)[8]) const {
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
   }
-  static __device__ __forceinline__ void store(float* row, int sub, const float (&x)[8]) {
-    reinterpret_cast<float4*>(row)[2 * sub] = make_float4(x[0], x[1], x[2], x[3]);
-    reinterpret_cast<float4*>(row)[2 * sub + 1] = make_float4(x[4], x[5], x[6], x[7]);
-  }
 };
+template <typename T>
+__device__ __forceinline__ void row8_load(const T* row, int sub, float (&x)[8]) {
+  Raw8<T> r;
+  r.load(row, sub);
+  r.values(x);
+}
+__device__ __forceinline__ void row8_store(__nv_bfloat16* row, int sub, const float (&x)[8]) {
+  uint4 u;
+  u.x = pack_bf16x2(x[0], x[1]); u.y = pack_bf16x2(x[2], x[3]);
+  u.z = pack_bf16x2(x[4], x[5]); u.w = pack_bf16x2(x[6], x[7]);
+  reinterpret_cast<uint4*>(row)[sub] = u;
+}
+__device__ __forceinline__ void row8_store(float* row, int sub, const float (&x)[8]) {
+  reinterpret_cast<float4*>(row)[2 * sub] = make_float4(x[0], x[1], x[2], x[3]);
+  reinterpret_cast<float4*>(row)[2 * sub + 1] = make_float4(x[4], x[5], x[6], x[7]);
+}
 
 // sum over the eight lanes of a group (every lane gets it; same order in every group)
 __device__ __forceinline__ float group8_sum(float v, unsigned gmask) {
@@ -474,29 +485,6 @@ __device__ __forceinline__ float group8_sum_scatter4(const float (&v)[4], int su
   const float b = keep + __shfl_xor_sync(gmask, give, 2);
   return b + __shfl_xor_sync(gmask, b, 1);
 }
-
-// Raw values of one lane's eighth of a row: loads that are in flight while others are worked on.
-template <typename T> struct Raw8;
-template <> struct Raw8<__nv_bfloat16> {
-  uint4 u;
-  __device__ __forceinline__ void load(const __nv_bfloat16* row, int sub) { u = reinterpret_cast<const uint4*>(row)[sub]; }
-  __device__ __forceinline__ void values(float (&x)[8]) const {
-    x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
-    x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
-    x[4] = __uint_as_float(u.z << 16); x[5] = __uint_as_float(u.z & 0xffff0000u);
-    x[6] = __uint_as_float(u.w << 16); x[7] = __uint_as_float(u.w & 0xffff0000u);
-  }
-};
-template <> struct Raw8<float> {
-  float4 a, b;
-  __device__ __forceinline__ void load(const float* row, int sub) {
-    a = reinterpret_cast<const float4*>(row)[2 * sub];
-    b = reinterpret_cast<const float4*>(row)[2 * sub + 1];
-  }
-  __device__ __forceinline__ void values(float (&x)[8]) const {
-    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-  }
-};
 
 // What the tokens of a row that merge into one pivot add up to, in token order, held by eight lanes.
 struct MergeSums {
@@ -533,11 +521,11 @@ __device__ __forceinline__ void merge_into_pivot(const MergeParams& p, int seg, 
   k_old.values(o);
 #pragma unroll
   for (int e = 0; e < 8; ++e) o[e] = __fadd_rn(__fmul_rn(fo, o[e]), __fmul_rn(fn, m.K[e]));
-  Row8<T>::store(kb, sub, o);
+  row8_store(kb, sub, o);
   v_old.values(o);
 #pragma unroll
   for (int e = 0; e < 8; ++e) o[e] = __fadd_rn(__fmul_rn(fo, o[e]), __fmul_rn(fn, m.V[e]));
-  Row8<T>::store(vb, sub, o);
+  row8_store(vb, sub, o);
   if (sub == 0) {
     p.piv_W[seg] = denom;
     p.piv_S[seg] = __fadd_rn(S, m.S);
@@ -822,8 +810,8 @@ __global__ void __launch_bounds__(256, 4) rows_merge_kernel(const MergeParams p)
           const int code = __shfl_sync(gmask, code_l, src), pos = __shfl_sync(gmask, pos_l, src);
           const float a = __shfl_sync(gmask, a_l, src), s_t = __shfl_sync(gmask, s_l, src);
           float k[8], v[8];
-          Row8<T>::load(token_row_at<T>(p, h, code, pos, false), sub, k);
-          Row8<T>::load(token_row_at<T>(p, h, code, pos, true), sub, v);
+          row8_load(token_row_at<T>(p, h, code, pos, false), sub, k);
+          row8_load(token_row_at<T>(p, h, code, pos, true), sub, v);
           m.add(a, s_t, k, v);
         }
       }
@@ -1374,7 +1362,7 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
     {
       const int sg = __shfl_sync(gmask, my_seg, gbase + seed);
       float k[8];
-      Row8<T>::load(bK + static_cast<long long>(sg) * D, sub, k);
+      row8_load(bK + static_cast<long long>(sg) * D, sub, k);
       float ss = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss += k[e] * k[e];
@@ -1391,7 +1379,7 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
       if (c < B) {
         const int sg = __shfl_sync(gmask, my_seg, gbase + c);
         float k[8];
-        Row8<T>::load(bK + static_cast<long long>(sg) * D, sub, k);
+        row8_load(bK + static_cast<long long>(sg) * D, sub, k);
         float ss = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) ss += k[e] * k[e];
@@ -1415,8 +1403,8 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
         const float cn = __fdiv_rn(w[c], wden);
         const int sg = __shfl_sync(gmask, my_seg, gbase + c);
         float tk[8], tv[8];
-        Row8<T>::load(bK + static_cast<long long>(sg) * D, sub, tk);
-        Row8<T>::load(bV + static_cast<long long>(sg) * D, sub, tv);
+        row8_load(bK + static_cast<long long>(sg) * D, sub, tk);
+        row8_load(bV + static_cast<long long>(sg) * D, sub, tv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           nk[e] = __fadd_rn(nk[e], __fmul_rn(cn, tk[e]));
@@ -1455,7 +1443,7 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
       // keys normalised in the pool dtype, as the reference does here (stac/merger.py:493-495)
       auto load_normalised = [&](int seg, float (&out)[8]) {
         float pk[8];
-        Row8<T>::load(pK + static_cast<long long>(seg) * D, sub, pk);
+        row8_load(pK + static_cast<long long>(seg) * D, sub, pk);
         float ss = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) ss += pk[e] * pk[e];
@@ -1495,16 +1483,16 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
         const float denom = fmaxf(__fadd_rn(Wj, Wn), 1e-8f);
         const float fj = __fdiv_rn(Wj, denom), fk = __fdiv_rn(Wn, denom);
         float a[8], b[8];
-        Row8<T>::load(pK + static_cast<long long>(vseg) * D, sub, a);
-        Row8<T>::load(pK + static_cast<long long>(nseg) * D, sub, b);
+        row8_load(pK + static_cast<long long>(vseg) * D, sub, a);
+        row8_load(pK + static_cast<long long>(nseg) * D, sub, b);
 #pragma unroll
         for (int e = 0; e < 8; ++e) b[e] = __fadd_rn(__fmul_rn(fj, a[e]), __fmul_rn(fk, b[e]));
-        Row8<T>::store(pK + static_cast<long long>(nseg) * D, sub, b);
-        Row8<T>::load(pV + static_cast<long long>(vseg) * D, sub, a);
-        Row8<T>::load(pV + static_cast<long long>(nseg) * D, sub, b);
+        row8_store(pK + static_cast<long long>(nseg) * D, sub, b);
+        row8_load(pV + static_cast<long long>(vseg) * D, sub, a);
+        row8_load(pV + static_cast<long long>(nseg) * D, sub, b);
 #pragma unroll
         for (int e = 0; e < 8; ++e) b[e] = __fadd_rn(__fmul_rn(fj, a[e]), __fmul_rn(fk, b[e]));
-        Row8<T>::store(pV + static_cast<long long>(nseg) * D, sub, b);
+        row8_store(pV + static_cast<long long>(nseg) * D, sub, b);
         if (sub == 0) {
           p.piv_W[nseg] = denom;
           p.piv_S[nseg] = __fadd_rn(p.piv_S[vseg], p.piv_S[nseg]);
@@ -1513,8 +1501,8 @@ __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams
       }
       pseg = vseg;
     }
-    Row8<T>::store(pK + static_cast<long long>(pseg) * D, sub, nk);
-    Row8<T>::store(pV + static_cast<long long>(pseg) * D, sub, nv);
+    row8_store(pK + static_cast<long long>(pseg) * D, sub, nk);
+    row8_store(pV + static_cast<long long>(pseg) * D, sub, nv);
     if (sub == 0) {
       p.piv_W[pseg] = Wsum;
       p.piv_S[pseg] = sumS;
