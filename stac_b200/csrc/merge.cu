@@ -1578,22 +1578,24 @@ ScratchLayout scratch_layout(int heads, int ncap, int buf_cap) {
 template <typename T>
 int launch_merge(MergeParams& mp, cudaStream_t st) {
   if (cudaMemsetAsync(mp.plan, 0, kPlanSize * 4, st) != cudaSuccess) return STAC_ERR_CUDA;
-  const bool one_wave = mp.heads <= 2 * 148;
+  int dev, n_sm;
+  if (current_device(&dev) != STAC_OK || device_sm_count(dev, &n_sm) != STAC_OK) return STAC_ERR_CUDA;
+  const bool one_wave = mp.heads <= 2 * n_sm;
   if (launch_behind(one_wave ? sort_tokens_kernel<1024> : sort_tokens_kernel<512>, dim3(mp.heads), dim3(one_wave ? 1024 : 512), 0, st,
                     mp) != cudaSuccess)
     return STAC_ERR_CUDA;
   dim3 grid_a1((mp.ncap + 255) / 256, mp.heads);
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
   if (launch_behind(tokens_sim_merge_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(rows_merge_kernel<T>, dim3(148 * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(rows_merge_kernel<T>, dim3(n_sm * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_rank_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(scan_rows_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 0) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(scan_rows_kernel, dim3(mp.heads), dim3(1024), 0, st, mp, 1) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_phase_b1a_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(rows_phase_b1m_kernel<T, 2>, dim3(148 * 6), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(rows_phase_b1m_kernel<T, 2>, dim3(n_sm * 6), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(tokens_place_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(rows_phase_b2_kernel<T>, dim3(148 * 16), dim3(128), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(finalize_kernel<T>, dim3(148 * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;   // grid-stride over the freed ids (known on the device only)
+  if (launch_behind(rows_phase_b2_kernel<T>, dim3(n_sm * 16), dim3(128), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  if (launch_behind(finalize_kernel<T>, dim3(n_sm * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;   // grid-stride over the freed ids (known on the device only)
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
