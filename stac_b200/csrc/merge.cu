@@ -551,7 +551,7 @@ __device__ __forceinline__ void merge_into_pivot(const MergeParams& p, int seg, 
 // queued for rows_merge_kernel.
 // (As two kernels, which read a row's tokens twice and found them again through lists in memory, similarities
 // and merges took 288 + 293 us with 384 heads of 8328 tokens in a bounded memory, 102 + 166 us with 384 heads of 1041
-// tokens, 31 + 51 us with 16 heads of 8328 fp32 tokens; now 394 + 10, 162 + 2, 67 + 2.  Eight lanes taking a whole row
+// tokens, 31 + 51 us with 16 heads of 8328 fp32 tokens; now 394 + 10, 162 + 2, 62 + 2.  Eight lanes taking a whole row
 // for comparing and merging in one go were slower, 414, 200 and 95 us: the four rows of a warp diverge.)
 constexpr int kTokBlock = 256;
 constexpr int kShortRow = 8;           // one lane per token
@@ -655,10 +655,17 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
     const int np = npiv_s[first];
     const int4 sg = segs[first];
     const int seg[kMaxP] = {sg.x, sg.y, sg.z, sg.w};
-    Raw8<T> rp[kMaxP];
+    // fp32 rows two pivots at a time: four do not fit into the registers beside the token's, and a spilled load is a load that
+    // is waited for.  (16 heads of 8328 fp32 tokens: 66.7 -> 61.5 us, the first four calls on a fresh memory 50.4 -> 45.3; three
+    // CTAs per SM, without any spill, 80 us.)
+    constexpr int kAtOnce = sizeof(T) == 4 ? 2 : kMaxP;
+    Raw8<T> rp[kAtOnce];
+    auto load_pivots = [&](int q0) {
 #pragma unroll
-    for (int q = 0; q < kMaxP; ++q)
-      if (q < np) rp[q].load(static_cast<const T*>(p.piv_K) + static_cast<long long>(seg[q]) * p.D, sub);
+      for (int q = 0; q < kAtOnce; ++q)
+        if (q0 + q < np) rp[q].load(static_cast<const T*>(p.piv_K) + static_cast<long long>(seg[q0 + q]) * p.D, sub);
+    };
+    load_pivots(0);
     float k[8];
     next_k.values(k);
     if (e + kStep < n) next_k.load(key_row(list[e + kStep] & 0xfff), sub);
@@ -667,17 +674,22 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
     for (int x = 0; x < 8; ++x) kk = fmaf(k[x], k[x], kk);
     float dot[kMaxP], nrm[kMaxP];
 #pragma unroll
-    for (int q = 0; q < kMaxP; ++q) {
-      dot[q] = nrm[q] = 0.f;
-      if (q < np) {
-        float pk[8];
-        rp[q].values(pk);
+    for (int q0 = 0; q0 < kMaxP; q0 += kAtOnce) {
 #pragma unroll
-        for (int x = 0; x < 8; ++x) {
-          dot[q] = fmaf(k[x], pk[x], dot[q]);
-          nrm[q] = fmaf(pk[x], pk[x], nrm[q]);
+      for (int q = 0; q < kAtOnce; ++q) {
+        float pk[8], d = 0.f, pp = 0.f;
+        if (q0 + q < np) {
+          rp[q].values(pk);
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            d = fmaf(k[x], pk[x], d);
+            pp = fmaf(pk[x], pk[x], pp);
+          }
         }
+        dot[q0 + q] = d;
+        nrm[q0 + q] = pp;
       }
+      if (q0 + kAtOnce < kMaxP) load_pivots(q0 + kAtOnce);
     }
     const float den_k = fmaxf(sqrtf(group8_sum(kk, gmask)), 1e-6f);
     // lanes 2 q and 2 q + 1 both finish pivot q
