@@ -675,3 +675,47 @@ def test_launches_are_counted_where_they_are_made():
         before = _lib.kernel_launches()
         ops.attn_colsum(q, k, v, T, score_update=(scores, counts, T, 0, M, 0.9))
         assert _lib.kernel_launches() - before == want
+
+
+@pytest.mark.parametrize("Tn", [2049, 4097, 8328])      # second listing round, past the registers, the pool-stress length
+def test_sort_of_many_heads_equals_the_sort_of_few(Tn):
+    """300 heads take the sort's CTAs of 512 threads, four of them the ones of 1024 (which are compared with the oracle):
+    the same tokens leave the same slots, contents and carried tokens, bit for bit."""
+    from stac_b200 import _lib
+    from stac_b200.stac.merger import VoxelKVMerger
+    H, few, D, NV = 300, [0, 1, 147, 299], 64, Tn // 5
+    g = torch.Generator(device=DEV).manual_seed(Tn)
+
+    def memory(heads):
+        return VoxelKVMerger(heads, D, init_voxels=NV, pivot_cap=4, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8,
+                             score_thresh=0.1, dtype=torch.bfloat16, device=DEV, allocator="segment", seg_size=1, slab_cap=16)
+
+    def contents(vm, heads):
+        vm._pull_meta()
+        cur, n = vm._over[vm._over_cur], vm._meta.cpu().tolist()[_lib.META_OVER_COUNT]
+        hv = cur["hv"][:n].long()
+        res = []
+        for i, h in enumerate(heads):
+            for cnt, seg, fields in ((vm._buf_row_cnt, vm._buf_row_seg, (vm._buf_K, vm._buf_V, vm._buf_S)),
+                                     (vm._piv_row_cnt, vm._piv_row_seg, (vm._piv_K, vm._piv_V, vm._piv_W, vm._piv_S, vm._piv_C))):
+                s = seg[h, :NV]
+                res += [cnt[h, :NV].clone(), s >= 0] + [f[s[s >= 0].long()] for f in fields]
+            mine = hv[:, 0] == h
+            res += [hv[mine, 1], cur["K"][:n][mine], cur["V"][:n][mine], cur["S"][:n][mine]]
+        return res
+
+    many, small = memory(H), memory(len(few))
+    dirs = torch.randn(NV, D, device=DEV, generator=g)
+    for step in range(3):
+        vx = torch.randint(0, NV, (H, Tn), device=DEV, generator=g)
+        K = torch.randn(H, Tn, D, device=DEV, generator=g)
+        near = torch.rand(H, Tn, 1, device=DEV, generator=g) < 0.6
+        K = torch.where(near, dirs[vx] + 0.2 * K, K).to(torch.bfloat16)
+        V = torch.randn(H, Tn, D, device=DEV, generator=g).to(torch.bfloat16)
+        S = torch.exp(torch.randint(0, 4, (H, Tn), device=DEV, generator=g).float())      # ties: by arrival
+        vx = vx.int()
+        many.insert_and_merge(K, V, S, None, vx, NV)
+        small.insert_and_merge(K[few].contiguous(), V[few].contiguous(), S[few].contiguous(), None, vx[few].contiguous(), NV)
+        a, b = contents(many, few), contents(small, range(len(few)))
+        assert all(torch.equal(x, y) for x, y in zip(a, b)), step
+    assert sum(int(x.numel()) for x in b) > 0 and many._piv_row_cnt[few].sum() > 0
