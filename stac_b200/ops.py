@@ -103,10 +103,12 @@ def _kv_strides(t, layout):
 
 def _check_score_update(scores, counts, row_stride, H, T_hot, device):
     """The kernel writes [H, T_hot] fp32 scores and counts at ``row_stride`` and is given pointers only."""
-    for t in (scores, counts):
-        assert t.dtype == torch.float32 and t.device == device, "running scores and counts: fp32 on the queries' device"
-        assert t.dim() == 2 and t.shape[0] == H and t.shape[1] >= T_hot, "running scores and counts: [H, >= T_hot]"
-        assert t.stride() == (row_stride, 1) and (H == 1 or row_stride >= T_hot), "running scores and counts: strides"
+    assert scores.dtype is counts.dtype is torch.float32 and scores.device == counts.device == device, \
+        "running scores and counts: fp32 on the queries' device"
+    assert scores.stride() == counts.stride() == (row_stride, 1) and (H == 1 or row_stride >= T_hot), \
+        "running scores and counts: strides"
+    (hs, ws), (hc, wc) = scores.shape, counts.shape
+    assert hs == hc == H and ws >= T_hot and wc >= T_hot, "running scores and counts: [H, >= T_hot]"
 
 
 def attn_colsum(q, k_hot, v_hot, T_hot, k_ret=None, v_ret=None, bias_ret=None, T_ret=0, *,
