@@ -560,10 +560,11 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
   constexpr int kAll = kTokBlock + kShortRow;
   constexpr int kNoKey = -1;           // not a voxel id
-  __shared__ int key_s[kShortRow + kAll];        // voxel ids from eight tokens before to eight behind
+  __shared__ int key_s[kAll + 2 * kShortRow];    // voxel ids from eight tokens before to eight behind, and eight of none
   __shared__ uintptr_t krow_s[kAll];             // address of the token's key row (16-byte aligned); bit 0: a carried token
   __shared__ float score_s[kAll], sim_s[kAll];
-  __shared__ signed char best_s[kAll];           // pivot that the token merges into, -1 = none
+  constexpr int kQueued = -2;
+  __shared__ signed char best_s[kAll];           // pivot that the token merges into, -1 = none, kQueued = its row is a longer one
   __shared__ int4 segs[kTokBlock];
   __shared__ unsigned char npiv_s[kTokBlock], len_s[kTokBlock];   // len: tokens of the short row that starts here
   __shared__ unsigned short list[kAll];          // token, (tokens of its row before it) << 12; then rows to merge
@@ -616,6 +617,7 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
   if (t < kShortRow) {
     keep(t + kTokBlock, key_x, code_x, pos_x, score_x);
     key_s[t] = i0 > 0 ? static_cast<int>(keys[i0 - kShortRow + t]) : kNoKey;
+    key_s[kShortRow + kAll + t] = kNoKey;
   }
   if (mine) {
     p.tok_score[hb + i] = score;
@@ -630,9 +632,14 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
     const int* k = key_s + kShortRow + t;
     const int key = k[0];
     if (key == kNoKey || (t < kTokBlock && npiv_s[t] == 0)) return;
-    int before = 0, behind = 1;
-    while (before < kShortRow && k[-before - 1] == key) ++before;
-    while (before + behind <= kShortRow && t + behind < kAll && k[behind] == key) ++behind;
+    // tokens of the row on either side, up to eight: equal keys lie side by side
+    auto run = [&](int dir) {
+      if (k[8 * dir] == key) return 8;
+      int n = k[4 * dir] == key ? 4 : 0;
+      if (k[(n + 2) * dir] == key) n += 2;
+      return k[(n + 1) * dir] == key ? n + 1 : n;
+    };
+    const int before = run(-1), behind = 1 + run(1);
     const bool is_short = before + behind <= kShortRow;
     const int first = is_short ? t - before : t;
     if (first < 0 || first >= kTokBlock || npiv_s[first] == 0) return;
@@ -716,13 +723,19 @@ __global__ void __launch_bounds__(kTokBlock, 4) tokens_sim_merge_kernel(const Me
           sim_s[tk] = best_sim;
           atomicOr(&todo_mask[first >> 5], 1u << (first & 31));
         } else {
-          const int ri = p.tok_row[o];
-          if (atomicExch(&p.row_flag[hb + ri], 1) == 0) p.merge_list[list_push(&p.plan[kPlanMergeCount])] = make_int2(h, ri);
+          best_s[tk] = kQueued;
         }
       }
     }
   }
   __syncthreads();
+  // Longer rows are queued behind the comparing, by the first of several neighbouring tokens: with many heads the loop above
+  // is bound by its instructions.  (384 heads of 8328 tokens, rows of 12: 652 -> 606 us against every token for itself;
+  // the runs of equal keys counted in four looks instead of a loop: -> 582.)
+  if (best_s[t] == kQueued && !(t > 0 && best_s[t - 1] == kQueued && key_s[kShortRow + t - 1] == key)) {
+    const int ri = p.tok_row[hb + i];
+    if (atomicExch(&p.row_flag[hb + ri], 1) == 0) p.merge_list[list_push(&p.plan[kPlanMergeCount])] = make_int2(h, ri);
+  }
   if ((todo_mask[t >> 5] >> lane) & 1u) list[list_push(&n_todo)] = static_cast<unsigned short>(t);
   __syncthreads();
   const int n_rows = n_todo;
