@@ -95,10 +95,9 @@ def _attn_workspace(device, M, H):
 
 def _kv_strides(t, layout):
     """(row_stride, head_stride) in elements for a [H,T,D] ('htd') or [T,H,D] ('thd') tensor."""
-    assert t.stride(-1) == 1
-    if layout == "htd":
-        return t.stride(1), t.stride(0)
-    return t.stride(0), t.stride(1)
+    outer, inner, last = t.stride()
+    assert last == 1
+    return (inner, outer) if layout == "htd" else (outer, inner)
 
 
 def _check_score_update(scores, counts, row_stride, H, T_hot, device):
