@@ -550,8 +550,9 @@ __device__ __forceinline__ void merge_into_pivot(const MergeParams& p, int seg, 
 // own; only that CTA looks at its pivots, so all of its similarities are taken before.  Longer rows are
 // queued for rows_merge_kernel.
 // (As two kernels, which read a row's tokens twice and found them again through lists in memory, similarities
-// and merges took 288 + 293 us with 384 heads of 8328 tokens in a bounded memory, 102 + 166 us with 384 heads of 1041
-// tokens, 31 + 51 us with 16 heads of 8328 fp32 tokens; now 394 + 10, 162 + 2, 62 + 2.  Eight lanes taking a whole row
+// and merges took 285 + 287 us with 384 heads of 8328 tokens in a bounded memory, 103 + 166 us with 384 heads of 1041
+// tokens, 31 + 52 us with 16 heads of 8328 fp32 tokens, where most rows merge; now 364 + 25, 160 + 2, 61 + 2.  Where few
+// do, in the first calls on the first and the last, 57 + 24 and 25 + 31 then, 71 + 17 and 45 + 22 now.  Eight lanes taking a whole row
 // for comparing and merging in one go were slower, 414, 200 and 95 us: the four rows of a warp diverge.)
 constexpr int kTokBlock = 256;
 constexpr int kShortRow = 8;           // one lane per token
