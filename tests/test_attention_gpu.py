@@ -77,10 +77,10 @@ def test_one_to_nine_key_tiles(M, H, T_hot, T_ret):
     _assert_close(*_run_two_segment(M, H, T_hot, T_ret, seed=T_hot + T_ret))
 
 
-@pytest.mark.parametrize("T_hot,T_ret", [(336, 0), (600, 70), (1008, 0), (1100, 0), (1150, 90), (1400, 20)])
+@pytest.mark.parametrize("T_hot,T_ret", [(336, 0), (672, 0), (600, 70), (1008, 0), (1100, 0), (1150, 90), (1400, 20)])
 @pytest.mark.parametrize("M,H", [(130, 2), (2600, 8)])
 def test_scores_wait_for_the_values_of_the_tile_before_them(M, H, T_hot, T_ret):
-    """3, 7, 9, 10, 12 and 14 key tiles, in the second shape cut over the SMs at many offsets, so that segments of every
+    """3, 6, 7, 9, 10, 12 and 14 key tiles, in the second shape cut over the SMs at many offsets, so that segments of every
     short length occur: scores take over the columns of probabilities only when P V has read them (same bits
     every run)."""
     got, ref = _run_two_segment(M, H, T_hot, T_ret, seed=T_hot + T_ret)
