@@ -847,15 +847,11 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const bool is_ret = j >= n_hot;
         const int n0 = (is_ret ? j - n_hot : j) * kFT;
         const int valid = min(kFT, (is_ret ? p.T_ret : p.T_hot) - n0);
-        named_bar_sync(1 + g, 128);
-        bool live = false;
-        if (row < kFT) {
-          float bv = -INFINITY;
-          if (row < valid) bv = is_ret ? p.bias_ret[h * p.bias_head_stride + n0 + row] * kLog2e : 0.f;
-          sm.bias2[g][row] = bv;
-          live = bv != -INFINITY;
-        }
-        const bool tile_live = named_bar_or(1 + g, 128, live);   // false: every key of the tile is masked (padding behind the valid pivots)
+        float bv = -INFINITY;
+        if (row < valid) bv = is_ret ? p.bias_ret[h * p.bias_head_stride + n0 + row] * kLog2e : 0.f;
+        named_bar_sync(1 + g, 128);   // the bias is on its way while the warpgroup meets
+        if (row < kFT) sm.bias2[g][row] = bv;
+        const bool tile_live = named_bar_or(1 + g, 128, bv != -INFINITY);   // false: every key of the tile is masked (padding behind the valid pivots)
         any_live = any_live || tile_live;
         mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
         tc_fence_after();
