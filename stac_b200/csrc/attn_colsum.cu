@@ -544,16 +544,21 @@ struct FwdWalk {
 // are handled two at a time with the packed fp32 instructions (scale-and-subtract, row sums).
 // The pairs whose bit is set in kFastPairMask take their exponentials on the FMA pipes (cubic,
 // 8.6e-5 relative, far below the bf16 rounding of P) to relieve the exponential unit.
+// Their arguments go into a running maximum: 2^128 and more, which the exponential unit turns into infinities that the
+// row sum shows, would wrap there.
 template <int kJ>
-__device__ __forceinline__ uint64_t fast_exp_pair(uint64_t x2) {
-  if ((kFastPairMask >> (kJ & 15)) & 1u) return poly_exp2_x2(x2);
+__device__ __forceinline__ uint64_t fast_exp_pair(uint64_t x2, float& top) {
   float x0, x1;
   unpack_f32x2(x2, x0, x1);
+  if constexpr ((kFastPairMask >> (kJ & 15)) & 1u) {
+    top = fmax3(top, x0, x1);
+    return poly_exp2_x2(x2);
+  }
   return pack_f32x2(fast_exp2(x0), fast_exp2(x1));
 }
 template <bool kBias, int kN, int kI = 0>
 __device__ __forceinline__ void fast_exp_chunk(const uint32_t (&s)[32], uint32_t (&pk)[16], const float* bias2,
-                                               uint64_t c2c2, uint64_t negm2, uint64_t& l0, uint64_t& l1) {
+                                               uint64_t c2c2, uint64_t negm2, uint64_t& l0, uint64_t& l1, float& top) {
   if constexpr (kI < kN) {
     uint64_t x0 = pack_f32x2(__uint_as_float(s[kI + 0]), __uint_as_float(s[kI + 1]));
     uint64_t x1 = pack_f32x2(__uint_as_float(s[kI + 2]), __uint_as_float(s[kI + 3]));
@@ -565,7 +570,7 @@ __device__ __forceinline__ void fast_exp_chunk(const uint32_t (&s)[32], uint32_t
       x0 = fma_f32x2(x0, c2c2, negm2);
       x1 = fma_f32x2(x1, c2c2, negm2);
     }
-    const uint64_t e0 = fast_exp_pair<kI / 2>(x0), e1 = fast_exp_pair<kI / 2 + 1>(x1);
+    const uint64_t e0 = fast_exp_pair<kI / 2>(x0, top), e1 = fast_exp_pair<kI / 2 + 1>(x1, top);
     l0 = add_f32x2(l0, e0);
     l1 = add_f32x2(l1, e1);
     float a0, a1, a2, a3;
@@ -573,7 +578,7 @@ __device__ __forceinline__ void fast_exp_chunk(const uint32_t (&s)[32], uint32_t
     unpack_f32x2(e1, a2, a3);
     pk[kI / 2] = pack_bf16x2(a0, a1);
     pk[kI / 2 + 1] = pack_bf16x2(a2, a3);
-    fast_exp_chunk<kBias, kN, kI + 4>(s, pk, bias2, c2c2, negm2, l0, l1);
+    fast_exp_chunk<kBias, kN, kI + 4>(s, pk, bias2, c2c2, negm2, l0, l1, top);
   }
 }
 
@@ -772,6 +777,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     uint32_t ra[32], rb[32], pk[16];   // rb: the read-out of O
     const uint32_t s_addr = tmem + lane_base + g * kFT;
     bool overflow = false;
+    float top = 0.f;          // largest exponent (relative to the row reference) that the FMA pipes were given
     FwdWalk walk(p, n_tiles);
     int seg = 0, item, t0, t1;
     int c_base = 0;   // key tiles of earlier segments
@@ -817,13 +823,13 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
         for (int ch = 0; ch < kFT / 32; ++ch) {
           tmem_ld_wait();
-          fast_exp_chunk<kBias, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1);
+          fast_exp_chunk<kBias, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1, top);
           if (ch + 1 < kFT / 32) tmem_ld32(s_addr + 32 * (ch + 1), ra);
           else tmem_ld16(s_addr + 32 * (ch + 1), ra);
           tmem_st16(s_addr + 16 * ch, pk);
         }
         tmem_ld_wait();
-        fast_exp_chunk<kBias, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1);
+        fast_exp_chunk<kBias, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1, top);
         tmem_st8(s_addr + (kFT - 16) / 2, pk);
         tmem_st_wait();
         tc_fence_before();
@@ -995,6 +1001,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       c_base += len;
     }
+    overflow = overflow || top >= 128.f;
     if (__any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(p.fallback, 1);
   }
   tc_fence_before();

@@ -159,6 +159,25 @@ def test_scores_far_above_the_first_keys(M, H, T_hot):
     np.testing.assert_allclose(cs, cs_ref, rtol=1e-3, atol=1e-6)
 
 
+def test_one_key_far_above_the_first_keys():
+    """A single key 2^144 above the row reference, at every place of a chunk of 32: whichever pipe its exponential runs on,
+    the call is recomputed by the exact kernel (one call per place: any flagged row recomputes a whole call)."""
+    from stac_b200 import ops
+    rs = np.random.RandomState(8)
+    M, T, dev = 40, 300, torch.device("cuda:0")
+    u = rs.randn(64).astype(np.float32)
+    u /= np.linalg.norm(u)
+    q = _bf16(8 * u + 0.1 * rs.randn(M, 1, 64).astype(np.float32))
+    v = _bf16(rs.randn(1, T, 64).astype(np.float32))
+    for place in range(224, 224 + 32):
+        k = rs.randn(1, T, 64).astype(np.float32)
+        k[0, place] = 100 * u
+        k = _bf16(k)
+        got = ops.attn_colsum(q.to(dev), k.to(dev), v.to(dev), T, want_lse=True)
+        ref = oracle_attn(q.float().numpy(), k.float().numpy().transpose(1, 0, 2), v.float().numpy().transpose(1, 0, 2), None)
+        _assert_close([x.float().cpu().numpy() for x in got], ref)
+
+
 @pytest.mark.parametrize("shift", [-40.0, 30.0])
 def test_large_bias(shift):
     got, ref = _run_two_segment(200, 2, 300, 260, seed=13, bias_shift=shift)
