@@ -454,9 +454,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // CTA per SM and cuts that unit sequence into equal contiguous ranges (no partly filled last
 // wave); a CTA walks its range segment by segment, a segment being a run of key tiles of one
 // item.  An item on a cut is computed in two parts by two CTAs, each with its own row
-// references; the parts (unnormalised accumulator, row sums, references) go to a workspace, each
-// CTA counts its arrival at the cut and the one that arrives second joins the two parts (plain
-// split-softmax algebra, operands in a fixed order: same bits whichever CTA does it).  With at
+// references; the CTA that arrives first at a cut leaves its part (unnormalised accumulator, row sums, references) in a
+// workspace, and the one that arrives second joins it with its own, which stays in registers (plain
+// split-softmax algebra, operands in a fixed order: same bits whichever CTA does it).  Cuts cost a call about 3 us
+// (6 when both parts went through memory, rows of 256 bytes per thread).  With at
 // most half as many items as SMs every item is cut in exactly two halves instead.  Barrier
 // phases, the stages and the score buffers run on across segments; the query tile, the row references and the
 // partial row sums are double buffered by segment parity, and so are the barriers that several warpgroups
@@ -491,8 +492,8 @@ struct FastSmem {
   uint8_t v[kFastWgs][kFastTileBytes];
   float bias2[kFastWgs][kBN];
   float m_ref[2][kBM];                          // row references of the segment (parity)
-  float lpart[2][kFastWgs - 1][kBM];            // row sums of warpgroups 1.. (segment parity)
-  int live[2][kFastWgs - 1];                    // did warpgroup 1.. see a key that is not masked (segment parity)
+  float lpart[2][kFastWgs][kBM];                // row sums of the warpgroups (segment parity)
+  int live[2][kFastWgs];                        // did a warpgroup see a key that is not masked (segment parity)
   uint64_t q_full[2];
   uint64_t q_empty[2];
   uint64_t k_full[kFastWgs];
@@ -501,11 +502,11 @@ struct FastSmem {
   uint64_t p_full[kFastWgs];     // its probabilities are in TMEM
   uint64_t pv_done[kFastWgs];    // the P V MMAs that read them are done: scores may overwrite them, values theirs
   uint64_t ref_ready[2];
-  uint64_t l_ready[2];           // warpgroups 1.. have published their row sums of the segment (parity)
+  uint64_t l_ready[2];           // the other warpgroups have published their row sums of the segment (parity)
   uint64_t o_done;               // all P V MMAs of the segment are complete
   uint64_t o_free;               // the segment's accumulator has been read out of TMEM
   uint32_t tmem_base;
-  int join_flag;                 // arrival count seen at a cut (1: the other part is complete)
+  int join_flag[kFastWgs];       // arrival count seen at a cut (1: the other part is complete), of the warpgroup that closes a segment
 };
 
 // The (item, key tile) units of one CTA, walked segment by segment: a segment is a run of key
@@ -792,12 +793,14 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       bool have_ref = false;
       bool any_live = false;  // some key tile of this warpgroup in this segment had a key that is not masked
       int x = (g - c_base) & (kFastWgs - 1);
-      // The reference of the segment, at the first tile of this warpgroup; the first 32 scores are in ra behind it.
+      // The reference of the segment, at the first tile of this warpgroup.
       auto reference = [&](bool need_bias) {
-        have_ref = true;
+        mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
+        tc_fence_after();
         if (x == 0) {
           // exact row maximum of the segment's first tile = the row's reference for the segment
           float mx = -INFINITY;
+          tmem_ld32(s_addr, ra);
 #pragma unroll
           for (int ch = 0; ch < kFT / 32; ++ch) {
             tmem_ld_wait();
@@ -807,7 +810,6 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           }
           tmem_ld_wait();
           mx = fast_max_chunk<16>(ra, bias2 + kFT - 16, need_bias, c2, mx);
-          tmem_ld32(s_addr, ra);
           m_ref = (mx == -INFINITY) ? 0.f : mx;
           sm.m_ref[sb][row] = m_ref;
           mbar_arrive(&sm.ref_ready[sb]);
@@ -816,6 +818,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           m_ref = sm.m_ref[sb][row];
         }
         negm2 = pack_f32x2(-m_ref, -m_ref);
+        have_ref = true;
       };
       // Scores -> probabilities in place, chunk by chunk: load, wait, convert, store.
       auto convert = [&](auto bias_tag) {
@@ -838,12 +841,12 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // whole tiles of the hot cache: no bias, nothing masked
       const int n_plain = min(len, p.T_hot / kFT - t0);
       any_live = x < n_plain;
+      if (x < n_plain) reference(false);
 #pragma unroll 1
       for (; x < n_plain; x += kFastWgs, ++round) {
         mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
         tc_fence_after();
         tmem_ld32(s_addr, ra);
-        if (!have_ref) reference(false);
         convert(std::false_type{});
       }
       // the ragged last tile of the hot cache, the retrieved pivots
@@ -859,9 +862,11 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (row < kFT) sm.bias2[g][row] = bv;
         const bool tile_live = named_bar_or(1 + g, 128, bv != -INFINITY);   // false: every key of the tile is masked (padding behind the valid pivots)
         any_live = any_live || tile_live;
+        const bool first = !have_ref;
+        if (first) reference(true);
         mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
         tc_fence_after();
-        if (!tile_live && have_ref) {
+        if (!tile_live && !first) {
           // nothing to exponentiate: all probabilities of this tile are zero
 #pragma unroll
           for (int i = 0; i < 16; ++i) pk[i] = 0u;
@@ -874,7 +879,6 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           continue;
         }
         tmem_ld32(s_addr, ra);
-        if (!have_ref) reference(true);
         convert(std::true_type{});
       }
       // ---- end of the segment
@@ -883,22 +887,23 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       unpack_f32x2(l1, lc, ld);
       const float lsum = (la + lb) + (lc + ld);
       overflow = overflow || !(lsum <= kFastRowSumLimit);   // also true for NaN
-      if (g != 0) {
-        sm.lpart[sb][g - 1][row] = lsum;
-        if (row == 0) sm.live[sb][g - 1] = any_live ? 1 : 0;
+      sm.lpart[sb][g][row] = lsum;
+      if (row == 0) sm.live[sb][g] = any_live ? 1 : 0;
+      if (g != ((c_base + len - 1) & (kFastWgs - 1))) {
         mbar_arrive(&sm.l_ready[sb]);
       } else {
-        if (!have_ref) {
-          mbar_wait(&sm.ref_ready[sb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-          m_ref = sm.m_ref[sb][row];
-        }
+        // The warpgroup of the last tile closes the segment: its next tile is three tiles into the next segment, where the
+        // others are working meanwhile.  (Every segment of a CTA behind its first adds 1.0 us to this kernel; 2.5 when
+        // warpgroup 0 closed them all, whose next tile was often the first of the next segment.)
         mbar_wait(&sm.l_ready[sb], (seg >> 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-        const float l = ((lsum + sm.lpart[sb][0][row]) + sm.lpart[sb][1][row]) + sm.lpart[sb][2][row];
+        const float l = ((sm.lpart[sb][0][row] + sm.lpart[sb][1][row]) + sm.lpart[sb][2][row]) + sm.lpart[sb][3][row];
         // A segment whose keys are all masked has no reference (m_ref is a placeholder): it must not
         // take part in a join.  A segment with live keys whose probabilities all underflowed (its
         // first tile was masked, so the placeholder was used, and the live scores lie far below
         // it) cannot be represented: the exact kernel redoes the call.
-        const bool seg_live = any_live || sm.live[sb][0] != 0 || sm.live[sb][1] != 0 || sm.live[sb][2] != 0;
+        bool seg_live = any_live;
+#pragma unroll
+        for (int w = 0; w < kFastWgs; ++w) seg_live = seg_live || (w != g && sm.live[sb][w] != 0);
         if (seg_live && !(l > 0.f)) overflow = true;
         mbar_wait(&sm.o_done, seg & 1, p.err, DEV_TIMEOUT_MMA);
         tc_fence_after();
@@ -936,32 +941,39 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             p.lse2[static_cast<long long>(h) * p.lse2_stride + mrow] = l2;
           }
         } else {
-          // part of an item: unnormalised accumulator, row sum and row reference go to this
-          // CTA's slot (slot 1: the item starts here and ends in the next CTA; slot 0: it began
-          // in the previous CTA).  Whichever of the two CTAs gets there second joins the parts.
+          // Part of an item: whichever of the two CTAs gets there second joins the parts.  The first one leaves its
+          // unnormalised accumulator, row sums and references in its slot (slot 1: the item starts here and ends in the
+          // next CTA; slot 0: it began in the previous CTA) and counts its arrival.  The parts lie with a row's 16-byte pieces
+          // kBM rows apart, so that a warp writes and reads whole lines.
           const bool first_part = t0 == 0;
           const int cut = first_part ? blockIdx.x : blockIdx.x - 1;   // between CTA cut and cut + 1
-          float* slot = p.part + static_cast<size_t>(2 * blockIdx.x + (first_part ? 1 : 0)) * kPartFloats;
-          float4* orow = reinterpret_cast<float4*>(slot + row * kD);
-#pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
-            orow[q4] = make_float4(__uint_as_float(ra[q4 * 4 + 0]), __uint_as_float(ra[q4 * 4 + 1]),
-                                   __uint_as_float(ra[q4 * 4 + 2]), __uint_as_float(ra[q4 * 4 + 3]));
-#pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
-            orow[8 + q4] = make_float4(__uint_as_float(rb[q4 * 4 + 0]), __uint_as_float(rb[q4 * 4 + 1]),
-                                       __uint_as_float(rb[q4 * 4 + 2]), __uint_as_float(rb[q4 * 4 + 3]));
-          slot[kBM * kD + row] = l;
           const float m_pub = seg_live ? m_ref : -INFINITY;
-          slot[kBM * kD + kBM + row] = m_pub;
-          __threadfence();                       // this thread's part is visible device-wide ...
-          named_bar_sync(6, 128);                // ... and so is every other row's
-          if (row == 0) sm.join_flag = atomicAdd(p.part_count + cut, 1);
-          named_bar_sync(6, 128);
-          if (sm.join_flag == 1) {
+          if (row == 0) sm.join_flag[g] = ld_acquire(p.part_count + cut);
+          named_bar_sync(1 + g, 128);
+          bool second = sm.join_flag[g] == 1;          // usually: the item's other CTA began with it, or ended with it long ago
+          if (!second) {
+            float* slot = p.part + static_cast<size_t>(2 * blockIdx.x + (first_part ? 1 : 0)) * kPartFloats;
+            float4* orow = reinterpret_cast<float4*>(slot) + row;
+#pragma unroll
+            for (int q4 = 0; q4 < 8; ++q4)
+              orow[q4 * kBM] = make_float4(__uint_as_float(ra[q4 * 4 + 0]), __uint_as_float(ra[q4 * 4 + 1]),
+                                           __uint_as_float(ra[q4 * 4 + 2]), __uint_as_float(ra[q4 * 4 + 3]));
+#pragma unroll
+            for (int q4 = 0; q4 < 8; ++q4)
+              orow[(8 + q4) * kBM] = make_float4(__uint_as_float(rb[q4 * 4 + 0]), __uint_as_float(rb[q4 * 4 + 1]),
+                                                 __uint_as_float(rb[q4 * 4 + 2]), __uint_as_float(rb[q4 * 4 + 3]));
+            slot[kBM * kD + row] = l;
+            slot[kBM * kD + kBM + row] = m_pub;
+            __threadfence();                           // this thread's part is visible device-wide ...
+            named_bar_sync(1 + g, 128);                // ... and so is every other row's
+            if (row == 0) sm.join_flag[g] = atomicAdd(p.part_count + cut, 1);
+            named_bar_sync(1 + g, 128);
+            second = sm.join_flag[g] == 1;
+          }
+          if (second) {
             // the other CTA's part was complete before its counter increment, which came first
             __threadfence();
-            if (row == 0) p.part_count[cut] = 0;   // both have arrived: ready for the next call
+            if (row == 0) p.part_count[cut] = 0;       // both have arrived: ready for the next call
             const float* other = p.part + static_cast<size_t>(first_part ? 2 * (cut + 1) : 2 * cut + 1) * kPartFloats;
             const float lo_ = __ldcg(other + kBM * kD + row), mo_ = __ldcg(other + kBM * kD + kBM + row);
             // a = the part with the item's first tiles, b = the part with its last ones
@@ -974,7 +986,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const float lsum2 = __fmaf_rn(la, wa, __fmul_rn(lb, wb));
             const float inv = lsum2 > 0.f ? 1.f / lsum2 : 0.f;
             if (mrow < p.M) {
-              const float4* orow_o = reinterpret_cast<const float4*>(other + row * kD);
+              const float4* orow_o = reinterpret_cast<const float4*>(other) + row;
               __nv_bfloat16* dst = p.out + static_cast<long long>(mrow) * p.out_row_stride + h * kD;
               auto join = [&](uint32_t own, float oth) {
                 const float x = __uint_as_float(own);
@@ -983,7 +995,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               };
 #pragma unroll
               for (int q8 = 0; q8 < 8; ++q8) {
-                const float4 o0 = __ldcg(orow_o + 2 * q8), o1 = __ldcg(orow_o + 2 * q8 + 1);
+                const float4 o0 = __ldcg(orow_o + 2 * q8 * kBM), o1 = __ldcg(orow_o + (2 * q8 + 1) * kBM);
                 const uint32_t* r8 = q8 < 4 ? &ra[q8 * 8] : &rb[(q8 - 4) * 8];
                 uint4 val;
                 val.x = pack_bf16x2(join(r8[0], o0.x), join(r8[1], o0.y));

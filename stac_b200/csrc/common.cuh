@@ -315,6 +315,12 @@ __device__ __forceinline__ uint64_t poly_exp2_x2(uint64_t x2) {
                     __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
 }
 
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // three-input maximum (one instruction on sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
