@@ -643,12 +643,13 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   grid_dep_launch();
 
   if (p.zero_colsum != nullptr) {
-    // a slice of the column-sum output per CTA (the next kernel adds partial sums onto zeros)
+    // a slice of the column-sum output per CTA (the next kernel adds partial sums onto zeros; negative ones, so that the
+    // first of two additions to a key can be told from the second, see there)
     const long long total = static_cast<long long>(p.H) * p.zero_width;
     const long long lo = total * blockIdx.x / gridDim.x, hi = total * (blockIdx.x + 1) / gridDim.x;
     for (long long e = lo + threadIdx.x; e < hi; e += kFastThreads) {
       const long long hh = e / p.zero_width;
-      p.zero_colsum[hh * p.zero_stride + (e - hh * p.zero_width)] = 0.f;
+      p.zero_colsum[hh * p.zero_stride + (e - hh * p.zero_width)] = -0.f;
     }
   }
 
@@ -1088,7 +1089,7 @@ struct ColParams {
   // an item has at most two parts, added onto the zeroed output with one atomic each.
   float* parts;       // [2 * gridDim.x][kColGroup * kBN]
   int* part_count;    // [n_items], zero on entry, left zero
-  // Running scores that the column sums of the hot keys go into (stac/h2o.py:177-216), or nullptr (no atomics then):
+  // Running scores that the column sums of the hot keys go into (stac/h2o.py:177-216), or nullptr:
   // s = colsum * T_hot / Tq; an old key's score decays, score * temperature + s (two roundings, as mul_ then
   // add_), a new one's is s; counts += 1.
   float* scores;      // [H, score_stride]
@@ -1458,19 +1459,31 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (masked) sum = 0.f;
       }
       float* dst = p.colsum + static_cast<long long>(h) * p.colsum_stride + (is_ret ? p.T_hot : 0) + n0 + key;
-      auto finish = [&](float total) {
-        *dst = total;
+      auto update_score = [&](float total) {
         if (p.scores != nullptr && !is_ret) {
           const float sc = __fdiv_rn(__fmul_rn(total, static_cast<float>(p.T_hot)), p.tq);
           p.scores[score_at] = n0 + key >= p.old_T ? sc : __fadd_rn(__fmul_rn(old_score, p.temperature), sc);
           p.counts[score_at] = __fadd_rn(old_count, 1.0f);
         }
       };
+      auto finish = [&](float total) {
+        *dst = total;
+        update_score(total);
+      };
       constexpr int kSlot = kColGroup * kBN;
       if (i0 == 0 && i1 == nq) {
         if (key < valid) finish(sum);
       } else if (p.parts == nullptr) {
-        if (key < valid) atomicAdd(dst, sum);
+        if (key < valid) {
+          if (p.scores == nullptr || is_ret) {
+            atomicAdd(dst, sum);      // nothing to wait for
+          } else {
+            // Of the two additions onto -0 the first finds the sign bit, the second the other CTA's sum, which is +0 at
+            // least: the thread of the second has the total, with the bits that are in memory, and updates the score.
+            const float before = atomicAdd(dst, sum);
+            if (!signbit(before)) update_score(__fadd_rn(before, sum));
+          }
+        }
       } else {
         // CTA c owns the units [total * c / G, total * (c + 1) / G): owner(u) = ((u + 1) * G - 1) / total
         const long long total = static_cast<long long>(p.n_items) * nq, G = gridDim.x;
@@ -1723,15 +1736,19 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     cp.err = err;
     cp.split = (col_split || col_parts) ? 1 : 0;      // col_split: the forward kernel has cleared a.colsum
     cp.parts = col_parts ? part + kFwdPartElems : nullptr;
-    // running scores: updated by the thread that has a key's final sum; where atomics make it, by a launch behind
-    cp.scores = col_split ? nullptr : a.scores; cp.counts = a.counts; cp.score_stride = a.score_stride;
+    // Running scores: updated by the thread that has a key's final sum (1041 rows, 16 heads, 5600 keys 66.4 -> 65.2 us per
+    // call, 8328 + 2082 keys 110.6 -> 109.5, 2 us per layer of a stream, against a launch behind the kernel).  Below two items
+    // per SM, where nearly every item is cut, the launch stays: callers count a call's launches there (3800 keys 50.9
+    // against 49.7 us).
+    const bool scored_apart = col_split && col_items < 2 * n_sm;
+    cp.scores = scored_apart ? nullptr : a.scores; cp.counts = a.counts; cp.score_stride = a.score_stride;
     cp.old_T = a.old_T; cp.tq = static_cast<float>(a.score_Tq); cp.temperature = a.temperature;
     cp.part_count = ctl + kCtlColItems;
     const int grid_c = cp.split ? n_sm : cp.n_items;
     if (launch_behind(attn_colsum_kernel, dim3(grid_c), dim3(kColThreads), col_smem, stream, tm_qs, tm_kh, tm_kr,
                       cp) != cudaSuccess)
       return STAC_ERR_CUDA;
-    if (col_split && a.scores != nullptr)
+    if (scored_apart && a.scores != nullptr)
       return stac_scores_update(a.colsum, a.colsum_head_stride, a.scores, a.counts, a.score_stride, a.H, a.T_hot, a.old_T,
                                 a.score_Tq, a.temperature, reinterpret_cast<stac_stream_t>(stream));
   }

@@ -93,7 +93,7 @@ class HeavyHittersKV(KVManager):
 
     def _attend_and_score(self, query_states, slot, *retrieved):
         """Attention whose column sums go into the running scores of the hot keys in the same call: in the kernel
-        that makes them where the heads are few (24 layers, 2 heads: 2911 -> 2870 us per step)."""
+        that makes them (24 layers, 2 heads: 2911 -> 2870 us per step; 16 heads: 3469 -> 3415)."""
         Tq, T_live = query_states.shape[1], self._offset_hot[slot]
         update = None
         if T_live > 0:
