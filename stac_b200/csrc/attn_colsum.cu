@@ -33,9 +33,9 @@ constexpr int kFwdStages = 4;
 constexpr int kFwdThreads = 384;       // warpgroup 0: warp 0 TMA, warp 1 MMA (2, 3 idle); warpgroups 1, 2: softmax
 static_assert(128 * 40 + 256 * 232 <= kFwdThreads * ((65536 / kFwdThreads) / 8 * 8),
               "exact forward kernel: setmaxnreg targets exceed the CTA's register allocation");
-constexpr int kColGroup = 3;           // key tiles per item = exponent warpgroups of the column-sum kernel
-constexpr int kColStages = kColGroup == 4 ? 3 : 4;
-constexpr int kColThreads = 128 + kColGroup * 128;   // warpgroup 0 control (warp 0 TMA, warp 1 MMA issue), then exponent
+constexpr int kColGroup = 3;           // key tiles per item = exponent warpgroups of the column-sum kernel (two or one in short calls)
+constexpr int kColStages = 4;
+constexpr int col_threads(int group) { return 128 + group * 128; }   // warpgroup 0 control (warp 0 TMA, warp 1 MMA issue), then exponent
 #ifndef STAC_COL_PAIR_MASK
 #define STAC_COL_PAIR_MASK 0x88
 #endif
@@ -48,13 +48,12 @@ constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;   // which of 8 consecutiv
 // exponent warps read nothing from shared memory; 0: they read it per score (LDS.128 per four).
 constexpr bool kColFoldLse = STAC_COL_FOLD_LSE != 0;
 constexpr int kColXBytes = 128 * 32;   // 128 rows x 16 bf16, no swizzle: [16 row groups][2 K chunks][8 rows][16 B]
-constexpr int kColCtlRegs = 56;
-constexpr int kColExpRegs = kColGroup == 4 ? 104 : 152;
+constexpr int kColCtlRegs = 56, kColExpRegs = 152;
 // setmaxnreg only moves registers inside the CTA's allocation, which is fixed at launch to
 // (registers per thread the launch bound allows, a multiple of 8) x threads.  A request beyond
 // what the control warpgroup released would wait forever.
-constexpr int kColLaunchRegs = (65536 / kColThreads) / 8 * 8;
-static_assert(128 * kColCtlRegs + (kColThreads - 128) * kColExpRegs <= kColThreads * kColLaunchRegs,
+constexpr int kColLaunchRegs = (65536 / col_threads(kColGroup)) / 8 * 8;
+static_assert(128 * kColCtlRegs + 128 * kColGroup * kColExpRegs <= col_threads(kColGroup) * kColLaunchRegs,
               "column-sum kernel: setmaxnreg targets exceed the CTA's register allocation");
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -1027,7 +1026,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------
-// Column sums.  An item = (head, group of kColGroup 128-key tiles), head-major; its units are the
+// Column sums.  An item = (head, group of kGroup 128-key tiles: kColGroup, or two or one in short calls), head-major; its units are the
 // 128-row query tiles.  All units of the launch form one sequence that is cut into equal
 // contiguous ranges, one per persistent CTA, so every SM gets the same amount of work; an item
 // that straddles a cut is finished by two CTAs, each adding its partial sums to the zeroed
@@ -1037,7 +1036,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 // (N = 64, two 64-column TMEM buffers per key tile); warpgroup w owns key tile w, one key
 // (TMEM lane) per thread, so a thread's column sum never leaves its registers.  Three exponent
 // warps per scheduler keep the exp2 unit busier than two did (85 % against 75 % of the active
-// cycles); a fourth (kColGroup = 4, 104 registers per thread) measured the same as three.
+// cycles); a fourth (104 registers per thread) measured the same as three.
 // The last query tile is ragged unless M_sub is a multiple of 128 (one frame of 1041 tokens fills 17
 // of its rows): its second half is not scored when no row lies in it, and of the half that holds
 // the last row only the 16-row pieces up to that row are exponentiated.
@@ -1046,11 +1045,11 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 // lse2 holds the row log-sum-exp in the log2 domain; rows past M_sub read as +inf so that
 // padded query columns contribute exp2(-inf) = 0.
 // ---------------------------------------------------------------------------------------
-constexpr int kColExpThreads = kColGroup * 128;
 constexpr int kColHalf = 64;           // query rows per score buffer
 
+template <int kGroup>
 struct ColSmem {
-  uint8_t k[2][kColGroup][kTileBytes];  // [item parity][key tile of the group]
+  uint8_t k[2][kGroup][kTileBytes];     // [item parity][key tile of the group]
   uint8_t q[kColStages][kTileBytes];
   uint64_t k_full[2];
   uint64_t k_empty[2];
@@ -1162,8 +1161,8 @@ __device__ __forceinline__ void col_exp_chunk16(const uint32_t (&s)[32], const f
 // A 64-row half is read from TMEM in four pieces of 16 rows, the next piece always in flight
 // (the first piece of the next half included: its buffer does not depend on this warpgroup
 // finishing the current one).  `tail` > 0: the last half has only that many pieces with rows (1 to 3).
-template <bool kFast>
-__device__ __forceinline__ float col_item_sum(ColSmem& sm, const ColParams& p, uint32_t t_base, const float* nl_item,
+template <bool kFast, class Smem>
+__device__ __forceinline__ float col_item_sum(Smem& sm, const ColParams& p, uint32_t t_base, const float* nl_item,
                                               int n_half, int tail, int& ui, float c2, float b2_in) {
   uint32_t ra[32], rb[32];   // 16 registers of each are used
   float a0 = 0.f;
@@ -1231,11 +1230,14 @@ __device__ __forceinline__ float col_item_sum(ColSmem& sm, const ColParams& p, u
   return a0 + ((b0 + b1) + (b2 + b3));
 }
 
-__global__ void __launch_bounds__(kColThreads, 1)
+template <int kGroup>
+__global__ void __launch_bounds__(col_threads(kGroup), 1)
 attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k_hot,
                    const __grid_constant__ CUtensorMap tm_k_ret, const ColParams p) {
   extern __shared__ uint8_t smem_raw[];
-  ColSmem& sm = *reinterpret_cast<ColSmem*>(align1024(smem_raw));
+  using Smem = ColSmem<kGroup>;
+  Smem& sm = *reinterpret_cast<Smem*>(align1024(smem_raw));
+  constexpr int kExpThreads = kGroup * 128;
   STAC_TS(2, false);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1246,7 +1248,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&sm.k_full[i], 1);
       mbar_init(&sm.k_empty[i], 1);
       mbar_init(&sm.s_full[i], 1);
-      mbar_init(&sm.s_free[i], kColExpThreads);
+      mbar_init(&sm.s_free[i], kExpThreads);
     }
     for (int s = 0; s < kColStages; ++s) {
       mbar_init(&sm.q_full[s], 1);
@@ -1277,7 +1279,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   grid_dep_wait();
 
   if (warp < 4) {
-    setmaxnreg_dec<kColCtlRegs>();
+    if constexpr (kGroup == kColGroup) setmaxnreg_dec<kColCtlRegs>();   // (smaller CTAs have registers enough)
     if (warp == 0 && lane == 0) {
       // ------------------------------------------------------------------ TMA producer
       tma_prefetch_desc(&tm_q);
@@ -1288,10 +1290,10 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int h = item / p.n_groups, grp = item - h * p.n_groups;   // head-major item order
         const int kb = n & 1;
         if (n >= 2) mbar_wait(&sm.k_empty[kb], ((n >> 1) - 1) & 1, p.err, DEV_TIMEOUT_CONSUMER);
-        mbar_arrive_expect_tx(&sm.k_full[kb], kColGroup * kTileBytes);
+        mbar_arrive_expect_tx(&sm.k_full[kb], kGroup * kTileBytes);
 #pragma unroll
-        for (int t = 0; t < kColGroup; ++t) {
-          const int j = min(kColGroup * grp + t, p.n_tiles - 1);
+        for (int t = 0; t < kGroup; ++t) {
+          const int j = min(kGroup * grp + t, p.n_tiles - 1);
           if (j < p.n_hot_tiles) tma_load_3d(sm.k[kb][t], &tm_k_hot, &sm.k_full[kb], 0, j * kBN, h);
           else tma_load_3d(sm.k[kb][t], &tm_k_ret, &sm.k_full[kb], 0, (j - p.n_hot_tiles) * kBN, h);
         }
@@ -1354,7 +1356,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       for (; walk.next(item, i0, i1); ++n) {
         const int kb = n & 1;
         mbar_wait(&sm.k_full[kb], (n >> 1) & 1, p.err, DEV_TIMEOUT_TMA);
-        const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(kb * kColGroup * (kTileBytes >> 4));
+        const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(kb * kGroup * (kTileBytes >> 4));
         for (int i = i0; i < i1; ++i) {
           mbar_wait(&sm.q_full[s], s_round & 1, p.err, DEV_TIMEOUT_TMA);
           if (kColFoldLse) mbar_wait(&sm.x_full[s], s_round & 1, p.err, DEV_TIMEOUT_CONSUMER);
@@ -1370,7 +1372,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tc_fence_after();
             if (elect_one()) {
 #pragma unroll
-              for (int t = 0; t < kColGroup; ++t) {
+              for (int t = 0; t < kGroup; ++t) {
                 const uint64_t kd = k_desc + static_cast<uint64_t>(t * (kTileBytes >> 4));
                 umma_ss(d + t * 128, kd, q_desc, idesc, 0u);
                 umma_ss(d + t * 128, kd + 2, q_desc + 2, idesc, 1u);
@@ -1396,7 +1398,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     }
   } else {
     // ------------------------------------------------------------------ exponent warpgroups
-    setmaxnreg_inc<kColExpRegs>();
+    if constexpr (kGroup == kColGroup) setmaxnreg_inc<kColExpRegs>();
     const int w = (warp - 4) >> 2;   // which key tile of the group
     const int wq = warp & 3;
     const int key = wq * 32 + lane;  // key inside the tile = TMEM lane
@@ -1413,16 +1415,16 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       float* nl_s = sm.lse2;
       if (!kColFoldLse && h != cur_h) {
         cur_h = h;
-        named_bar_sync(1, kColExpThreads);   // everyone is done with the previous head's values
-        for (int r = tid; r < nq * kBM; r += kColExpThreads) {
+        named_bar_sync(1, kExpThreads);   // everyone is done with the previous head's values
+        for (int r = tid; r < nq * kBM; r += kExpThreads) {
           float v = -INFINITY;
           if (r < p.M_sub)
             v = -p.lse2[static_cast<long long>(h) * p.lse2_stride + static_cast<long long>(r) * p.row_stride];
           nl_s[r] = v;
         }
-        named_bar_sync(1, kColExpThreads);
+        named_bar_sync(1, kExpThreads);
       }
-      const int j = kColGroup * grp + w;
+      const int j = kGroup * grp + w;
       const bool exists = j < p.n_tiles;
       const bool is_ret = j >= p.n_hot_tiles;
       const int n0 = (is_ret ? j - p.n_hot_tiles : j) * kBN;
@@ -1470,7 +1472,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         *dst = total;
         update_score(total);
       };
-      constexpr int kSlot = kColGroup * kBN;
+      constexpr int kSlot = kGroup * kBN;
       if (i0 == 0 && i1 == nq) {
         if (key < valid) finish(sum);
       } else if (p.parts == nullptr) {
@@ -1492,9 +1494,9 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         float* slot = p.parts + static_cast<size_t>(2 * blockIdx.x + (i0 > 0 ? 0 : 1)) * kSlot;
         slot[w * kBN + key] = key < valid ? sum : 0.f;
         __threadfence();                          // this thread's part is visible device-wide ...
-        named_bar_sync(1, kColExpThreads);        // ... and so is every other key's
+        named_bar_sync(1, kExpThreads);        // ... and so is every other key's
         if (tid == 0) sm.join_flag = atomicAdd(p.part_count + item, 1);
-        named_bar_sync(1, kColExpThreads);
+        named_bar_sync(1, kExpThreads);
         if (sm.join_flag == c_last - c_first) {
           // every other part was complete before its counter increment, which came earlier
           __threadfence();
@@ -1609,8 +1611,11 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   float corr;
   attn_subsample_plan(a.M, a.subsample_ratio, &m_sub, &stride, &corr);
   const int nq = (m_sub + kBM - 1) / kBM;
-  const int col_smem = static_cast<int>(sizeof(ColSmem)) + (kColFoldLse ? 0 : nq * kBM * 4) + 1024;
-  if (col_smem > 227 * 1024) return STAC_ERR_BAD_ARG;
+  auto col_smem = [&](int group) {
+    const size_t fixed = group == 1 ? sizeof(ColSmem<1>) : group == 2 ? sizeof(ColSmem<2>) : sizeof(ColSmem<3>);
+    return static_cast<int>(fixed) + (kColFoldLse ? 0 : nq * kBM * 4) + 1024;
+  };
+  if (col_smem(kColGroup) > 227 * 1024) return STAC_ERR_BAD_ARG;
   const int fast_smem = static_cast<int>(sizeof(FastSmem)) + 1024;
   if (attr_done.needs_setup(dev)) {
     if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem) != cudaSuccess)
@@ -1618,9 +1623,9 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     if (cudaFuncSetAttribute(attn_fwd_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fast_smem) !=
         cudaSuccess)
       return STAC_ERR_CUDA;
-    if (cudaFuncSetAttribute(attn_colsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
-        cudaSuccess)
-      return STAC_ERR_CUDA;
+    for (auto* kernel : {attn_colsum_kernel<1>, attn_colsum_kernel<2>, attn_colsum_kernel<kColGroup>})
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+        return STAC_ERR_CUDA;
     attr_done.mark(dev);
   }
 
@@ -1698,12 +1703,21 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   // the output for that; a join through the workspace took 1 to 2 us more per call).  With fewer items (few heads,
   // short key ranges) and a workspace, the units are still cut evenly; an item may then have three or more parts,
   // which go through the workspace and are added in CTA order by the CTA that finishes last.
-  const int col_items = ((fp.n_hot_tiles + fp.n_ret_tiles + kColGroup - 1) / kColGroup) * a.H;
+  const int col_tiles = fp.n_hot_tiles + fp.n_ret_tiles;
+  auto items_of = [&](int group) { return (col_tiles + group - 1) / group * a.H; };
+  const int col_items = items_of(kColGroup);
   const bool col_split = a.colsum != nullptr && col_items >= n_sm;
   // (worth it from about six units per CTA: below that the extra key-tile loads and the join of a
   // CTA that touches two items cost more than the even cut gains; measured at M = 1041, N = 2082)
   const bool col_parts = a.colsum != nullptr && !col_split && part != nullptr && n_sm <= kFastMaxCtas &&
                          static_cast<long long>(col_items) * nq >= 6ll * n_sm;
+  // Where a call is one wave of one item per CTA, smaller groups fill more SMs as long as they are still one wave: a CTA's
+  // query tiles then take an exponent unit less time each, although fewer warps keep it busy.  us per call with groups of
+  // three / two / one (where that is one wave): M 1041, N 2082, 16 heads 37.6 / 34.6; M 1041, N 1041 32.6 / 29.0 / 27.6; M 200,
+  // N 300, 2 heads 16.6 / 15.6 / 14.8; M 4164, N 1041, 2 heads 69.9 / 55.6 / 44.7.  Same sums in the same order.
+  int col_group = kColGroup;
+  if (!col_split && !col_parts)
+    while (col_group > 1 && items_of(col_group - 1) <= n_sm) --col_group;
   // Every call leaves the control words as it found them, so a workspace that was zeroed once needs no
   // clearing: one memset less per call, and the forward kernel follows the kernel before it directly
   // (M = 1041, N = 2082, H = 16: 42.5 -> 38.2 us per call).
@@ -1727,7 +1741,7 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     cp.T_hot = a.T_hot; cp.T_ret = a.T_ret;
     cp.n_hot_tiles = fp.n_hot_tiles; cp.n_q_tiles = nq;
     cp.n_tiles = fp.n_hot_tiles + fp.n_ret_tiles;
-    cp.n_groups = (cp.n_tiles + kColGroup - 1) / kColGroup;
+    cp.n_groups = (cp.n_tiles + col_group - 1) / col_group;
     cp.n_items = cp.n_groups * a.H;
     cp.scale_log2 = scale_log2; cp.correction = corr;
     cp.bias_ret = a.bias_ret; cp.bias_head_stride = a.bias_head_stride;
@@ -1745,8 +1759,10 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     cp.old_T = a.old_T; cp.tq = static_cast<float>(a.score_Tq); cp.temperature = a.temperature;
     cp.part_count = ctl + kCtlColItems;
     const int grid_c = cp.split ? n_sm : cp.n_items;
-    if (launch_behind(attn_colsum_kernel, dim3(grid_c), dim3(kColThreads), col_smem, stream, tm_qs, tm_kh, tm_kr,
-                      cp) != cudaSuccess)
+    auto* const col_kernel = col_group == 1 ? attn_colsum_kernel<1> : col_group == 2 ? attn_colsum_kernel<2>
+                                                                                     : attn_colsum_kernel<kColGroup>;
+    if (launch_behind(col_kernel, dim3(grid_c), dim3(col_threads(col_group)), col_smem(col_group), stream, tm_qs, tm_kh,
+                      tm_kr, cp) != cudaSuccess)
       return STAC_ERR_CUDA;
     if (scored_apart && a.scores != nullptr)
       return stac_scores_update(a.colsum, a.colsum_head_stride, a.scores, a.counts, a.score_stride, a.H, a.T_hot, a.old_T,

@@ -105,6 +105,16 @@ def test_units_split_over_all_sms():
     assert np.array_equal(got[2], again[2])          # shared items sum to the same bits every run
 
 
+@pytest.mark.parametrize("M,H,T_hot,T_ret", [
+    (130, 4, 4736, 0),      # 148 key tiles: groups of one
+    (130, 4, 4737, 0),      # one tile more: groups of two, the last of a head half empty
+    (70, 4, 4600, 129),     # hot and retrieved tiles in one group of two
+    (130, 4, 9470, 2),      # 75 groups of two: of three
+])
+def test_column_sum_groups_of_one_two_and_three_tiles(M, H, T_hot, T_ret):
+    _assert_close(*_run_two_segment(M, H, T_hot, T_ret, seed=M + T_hot))
+
+
 def test_forward_units_split_over_all_sms():
     """More (head, query tile) items than SMs: the forward kernel runs one CTA per SM over equal
     ranges of (item, key tile) units; items on a cut are computed in two parts and joined."""
