@@ -281,6 +281,37 @@ def test_leading_masked_tile_then_faint_keys():
     _assert_close((out.float().cpu().numpy(), lse.cpu().numpy(), cs.cpu().numpy()), (o_ref, lse_ref, cs_ref))
 
 
+@pytest.mark.parametrize("M,H,N", [(70, 2, 1), (130, 2, 112), (130, 3, 449), (257, 2, 1000), (2600, 8, 900), (1100, 2, 2000)])
+@pytest.mark.parametrize("kind", ["counts", "mask", "lowest", "huge", "scale"])
+def test_a_bias_on_every_key(M, H, N, kind):
+    """The bias goes through the tensor core before the scale: log counts with masked keys and whole masked tiles (first, middle,
+    last of a head), a type's lowest value as the mask, finite biases that do not fit before the scale (recomputed by the
+    exact kernel), a scale that is not a power of two.  One CTA per item, items cut over the SMs, items in halves."""
+    from stac_b200 import ops
+    rs = np.random.RandomState(M + N)
+    q, k, v = (_bf16(rs.randn(*s).astype(np.float32)) for s in ((M, H, 64), (N, H, 64), (N, H, 64)))
+    bias = np.log(rs.randint(1, 9, size=(H, N)).astype(np.float32))
+    scale = 0.1 if kind == "scale" else 0.125
+    if kind == "huge":
+        bias -= np.float32(3e37)       # eight times that is beyond 1e38
+    elif kind != "counts" and N > 1:
+        masked = rs.rand(H, N) < 0.25
+        for h, tile in ((0, 0), (1, 3), (H - 1, (N - 1) // 112)):
+            masked[h, 112 * tile:112 * (tile + 1)] = N > 112
+        bias[masked] = np.finfo(np.float32).min if kind == "lowest" else -np.inf
+    dev = torch.device("cuda:0")
+    status = ops.DeviceStatus(dev)
+    got = ops.attn_colsum(q.to(dev), None, None, 0, k.to(dev), v.to(dev), torch.from_numpy(bias).to(dev), N, layout="thd",
+                          scale=scale, want_lse=True, status=status)
+    torch.cuda.synchronize()
+    status.raise_if_set("attention")
+    o, lse, cs = oracle_attn(q.float().numpy(), k.float().numpy(), v.float().numpy(), bias, scale=scale)
+    got = [x.float().cpu().numpy() for x in got]
+    if kind == "huge":
+        cs = got[2]      # column sums are computed for log-sum-exps up to 1e29
+    _assert_close(got, (o, lse, cs))
+
+
 def test_calls_replay_from_a_cuda_graph():
     """The entry point neither allocates nor synchronises, so calls can be captured into a CUDA
     graph (the programmatic-serialization edges between its kernels included); a replay gives the
