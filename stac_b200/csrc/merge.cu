@@ -208,13 +208,187 @@ __device__ __forceinline__ int4 block_scan4(int4 v, int4* warp_sums, int4* total
 }
 
 // ------------------------------------------------------------------------------------ sort
-// Threads: 1024, two CTAs per SM, as long as that is one wave of heads, else 512 and four per SM: the kernel is
-// a chain of latencies and barriers, and a second wave costs as much as the first.
-// (384 heads: 8328 tokens each 121 -> 106 us, 1041 each 31.9 -> 19.3 us.  16 heads, 8328 tokens: 44.7 -> 34.3 us since
-// the digits are counted with shared-memory adds; matching the lanes of a warp first cost more than the adds'
-// conflicts.)
-template <int kThreads>
-__global__ void __launch_bounds__(kThreads, 2048 / kThreads) sort_tokens_kernel(const MergeParams p) {
+// A CTA per head: a chain of latencies and barriers, so that a second wave of CTAs costs as much as the first.  The
+// number of heads decides how many have to share an SM (see launch_merge).
+// (Digits are counted with shared-memory adds; matching the lanes of a warp first cost more than the adds' conflicts.)
+// Lanes of the warp that are `in` and have this lane's digit, by eight ballots.  (__match_any_sync takes longer the more digits
+// there are: 16 heads of 8328 tokens, the first scatter 16.3 thousand cycles with it, 9.2 with ballots.)
+__device__ __forceinline__ unsigned same_digit(bool in, unsigned digit) {
+  unsigned peers = __ballot_sync(kFull, in);
+#pragma unroll
+  for (int bit = 0; bit < 8; ++bit) {
+    const bool set = (digit >> bit) & 1u;
+    const unsigned m = __ballot_sync(kFull, set);
+    peers &= set ? m : ~m;
+  }
+  return peers;
+}
+
+// Lists of up to kThreads * kItems tokens and voxel ids of 16 bits are sorted in shared memory (sort_tokens_shared), others
+// through the lists in global memory (the rest of this kernel).
+__device__ __forceinline__ int warp_scan_sum(int v, int lane) {      // inclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
+}
+
+// One word per token, voxel id above its place in the list (evicted tokens by position, then carried ones), in one array: a
+// warp takes its part of it into registers before a pass scatters.  Tokens that are not valid take the id 0xFFFF and end
+// up behind the others, so nothing is compacted first; rows are found in one sweep.
+// (8328 tokens each: 16 heads 34.5 -> 21.4 us, 384 heads 105.5 -> 70.3; 4164 each, 384 heads 54.5 -> 44.5; 1041 each, 384 heads
+// 19.4 -> 14.1.  The lists in global memory cost a scattered 4-byte write per key, value and pass, and a round trip
+// to L2 around every block scan, one per 4 kThreads tokens.)
+template <int kThreads, int kItems>
+__device__ __forceinline__ void sort_tokens_shared(const MergeParams& p, int h, int os, int n_items, unsigned* buf, int* hist) {
+  constexpr int kWarps = kThreads / 32, kHistRow = 257;
+  constexpr unsigned kNone = 0xFFFFu;
+  __shared__ int counts[kWarps];
+  __shared__ int scan_sums[32];
+  __shared__ int scan_total, n_new_valid, n_valid;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int chunk = ((n_items + kWarps - 1) / kWarps + 31) / 32 * 32;    // items per warp, at most 32 kItems
+  const int c0 = warp * chunk, c1 = min(n_items, c0 + chunk);
+  if (threadIdx.x == 0) n_new_valid = n_valid = 0;
+  const int n_it = (max(c1 - c0, 0) + 31) / 32;        // rounds of 32 items in which this warp has any
+  unsigned item[kItems];
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {       // positions first, so that all loads of a thread are in flight together
+    const int i = c0 + t * 32 + lane;
+    item[t] = i;
+    if (t < n_it && p.idx != nullptr && i < c1 && i < p.n_new) item[t] = p.idx[static_cast<long long>(h) * p.n_new + i];
+  }
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {
+    if (t < n_it) {
+      const int i = c0 + t * 32 + lane;
+      int vx = -1;
+      if (i < c1) vx = i < p.n_new ? p.vx_src[h * p.meta_head_stride + static_cast<int>(item[t])] : p.over_hv_in[2 * (os + i - p.n_new) + 1];
+      item[t] = vx;
+    }
+  }
+  int* my_hist = hist + warp * kHistRow;
+  auto clear_hist = [&] {
+    for (int i = lane; i < 256; i += 32) my_hist[i] = 0;
+    __syncwarp();
+  };
+  auto count = [&](unsigned w, int shift) { atomicAdd(&my_hist[(w >> shift) & 255u], 1); };
+  clear_hist();
+  __syncthreads();
+  int new_valid = 0, valid = 0;
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {
+    if (t < n_it) {
+      const int i = c0 + t * 32 + lane;
+      const bool ok = static_cast<int>(item[t]) >= 0 && static_cast<int>(item[t]) < p.voxel_used;
+      new_valid += __popc(__ballot_sync(kFull, ok && i < p.n_new));
+      valid += __popc(__ballot_sync(kFull, ok));
+      item[t] = (ok ? item[t] << 16 : kNone << 16) | static_cast<unsigned>(i);
+      if (i < c1) {
+        buf[i] = item[t];
+        count(item[t], 16);
+      }
+    }
+  }
+  if (lane == 0) {
+    atomicAdd(&n_new_valid, new_valid);
+    atomicAdd(&n_valid, valid);
+  }
+#pragma unroll 1
+  for (int shift = 16; shift < 32; shift += 8) {
+    if (shift > 16) {
+      clear_hist();
+      for (int t = 0; t < n_it; ++t)
+        if (c0 + t * 32 + lane < c1) count(buf[c0 + t * 32 + lane], shift);
+    }
+    __syncthreads();
+    // exclusive scan of the counters in (digit, warp) order: 8 consecutive entries per thread
+    int loc[8];
+    int sum = 0;
+    constexpr int kParts = kWarps / 8;      // threads per digit
+    int* of_thread = hist + (threadIdx.x % kParts) * 8 * kHistRow + threadIdx.x / kParts;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      loc[e] = of_thread[e * kHistRow];
+      sum += loc[e];
+    }
+    int run = block_scan<kWarps>(sum, scan_sums, &scan_total);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      of_thread[e * kHistRow] = run;
+      run += loc[e];
+    }
+#pragma unroll
+    for (int t = 0; t < kItems; ++t)
+      if (t < n_it && c0 + t * 32 + lane < c1) item[t] = buf[c0 + t * 32 + lane];
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+      if (t < n_it) {                       // warp-uniform
+        const bool in = c0 + t * 32 + lane < c1;
+        const unsigned d = (item[t] >> shift) & 255u;
+        const unsigned peers = same_digit(in, d);
+        const unsigned before = peers & ((1u << lane) - 1);
+        if (in) buf[my_hist[d] + __popc(before)] = item[t];
+        __syncwarp();
+        if (in && before == 0) my_hist[d] += __popc(peers);
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+  }
+  // rows of the sorted list: a bit per item that starts one, then everything that is known about the items
+  const int n = n_valid, c1_valid = min(c1, n);
+  unsigned starts = 0;
+  int n_starts = 0;
+  for (int t = 0; t < n_it; ++t) {
+    const int i = c0 + t * 32 + lane;
+    const bool start = i < c1_valid && (i == 0 || buf[i - 1] >> 16 != buf[i] >> 16);
+    starts |= (start ? 1u : 0u) << t;
+    n_starts += __popc(__ballot_sync(kFull, start));
+  }
+  if (lane == 0) counts[warp] = n_starts;
+  __syncthreads();
+  const int incl = warp_scan_sum(lane < kWarps ? counts[lane] : 0, lane);
+  int r0 = warp > 0 ? __shfl_sync(kFull, incl, warp - 1) : 0;      // rows that start before this warp's items
+  const int n_rows = __shfl_sync(kFull, incl, kWarps - 1);
+  const long long hb = static_cast<long long>(h) * p.ncap;
+  unsigned int* keys = ((p.passes & 1) ? p.keys_b : p.keys_a) + hb;
+  int* codes = ((p.passes & 1) ? p.vals_b : p.vals_a) + hb;
+  int* rst = p.row_start + static_cast<long long>(h) * (p.ncap + 1);
+  for (int t = 0; t < n_it; ++t) {
+    const int i = c0 + t * 32 + lane;
+    const unsigned m = __ballot_sync(kFull, (starts >> t) & 1u);
+    if (i < c1_valid) {
+      const int r = r0 + __popc(m & (0xffffffffu >> (31 - lane))) - 1;
+      const unsigned key = buf[i] >> 16;
+      const int at = static_cast<int>(buf[i] & 0xFFFFu);
+      keys[i] = key;
+      codes[i] = at < p.n_new ? at : ~(os + at - p.n_new);
+      p.tok_row[hb + i] = r;
+      if ((starts >> t) & 1u) {
+        p.row_vx[hb + r] = static_cast<int>(key);
+        rst[r] = i;
+        p.row_flag[hb + r] = 0;
+      }
+      // the token behind kLongRow others of its row lists it
+      if (i >= kLongRow && buf[i - kLongRow] >> 16 == key && (i == kLongRow || buf[i - kLongRow - 1] >> 16 != key))
+        p.long_list[list_push(&p.plan[kPlanLongCount])] = make_int2(h, r);
+    }
+    r0 += __popc(m);
+  }
+  if (threadIdx.x == 0) {
+    rst[n_rows] = n;
+    p.n_rows[h] = n_rows;
+    p.n_tok[h] = n;
+    if (n_new_valid > 0) atomicOr(&p.plan[kPlanAnyValid], 1);
+  }
+}
+
+template <int kThreads, int kMinCtas, int kItems>
+__global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const MergeParams p) {
   constexpr int kWarps = kThreads / 32;
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
   // Digit counters, [warp][digit]: a warp's lanes count different digits of the same warp, so neighbouring
@@ -222,11 +396,19 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) sort_tokens_kernel(
   // digit, read without conflicts too.  ([digit][warp] put all of a warp's counters in one bank.)
   // (384 heads, 8328 tokens each: insert + retrieval 1112 -> 1068 us; 16 heads, fp32: 278 -> 263 us.)
   constexpr int kHistRow = 257;
-  __shared__ int hist[kHistRow * kWarps];
+  extern __shared__ int sort_smem[];
+  int* hist = sort_smem;               // [kHistRow * kWarps]
   __shared__ int warp_sums[32];
   __shared__ int sh_total;
   __shared__ int sh_carry;
   const int h = blockIdx.x;
+  if constexpr (kItems > 0) {
+    const int os = p.over_start_in[h], n_items = p.n_new + p.over_start_in[h + 1] - os;
+    if (n_items <= min(p.ncap, kThreads * kItems) && p.voxel_used <= 0xFFFF) {
+      sort_tokens_shared<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem + kHistRow * kWarps), hist);
+      return;
+    }
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned int* ka = p.keys_a + static_cast<long long>(h) * p.ncap;
   unsigned int* kb = p.keys_b + static_cast<long long>(h) * p.ncap;
@@ -333,8 +515,8 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) sort_tokens_kernel(
     }
     __syncthreads();
     auto scatter = [&](bool in, unsigned int key, int val) {
-      const unsigned int d = in ? ((key >> shift) & 255u) : (256u + lane);
-      const unsigned int peers = __match_any_sync(kFull, d);
+      const unsigned int d = (key >> shift) & 255u;
+      const unsigned int peers = same_digit(in, d);
       const unsigned int before = peers & ((1u << lane) - 1);
       if (in) {
         const int dst = my_hist[d] + __popc(before);
@@ -1601,15 +1783,35 @@ ScratchLayout scratch_layout(int heads, int ncap, int buf_cap) {
   return L;
 }
 
+// One wave of CTAs wherever there can be one, a second wave costs as much as the first: a head has an SM to itself, shares it
+// with one other head, or with two or three, whose shared memory holds 8704 or 2048 tokens each; more heads with longer lists
+// sort in global memory.
+cudaError_t launch_sort(const MergeParams& mp, int dev, int n_sm, cudaStream_t st) {
+  auto launch = [&](auto* kernel, int threads, int items) {
+    return launch_behind(kernel, dim3(mp.heads), dim3(threads), (257 * (threads / 32) + threads * items) * 4, st, mp);
+  };
+  static PerDeviceFlag attr_done;       // the shared-memory opt-in is made once per device
+  if (attr_done.needs_setup(dev)) {
+    for (auto* kernel : {sort_tokens_kernel<1024, 1, 9>, sort_tokens_kernel<1024, 2, 9>, sort_tokens_kernel<512, 3, 17>,
+                         sort_tokens_kernel<512, 4, 4>}) {
+      const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
+      if (rc != cudaSuccess) return rc;
+    }
+    attr_done.mark(dev);
+  }
+  if (mp.heads <= n_sm) return launch(sort_tokens_kernel<1024, 1, 9>, 1024, 9);
+  if (mp.heads <= 2 * n_sm) return launch(sort_tokens_kernel<1024, 2, 9>, 1024, 9);
+  if (mp.heads <= 4 * n_sm && mp.n_new <= 1536) return launch(sort_tokens_kernel<512, 4, 4>, 512, 4);   // (512 carried ones)
+  if (mp.heads <= 3 * n_sm) return launch(sort_tokens_kernel<512, 3, 17>, 512, 17);
+  return launch(sort_tokens_kernel<512, 4, 0>, 512, 0);
+}
+
 template <typename T>
 int launch_merge(MergeParams& mp, cudaStream_t st) {
   if (cudaMemsetAsync(mp.plan, 0, kPlanSize * 4, st) != cudaSuccess) return STAC_ERR_CUDA;
   int dev, n_sm;
   if (current_device(&dev) != STAC_OK || device_sm_count(dev, &n_sm) != STAC_OK) return STAC_ERR_CUDA;
-  const bool one_wave = mp.heads <= 2 * n_sm;
-  if (launch_behind(one_wave ? sort_tokens_kernel<1024> : sort_tokens_kernel<512>, dim3(mp.heads), dim3(one_wave ? 1024 : 512), 0, st,
-                    mp) != cudaSuccess)
-    return STAC_ERR_CUDA;
+  if (launch_sort(mp, dev, n_sm, st) != cudaSuccess) return STAC_ERR_CUDA;
   dim3 grid_a1((mp.ncap + 255) / 256, mp.heads);
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
   if (launch_behind(tokens_sim_merge_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;

@@ -677,6 +677,39 @@ def test_launches_are_counted_where_they_are_made():
         assert _lib.kernel_launches() - before == want
 
 
+@pytest.mark.parametrize("heads,Tn,voxels,used", [
+    (4, 1, 3, 3), (4, 33, 5, 5), (4, 1500, 300, 70000),     # one token; lists in shared and in global memory (ids above 16 bits)
+    (200, 2500, 500, 500),                                  # two heads per SM
+    (300, 1500, 40, 40), (300, 1537, 300, 300),             # four per SM (in the second call more carried tokens than it holds), three
+    (300, 9000, 1800, 1800), (460, 1600, 300, 300),         # too long for three per SM; more heads than three per SM
+])
+def test_sorts_of_all_shapes_give_the_same_memory(heads, Tn, voxels, used):
+    """The list of a head is sorted in shared memory by CTAs of three shapes, or in global memory: the same tokens in two of the
+    ``heads``, and alone in a memory of two heads whose lists are sorted in shared memory, leave the same rows."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    D, two = 64, [0, heads - 1]
+    g = torch.Generator(device=DEV).manual_seed(Tn)
+    many, small = (VoxelKVMerger(h, D, init_voxels=n, pivot_cap=4, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8, score_thresh=0.1,
+                                 dtype=torch.bfloat16, device=DEV, allocator="segment", seg_size=1, slab_cap=16)
+                   for h, n in ((heads, used), (2, voxels)))
+
+    def rows(vm, which):
+        res = []
+        for cnt, seg, fields in ((vm._buf_row_cnt, vm._buf_row_seg, (vm._buf_K, vm._buf_V, vm._buf_S)),
+                                 (vm._piv_row_cnt, vm._piv_row_seg, (vm._piv_K, vm._piv_V, vm._piv_W, vm._piv_S, vm._piv_C))):
+            s = seg[which, :voxels]
+            res += [cnt[which, :voxels], s >= 0] + [f[s[s >= 0].long()] for f in fields]
+        return res
+
+    for step in range(3):
+        vx = torch.randint(-1, voxels, (heads, Tn), device=DEV, generator=g).int()     # -1: not in the memory
+        K, V = (torch.randn(heads, Tn, D, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+        S = torch.exp(torch.randint(0, 4, (heads, Tn), device=DEV, generator=g).float())
+        many.insert_and_merge(K, V, S, None, vx, used)
+        small.insert_and_merge(K[two].contiguous(), V[two].contiguous(), S[two].contiguous(), None, vx[two].contiguous(), voxels)
+        assert all(torch.equal(a, b) for a, b in zip(rows(many, two), rows(small, [0, 1]))), step
+
+
 @pytest.mark.parametrize("Tn", [2049, 4097, 8328])      # second listing round, past the registers, the pool-stress length
 def test_sort_of_many_heads_equals_the_sort_of_few(Tn):
     """300 heads take the sort's CTAs of 512 threads, four of them the ones of 1024 (which are compared with the oracle):
