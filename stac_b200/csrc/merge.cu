@@ -140,6 +140,7 @@ struct MergeParams {
   int2* merge_list;    // [heads*ncap] rows (head, row index) of more than kShortRow tokens with at least one merging token
   int passes;          // radix passes (8 bits each)
   int seg_vec;         // 1: the pivot segments of a row are one aligned 16-byte vector
+  int buf_seg_vec;     // 1: the buffer segments of a row are two of them
   int* err;
 };
 
@@ -1034,10 +1035,28 @@ __global__ void __launch_bounds__(256, 4) rows_merge_kernel(const MergeParams p)
 // the row's pivots times score_thresh (stac/merger.py:735-745).
 __device__ __forceinline__ float row_gate(const MergeParams& p, long long r, int npiv) {
   float sumS = 0.f, sumC = 0.f;
-  for (int q = 0; q < npiv; ++q) {
-    const int seg = p.piv_row_seg[r * p.P + q];
-    sumS = __fadd_rn(sumS, p.piv_S[seg]);
-    sumC = __fadd_rn(sumC, p.piv_C[seg]);
+  if (p.seg_vec) {       // all loads side by side
+    const int4 sg = reinterpret_cast<const int4*>(p.piv_row_seg)[r];
+    const int seg[kMaxP] = {sg.x, sg.y, sg.z, sg.w};
+    float S[kMaxP], C[kMaxP];
+#pragma unroll
+    for (int q = 0; q < kMaxP; ++q) {
+      S[q] = q < npiv ? p.piv_S[seg[q]] : 0.f;
+      C[q] = q < npiv ? p.piv_C[seg[q]] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < kMaxP; ++q) {
+      if (q < npiv) {
+        sumS = __fadd_rn(sumS, S[q]);
+        sumC = __fadd_rn(sumC, C[q]);
+      }
+    }
+  } else {
+    for (int q = 0; q < npiv; ++q) {
+      const int seg = p.piv_row_seg[r * p.P + q];
+      sumS = __fadd_rn(sumS, p.piv_S[seg]);
+      sumC = __fadd_rn(sumC, p.piv_C[seg]);
+    }
   }
   return __fmul_rn(__fdiv_rn(sumS, fmaxf(sumC, 1e-6f)), p.score_thresh);
 }
@@ -1148,6 +1167,79 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
   const int nbuf = p.buf_row_cnt[r];
   const float* tscore = p.tok_score + hb;
   int* tdest = p.tok_dest + hb;
+  int* od = p.old_dest + (hb + ri) * kMaxB;
+  auto publish = [&](int n_sel) {
+    const int n_cand = nbuf + n_sel;
+    const int newcnt = min(p.B, n_cand);
+    const int full = (n_sel > 0 && newcnt == p.B) ? 1 : 0;
+    int4 info;
+    info.x = newcnt - nbuf;
+    info.y = max(0, n_cand - p.B);
+    info.z = full | ((full && npiv < p.P) ? 2 : 0) | (nbuf << 4);
+    info.w = n_sel;
+    p.row_info[hb + ri] = info;
+  };
+  if (s1 - s0 <= kShortRow) {
+    // Most rows: all tokens in registers, their loads and those of the buffer's segments side by side.  (Token by token, as
+    // below, with scores read again for every comparison: 75.6 against 59.0 us in this kernel with 384 heads of
+    // 8328 tokens, 63.4 against 50.6 with 4164, 15.4 against 8.9 with 16 heads.)
+    const int n = s1 - s0;
+    float sc[kShortRow], sim[kShortRow];
+    int seg[kMaxB];
+#pragma unroll
+    for (int j = 0; j < kShortRow; ++j) {
+      sc[j] = j < n ? tscore[s0 + j] : 0.f;
+      sim[j] = j < n && npiv > 0 ? p.tok_sim[hb + s0 + j] : -INFINITY;
+    }
+#pragma unroll
+    for (int c = 0; c < kMaxB; c += 4) {
+      if (p.buf_seg_vec) {
+        const int4 sg = c < nbuf ? reinterpret_cast<const int4*>(p.buf_row_seg)[r * 2 + c / 4] : make_int4(0, 0, 0, 0);
+        seg[c] = sg.x; seg[c + 1] = sg.y; seg[c + 2] = sg.z; seg[c + 3] = sg.w;
+      } else {
+#pragma unroll
+        for (int e = c; e < c + 4; ++e) seg[e] = e < nbuf ? p.buf_row_seg[r * p.B + e] : 0;
+      }
+    }
+    const float gate = npiv > 0 ? row_gate(p, r, npiv) : -INFINITY;
+    unsigned sel = 0u;
+#pragma unroll
+    for (int j = 0; j < kShortRow; ++j)
+      if (j < n && (npiv == 0 || (sim[j] < p.replace_thresh && fmaxf(sc[j], 1e-6f) > gate))) sel |= 1u << j;
+    int old_rank[kMaxB];       // buffered tokens are stored in rank order
+#pragma unroll
+    for (int c = 0; c < kMaxB; ++c) old_rank[c] = c;
+    if (sel == 0u) {           // nothing to buffer: everything stays in its place
+#pragma unroll
+      for (int j = 0; j < kShortRow; ++j)
+        if (j < n) tdest[s0 + j] = -1;
+    } else {
+      float ex[kMaxB];
+#pragma unroll
+      for (int c = 0; c < kMaxB; ++c) ex[c] = c < nbuf ? p.buf_S[seg[c]] : 0.f;
+#pragma unroll
+      for (int c = 0; c < kMaxB; ++c)
+#pragma unroll
+        for (int j = 0; j < kShortRow; ++j) old_rank[c] += ((sel >> j) & 1u) && sc[j] > ex[c] ? 1 : 0;
+#pragma unroll
+      for (int j = 0; j < kShortRow; ++j) {
+        if (j < n) {
+          int rank = 0;
+#pragma unroll
+          for (int c = 0; c < kMaxB; ++c) rank += c < nbuf && ex[c] >= sc[j] ? 1 : 0;
+#pragma unroll
+          for (int j2 = 0; j2 < kShortRow; ++j2)
+            rank += ((sel >> j2) & 1u) && (j2 < j ? sc[j2] >= sc[j] : sc[j2] > sc[j]) ? 1 : 0;
+          tdest[s0 + j] = (sel >> j) & 1u ? rank : -1;
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kMaxB; c += 4)      // (places behind the buffered ones are not read)
+      if (c < nbuf) *reinterpret_cast<int4*>(od + c) = make_int4(old_rank[c], old_rank[c + 1], old_rank[c + 2], old_rank[c + 3]);
+    publish(__popc(sel));
+    return;
+  }
   unsigned sel_mask = 0u;      // bit j: token s0 + j goes to the buffer
   if (npiv > 0) {
     const float gate = row_gate(p, r, npiv);
@@ -1159,8 +1251,6 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
   float ex[kMaxB];
 #pragma unroll
   for (int c = 0; c < kMaxB; ++c) ex[c] = (c < nbuf) ? p.buf_S[p.buf_row_seg[r * p.B + c]] : 0.f;
-  const int n_sel = __popc(sel_mask);
-  int* od = p.old_dest + (hb + ri) * kMaxB;
 #pragma unroll
   for (int c = 0; c < kMaxB; ++c) {
     if (c < nbuf) {
@@ -1185,15 +1275,7 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
     }
     tdest[i] = rank;
   }
-  const int n_cand = nbuf + n_sel;
-  const int newcnt = min(p.B, n_cand);
-  const int full = (n_sel > 0 && newcnt == p.B) ? 1 : 0;
-  int4 info;
-  info.x = newcnt - nbuf;
-  info.y = max(0, n_cand - p.B);
-  info.z = full | ((full && npiv < p.P) ? 2 : 0) | (nbuf << 4);
-  info.w = n_sel;
-  p.row_info[hb + ri] = info;
+  publish(__popc(sel_mask));
 }
 
 // One thread per row; the rows with more than kLongRow tokens are listed and ranked by a warp each, which
@@ -1907,6 +1989,7 @@ int stac_merge_insert(const stac_pool* pool, const stac_evicted* ev, void* scrat
   int bits = 1;
   while ((1ll << bits) < pool->voxel_used) ++bits;
   mp.passes = (bits + 7) / 8;
+  mp.buf_seg_vec = mp.B == stac::kMaxB && (reinterpret_cast<uintptr_t>(mp.buf_row_seg) & 15) == 0 ? 1 : 0;
   mp.seg_vec = mp.P == 4 && (reinterpret_cast<uintptr_t>(mp.piv_row_seg) & 15) == 0 ? 1 : 0;
   mp.err = dev_status;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
