@@ -41,7 +41,7 @@ class LaggedInts:
 
     def __init__(self, n):
         self.pin = torch.zeros(n, dtype=torch.int32).pin_memory()
-        self.event = None
+        self.event, self.waiting = None, False      # one event, recorded again by every push
         self.parts = {}      # sizes of the pushed tensors -> the slices of `pin` that they go to
 
     def push(self, *tensors):
@@ -51,17 +51,19 @@ class LaggedInts:
             parts = self.parts[sizes] = self.pin[:sum(sizes)].split(sizes)
         for part, t in zip(parts, tensors):
             part.copy_(t.reshape(-1), non_blocking=True)
-        self.event = torch.cuda.Event()
+        if self.event is None:
+            self.event = torch.cuda.Event()
         self.event.record()
+        self.waiting = True
 
     def pending(self):
-        return self.event is not None
+        return self.waiting
 
     def pull(self):
-        if self.event is None:
+        if not self.waiting:
             return None
         self.event.synchronize()
-        self.event = None
+        self.waiting = False
         return self.pin.tolist()
 
 
