@@ -112,6 +112,29 @@ def test_upsert_of_a_long_chunk_sorts_its_new_keys_outside_shared_memory():
         t_gpu.upsert_points(torch.zeros((131073, 3)))
 
 
+@pytest.mark.parametrize("T,n_recent,n_pinned,k", [(3, 1, 1, 0), (2047, 500, 0, 700), (2049, 0, 1, 1024), (4500, 1000, 37, 2000)])
+def test_h2o_select_of_many_rows(T, n_recent, n_pinned, k):
+    """More rows than two CTAs per SM hold take the smaller CTAs: the same positions."""
+    from stac_b200 import _lib
+    rs = np.random.RandomState(T)
+    rows = 310
+    scores = rs.rand(rows, T).astype(np.float32)
+    scores[5] = 0.5
+    scores[6] = np.round(scores[6], 2)
+    pinned = np.arange(n_pinned)
+    base = np.zeros(T, np.uint8)
+    base[T - n_recent:] = 1
+    base[pinned] = 1
+    n_keep = int(base.sum()) + k
+    keep = torch.empty((rows, n_keep), dtype=torch.int32, device=DEV)
+    drop = torch.empty((rows, T - n_keep), dtype=torch.int32, device=DEV)
+    assert _lib.lib().stac_h2o_select(_lib.ptr(torch.from_numpy(scores).to(DEV)), T, rows, _lib.ptr(torch.from_numpy(base).to(DEV)), T,
+                                      n_keep, _lib.ptr(keep), _lib.ptr(drop), _lib.stream_ptr()) == 0
+    keep, drop = keep.cpu().numpy(), drop.cpu().numpy()
+    assert np.array_equal(keep, h2o_keep_indices(scores, T, n_recent, pinned, k, 0))
+    assert np.array_equal(np.sort(np.concatenate([keep, drop], 1), 1), np.tile(np.arange(T), (rows, 1))) and (np.diff(drop) > 0).all()
+
+
 @pytest.mark.parametrize("T,n_recent,n_pinned,k", [(700, 200, 100, 150), (15615, 8328, 1041, 2082),
                                                      (333, 50, 0, 1), (1200, 100, 37, 1063)])
 def test_h2o_select_bit_exact(T, n_recent, n_pinned, k):
