@@ -39,7 +39,8 @@ constexpr int col_threads(int group) { return 128 + group * 128; }   // warpgrou
 #ifndef STAC_COL_PAIR_MASK
 #define STAC_COL_PAIR_MASK 0x88
 #endif
-constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;   // which of 8 consecutive PAIRS of exponentials of the column-sum kernel run on the FMA pipes
+// which of 8 consecutive PAIRS of exponentials of the column-sum kernel run on the FMA pipes
+constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;
 #ifndef STAC_COL_FOLD_LSE
 #define STAC_COL_FOLD_LSE 1
 #endif
@@ -486,13 +487,16 @@ constexpr int kFastCtlRegs = 64, kFastSoftmaxRegs = 104;
 static_assert(128 * kFastCtlRegs + 128 * kFastWgs * kFastSoftmaxRegs <= kFastThreads * ((65536 / kFastThreads) / 8 * 8),
               "fast forward kernel: setmaxnreg targets exceed the CTA's register allocation");
 
+template <bool kAllBiased>
 struct FastSmem {
   uint8_t q[2][kTileBytes];                     // query tile of the segment (parity)
   uint8_t k[kFastWgs][kFastTileBytes];
   uint8_t v[kFastWgs][kFastTileBytes];
-  float bias2[kFastWgs][kBN];                   // the biases of a tile (hot keys and pivots in one call)
-  alignas(16) uint8_t ax[kXBytes];              // a bias on every key: ones in K columns 0..2, same for every query
-  alignas(16) uint8_t bx[kFastWgs][kFT * 32];   // and per key its bias as three bf16
+  // Hot keys and pivots: the biases of a tile.  A bias on every key: ones in K columns 0..2, same for every query, and per
+  // key its bias as three bf16.  (Both in either variant: 1041 rows, 2082 keys 17.49 -> 17.66 us in this kernel.)
+  float bias2[kAllBiased ? 1 : kFastWgs][kBN];
+  alignas(16) uint8_t ax[kAllBiased ? kXBytes : 16];
+  alignas(16) uint8_t bx[kAllBiased ? kFastWgs : 1][kAllBiased ? kFT * 32 : 16];
   float m_ref[2][kBM];                          // row references of the segment (parity)
   float lpart[2][kFastWgs][kBM];                // row sums of the warpgroups (segment parity)
   int live[2][kFastWgs];                        // did a warpgroup see a key that is not masked (segment parity)
@@ -613,7 +617,8 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_v_hot, const __grid_constant__ CUtensorMap tm_k_ret,
                      const __grid_constant__ CUtensorMap tm_v_ret, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
-  FastSmem& sm = *reinterpret_cast<FastSmem*>(align1024(smem_raw));
+  using Smem = FastSmem<kAllBiased>;
+  Smem& sm = *reinterpret_cast<Smem*>(align1024(smem_raw));
   STAC_TS(0, false);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1040,6 +1045,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const bool first_part = t0 == 0;
           const int cut = first_part ? blockIdx.x : blockIdx.x - 1;   // between CTA cut and cut + 1
           const float m_pub = seg_live ? m_ref : -INFINITY;
+          named_bar_sync(1 + g, 128);              // nobody reads the word of the segment before any more
           if (row == 0) sm.join_flag[g] = ld_acquire(p.part_count + cut);
           named_bar_sync(1 + g, 128);
           bool second = sm.join_flag[g] == 1;          // usually: the item's other CTA began with it, or ended with it long ago
@@ -1708,12 +1714,13 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     return static_cast<int>(fixed) + (kColFoldLse ? 0 : nq * kBM * 4) + 1024;
   };
   if (col_smem(kColGroup) > 227 * 1024) return STAC_ERR_BAD_ARG;
-  const int fast_smem = static_cast<int>(sizeof(FastSmem)) + 1024;
+  const bool all_biased = a.T_hot == 0;
+  const int fast_smem = static_cast<int>(all_biased ? sizeof(FastSmem<true>) : sizeof(FastSmem<false>)) + 1024;
   if (attr_done.needs_setup(dev)) {
     if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem) != cudaSuccess)
       return STAC_ERR_CUDA;
     for (auto* kernel : {attn_fwd_fast_kernel<false>, attn_fwd_fast_kernel<true>})
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fast_smem) != cudaSuccess)
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FastSmem<true>) + 1024) != cudaSuccess)
         return STAC_ERR_CUDA;
     for (auto* kernel : {attn_colsum_kernel<1>, attn_colsum_kernel<2>, attn_colsum_kernel<kColGroup>})
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
@@ -1821,7 +1828,7 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   fp.zero_colsum = col_split ? a.colsum : nullptr;
   fp.zero_stride = a.colsum_head_stride;
   fp.zero_width = a.T_hot + a.T_ret;
-  if (launch_behind(a.T_hot > 0 ? attn_fwd_fast_kernel<false> : attn_fwd_fast_kernel<true>, dim3(grid_fast), dim3(kFastThreads), fast_smem, stream, tm_q, tf_kh, tf_vh,
+  if (launch_behind(all_biased ? attn_fwd_fast_kernel<true> : attn_fwd_fast_kernel<false>, dim3(grid_fast), dim3(kFastThreads), fast_smem, stream, tm_q, tf_kh, tf_vh,
                     tf_kr, tf_vr, fp) != cudaSuccess)
     return STAC_ERR_CUDA;
   if (launch_behind(attn_fwd_kernel, grid_f, dim3(kFwdThreads), fwd_smem, stream, tm_q, tm_kh, tm_vh, tm_kr, tm_vr,
