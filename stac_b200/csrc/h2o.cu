@@ -541,7 +541,8 @@ int stac_h2o_select(const float* scores, int64_t row_stride, int n_rows, const u
     attr_done.mark(dev);
   }
   const bool one_wave = n_rows <= 2 * n_sm;
-  if (stac::launch_behind(one_wave ? stac::h2o_select_kernel<1024> : stac::h2o_select_kernel<512>, dim3(n_rows), dim3(one_wave ? 1024 : 512), smem, reinterpret_cast<cudaStream_t>(stream),
+  if (stac::launch_behind(one_wave ? stac::h2o_select_kernel<1024> : stac::h2o_select_kernel<512>, dim3(n_rows),
+                          dim3(one_wave ? 1024 : 512), smem, reinterpret_cast<cudaStream_t>(stream),
                           scores, row_stride, is_base, T, n_keep, keep_idx, drop_idx) != cudaSuccess)
     return STAC_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;

@@ -267,7 +267,10 @@ __device__ __forceinline__ void sort_tokens_shared(const MergeParams& p, int h, 
     if (t < n_it) {
       const int i = c0 + t * 32 + lane;
       int vx = -1;
-      if (i < c1) vx = i < p.n_new ? p.vx_src[h * p.meta_head_stride + static_cast<int>(item[t])] : p.over_hv_in[2 * (os + i - p.n_new) + 1];
+      if (i < c1) {
+        vx = i < p.n_new ? p.vx_src[h * p.meta_head_stride + static_cast<int>(item[t])]
+                         : p.over_hv_in[2 * (os + i - p.n_new) + 1];
+      }
       item[t] = vx;
     }
   }
