@@ -1172,7 +1172,7 @@ struct ColParams {
   int n_q_tiles;
   int split;       // 1: units are cut evenly over the grid (items may be shared by two CTAs)
   float scale_log2;
-  float correction;
+  float correction, fast_correction;     // fast: of sums with a share of their exponentials on the FMA pipes
   const float* bias_ret;
   long long bias_head_stride;
   const float* lse2;
@@ -1554,7 +1554,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       float sum = warp_fast ? col_item_sum<true>(sm, p, t_base, nl_item, n_half, tail, ui, c2, 0.f)
                             : col_item_sum<false>(sm, p, t_base, nl_item, n_half, tail, ui, c2, b2_in);
       if (key < valid) {
-        sum *= p.correction;
+        sum *= warp_fast ? p.fast_correction : p.correction;
         if (b2_small) sum *= exp2f(b2);
         if (masked) sum = 0.f;
       }
@@ -1848,7 +1848,7 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     // of that kernel variant 1.0e-7 -> 0.5e-7).  Other calls keep their bits: selections compare sums that tie.
     constexpr float kCubicMean = 8.24e-6f * 0.25f;
     static_assert(kColPairMask == 0x88u, "a quarter of the pairs");
-    cp.scale_log2 = scale_log2; cp.correction = a.T_hot > 0 ? corr : corr * (1.f - kCubicMean);
+    cp.scale_log2 = scale_log2; cp.correction = corr; cp.fast_correction = all_biased ? corr * (1.f - kCubicMean) : corr;
     cp.bias_ret = a.bias_ret; cp.bias_head_stride = a.bias_head_stride;
     cp.lse2 = lse2; cp.lse2_stride = a.M;
     cp.colsum = a.colsum; cp.colsum_stride = a.colsum_head_stride;
