@@ -287,7 +287,8 @@ __device__ __forceinline__ void sort_tokens_shared(const MergeParams& p, int h, 
   for (int t = 0; t < kItems; ++t) {
     if (t < n_it) {
       const int i = c0 + t * 32 + lane;
-      const bool ok = static_cast<int>(item[t]) >= 0 && static_cast<int>(item[t]) < p.voxel_used;
+      // (carried tokens are valid whatever the voxel count of this call is)
+      const bool ok = item[t] < (i < p.n_new ? static_cast<unsigned>(p.voxel_used) : kNone);
       new_valid += __popc(__ballot_sync(kFull, ok && i < p.n_new));
       valid += __popc(__ballot_sync(kFull, ok));
       item[t] = (ok ? item[t] << 16 : kNone << 16) | static_cast<unsigned>(i);
