@@ -39,8 +39,7 @@ constexpr int col_threads(int group) { return 128 + group * 128; }   // warpgrou
 #ifndef STAC_COL_PAIR_MASK
 #define STAC_COL_PAIR_MASK 0x88
 #endif
-// which of 8 consecutive PAIRS of exponentials of the column-sum kernel run on the FMA pipes
-constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;
+constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;   // which of 8 consecutive PAIRS of exponentials of the column-sum kernel run on the FMA pipes
 #ifndef STAC_COL_FOLD_LSE
 #define STAC_COL_FOLD_LSE 1
 #endif
@@ -48,7 +47,7 @@ constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;
 // K = 16 step whose operands are a tile of ones and the row values split into three bf16), so the
 // exponent warps read nothing from shared memory; 0: they read it per score (LDS.128 per four).
 constexpr bool kColFoldLse = STAC_COL_FOLD_LSE != 0;
-constexpr int kXBytes = 128 * 32;      // 128 rows x 16 bf16, no swizzle: [16 row groups][2 K chunks][8 rows][16 B]
+constexpr int kColXBytes = 128 * 32;   // 128 rows x 16 bf16, no swizzle: [16 row groups][2 K chunks][8 rows][16 B]
 constexpr int kColCtlRegs = 56, kColExpRegs = 152;
 // setmaxnreg only moves registers inside the CTA's allocation, which is fixed at launch to
 // (registers per thread the launch bound allows, a multiple of 8) x threads.  A request beyond
@@ -83,7 +82,6 @@ struct FwdParams {
   int T_hot, T_ret;
   int n_hot_tiles, n_ret_tiles;
   float scale_log2;
-  float inv_scale;           // fast kernel, calls whose keys all have a bias: it enters the scores before the scale
   const float* bias_ret;
   long long bias_head_stride;
   __nv_bfloat16* out;
@@ -487,23 +485,17 @@ constexpr int kFastCtlRegs = 64, kFastSoftmaxRegs = 104;
 static_assert(128 * kFastCtlRegs + 128 * kFastWgs * kFastSoftmaxRegs <= kFastThreads * ((65536 / kFastThreads) / 8 * 8),
               "fast forward kernel: setmaxnreg targets exceed the CTA's register allocation");
 
-template <bool kAllBiased>
 struct FastSmem {
   uint8_t q[2][kTileBytes];                     // query tile of the segment (parity)
   uint8_t k[kFastWgs][kFastTileBytes];
   uint8_t v[kFastWgs][kFastTileBytes];
-  // Hot keys and pivots: the biases of a tile.  A bias on every key: ones in K columns 0..2, same for every query, and per
-  // key its bias as three bf16.  (Both in either variant: 1041 rows, 2082 keys 17.49 -> 17.66 us in this kernel.)
-  float bias2[kAllBiased ? 1 : kFastWgs][kBN];
-  alignas(16) uint8_t ax[kAllBiased ? kXBytes : 16];
-  alignas(16) uint8_t bx[kAllBiased ? kFastWgs : 1][kAllBiased ? kFT * 32 : 16];
+  float bias2[kFastWgs][kBN];
   float m_ref[2][kBM];                          // row references of the segment (parity)
   float lpart[2][kFastWgs][kBM];                // row sums of the warpgroups (segment parity)
   int live[2][kFastWgs];                        // did a warpgroup see a key that is not masked (segment parity)
   uint64_t q_full[2];
   uint64_t q_empty[2];
   uint64_t k_full[kFastWgs];
-  uint64_t x_full[kFastWgs];     // the bias operand of a tile is written
   uint64_t v_full[kFastWgs];
   uint64_t s_full[kFastWgs];     // scores of a tile are in TMEM; the place of its keys is free again
   uint64_t p_full[kFastWgs];     // its probabilities are in TMEM
@@ -550,21 +542,21 @@ struct FwdWalk {
 
 // kN scores -> kN probabilities relative to the row reference, packed as bf16 pairs.  Scores
 // are handled two at a time with the packed fp32 instructions (scale-and-subtract, row sums).
-// The pairs whose bit is set in kFastPairMask take their exponentials on the FMA pipes (cubic, 8.6e-5 relative, or
-// quintic, 1.6e-7: both far below the bf16 rounding of P) to relieve the exponential unit.
+// The pairs whose bit is set in kFastPairMask take their exponentials on the FMA pipes (cubic,
+// 8.6e-5 relative, far below the bf16 rounding of P) to relieve the exponential unit.
 // Their arguments go into a running maximum: 2^128 and more, which the exponential unit turns into infinities that the
 // row sum shows, would wrap there.
-template <int kDegree, int kJ>
+template <int kJ>
 __device__ __forceinline__ uint64_t fast_exp_pair(uint64_t x2, float& top) {
   float x0, x1;
   unpack_f32x2(x2, x0, x1);
   if constexpr ((kFastPairMask >> (kJ & 15)) & 1u) {
     top = fmax3(top, x0, x1);
-    return poly_exp2_x2<kDegree>(x2);
+    return poly_exp2_x2(x2);
   }
   return pack_f32x2(fast_exp2(x0), fast_exp2(x1));
 }
-template <bool kBias, int kDegree, int kN, int kI = 0>
+template <bool kBias, int kN, int kI = 0>
 __device__ __forceinline__ void fast_exp_chunk(const uint32_t (&s)[32], uint32_t (&pk)[16], const float* bias2,
                                                uint64_t c2c2, uint64_t negm2, uint64_t& l0, uint64_t& l1, float& top) {
   if constexpr (kI < kN) {
@@ -578,7 +570,7 @@ __device__ __forceinline__ void fast_exp_chunk(const uint32_t (&s)[32], uint32_t
       x0 = fma_f32x2(x0, c2c2, negm2);
       x1 = fma_f32x2(x1, c2c2, negm2);
     }
-    const uint64_t e0 = fast_exp_pair<kDegree, kI / 2>(x0, top), e1 = fast_exp_pair<kDegree, kI / 2 + 1>(x1, top);
+    const uint64_t e0 = fast_exp_pair<kI / 2>(x0, top), e1 = fast_exp_pair<kI / 2 + 1>(x1, top);
     l0 = add_f32x2(l0, e0);
     l1 = add_f32x2(l1, e1);
     float a0, a1, a2, a3;
@@ -586,7 +578,7 @@ __device__ __forceinline__ void fast_exp_chunk(const uint32_t (&s)[32], uint32_t
     unpack_f32x2(e1, a2, a3);
     pk[kI / 2] = pack_bf16x2(a0, a1);
     pk[kI / 2 + 1] = pack_bf16x2(a2, a3);
-    fast_exp_chunk<kBias, kDegree, kN, kI + 4>(s, pk, bias2, c2c2, negm2, l0, l1, top);
+    fast_exp_chunk<kBias, kN, kI + 4>(s, pk, bias2, c2c2, negm2, l0, l1, top);
   }
 }
 
@@ -603,22 +595,12 @@ __device__ __forceinline__ float fast_max_chunk(const uint32_t (&s)[32], const f
   return mx;
 }
 
-// kAllBiased: every key has a bias (no hot segment).  It is then added to the scores by the tensor core, bias / scale split into
-// three bf16 (all bits of it where the scale is a power of two) times ones in a K = 16 step of its own, and the loop is the
-// one of keys without a bias; the warpgroup writes the operand of its next tile while it would wait for that tile's
-// scores anyway.  us in this kernel: 2603 rows, 6247 keys, 12 heads 79.8 -> 72.6, 4164 rows, 9000 keys 157.9 -> 139.9 (added in the
-// softmax warps: two barriers per tile, a shared load and two more additions per four scores; without a bias 69 and 134).
-// Written by the loading warps instead: 88 to 100 us, they get too few issue slots.  The exponentials on the FMA pipes
-// take the quintic here.  Calls with hot keys and pivots keep the addition in the softmax warps: a score's last
-// bits differ between the two ways, and so would the tokens that a selection keeps among scores that tie.
-template <bool kAllBiased>
 __global__ void __launch_bounds__(kFastThreads, 1)
 attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k_hot,
                      const __grid_constant__ CUtensorMap tm_v_hot, const __grid_constant__ CUtensorMap tm_k_ret,
                      const __grid_constant__ CUtensorMap tm_v_ret, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
-  using Smem = FastSmem<kAllBiased>;
-  Smem& sm = *reinterpret_cast<Smem*>(align1024(smem_raw));
+  FastSmem& sm = *reinterpret_cast<FastSmem*>(align1024(smem_raw));
   STAC_TS(0, false);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -635,7 +617,6 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     mbar_init(&sm.o_done, 1);
     for (int b = 0; b < kFastWgs; ++b) {
       mbar_init(&sm.k_full[b], 1);
-      if (kAllBiased) mbar_init(&sm.x_full[b], 128);
       mbar_init(&sm.v_full[b], 1);
       mbar_init(&sm.s_full[b], 1);
       mbar_init(&sm.p_full[b], 128);
@@ -643,18 +624,6 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
     mbar_init(&sm.o_free, 128);
     mbar_fence_init();
-  }
-  if (kAllBiased && threadIdx.x >= 128) {
-    // the constant operand, and what stays zero of the other one (its thread writes the rest and fences)
-    const int g = (threadIdx.x >> 7) - 1, at = ((threadIdx.x & 127) >> 3) * 256 + (threadIdx.x & 7) * 16;
-    uint4* x_row = reinterpret_cast<uint4*>(sm.bx[g] + at);
-    if ((threadIdx.x & 127) < kFT) x_row[0] = x_row[8] = make_uint4(0u, 0u, 0u, 0u);
-    if (g == 0) {
-      uint4* one_row = reinterpret_cast<uint4*>(sm.ax + at);
-      one_row[0] = make_uint4(0x3F803F80u, 0x00003F80u, 0u, 0u);
-      one_row[8] = make_uint4(0u, 0u, 0u, 0u);
-      fence_proxy_async_smem();
-    }
   }
   if (warp == 1) {
     tmem_alloc(&sm.tmem_base, 512);
@@ -734,8 +703,6 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       constexpr uint32_t idesc_s = umma_idesc_bf16(kBM, kFT, 0);
       const uint64_t q_desc0 = smem_desc_sw128(smem_u32(sm.q[0]));
       const uint64_t k_desc0 = smem_desc_sw128(smem_u32(sm.k[0]));
-      const uint64_t ax_desc = smem_desc_nosw(smem_u32(sm.ax), 128, 256);
-      const uint64_t bx_desc0 = smem_desc_nosw(smem_u32(sm.bx[0]), 128, 256);
       FwdWalk walk(p, n_tiles);
       int item, t0, t1;
       uint32_t b = 0, par = 1;     // stage and buffer of the tile, phase of their previous use
@@ -749,13 +716,10 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(b * (kFastTileBytes >> 4));
           const uint32_t d = tmem + b * kFT;
           mbar_wait(&sm.k_full[b], par ^ 1, p.err, DEV_TIMEOUT_TMA);
-          if (kAllBiased) mbar_wait(&sm.x_full[b], par ^ 1, p.err, DEV_TIMEOUT_CONSUMER);
           if (reused) mbar_wait(&sm.pv_done[b], par, p.err, DEV_TIMEOUT_CONSUMER);
           tc_fence_after();
           if (elect_one()) {
-            // (the bias first: with the scores on top of it one sum less is rounded)
-            if (kAllBiased) umma_ss(d, ax_desc, bx_desc0 + static_cast<uint64_t>(b * (kFT * 32 >> 4)), idesc_s, 0u);
-            umma_ss(d, q_desc, k_desc, idesc_s, kAllBiased ? 1u : 0u);
+            umma_ss(d, q_desc, k_desc, idesc_s, 0u);
             umma_ss(d, q_desc + 2, k_desc + 2, idesc_s, 1u);
             umma_ss(d, q_desc + 4, k_desc + 4, idesc_s, 1u);
             umma_ss(d, q_desc + 6, k_desc + 6, idesc_s, 1u);
@@ -819,42 +783,6 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     int seg = 0, item, t0, t1;
     int c_base = 0;   // key tiles of earlier segments
     int round = 0;    // tiles that this warpgroup has behind it
-    // kAllBiased from here on: bias of key `row` of tile j, -inf for places behind the last key
-    bool live = true; // false: every key of this warpgroup's next tile is masked
-    auto load_bias = [&](int h, int j) {
-      const int key = j * kFT + row;
-      return row < kFT && key < p.T_ret ? p.bias_ret[h * p.bias_head_stride + key] : -INFINITY;
-    };
-    auto write_bias = [&](float bias) {
-      const float b2 = bias * kLog2e;
-      float x = bias * p.inv_scale;
-      if (!(fabsf(x) < 1e38f)) {
-        if (fabsf(b2) == INFINITY) {
-          x = copysignf(b2, b2 * p.inv_scale);     // a mask: the infinity that the scale turns into this one
-        } else if (b2 == b2) {
-          atomicOr(p.fallback, 1);                 // finite, but not before the scale: the exact kernel adds it behind it
-          x = 0.f;
-        }
-      }
-      if (row < kFT) *reinterpret_cast<uint2*>(sm.bx[g] + (row >> 3) * 256 + (row & 7) * 16) = split_bf16x3(x);
-      fence_proxy_async_smem();
-      mbar_arrive(&sm.x_full[g]);
-      live = named_bar_or(1 + g, 128, b2 != -INFINITY);
-    };
-    // The same for the warpgroup's first tile behind `base` tiles, which is in the next segment or one behind it.
-    auto write_bias_ahead = [&](int base) {
-      FwdWalk ahead = walk;
-      int item_a, t0_a, t1_a;
-      while (ahead.next(item_a, t0_a, t1_a)) {
-        const int j = t0_a + ((g - base) & (kFastWgs - 1));
-        if (j < t1_a) {
-          write_bias(load_bias(item_a / p.n_q_tiles, j));
-          break;
-        }
-        base += t1_a - t0_a;
-      }
-    };
-    if constexpr (kAllBiased) write_bias_ahead(0);
     for (; walk.next(item, t0, t1); ++seg) {
       const int h = item / p.n_q_tiles, m_tile = item - h * p.n_q_tiles;
       const int len = t1 - t0;
@@ -895,53 +823,21 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // Scores -> probabilities in place, chunk by chunk: load, wait, convert, store.
       auto convert = [&](auto bias_tag) {
         constexpr bool kBias = decltype(bias_tag)::value;
-        constexpr int kDegree = kAllBiased ? 5 : 3;
 #pragma unroll
         for (int ch = 0; ch < kFT / 32; ++ch) {
           tmem_ld_wait();
-          fast_exp_chunk<kBias, kDegree, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1, top);
+          fast_exp_chunk<kBias, 32>(ra, pk, bias2 + 32 * ch, c2c2, negm2, l0, l1, top);
           if (ch + 1 < kFT / 32) tmem_ld32(s_addr + 32 * (ch + 1), ra);
           else tmem_ld16(s_addr + 32 * (ch + 1), ra);
           tmem_st16(s_addr + 16 * ch, pk);
         }
         tmem_ld_wait();
-        fast_exp_chunk<kBias, kDegree, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1, top);
+        fast_exp_chunk<kBias, 16>(ra, pk, bias2 + kFT - 16, c2c2, negm2, l0, l1, top);
         tmem_st8(s_addr + (kFT - 16) / 2, pk);
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(&sm.p_full[g]);
       };
-      // all probabilities of a tile are zero: nothing to exponentiate
-      auto convert_masked = [&] {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) pk[i] = 0u;
-#pragma unroll
-        for (int ch = 0; ch < kFT / 32; ++ch) tmem_st16(s_addr + 16 * ch, pk);
-        tmem_st8(s_addr + (kFT - 16) / 2, pk);
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(&sm.p_full[g]);
-      };
-      if constexpr (kAllBiased) {
-        if (x < len) reference(false);
-#pragma unroll 1
-        for (; x < len; x += kFastWgs, ++round) {
-          const bool more = x + kFastWgs < len;
-          float bias = 0.f;     // of the next tile, on its way during this one
-          if (more) bias = load_bias(h, t0 + x + kFastWgs);
-          any_live = any_live || live;
-          mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
-          tc_fence_after();
-          if (live) {
-            tmem_ld32(s_addr, ra);
-            convert(std::false_type{});
-          } else {
-            convert_masked();
-          }
-          if (more) write_bias(bias);
-        }
-        if (((g - c_base) & (kFastWgs - 1)) < len) write_bias_ahead(c_base + len);   // else that is done already
-      } else {
       // whole tiles of the hot cache: no bias, nothing masked
       const int n_plain = min(len, p.T_hot / kFT - t0);
       any_live = x < n_plain;
@@ -971,12 +867,19 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         mbar_wait(&sm.s_full[g], round & 1, p.err, DEV_TIMEOUT_MMA);
         tc_fence_after();
         if (!tile_live && !first) {
-          convert_masked();
+          // nothing to exponentiate: all probabilities of this tile are zero
+#pragma unroll
+          for (int i = 0; i < 16; ++i) pk[i] = 0u;
+#pragma unroll
+          for (int ch = 0; ch < kFT / 32; ++ch) tmem_st16(s_addr + 16 * ch, pk);
+          tmem_st8(s_addr + (kFT - 16) / 2, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          mbar_arrive(&sm.p_full[g]);
           continue;
         }
         tmem_ld32(s_addr, ra);
         convert(std::true_type{});
-      }
       }
       // ---- end of the segment
       float la, lb, lc, ld;
@@ -1158,8 +1061,8 @@ struct ColSmem {
   uint64_t x_full[kColStages];            // the row-term operand of a query stage is written
   uint32_t tmem_base;
   int join_flag;                          // arrival count seen at a shared item
-  alignas(16) uint8_t ax[kXBytes];     // ones in K columns 0..2, same for every key
-  alignas(16) uint8_t bx[kColStages][kXBytes];   // per query row: -lse2 / c2 as hi, mid, lo bf16
+  alignas(16) uint8_t ax[kColXBytes];     // ones in K columns 0..2, same for every key
+  alignas(16) uint8_t bx[kColStages][kColXBytes];   // per query row: -lse2 / c2 as hi, mid, lo bf16
   alignas(16) float lse2[4];  // (without the fold) flexible: n_q_tiles * 128 floats follow (negated, one head)
 };
 
@@ -1172,7 +1075,7 @@ struct ColParams {
   int n_q_tiles;
   int split;       // 1: units are cut evenly over the grid (items may be shared by two CTAs)
   float scale_log2;
-  float correction, fast_correction;     // fast: of sums with a share of their exponentials on the FMA pipes
+  float correction;
   const float* bias_ret;
   long long bias_head_stride;
   const float* lse2;
@@ -1230,7 +1133,7 @@ struct ColWalk {
 template <int kJ>
 __device__ __forceinline__ uint64_t col_exp_pair(uint64_t s2, uint64_t c2c2, float n0, float n1) {
   const uint64_t x2 = kColFoldLse ? mul_f32x2(s2, c2c2) : fma_f32x2(s2, c2c2, pack_f32x2(n0, n1));
-  if ((kColPairMask >> kJ) & 1u) return poly_exp2_x2<3>(x2);
+  if ((kColPairMask >> kJ) & 1u) return poly_exp2_x2(x2);
   float x0, x1;
   unpack_f32x2(x2, x0, x1);
   return pack_f32x2(fast_exp2(x0), fast_exp2(x1));
@@ -1478,7 +1381,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 umma_ss(d + t * 128, kd + 6, q_desc + 6, idesc, 1u);
                 // the 64 rows of this half: eight row groups of 256 bytes further in the operand
                 if (kColFoldLse)
-                  umma_ss(d + t * 128, ax_desc, bx_desc0 + static_cast<uint64_t>((s * kXBytes + half * 2048) >> 4),
+                  umma_ss(d + t * 128, ax_desc, bx_desc0 + static_cast<uint64_t>((s * kColXBytes + half * 2048) >> 4),
                           idesc, 1u);
               }
               umma_commit(&sm.s_full[g]);
@@ -1554,7 +1457,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       float sum = warp_fast ? col_item_sum<true>(sm, p, t_base, nl_item, n_half, tail, ui, c2, 0.f)
                             : col_item_sum<false>(sm, p, t_base, nl_item, n_half, tail, ui, c2, b2_in);
       if (key < valid) {
-        sum *= warp_fast ? p.fast_correction : p.correction;
+        sum *= p.correction;
         if (b2_small) sum *= exp2f(b2);
         if (masked) sum = 0.f;
       }
@@ -1714,14 +1617,13 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     return static_cast<int>(fixed) + (kColFoldLse ? 0 : nq * kBM * 4) + 1024;
   };
   if (col_smem(kColGroup) > 227 * 1024) return STAC_ERR_BAD_ARG;
-  const bool all_biased = a.T_hot == 0;
-  const int fast_smem = static_cast<int>(all_biased ? sizeof(FastSmem<true>) : sizeof(FastSmem<false>)) + 1024;
+  const int fast_smem = static_cast<int>(sizeof(FastSmem)) + 1024;
   if (attr_done.needs_setup(dev)) {
     if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem) != cudaSuccess)
       return STAC_ERR_CUDA;
-    for (auto* kernel : {attn_fwd_fast_kernel<false>, attn_fwd_fast_kernel<true>})
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FastSmem<true>) + 1024) != cudaSuccess)
-        return STAC_ERR_CUDA;
+    if (cudaFuncSetAttribute(attn_fwd_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fast_smem) !=
+        cudaSuccess)
+      return STAC_ERR_CUDA;
     for (auto* kernel : {attn_colsum_kernel<1>, attn_colsum_kernel<2>, attn_colsum_kernel<kColGroup>})
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
         return STAC_ERR_CUDA;
@@ -1771,7 +1673,6 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   fp.n_hot_tiles = (a.T_hot + kBN - 1) / kBN;
   fp.n_ret_tiles = (a.T_ret + kBN - 1) / kBN;
   fp.scale_log2 = scale_log2;
-  fp.inv_scale = 1.f / a.scale;
   fp.bias_ret = a.bias_ret; fp.bias_head_stride = a.bias_head_stride;
   fp.out = static_cast<__nv_bfloat16*>(a.out); fp.out_row_stride = a.out_row_stride;
   fp.lse = a.lse; fp.lse2 = lse2; fp.lse2_stride = a.M;
@@ -1828,7 +1729,7 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   fp.zero_colsum = col_split ? a.colsum : nullptr;
   fp.zero_stride = a.colsum_head_stride;
   fp.zero_width = a.T_hot + a.T_ret;
-  if (launch_behind(all_biased ? attn_fwd_fast_kernel<true> : attn_fwd_fast_kernel<false>, dim3(grid_fast), dim3(kFastThreads), fast_smem, stream, tm_q, tf_kh, tf_vh,
+  if (launch_behind(attn_fwd_fast_kernel, dim3(grid_fast), dim3(kFastThreads), fast_smem, stream, tm_q, tf_kh, tf_vh,
                     tf_kr, tf_vr, fp) != cudaSuccess)
     return STAC_ERR_CUDA;
   if (launch_behind(attn_fwd_kernel, grid_f, dim3(kFwdThreads), fwd_smem, stream, tm_q, tm_kh, tm_vh, tm_kr, tm_vr,
@@ -1843,12 +1744,7 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     cp.n_tiles = fp.n_hot_tiles + fp.n_ret_tiles;
     cp.n_groups = (cp.n_tiles + col_group - 1) / col_group;
     cp.n_items = cp.n_groups * a.H;
-    // Calls whose keys all have a bias: the mean of the cubic's error, weighted with what it approximates, times its share
-    // leaves the sums (2.1e-6 of them; error against 64 bits at 4164 rows, 9000 keys 1.5e-6 -> 0.7e-6, of the log-sum-exps
-    // of that kernel variant 1.0e-7 -> 0.5e-7).  Other calls keep their bits: selections compare sums that tie.
-    constexpr float kCubicMean = 8.24e-6f * 0.25f;
-    static_assert(kColPairMask == 0x88u, "a quarter of the pairs");
-    cp.scale_log2 = scale_log2; cp.correction = corr; cp.fast_correction = all_biased ? corr * (1.f - kCubicMean) : corr;
+    cp.scale_log2 = scale_log2; cp.correction = corr;
     cp.bias_ret = a.bias_ret; cp.bias_head_stride = a.bias_head_stride;
     cp.lse2 = lse2; cp.lse2_stride = a.M;
     cp.colsum = a.colsum; cp.colsum_stride = a.colsum_head_stride;

@@ -280,33 +280,21 @@ __device__ __forceinline__ uint64_t add_rm_f32x2(uint64_t a, uint64_t b) {
 }
 
 // exp2 of two values on the FMA / integer pipes instead of the exponential unit: x = n + f with n = floor(x), 2^f
-// from a polynomial on [0, 1), n added to the exponent field.  x + 1.5 * 2^23 rounded towards -inf leaves n in the
-// low mantissa bits.  Inputs below -127 (and -inf) give exactly 0; inputs of 128 and more wrap (callers check).
-// Range reduction and polynomial use packed instructions (six for the pair with the cubic, eight with the
-// quintic), the clamp and the exponent are per value.  kDegree 3: largest relative error 8.6e-5.  kDegree 5: 1.6e-7, as
-// good as the exponential unit (minimax under p(0) = 1 and a zero mean of the error weighted by 2^f, by linear
-// programming).
-template <int kDegree>
+// from a cubic fitted to [0, 1) (largest relative error 8.6e-5), n added to the exponent field.  x + 1.5 * 2^23 rounded
+// towards -inf leaves n in the low mantissa bits.  Inputs below -127 (and -inf) give exactly 0; NaN does too and
+// inputs of 128 and more wrap (callers check).  Costs about as many issue slots as two ex2.approx occupy the exponential
+// unit: range reduction and cubic use packed instructions (six for the pair), the clamp and the exponent are per value.
 __device__ __forceinline__ uint64_t poly_exp2_x2(uint64_t x2) {
-  static_assert(kDegree == 3 || kDegree == 5, "fitted for these");
-  auto both = [](float c) { return pack_f32x2(c, c); };
   float x0, x1;
   unpack_f32x2(x2, x0, x1);
   x2 = pack_f32x2(fmaxf(x0, -127.f), fmaxf(x1, -127.f));
-  const uint64_t t2 = add_rm_f32x2(x2, both(12582912.f));
-  const uint64_t u2 = add_f32x2(t2, both(-12582912.f));
-  const uint64_t f2 = fma_f32x2(u2, both(-1.f), x2);
-  uint64_t p2;
-  if constexpr (kDegree == 3) {
-    p2 = fma_f32x2(both(0.07706617563962936f), f2, both(0.22764593362808228f));
-    p2 = fma_f32x2(p2, f2, both(0.6951165795326233f));
-  } else {
-    p2 = fma_f32x2(both(0.0018599523464217782f), f2, both(0.009033777751028538f));
-    p2 = fma_f32x2(p2, f2, both(0.05578712373971939f));
-    p2 = fma_f32x2(p2, f2, both(0.24016796052455902f));
-    p2 = fma_f32x2(p2, f2, both(0.69315105676651f));
-  }
-  p2 = fma_f32x2(p2, f2, both(1.f));
+  const uint64_t t2 = add_rm_f32x2(x2, pack_f32x2(12582912.f, 12582912.f));
+  const uint64_t u2 = add_f32x2(t2, pack_f32x2(-12582912.f, -12582912.f));
+  const uint64_t f2 = fma_f32x2(u2, pack_f32x2(-1.f, -1.f), x2);
+  uint64_t p2 = fma_f32x2(pack_f32x2(0.07706617563962936f, 0.07706617563962936f), f2,
+                          pack_f32x2(0.22764593362808228f, 0.22764593362808228f));
+  p2 = fma_f32x2(p2, f2, pack_f32x2(0.6951165795326233f, 0.6951165795326233f));
+  p2 = fma_f32x2(p2, f2, pack_f32x2(1.f, 1.f));
   float p0, p1, t0, t1;
   unpack_f32x2(p2, p0, p1);
   unpack_f32x2(t2, t0, t1);
@@ -331,16 +319,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
-}
-
-// v as the sum of three bf16 (its 24 bits, eight at a time), K columns 0, 1 and 2 of an operand row: a tensor core that
-// multiplies it with (1, 1, 1, 0, ...) adds v to a score.  Infinities and NaN stay what they are.
-__device__ __forceinline__ uint2 split_bf16x3(float v) {
-  const uint32_t hi = __float_as_uint(v) & 0xFFFF0000u;
-  const float r1 = fabsf(v) < INFINITY ? v - __uint_as_float(hi) : 0.f;
-  const uint32_t mid = __float_as_uint(r1) & 0xFFFF0000u;
-  const float lo = r1 - __uint_as_float(mid);
-  return make_uint2(__byte_perm(v != v ? 0x7FFF0000u : hi, mid, 0x7632), __float_as_uint(lo) >> 16);
 }
 
 // Warpgroup-wide register re-allocation (all four warps of a warpgroup must execute it).

@@ -282,23 +282,23 @@ def test_leading_masked_tile_then_faint_keys():
 
 
 @pytest.mark.parametrize("M,H,N", [(70, 2, 1), (130, 2, 112), (130, 3, 449), (257, 2, 1000), (2600, 8, 900), (1100, 2, 2000)])
-@pytest.mark.parametrize("kind", ["counts", "mask", "lowest", "huge", "scale"])
+@pytest.mark.parametrize("kind", ["counts", "mask", "lowest", "faint", "huge", "scale"])
 def test_a_bias_on_every_key(M, H, N, kind):
-    """The bias goes through the tensor core before the scale: log counts with masked keys and whole masked tiles (first, middle,
-    last of a head), a type's lowest value as the mask, finite biases that do not fit before the scale (recomputed by the
-    exact kernel), a scale that is not a power of two.  One CTA per item, items cut over the SMs, items in halves."""
+    """Log counts with masked keys and whole masked tiles (first, middle, last of a head), a type's lowest value and a finite one
+    within its range as the mask, biases that swallow the scores, a scale that is not a power of two.  One CTA per item,
+    items cut over the SMs, items in halves."""
     from stac_b200 import ops
     rs = np.random.RandomState(M + N)
     q, k, v = (_bf16(rs.randn(*s).astype(np.float32)) for s in ((M, H, 64), (N, H, 64), (N, H, 64)))
     bias = np.log(rs.randint(1, 9, size=(H, N)).astype(np.float32))
     scale = 0.1 if kind == "scale" else 0.125
     if kind == "huge":
-        bias -= np.float32(3e37)       # eight times that is beyond 1e38
+        bias -= np.float32(3e37)
     elif kind != "counts" and N > 1:
         masked = rs.rand(H, N) < 0.25
         for h, tile in ((0, 0), (1, 3), (H - 1, (N - 1) // 112)):
             masked[h, 112 * tile:112 * (tile + 1)] = N > 112
-        bias[masked] = np.finfo(np.float32).min if kind == "lowest" else -np.inf
+        bias[masked] = {"lowest": np.finfo(np.float32).min, "faint": np.float32(-3e37)}.get(kind, -np.inf)
     dev = torch.device("cuda:0")
     status = ops.DeviceStatus(dev)
     got = ops.attn_colsum(q.to(dev), None, None, 0, k.to(dev), v.to(dev), torch.from_numpy(bias).to(dev), N, layout="thd",
@@ -306,10 +306,31 @@ def test_a_bias_on_every_key(M, H, N, kind):
     torch.cuda.synchronize()
     status.raise_if_set("attention")
     o, lse, cs = oracle_attn(q.float().numpy(), k.float().numpy(), v.float().numpy(), bias, scale=scale)
-    got = [x.float().cpu().numpy() for x in got]
     if kind == "huge":
-        cs = got[2]      # column sums are computed for log-sum-exps up to 1e29
-    _assert_close(got, (o, lse, cs))
+        cs = np.zeros_like(cs)       # rows whose log-sum-exp is beyond 1e29 add nothing to the column sums
+    _assert_close([x.float().cpu().numpy() for x in got], (o, lse, cs))
+
+
+@pytest.mark.parametrize("shift", [-40.0, 30.0, 300.0])
+@pytest.mark.parametrize("scale", [0.125, 0.1])
+def test_a_bias_far_from_zero_is_added_behind_the_scale(shift, scale):
+    """One rounding of the exponents at the bias's size.  Column sums: half an ulp of the biased exponent and half an ulp of the
+    row's log-sum-exp, both in log2 units, beside a quarter of the cubic's mean error (8.24e-6).  Log-sum-exps: four
+    such roundings (bias, exponent, sum with the reference, change of base) beside 1.4e-5 for the cubic in an eighth of 300 keys."""
+    from stac_b200 import ops
+    M, N, H = 500, 300, 4
+    rs = np.random.RandomState(21)
+    q, k, v = (_bf16(rs.randn(*s).astype(np.float32)) for s in ((M, H, 64), (N, H, 64), (N, H, 64)))
+    bias = np.log(rs.randint(1, 9, size=(H, N))).astype(np.float32) + np.float32(shift)
+    dev = torch.device("cuda:0")
+    _, lse, cs = ops.attn_colsum(q.to(dev), None, None, 0, k.to(dev), v.to(dev), torch.from_numpy(bias).to(dev), N, layout="thd",
+                                 scale=scale, want_lse=True)
+    s = torch.einsum("mhd,nhd->hmn", q.double(), k.double()) * scale + torch.from_numpy(bias).double()[:, None]
+    lse_ref = s.logsumexp(-1)
+    cs_ref = (s - lse_ref[..., None]).exp().sum(1)
+    rounding = float(np.spacing(np.float32(abs(shift) * 1.4427))) * 0.6931
+    assert ((cs.cpu().double() - cs_ref).norm() / cs_ref.norm()).item() <= 2.1e-6 + rounding
+    assert (lse.cpu().double() - lse_ref).abs().max().item() <= 1.4e-5 + 2 * rounding
 
 
 def test_calls_replay_from_a_cuda_graph():
