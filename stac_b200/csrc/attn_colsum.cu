@@ -545,13 +545,13 @@ struct FwdWalk {
 // The pairs whose bit is set in kFastPairMask take their exponentials on the FMA pipes (cubic,
 // 8.6e-5 relative, far below the bf16 rounding of P) to relieve the exponential unit.
 // Their arguments go into a running maximum: 2^128 and more, which the exponential unit turns into infinities that the
-// row sum shows, would wrap there.
+// row sum shows, would wrap there, and NaN would be a probability of zero.
 template <int kJ>
 __device__ __forceinline__ uint64_t fast_exp_pair(uint64_t x2, float& top) {
   float x0, x1;
   unpack_f32x2(x2, x0, x1);
   if constexpr ((kFastPairMask >> (kJ & 15)) & 1u) {
-    top = fmax3(top, x0, x1);
+    top = fmax3_nan(top, x0, x1);
     return poly_exp2_x2(x2);
   }
   return pack_f32x2(fast_exp2(x0), fast_exp2(x1));
@@ -1014,7 +1014,7 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       c_base += len;
     }
-    overflow = overflow || top >= 128.f;
+    overflow = overflow || !(top < 128.f);   // also true for NaN
     if (__any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(p.fallback, 1);
   }
   tc_fence_before();

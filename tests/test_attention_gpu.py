@@ -188,6 +188,25 @@ def test_one_key_far_above_the_first_keys():
         _assert_close([x.float().cpu().numpy() for x in got], ref)
 
 
+@pytest.mark.parametrize("what", ["key", "bias"])
+def test_nan_at_every_place(what):
+    """A NaN key, or a NaN bias of a pivot, at every place of a chunk of 32: every output row of its head is NaN, whichever pipe its
+    exponential runs on, and the other head's are not."""
+    from stac_b200 import ops
+    M, T, dev = 40, 336, torch.device("cuda:0")      # whole tiles of 112 keys
+    g = torch.Generator().manual_seed(3)
+    q, k, v, kr, vr = (torch.randn(*s, generator=g).to(torch.bfloat16).to(dev) for s in ((M, 2, 64),) + ((2, T, 64),) * 4)
+    for place in range(128, 128 + 32):
+        k2, br = k.clone(), torch.zeros(2, T, device=dev)
+        if what == "key":
+            k2[0, place] = float("nan")
+        else:
+            br[0, place] = float("nan")
+        out, lse, _ = ops.attn_colsum(q, k2, v, T, kr, vr, br, T, want_lse=True)
+        assert out[:, 0].isnan().all() and lse[0].isnan().all(), place
+        assert out[:, 1].isfinite().all() and lse[1].isfinite().all(), place
+
+
 @pytest.mark.parametrize("shift", [-40.0, 30.0])
 def test_large_bias(shift):
     got, ref = _run_two_segment(200, 2, 300, 260, seed=13, bias_shift=shift)
