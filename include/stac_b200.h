@@ -104,9 +104,9 @@ int stac_attn_colsum_kept(const void* q, int64_t q_row_stride,
                           int* dev_status, stac_stream_t stream);
 
 /* The same with a kept workspace, and the running scores of the hot keys updated from their column sums by the
- * kernel that makes them, or by a launch behind it where nearly every sum is added up by two CTAs: the effect of
- * stac_scores_update(colsum, ..., T_live = T_hot, old_T, Tq, temperature) behind the call, bit for bit.  `colsum`
- * must not be NULL, and the rows of `scores` and `counts` must not overlap: score_row_stride >= T_hot where H > 1. */
+ * kernel that makes them: the effect of stac_scores_update(colsum, ..., T_live = T_hot, old_T, Tq, temperature) behind
+ * the call, bit for bit.  `colsum` must not be NULL, and the rows of `scores` and `counts` must not overlap:
+ * score_row_stride >= T_hot where H > 1. */
 int stac_attn_colsum_scored(const void* q, int64_t q_row_stride,
                             const void* k_hot, const void* v_hot, int64_t hot_row_stride, int64_t hot_head_stride, int T_hot,
                             const void* k_ret, const void* v_ret, int64_t ret_row_stride, int64_t ret_head_stride, int T_ret,

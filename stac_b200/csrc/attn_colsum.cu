@@ -1751,12 +1751,9 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     cp.err = err;
     cp.split = (col_split || col_parts) ? 1 : 0;      // col_split: the forward kernel has cleared a.colsum
     cp.parts = col_parts ? part + kFwdPartElems : nullptr;
-    // Running scores: updated by the thread that has a key's final sum (1041 rows, 16 heads, 5600 keys 66.4 -> 65.2 us per
-    // call, 8328 + 2082 keys 110.6 -> 109.5, 2 us per layer of a stream, against a launch behind the kernel).  Below two items
-    // per SM, where nearly every item is cut, the launch stays: callers count a call's launches there (3800 keys 50.9
-    // against 49.7 us).
-    const bool scored_apart = col_split && col_items < 2 * n_sm;
-    cp.scores = scored_apart ? nullptr : a.scores; cp.counts = a.counts; cp.score_stride = a.score_stride;
+    // Running scores: updated by the thread that has a key's final sum.  (us per call with a launch behind the kernel instead,
+    // 16 heads: 128 rows, 3800 keys 32.4 against 31.0, 1041 rows, 3800 keys 51.1 against 49.6, 5600 keys 66.8 against 65.5.)
+    cp.scores = a.scores; cp.counts = a.counts; cp.score_stride = a.score_stride;
     cp.old_T = a.old_T; cp.tq = static_cast<float>(a.score_Tq); cp.temperature = a.temperature;
     cp.part_count = ctl + kCtlColItems;
     const int grid_c = cp.split ? n_sm : cp.n_items;
@@ -1765,9 +1762,6 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
     if (launch_behind(col_kernel, dim3(grid_c), dim3(col_threads(col_group)), col_smem(col_group), stream, tm_qs, tm_kh,
                       tm_kr, cp) != cudaSuccess)
       return STAC_ERR_CUDA;
-    if (scored_apart && a.scores != nullptr)
-      return stac_scores_update(a.colsum, a.colsum_head_stride, a.scores, a.counts, a.score_stride, a.H, a.T_hot, a.old_T,
-                                a.score_Tq, a.temperature, reinterpret_cast<stac_stream_t>(stream));
   }
   return STAC_OK;
 }

@@ -521,11 +521,11 @@ def test_ragged_last_query_tile(M, H, T_hot, T_ret):
 
 @pytest.mark.parametrize("M,H,T_hot,T_ret,old_T,ratio", [
     (130, 2, 300, 90, 170, 1.0),          # one CTA per item: updated by the kernel
-    (1041, 16, 3400, 140, 2359, 1.0),     # items shared by two CTAs: by a launch behind it
+    (1041, 16, 3400, 140, 2359, 1.0),     # one to two items per SM, nearly all shared by two CTAs: by the thread that adds second
     (2600, 3, 6000, 0, 0, 1.0),           # by three and more: by the CTA that joins them
     (900, 5, 1500, 260, 1500, 0.25),      # rows left out; no new key
     (2600, 3, 5900, 200, 4000, 1.0),      # hot and retrieved tiles in one group of items shared by three CTAs
-    (300, 16, 7300, 200, 5000, 1.0),      # two and more items per SM, some shared by two CTAs: by the thread that adds second
+    (300, 16, 7300, 200, 5000, 1.0),      # two and more items per SM, some shared by two CTAs
 ])
 def test_scores_updated_by_the_column_sum_kernel(M, H, T_hot, T_ret, old_T, ratio):
     """The running scores and counts get the bits that the update behind the call gives; the other outputs, the keys
