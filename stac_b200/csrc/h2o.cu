@@ -66,8 +66,11 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total_out)
 // One CTA per (layer, head) row.  Positions flagged in `is_base` (pinned and recent tokens)
 // are always kept; of the others the `k` highest scores are kept (ties: lower position
 // first).  Emits the kept positions and the dropped positions, both ascending.
-// 1024 threads, two CTAs per SM, as long as that is one wave of rows, else 512 and up to four: the kernel is a
-// chain of latencies and barriers.  (384 rows: 8328 tokens 38.9 -> 33.4 us, 15615 tokens 60.2 -> 57.4.)
+// 1024 threads, two CTAs per SM, as long as that is one wave of rows, else 512 where three of them or four share an SM:
+// the kernel is a chain of latencies and barriers.  (384 rows, 1024 against 512 threads: 8328 tokens 37.0, 30.9 us, 15615
+// tokens 55.0, 51.3, 18600 tokens 65.3, 62.1.)  A row's keys lie in shared memory: from 18881 tokens only two fit an SM,
+// from 28 thousand only one, and the larger CTAs have twice the warps there (19500 tokens 67.3, 80.8, 33000 tokens 139, 192).
+constexpr int kSelectStaticSmem = 1280;      // counters and such, rounded up
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 h2o_select_kernel(const float* __restrict__ scores, long long row_stride, const unsigned char* __restrict__ is_base,
@@ -540,9 +543,11 @@ int stac_h2o_select(const float* scores, int64_t row_stride, int n_rows, const u
         return STAC_ERR_CUDA;
     attr_done.mark(dev);
   }
-  const bool one_wave = n_rows <= 2 * n_sm;
-  if (stac::launch_behind(one_wave ? stac::h2o_select_kernel<1024> : stac::h2o_select_kernel<512>, dim3(n_rows),
-                          dim3(one_wave ? 1024 : 512), smem, reinterpret_cast<cudaStream_t>(stream),
+  // (228 KB per SM, 1 KB of it per CTA for the system)
+  const bool three_per_sm = 3 * (smem + stac::kSelectStaticSmem + 1024) <= 228 * 1024;
+  const bool small = n_rows > 2 * n_sm && three_per_sm;
+  if (stac::launch_behind(small ? stac::h2o_select_kernel<512> : stac::h2o_select_kernel<1024>, dim3(n_rows),
+                          dim3(small ? 512 : 1024), smem, reinterpret_cast<cudaStream_t>(stream),
                           scores, row_stride, is_base, T, n_keep, keep_idx, drop_idx) != cudaSuccess)
     return STAC_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;

@@ -112,7 +112,11 @@ def test_upsert_of_a_long_chunk_sorts_its_new_keys_outside_shared_memory():
         t_gpu.upsert_points(torch.zeros((131073, 3)))
 
 
-@pytest.mark.parametrize("T,n_recent,n_pinned,k", [(3, 1, 1, 0), (2047, 500, 0, 700), (2049, 0, 1, 1024), (4500, 1000, 37, 2000)])
+@pytest.mark.parametrize("T,n_recent,n_pinned,k", [
+    (3, 1, 1, 0), (2047, 500, 0, 700), (2049, 0, 1, 1024), (4500, 1000, 37, 2000),
+    (18880, 4164, 1041, 2082), (18881, 4164, 1041, 2082),      # the longest rows of which three fit an SM, one token more
+    (51200, 8328, 1041, 20000),                                # the longest rows that there are
+])
 def test_h2o_select_of_many_rows(T, n_recent, n_pinned, k):
     """More rows than two CTAs per SM hold take the smaller CTAs: the same positions."""
     from stac_b200 import _lib
@@ -133,6 +137,35 @@ def test_h2o_select_of_many_rows(T, n_recent, n_pinned, k):
     keep, drop = keep.cpu().numpy(), drop.cpu().numpy()
     assert np.array_equal(keep, h2o_keep_indices(scores, T, n_recent, pinned, k, 0))
     assert np.array_equal(np.sort(np.concatenate([keep, drop], 1), 1), np.tile(np.arange(T), (rows, 1))) and (np.diff(drop) > 0).all()
+
+
+def test_h2o_select_of_long_rows_takes_time_by_waves():
+    """Rows of which one fills an SM's shared memory: three waves take half as long again as two.  (With CTAs of half the threads
+    in the longer call they took 2.3 times as long.)"""
+    from stac_b200 import _lib
+    T, n_sm = 33000, torch.cuda.get_device_properties(0).multi_processor_count
+    scores = torch.rand((3 * n_sm, T), device=DEV)
+    base = torch.zeros(T, dtype=torch.uint8, device=DEV)
+    base[T // 2:] = 1
+    n_keep = int(base.sum()) + 4000
+    keep = torch.empty((3 * n_sm, n_keep), dtype=torch.int32, device=DEV)
+    drop = torch.empty((3 * n_sm, T - n_keep), dtype=torch.int32, device=DEV)
+
+    def best_of(rows):
+        times = []
+        for _ in range(20):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                assert _lib.lib().stac_h2o_select(_lib.ptr(scores), T, rows, _lib.ptr(base), T, n_keep, _lib.ptr(keep),
+                                                  _lib.ptr(drop), _lib.stream_ptr()) == 0
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    two, three = best_of(2 * n_sm), best_of(3 * n_sm)
+    assert three < 1.75 * two, (two, three)
 
 
 @pytest.mark.parametrize("T,n_recent,n_pinned,k", [(700, 200, 100, 150), (15615, 8328, 1041, 2082),
