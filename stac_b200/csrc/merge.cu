@@ -1289,7 +1289,11 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
 // voxels 1490 us per insert when the warps of the CTA that held a long row had to rank it, 767 us with
 // the list, 572 us with the scores passed between lanes instead of read one by one; 48 heads on 20 voxels 4966,
 // 2910 and 1938 us; 384 heads on 200 voxels 2816, 2378 and 2240 us.)
-__global__ void __launch_bounds__(256) rows_rank_kernel(const MergeParams p) {
+// kMinCtas: the rows of up to kShortRow tokens take 64 registers, with which four CTAs share an SM; for the longer ones, that wait
+// for more loads, six of 40 are better.  (us in this kernel with four and six, tokens and voxels of a head: 500 heads 4164, 300
+// 298, 251, 4164, 20 6063, 5561; 384 heads 1041, 20 338, 305; 500 heads 1500, 300 85, 90; 16 heads 8328, 6500 9.0, 11.8.)
+template <int kMinCtas>
+__global__ void __launch_bounds__(256, kMinCtas) rows_rank_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
   const int h = blockIdx.y;
   const int r0 = blockIdx.x * 256;
@@ -1905,7 +1909,10 @@ int launch_merge(MergeParams& mp, cudaStream_t st) {
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
   if (launch_behind(tokens_sim_merge_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_merge_kernel<T>, dim3(n_sm * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  if (launch_behind(rows_rank_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  // (as many tokens per voxel as that: most are in rows above kShortRow)
+  const bool long_rows = mp.n_new > kShortRow * static_cast<long long>(mp.voxel_used);
+  if (launch_behind(long_rows ? rows_rank_kernel<6> : rows_rank_kernel<4>, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess)
+    return STAC_ERR_CUDA;
   // (a CTA per head: with more than two per SM those of 512 threads are one wave; 384 heads, both launches
   // 55.1 -> 38.3 us in a bounded memory, 21.5 -> 15.6 in a stream of chunks of four frames)
   const bool two_per_sm = mp.heads <= 2 * n_sm;
