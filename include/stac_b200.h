@@ -265,7 +265,8 @@ enum stac_meta_index {       /* int32 counters in device memory, pool->meta[STAC
 typedef struct stac_pool {
   int heads, head_dim, elem_bytes;   /* elem_bytes: 2 = bf16, 4 = f32 storage of K and V */
   int pivot_cap, budget_cap;         /* P <= 4, B <= 8 */
-  int voxel_cap, voxel_used;         /* row stride per head; voxels known at the last insert */
+  int voxel_cap, voxel_used;         /* row stride per head; voxels known at the last insert: new tokens with
+                                        other ids are left out, carried ones are not */
   float sim_thresh, replace_thresh, score_thresh;
   void* buf_K; void* buf_V; float* buf_S;       /* [buf_cap][head_dim], [buf_cap] */
   int* buf_row_seg; int* buf_row_cnt; int* buf_free; int buf_cap;

@@ -243,8 +243,9 @@ __device__ __forceinline__ int warp_scan_sum(int v, int lane) {      // inclusiv
 // (8328 tokens each: 16 heads 34.5 -> 21.4 us, 384 heads 105.5 -> 70.3; 4164 each, 384 heads 54.5 -> 44.5; 1041 each, 384 heads
 // 19.4 -> 14.1.  The lists in global memory cost a scattered 4-byte write per key, value and pass, and a round trip
 // to L2 around every block scan, one per 4 kThreads tokens.)
+// False, with nothing written, if a carried token's id does not fit: carried tokens may lie above this call's voxel count.
 template <int kThreads, int kItems>
-__device__ __forceinline__ void sort_tokens_shared(const MergeParams& p, int h, int os, int n_items, unsigned* buf, int* hist) {
+__device__ __forceinline__ bool sort_tokens_shared(const MergeParams& p, int h, int os, int n_items, unsigned* buf, int* hist) {
   constexpr int kWarps = kThreads / 32, kHistRow = 257;
   constexpr unsigned kNone = 0xFFFFu;
   __shared__ int counts[kWarps];
@@ -310,6 +311,7 @@ __device__ __forceinline__ void sort_tokens_shared(const MergeParams& p, int h, 
         if (c0 + t * 32 + lane < c1) count(buf[c0 + t * 32 + lane], shift);
     }
     __syncthreads();
+    if (shift == 16 && n_valid - n_new_valid != n_items - p.n_new) return false;      // a carried token's id is too wide
     // exclusive scan of the counters in (digit, warp) order: 8 consecutive entries per thread
     int loc[8];
     int sum = 0;
@@ -391,6 +393,7 @@ __device__ __forceinline__ void sort_tokens_shared(const MergeParams& p, int h, 
     p.n_tok[h] = n;
     if (n_new_valid > 0) atomicOr(&p.plan[kPlanAnyValid], 1);
   }
+  return true;
 }
 
 template <int kThreads, int kMinCtas, int kItems>
@@ -407,13 +410,13 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const M
   __shared__ int warp_sums[32];
   __shared__ int sh_total;
   __shared__ int sh_carry;
+  __shared__ int n_passes;
   const int h = blockIdx.x;
   if constexpr (kItems > 0) {
     const int os = p.over_start_in[h], n_items = p.n_new + p.over_start_in[h + 1] - os;
-    if (n_items <= min(p.ncap, kThreads * kItems) && p.voxel_used <= 0xFFFF) {
-      sort_tokens_shared<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem + kHistRow * kWarps), hist);
+    if (n_items <= min(p.ncap, kThreads * kItems) && p.voxel_used <= 0xFFFF &&
+        sort_tokens_shared<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem + kHistRow * kWarps), hist))
       return;
-    }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned int* ka = p.keys_a + static_cast<long long>(h) * p.ncap;
@@ -462,13 +465,20 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const M
     if (threadIdx.x == 0) report_error(p.err, DEV_SORT_CAPACITY);
     n = p.ncap;
   }
+  unsigned int top = 0u;
   for (int o = os + threadIdx.x; o < oe; o += kThreads) {
     const int dst = n_valid + (o - os);
     if (dst < n) {
-      ka[dst] = static_cast<unsigned int>(p.over_hv_in[2 * o + 1]);
+      const unsigned int id = static_cast<unsigned int>(p.over_hv_in[2 * o + 1]);
+      ka[dst] = id;
       va[dst] = ~o;
+      top = max(top, id);
     }
   }
+  // Carried tokens may lie above this call's voxel count: all digits then, one more pass where that keeps their number odd (the
+  // kernels behind take the list from where p.passes leaves it).
+  const bool wide = __syncthreads_or(p.passes < 4 && (top >> (8 * p.passes)) != 0u);
+  if (threadIdx.x == 0) n_passes = wide ? 4 + (p.passes & 1) : p.passes;
   __syncthreads();
   // 3. stable LSD radix sort by voxel id.  Each warp owns a contiguous chunk of the list so
   //    that (warp, position in chunk) preserves the input order.
@@ -481,8 +491,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const M
   // loops.
   constexpr int kRegIt = 8;
   int* my_hist = hist + warp * kHistRow;
-  for (int pass = 0; pass < p.passes; ++pass) {
-    const int shift = pass * 8;
+  for (int pass = 0; pass < n_passes; ++pass) {
+    const int shift = min(pass, 3) * 8;      // (a fifth pass moves the sorted list)
     for (int i = threadIdx.x; i < kHistRow * kWarps; i += kThreads) hist[i] = 0;
     unsigned int kreg[kRegIt];
     int vreg[kRegIt];

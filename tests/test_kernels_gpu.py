@@ -769,6 +769,44 @@ def test_sorts_of_all_shapes_give_the_same_memory(heads, Tn, voxels, used):
         assert all(torch.equal(a, b) for a, b in zip(rows(many, two), rows(small, [0, 1]))), step
 
 
+@pytest.mark.parametrize("used,Tn", [(500, 700), (500, 9300), (200, 9300), (70000, 700)])
+def test_carried_tokens_above_the_voxel_count_of_a_call(used, Tn):
+    """Tokens that an insert carries over belong to their voxels whatever count the next one is given (the manager's only grows):
+    ids of 17 bits and the largest of 16, ids that share their low digits with ids below the count, in lists for shared
+    and for global memory, one, two and three digits."""
+    from stac_b200.stac.merger import VoxelKVMerger
+    H, D, voxels = 3, 64, 70000
+    ids = torch.tensor([44, 300, 180, 436, 65535, 65536 + 44, 69999], device=DEV, dtype=torch.int32)
+    g = torch.Generator(device=DEV).manual_seed(used + Tn)
+    a, b = (VoxelKVMerger(H, D, init_voxels=voxels, pivot_cap=4, budget_cap=8, sim_thresh=0.8, replace_thresh=0.8, score_thresh=0.1,
+                          dtype=torch.bfloat16, device=DEV, allocator="segment", seg_size=1, slab_cap=16) for _ in range(2))
+
+    def tokens(n, vx):
+        K, V = (torch.randn(H, n, D, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+        return K, V, torch.exp(torch.randn(H, n, device=DEV, generator=g)), None, vx
+
+    first = tokens(400, ids[torch.randint(0, len(ids), (H, 400), device=DEV, generator=g)])
+    for vm in (a, b):
+        vm.insert_and_merge(*first, voxels)
+    a._pull_meta()
+    assert a._over_max_head > 100
+    b.ensure_capacity = lambda n: None
+    b._voxel_offset = used
+    second = tokens(Tn, torch.randint(0, min(used, 500), (H, Tn), device=DEV, generator=g).int())
+    a.insert_and_merge(*second, voxels)
+    b.insert_and_merge(*second, used)
+    for name in ("_buf_row_cnt", "_piv_row_cnt", "_buf_row_seg", "_piv_row_seg", "_meta"):
+        assert torch.equal(getattr(a, name), getattr(b, name)), name
+    for cnt, seg, fields in (("_buf_row_cnt", "_buf_row_seg", ("_buf_K", "_buf_V", "_buf_S")),
+                             ("_piv_row_cnt", "_piv_row_seg", ("_piv_K", "_piv_V", "_piv_W", "_piv_S", "_piv_C"))):
+        live = getattr(a, seg)
+        live = live[live >= 0].long()
+        assert all(torch.equal(getattr(a, f)[live], getattr(b, f)[live]) for f in fields), cnt
+    n = int(a._over[a._over_cur]["start"][-1])
+    assert n > 0 and all(torch.equal(a._over[a._over_cur][f][:n], b._over[b._over_cur][f][:n]) for f in ("K", "V", "S", "hv"))
+    assert torch.equal(a._over[a._over_cur]["start"], b._over[b._over_cur]["start"])
+
+
 @pytest.mark.parametrize("Tn", [2049, 4097, 8328])      # second listing round, past the registers, the pool-stress length
 def test_sort_of_many_heads_equals_the_sort_of_few(Tn):
     """300 heads take the sort's CTAs of 512 threads, four of them the ones of 1024 (which are compared with the oracle):
