@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const M
     }
     __syncthreads();
     auto scatter = [&](bool in, unsigned int key, int val) {
-      const unsigned int d = (key >> shift) & 255u;
-      const unsigned int peers = same_digit(in, d);
+      const unsigned int d = in ? ((key >> shift) & 255u) : (256u + lane);
+      const unsigned int peers = __match_any_sync(kFull, d);
       const unsigned int before = peers & ((1u << lane) - 1);
       if (in) {
         const int dst = my_hist[d] + __popc(before);
