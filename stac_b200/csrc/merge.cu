@@ -1194,63 +1194,74 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
     p.row_info[hb + ri] = info;
   };
   if (s1 - s0 <= kShortRow) {
-    // Most rows: all tokens in registers, their loads and those of the buffer's segments side by side.  (Token by token, as
-    // below, with scores read again for every comparison: 75.6 against 59.0 us in this kernel with 384 heads of
-    // 8328 tokens, 63.4 against 50.6 with 4164, 15.4 against 8.9 with 16 heads.)
+    // Most rows: all tokens in registers, their loads side by side; the buffer's segments only where a token is selected.  (Token
+    // by token, as below, with scores read again for every comparison: 80.9 against 57.8 us in this kernel with 384 heads of
+    // 8328 tokens, 15.4 against 9.9 with 16 heads.)
     const int n = s1 - s0;
     float sc[kShortRow], sim[kShortRow];
-    int seg[kMaxB];
 #pragma unroll
     for (int j = 0; j < kShortRow; ++j) {
       sc[j] = j < n ? tscore[s0 + j] : 0.f;
       sim[j] = j < n && npiv > 0 ? p.tok_sim[hb + s0 + j] : -INFINITY;
-    }
-#pragma unroll
-    for (int c = 0; c < kMaxB; c += 4) {
-      if (p.buf_seg_vec) {
-        const int4 sg = c < nbuf ? reinterpret_cast<const int4*>(p.buf_row_seg)[r * 2 + c / 4] : make_int4(0, 0, 0, 0);
-        seg[c] = sg.x; seg[c + 1] = sg.y; seg[c + 2] = sg.z; seg[c + 3] = sg.w;
-      } else {
-#pragma unroll
-        for (int e = c; e < c + 4; ++e) seg[e] = e < nbuf ? p.buf_row_seg[r * p.B + e] : 0;
-      }
     }
     const float gate = npiv > 0 ? row_gate(p, r, npiv) : -INFINITY;
     unsigned sel = 0u;
 #pragma unroll
     for (int j = 0; j < kShortRow; ++j)
       if (j < n && (npiv == 0 || (sim[j] < p.replace_thresh && fmaxf(sc[j], 1e-6f) > gate))) sel |= 1u << j;
-    int old_rank[kMaxB];       // buffered tokens are stored in rank order
-#pragma unroll
-    for (int c = 0; c < kMaxB; ++c) old_rank[c] = c;
     if (sel == 0u) {           // nothing to buffer: everything stays in its place
 #pragma unroll
       for (int j = 0; j < kShortRow; ++j)
         if (j < n) tdest[s0 + j] = -1;
-    } else {
-      float ex[kMaxB];
 #pragma unroll
-      for (int c = 0; c < kMaxB; ++c) ex[c] = c < nbuf ? p.buf_S[seg[c]] : 0.f;
+      for (int c = 0; c < kMaxB; c += 4)      // (places behind the buffered ones are not read)
+        if (c < nbuf) *reinterpret_cast<int4*>(od + c) = make_int4(c, c + 1, c + 2, c + 3);
+      publish(0);
+      return;
+    }
+    float ex[kMaxB];           // buffered tokens are stored in rank order
 #pragma unroll
-      for (int c = 0; c < kMaxB; ++c)
+    for (int c = 0; c < kMaxB; c += 4) {
+      int4 sg = make_int4(0, 0, 0, 0);
+      if (p.buf_seg_vec) {
+        if (c < nbuf) sg = reinterpret_cast<const int4*>(p.buf_row_seg)[r * 2 + c / 4];
+      } else {
+        const int* row_seg = p.buf_row_seg + r * p.B;
+        if (c < nbuf) sg.x = row_seg[c];
+        if (c + 1 < nbuf) sg.y = row_seg[c + 1];
+        if (c + 2 < nbuf) sg.z = row_seg[c + 2];
+        if (c + 3 < nbuf) sg.w = row_seg[c + 3];
+      }
+      ex[c] = c < nbuf ? p.buf_S[sg.x] : 0.f;
+      ex[c + 1] = c + 1 < nbuf ? p.buf_S[sg.y] : 0.f;
+      ex[c + 2] = c + 2 < nbuf ? p.buf_S[sg.z] : 0.f;
+      ex[c + 3] = c + 3 < nbuf ? p.buf_S[sg.w] : 0.f;
+    }
 #pragma unroll
-        for (int j = 0; j < kShortRow; ++j) old_rank[c] += ((sel >> j) & 1u) && sc[j] > ex[c] ? 1 : 0;
+    for (int c = 0; c < kMaxB; c += 4) {
+      if (c < nbuf) {
+        int old_rank[4];
 #pragma unroll
-      for (int j = 0; j < kShortRow; ++j) {
-        if (j < n) {
-          int rank = 0;
+        for (int e = 0; e < 4; ++e) {
+          old_rank[e] = c + e;
 #pragma unroll
-          for (int c = 0; c < kMaxB; ++c) rank += c < nbuf && ex[c] >= sc[j] ? 1 : 0;
-#pragma unroll
-          for (int j2 = 0; j2 < kShortRow; ++j2)
-            rank += ((sel >> j2) & 1u) && (j2 < j ? sc[j2] >= sc[j] : sc[j2] > sc[j]) ? 1 : 0;
-          tdest[s0 + j] = (sel >> j) & 1u ? rank : -1;
+          for (int j = 0; j < kShortRow; ++j) old_rank[e] += ((sel >> j) & 1u) && sc[j] > ex[c + e] ? 1 : 0;
         }
+        *reinterpret_cast<int4*>(od + c) = make_int4(old_rank[0], old_rank[1], old_rank[2], old_rank[3]);
       }
     }
 #pragma unroll
-    for (int c = 0; c < kMaxB; c += 4)      // (places behind the buffered ones are not read)
-      if (c < nbuf) *reinterpret_cast<int4*>(od + c) = make_int4(old_rank[c], old_rank[c + 1], old_rank[c + 2], old_rank[c + 3]);
+    for (int j = 0; j < kShortRow; ++j) {
+      if (j < n) {
+        int rank = 0;
+#pragma unroll
+        for (int c = 0; c < kMaxB; ++c) rank += c < nbuf && ex[c] >= sc[j] ? 1 : 0;
+#pragma unroll
+        for (int j2 = 0; j2 < kShortRow; ++j2)
+          rank += ((sel >> j2) & 1u) && (j2 < j ? sc[j2] >= sc[j] : sc[j2] > sc[j]) ? 1 : 0;
+        tdest[s0 + j] = (sel >> j) & 1u ? rank : -1;
+      }
+    }
     publish(__popc(sel));
     return;
   }
@@ -1299,9 +1310,9 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
 // voxels 1490 us per insert when the warps of the CTA that held a long row had to rank it, 767 us with
 // the list, 572 us with the scores passed between lanes instead of read one by one; 48 heads on 20 voxels 4966,
 // 2910 and 1938 us; 384 heads on 200 voxels 2816, 2378 and 2240 us.)
-// kMinCtas: the rows of up to kShortRow tokens take 64 registers, with which four CTAs share an SM; for the longer ones, that wait
-// for more loads, six of 40 are better.  (us in this kernel with four and six, tokens and voxels of a head: 500 heads 4164, 300
-// 298, 251, 4164, 20 6063, 5561; 384 heads 1041, 20 338, 305; 500 heads 1500, 300 85, 90; 16 heads 8328, 6500 9.0, 11.8.)
+// kMinCtas: four CTAs per SM let the rows of up to kShortRow tokens have 64 registers, six 40.  Six are better wherever they find work,
+// most of all with longer rows, which wait for more loads.  (us in this kernel with four and six, tokens and voxels of a head: 384
+// heads 8328, 6500 63.2, 57.8, 8328, 300 721, 619; 148 heads 4164, 200 260, 238; 16 heads 8328, 6500 9.9, 11.2.)
 template <int kMinCtas>
 __global__ void __launch_bounds__(256, kMinCtas) rows_rank_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
@@ -1919,9 +1930,9 @@ int launch_merge(MergeParams& mp, cudaStream_t st) {
   dim3 grid_tok((mp.ncap + kTokBlock - 1) / kTokBlock, mp.heads);
   if (launch_behind(tokens_sim_merge_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_merge_kernel<T>, dim3(n_sm * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
-  // (as many tokens per voxel as that: most are in rows above kShortRow)
-  const bool long_rows = mp.n_new > kShortRow * static_cast<long long>(mp.voxel_used);
-  if (launch_behind(long_rows ? rows_rank_kernel<6> : rows_rank_kernel<4>, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess)
+  // (four CTAs per SM hold a thread per token: no row waits for a place)
+  const bool few_rows = static_cast<long long>(mp.heads) * mp.n_new <= 4ll * 256 * n_sm;
+  if (launch_behind(few_rows ? rows_rank_kernel<4> : rows_rank_kernel<6>, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess)
     return STAC_ERR_CUDA;
   // (a CTA per head: with more than two per SM those of 512 threads are one wave; 384 heads, both launches
   // 55.1 -> 38.3 us in a bounded memory, 21.5 -> 15.6 in a stream of chunks of four frames)

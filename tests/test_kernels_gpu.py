@@ -737,7 +737,7 @@ def test_launches_are_counted_where_they_are_made(M, H, T):
 
 @pytest.mark.parametrize("heads,Tn,voxels,used", [
     (4, 1, 3, 3), (4, 33, 5, 5), (4, 1500, 300, 70000),     # one token; lists in shared and in global memory (ids above 16 bits)
-    (4, 1500, 100, 70000),                                  # rows of 15 tokens, ranked by the kernels for long and for short rows
+    (4, 1500, 100, 70000), (200, 1500, 100, 70000),         # rows of 15 tokens; with both register budgets of the ranking
     (200, 2500, 500, 500),                                  # two heads per SM
     (300, 1500, 40, 40), (300, 1537, 300, 300),             # four per SM (in the second call more carried tokens than it holds), three
     (300, 9000, 1800, 1800), (460, 1600, 300, 300),         # too long for three per SM; more heads than three per SM
