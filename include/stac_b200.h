@@ -66,7 +66,8 @@ uint64_t stac_kernel_launches(void);
  *   bias_ret   f32 [H, >=T_ret], heads bias_head_stride apart: log C per pivot, -inf for padding
  *   lse        f32 [H, M] natural-log row log-sum-exp, or NULL
  *   colsum     f32 [H, colsum_head_stride]: entries [0,T_hot) hot keys, [T_hot, T_hot+T_ret)
- *              retrieved keys; or NULL to skip the column-sum pass
+ *              retrieved keys; or NULL to skip the column-sum pass.  Rows whose log-sum-exp is -inf or
+ *              beyond 1e29 in size add nothing
  *   workspace  scratch of at least stac_attn_workspace_bytes(M, H) bytes, 256-byte aligned, contents
  *              need no initialisation: the per-row log-sum-exps passed from the forward to the
  *              column-sum pass, a few flags and counters (cleared by the call), then ~11 MB for the

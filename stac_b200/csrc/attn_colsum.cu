@@ -39,7 +39,8 @@ constexpr int col_threads(int group) { return 128 + group * 128; }   // warpgrou
 #ifndef STAC_COL_PAIR_MASK
 #define STAC_COL_PAIR_MASK 0x88
 #endif
-constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;   // which of 8 consecutive PAIRS of exponentials of the column-sum kernel run on the FMA pipes
+// which of 8 consecutive PAIRS of exponentials of the column-sum kernel run on the FMA pipes
+constexpr unsigned kColPairMask = STAC_COL_PAIR_MASK;
 #ifndef STAC_COL_FOLD_LSE
 #define STAC_COL_FOLD_LSE 1
 #endif
@@ -860,7 +861,8 @@ attn_fwd_fast_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (row < valid) bv = is_ret ? p.bias_ret[h * p.bias_head_stride + n0 + row] * kLog2e : 0.f;
         named_bar_sync(1 + g, 128);   // the bias is on its way while the warpgroup meets
         if (row < kFT) sm.bias2[g][row] = bv;
-        const bool tile_live = named_bar_or(1 + g, 128, bv != -INFINITY);   // false: every key of the tile is masked (padding behind the valid pivots)
+        // false: every key of the tile is masked (padding behind the valid pivots)
+        const bool tile_live = named_bar_or(1 + g, 128, bv != -INFINITY);
         any_live = any_live || tile_live;
         const bool first = !have_ref;
         if (first) reference(true);
@@ -1403,7 +1405,7 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const int w = (warp - 4) >> 2;   // which key tile of the group
     const int wq = warp & 3;
     const int key = wq * 32 + lane;  // key inside the tile = TMEM lane
-    const int tid = threadIdx.x - 128;  // 0..383
+    const int tid = threadIdx.x - 128;  // 0..kExpThreads - 1
     const uint32_t t_base = tmem + (static_cast<uint32_t>(wq * 32) << 16) + w * 128;
     const float c2 = p.scale_log2;
     ColWalk walk(p);

@@ -576,7 +576,8 @@ int compact_launch(const int* keep_idx, long long keep_stride, int n_rows, int n
       return STAC_ERR_CUDA;
   }
   dim3 grid_m((T_buf + 255) / 256, n_rows);
-  if (stac::launch_behind(s_src != nullptr ? stac::compact_meta_kernel<true> : stac::compact_meta_kernel<false>, grid_m, dim3(256), 0, st, keep_idx, keep_stride, n_keep, T_buf,
+  auto* const meta_kernel = s_src != nullptr ? stac::compact_meta_kernel<true> : stac::compact_meta_kernel<false>;
+  if (stac::launch_behind(meta_kernel, grid_m, dim3(256), 0, st, keep_idx, keep_stride, n_keep, T_buf,
                           reinterpret_cast<const long long*>(ti_src), reinterpret_cast<long long*>(ti_dst), s_src,
                           s_dst, c_src, c_dst, vx_src, vx_dst) != cudaSuccess)
     return STAC_ERR_CUDA;
