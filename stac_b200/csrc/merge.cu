@@ -1194,21 +1194,25 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
     p.row_info[hb + ri] = info;
   };
   if (s1 - s0 <= kShortRow) {
-    // Most rows: all tokens in registers, their loads side by side; the buffer's segments only where a token is selected.  (Token
-    // by token, as below, with scores read again for every comparison: 80.9 against 57.8 us in this kernel with 384 heads of
-    // 8328 tokens, 15.4 against 9.9 with 16 heads.)
+    // Most rows: all tokens in registers; similarities become bits before the gate is there, and the buffer's segments are read only where a
+    // token is selected, so that few values are spilled.  (Token by token, as below, with scores read again for every comparison:
+    // 80.6 against 49.6 us in this kernel with 384 heads of 8328 tokens, 15.2 against 10.0 with 16 heads.)
     const int n = s1 - s0;
-    float sc[kShortRow], sim[kShortRow];
+    float sc[kShortRow];
+    unsigned sel = npiv == 0 ? (1u << n) - 1u : 0u;
+    if (npiv > 0) {
 #pragma unroll
-    for (int j = 0; j < kShortRow; ++j) {
-      sc[j] = j < n ? tscore[s0 + j] : 0.f;
-      sim[j] = j < n && npiv > 0 ? p.tok_sim[hb + s0 + j] : -INFINITY;
+      for (int j = 0; j < kShortRow; ++j)
+        if (j < n && p.tok_sim[hb + s0 + j] < p.replace_thresh) sel |= 1u << j;
     }
-    const float gate = npiv > 0 ? row_gate(p, r, npiv) : -INFINITY;
-    unsigned sel = 0u;
 #pragma unroll
-    for (int j = 0; j < kShortRow; ++j)
-      if (j < n && (npiv == 0 || (sim[j] < p.replace_thresh && fmaxf(sc[j], 1e-6f) > gate))) sel |= 1u << j;
+    for (int j = 0; j < kShortRow; ++j) sc[j] = j < n ? tscore[s0 + j] : 0.f;
+    if (npiv > 0) {
+      const float gate = row_gate(p, r, npiv);
+#pragma unroll
+      for (int j = 0; j < kShortRow; ++j)
+        if (!(fmaxf(sc[j], 1e-6f) > gate)) sel &= ~(1u << j);
+    }
     if (sel == 0u) {           // nothing to buffer: everything stays in its place
 #pragma unroll
       for (int j = 0; j < kShortRow; ++j)
@@ -1312,7 +1316,7 @@ __device__ __forceinline__ void rank_row_thread(const MergeParams& p, const int 
 // 2910 and 1938 us; 384 heads on 200 voxels 2816, 2378 and 2240 us.)
 // kMinCtas: four CTAs per SM let the rows of up to kShortRow tokens have 64 registers, six 40.  Six are better wherever they find work,
 // most of all with longer rows, which wait for more loads.  (us in this kernel with four and six, tokens and voxels of a head: 384
-// heads 8328, 6500 63.2, 57.8, 8328, 300 721, 619; 148 heads 4164, 200 260, 238; 16 heads 8328, 6500 9.9, 11.2.)
+// heads 8328, 6500 63, 50, 8328, 300 of 70000 721, 621; 148 heads 4164, 200 of 70000 260, 234; 16 heads 8328, 6500 9.9, 11.2.)
 template <int kMinCtas>
 __global__ void __launch_bounds__(256, kMinCtas) rows_rank_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
