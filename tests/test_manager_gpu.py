@@ -208,6 +208,18 @@ def test_window_manager_and_h2o_manager():
     assert np.array_equal(first[:tpf], np.arange(tpf)) and np.array_equal(first[tpf:], np.arange(5 * tpf, 7 * tpf))
 
 
+def test_values_of_two_batches_append_the_first():
+    """Keys have one batch; of values with more, the first is appended."""
+    from stac_b200.stac import KVManager
+    kv = KVManager(2, 3, 64, 8, chunk_size=2, buffer_size=6, recent_size=2, dtype=torch.bfloat16, device=torch.device(DEV))
+    kv.reset()
+    k, v = (torch.randn(n, 3, 16, 64, device=DEV).to(torch.bfloat16) for n in (1, 2))
+    kv.append_kv(k, v, 1)
+    assert torch.equal(kv.key_cache_hot[1, :, :16], k[0]) and torch.equal(kv.value_cache_hot[1, :, :16], v[0])
+    with pytest.raises(Exception):
+        kv.append_kv(k, v[0], 1)
+
+
 def test_cpu_spill_of_the_window_manager():
     """Buffers longer than gpu_limit frames: the oldest tokens of an append that does not fit go to
     the host buffer, plain attention still sees them, the host buffer raises when full
