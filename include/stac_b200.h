@@ -51,10 +51,11 @@ uint64_t stac_kernel_launches(void);
 
 /* Device integers on their way to the host: copies `na` ints from `a` to page-locked `host`, `nb` from `b` (or NULL) behind them,
  * and records `event` behind both, all on `stream`; nothing waits.  The event is one of stac_event_create, made with the stream's device
- * current; stac_event_wait returns when what the last recording was behind is complete. */
+ * current; stac_event_wait returns when what the last recording was behind is complete, stac_event_done says whether it is. */
 int stac_event_create(void** event);
 int stac_event_destroy(void* event);
 int stac_event_wait(void* event);
+int stac_event_done(void* event, int* done);
 int stac_ints_to_host(int* host, const int* a, int na, const int* b, int nb, void* event, stac_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------

@@ -100,6 +100,7 @@ SIGNATURES = {
     "stac_event_create": (c_int, [ctypes.POINTER(c_void_p)]),
     "stac_event_destroy": (c_int, [c_void_p]),
     "stac_event_wait": (c_int, [c_void_p]),
+    "stac_event_done": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "stac_ints_to_host": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p]),
     "stac_merge_scratch_bytes": (c_size_t, [c_int, c_int, c_int]),
     "stac_merge_insert": (c_int, [ctypes.POINTER(StacPool), ctypes.POINTER(StacEvicted), c_void_p, c_size_t, c_int,

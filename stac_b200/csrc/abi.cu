@@ -76,10 +76,18 @@ int stac_event_wait(void* event) {
   return cudaEventSynchronize(static_cast<cudaEvent_t>(event)) == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }
 
+int stac_event_done(void* event, int* done) {
+  if (event == nullptr || done == nullptr) return STAC_ERR_BAD_ARG;
+  const cudaError_t rc = cudaEventQuery(static_cast<cudaEvent_t>(event));
+  *done = rc == cudaSuccess ? 1 : 0;
+  if (rc != cudaSuccess) cudaGetLastError();      // (an answer, no error that a later call is to find)
+  return rc == cudaSuccess || rc == cudaErrorNotReady ? STAC_OK : STAC_ERR_CUDA;
+}
+
 int stac_ints_to_host(int* host, const int* a, int na, const int* b, int nb, void* event, stac_stream_t stream) {
-  if (host == nullptr || event == nullptr || a == nullptr || na <= 0 || nb < 0 || (nb > 0 && b == nullptr)) return STAC_ERR_BAD_ARG;
+  if (host == nullptr || event == nullptr || na < 0 || (na > 0 && a == nullptr) || nb < 0 || (nb > 0 && b == nullptr)) return STAC_ERR_BAD_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (cudaMemcpyAsync(host, a, sizeof(int) * na, cudaMemcpyDeviceToHost, st) != cudaSuccess) return STAC_ERR_CUDA;
+  if (na > 0 && cudaMemcpyAsync(host, a, sizeof(int) * na, cudaMemcpyDeviceToHost, st) != cudaSuccess) return STAC_ERR_CUDA;
   if (nb > 0 && cudaMemcpyAsync(host + na, b, sizeof(int) * nb, cudaMemcpyDeviceToHost, st) != cudaSuccess) return STAC_ERR_CUDA;
   return cudaEventRecord(static_cast<cudaEvent_t>(event), st) == cudaSuccess ? STAC_OK : STAC_ERR_CUDA;
 }

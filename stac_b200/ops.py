@@ -1,5 +1,6 @@
 """Thin torch-tensor wrappers over the C ABI (one function per entry point)."""
 
+import collections
 import ctypes
 import functools
 import math
@@ -41,14 +42,17 @@ class LaggedInts:
     one step ahead of the GPU.  ``pull`` returns None when nothing is pending."""
 
     def __init__(self, n):
+        _free_dropped()
         self.pin = torch.zeros(n, dtype=torch.int32).pin_memory()
         self.host, self.event, self.waiting = self.pin.data_ptr(), None, False      # one event, recorded again by every push
 
-    def push(self, first, second=None):
-        """Contiguous int32 tensors.  (Copies and event in one call of the library: 14 -> 5 us with two tensors against torch's.)"""
+    def push(self, *tensors):
+        """(Copies and event in one call of the library: 14 -> 5 us with two tensors against torch's.)"""
+        if len(tensors) not in (1, 2) or not all(t.is_cuda and t.dtype is torch.int32 and t.is_contiguous() for t in tensors):
+            tensors = (torch.cat([t.reshape(-1).to("cuda", torch.int32) for t in tensors]),)
+        first, second = tensors if len(tensors) == 2 else (tensors[0], None)
         n, m = first.numel(), 0 if second is None else second.numel()
-        assert first.dtype is torch.int32 and first.is_contiguous() and n + m <= self.pin.numel()
-        assert second is None or (second.dtype is torch.int32 and second.is_contiguous())
+        assert n + m <= self.pin.numel()
         if self.event is None:
             event = ctypes.c_void_p()
             check(_lib.lib().stac_event_create(ctypes.byref(event)), "stac_event_create")
@@ -60,26 +64,57 @@ class LaggedInts:
     def pending(self):
         return self.waiting
 
-    def _wait(self):
-        check(_lib.lib().stac_event_wait(self.event), "stac_event_wait")
-        self.waiting = False
+    def _arrive(self):
+        if self.waiting and self.event is not None:
+            check(_lib.lib().stac_event_wait(self.event), "stac_event_wait")
 
     def pull(self):
         if not self.waiting:
             return None
-        self._wait()
+        self._arrive()
+        self.waiting = False
         return self.pin.tolist()
 
+    # A copy, or what is unpickled, has memory of its own and no event.
+    def __getstate__(self):
+        self._arrive()
+        return self.pin.tolist(), self.waiting
+
+    def __setstate__(self, state):
+        values, waiting = state
+        self.__init__(len(values))
+        self.pin.copy_(torch.tensor(values, dtype=torch.int32))
+        self.waiting = waiting
+
     def __del__(self):
-        # (the page-locked memory may be handed to somebody else as soon as it is free: not before the copy has arrived)
+        # Whoever drops it may be a step ahead of the GPU, or in the middle of a graph capture, which a wait would spoil.
+        event = self.__dict__.pop("event", None)
         try:
-            if getattr(self, "waiting", False):
-                self._wait()
-            if getattr(self, "event", None) is not None:
-                _lib.lib().stac_event_destroy(self.event)
-                self.event = None
+            if event is not None and self.waiting:
+                _dropped.append((self.pin, event))
+            elif event is not None:
+                _lib.lib().stac_event_destroy(event)
         except Exception:       # the process or its context is on the way out
             pass
+
+
+# Page-locked memory (which may be handed to somebody else as soon as it is free) and events of mirrors that went away before their
+# copies had arrived; given back when the next mirror is made, so that there are never more than the GPU is behind.
+_dropped = collections.deque()
+
+
+def _free_dropped():
+    for _ in range(len(_dropped)):
+        try:
+            pin, event = _dropped.popleft()
+        except IndexError:      # another thread has it
+            return
+        done = ctypes.c_int(0)
+        _lib.lib().stac_event_done(event, ctypes.byref(done))
+        if done.value:
+            _lib.lib().stac_event_destroy(event)
+        else:
+            _dropped.append((pin, event))
 
 
 _workspaces = {}

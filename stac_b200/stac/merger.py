@@ -239,7 +239,7 @@ class VoxelKVMerger:
         """Enqueue the copy of the pool counters, the per-head overflow offsets and the status word
         to pinned host memory behind the insert that produced them; nothing waits here."""
         self._pushed_cur = self._over_cur
-        self._mirror.push(self._counters, self._status.word if self._status is not None else None)
+        self._mirror.push(self._counters, *([self._status.word] if self._status is not None else []))
 
     def _pull_meta(self):
         """Take in what the last insert left behind (waits for that insert if it is still running);

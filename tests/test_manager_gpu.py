@@ -429,3 +429,58 @@ def test_steady_state_steps_never_wait_for_the_gpu():
     info = kv.get_merger_info()
     assert info["pivot_pool_used"] > 0 and info["used_voxels"] == kv._vm.get_voxel_num()
     kv.free()
+
+
+def test_lagged_ints_are_dropped_without_a_wait():
+    """A mirror whose copy is still on its way goes away at once, also in the middle of a graph capture; its memory is nobody
+    else's until the copy has arrived."""
+    import time
+    from stac_b200 import ops
+    a, x = torch.arange(5, dtype=torch.int32, device=DEV), torch.zeros(3, device=DEV)
+    m = ops.LaggedInts(5)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(1_000_000_000)        # half a second
+    m.push(a)
+    where, t0 = m.host, time.perf_counter()
+    del m
+    assert time.perf_counter() - t0 < 0.2
+    others = [ops.LaggedInts(5) for _ in range(3)]
+    assert len(ops._dropped) == 1 and where not in [o.host for o in others]
+    torch.cuda.synchronize()
+    others.append(ops.LaggedInts(5))
+    assert not ops._dropped
+    m, g = others.pop(), torch.cuda.CUDAGraph()
+    m.push(a)
+    with torch.cuda.graph(g):
+        x += 1
+        del m
+        x += 1
+    g.replay()
+    assert x.tolist() == [2, 2, 2]
+    ops._free_dropped()
+    assert not ops._dropped
+
+
+def test_lagged_ints_and_their_copies():
+    """Copies and what is unpickled share neither memory nor event; whatever integers are pushed arrive as int32."""
+    import copy
+    import pickle
+    from stac_b200 import ops
+    a = torch.arange(6, dtype=torch.int32, device=DEV)
+    m = ops.LaggedInts(6)
+    assert m.pull() is None
+    m.push(a)
+    others = [copy.deepcopy(m), copy.copy(m), pickle.loads(pickle.dumps(m))]
+    assert len({o.host for o in others + [m]}) == 4 and all(o.host == o.pin.data_ptr() for o in others)
+    for i, o in enumerate(others):
+        assert o.pull() == list(range(6)) and o.pull() is None
+        o.push(a[:2] + 10 * i, a[:4])
+    assert m.pull() == list(range(6))
+    for i, o in enumerate(others):
+        assert o.pull() == [10 * i, 1 + 10 * i, 0, 1, 2, 3]
+    for pushed, want in (([a.long()], range(6)), ([a.view(3, 2).t()], [0, 2, 4, 1, 3, 5]), ([a[:1], a[1:3], a[3:]], range(6)),
+                         ([a[::2], a[:3].cpu()], [0, 2, 4, 0, 1, 2])):
+        m.push(*pushed)
+        assert m.pull() == list(want)
+    with pytest.raises(Exception):
+        m.push(a, a)
