@@ -1183,11 +1183,11 @@ attn_colsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-  // Launched with programmatic serialization behind the forward kernel: barriers and tensor memory are set up while that drains.
-  // The loading warp goes on, too: keys and queries were there before the forward kernel, which lets this one start only behind
-  // its own wait for what wrote them.  (us per call: M 2603, N 6247, 12 heads 94.0 -> 93.0, M 4164, 2 heads 96.3 -> 95.6, M 1041,
-  // N 2082 33.1 -> 32.8.)  The row log-sum-exps and the zeroed output are read and written only after this point.
-  if (warp != 0) grid_dep_wait();
+  // Launched with programmatic serialization behind the forward kernel: barriers and tensor memory are set up while that drains, and
+  // nothing in global memory is touched before this, neither the row log-sum-exps and the zeroed output, which that kernel writes, nor keys and
+  // queries, which one before it may have written: a thread sees those only behind a wait of its own.  (Keys and queries loaded ahead of it gave
+  // the same bits and took 0.3 to 1.0 us less of a call.)
+  grid_dep_wait();
 
   if (warp < 4) {
     if constexpr (kGroup == kColGroup) setmaxnreg_dec<kColCtlRegs>();   // (smaller CTAs have registers enough)

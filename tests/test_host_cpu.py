@@ -41,6 +41,20 @@ def test_library_exports_every_declared_symbol():
     assert lib.stac_voxel_scratch_bytes(10) == (10 + 16) * 8 + 16   # keys, key list padded to 16, counter
 
 
+def test_every_thread_waits_for_the_kernel_before():
+    """Kernels that may start while the one before them drains see what it and its predecessors wrote only in threads that have waited:
+    no condition stands in front of a wait, and every kernel that is launched that way has one."""
+    csrc = os.path.join(ROOT, "stac_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        kernels = re.split(r"\n__global__ ", re.sub(r"//[^\n]*", "", text))[1:]
+        for line in "\n".join(kernels).splitlines():
+            assert "grid_dep_wait()" not in line or line.strip() == "grid_dep_wait();", (name, line)
+        waiting = {re.search(r"(\w+_kernel)\s*\(", k).group(1): "  grid_dep_wait();" in k for k in kernels if re.search(r"(\w+_kernel)\s*\(", k)}
+        for launched in re.findall(r"launch(?:_clusters)?_behind\([^;]*?(\w+_kernel)\b", text):
+            assert waiting.get(launched, True), (name, launched)
+
+
 def test_struct_layout_matches_header():
     import ctypes
     from stac_b200 import _lib
