@@ -88,6 +88,12 @@ int stac_ints_to_host(int* host, const int* a, int na, const int* b, int nb, voi
  * ------------------------------------------------------------------------------------- */
 size_t stac_attn_workspace_bytes(int M, int H);
 
+/* How the forward kernel cuts a call on a device with n_sm SMs (host only): the number of its CTAs (0: bad sizes), and in `parts` how many equal
+ * ones each item (128 query rows of a head) has, in `cluster` whether a cluster joins them where the device has room for all (else, and
+ * always with 0, they go through the workspace).  One part and fewer CTAs than items: equal shares of all units.  The bits of an output depend on this
+ * plan, and the plan on these arguments alone. */
+int stac_attn_forward_plan(int M, int H, int T_hot, int T_ret, int n_sm, int workspace, int* parts, int* cluster);
+
 int stac_attn_colsum(const void* q, int64_t q_row_stride,
                      const void* k_hot, const void* v_hot, int64_t hot_row_stride, int64_t hot_head_stride, int T_hot,
                      const void* k_ret, const void* v_ret, int64_t ret_row_stride, int64_t ret_head_stride, int T_ret,

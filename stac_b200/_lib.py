@@ -58,6 +58,7 @@ SIGNATURES = {
     "stac_abi_version": (c_int, []),
     "stac_kernel_launches": (ctypes.c_uint64, []),
     "stac_attn_workspace_bytes": (c_size_t, [c_int, c_int]),
+    "stac_attn_forward_plan": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int)]),
     "stac_attn_colsum": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_i64, c_int, c_void_p, c_void_p,
                                  c_i64, c_i64, c_int, c_void_p, c_i64, c_void_p, c_i64, c_void_p, c_void_p, c_i64,
                                  c_int, c_int, c_int, c_f32, c_f32, c_void_p, c_size_t, c_void_p, c_void_p]),

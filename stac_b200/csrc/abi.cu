@@ -99,6 +99,11 @@ size_t stac_attn_workspace_bytes(int M, int H) {
   return lse_bytes + stac::attn_part_elems() * sizeof(float);
 }
 
+int stac_attn_forward_plan(int M, int H, int T_hot, int T_ret, int n_sm, int workspace, int* parts, int* cluster) {
+  if (M <= 0 || H <= 0 || T_hot < 0 || T_ret < 0 || T_hot + T_ret <= 0 || n_sm <= 0 || parts == nullptr || cluster == nullptr) return 0;
+  return stac::attn_forward_plan(M, H, T_hot, T_ret, n_sm, workspace != 0, parts, cluster);
+}
+
 }  // extern "C"
 
 namespace {

@@ -157,6 +157,7 @@ constexpr int kFastMaxCtas = 160;               // partial-result slots are prov
 // middle segment, i.e. one whose score buffer was last used inside the same segment
 constexpr int kFastMinSplitTiles = 2 * kFastWgs;
 constexpr int kFastMaxCluster = 8;              // the portable size
+static_assert(kPartFloats * 4 <= kFastWgs * kFastTileBytes, "a part that a cluster joins lies where the key tiles were");
 constexpr float kFastTileUs = 0.52f, kFastPartUs = 0.42f, kFastClusterUs = 2.2f, kFastWorkspaceUs = 3.2f;
 #ifndef STAC_FAST_PAIR_MASK
 #define STAC_FAST_PAIR_MASK 0x8080u
@@ -195,8 +196,10 @@ struct FastSmem {
 
 // The (item, key tile) units of one CTA, walked segment by segment: a segment is a run of key
 // tiles [t0, t1) of one item.  With `split` the units of the whole launch are cut into equal
-// contiguous ranges, one per CTA (an item on a cut is then finished by two CTAs); without it
-// CTA i owns item i.  Every role of the CTA walks the same sequence.
+// contiguous ranges, one per CTA: an item on a cut is then finished by two CTAs, or, with parts > 1 and parts * n_items CTAs,
+// every item by `parts` CTAs.  A cut total * c / (parts * n_items) = nt * c / parts falls on an item's end wherever c is a multiple of
+// `parts`, so that each of those CTAs has one segment, of one tile at least (parts <= nt): its part may lie in one place, and is
+// joined behind the walk.  Without `split` CTA i owns item i.  Every role of the CTA walks the same sequence.
 struct FwdWalk {
   int item, t0, left, nt;     // next item, its first tile, tiles of the CTA that are left, tiles per item
   __device__ FwdWalk(const FwdParams& p, int n_tiles) {
@@ -1466,7 +1469,7 @@ int make_map(CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint6
   return r == CUDA_SUCCESS ? STAC_OK : STAC_ERR_CUDA;
 }
 
-// Clusters of `size` CTAs of the forward kernel that can be resident at once.
+// Clusters of `size` CTAs of the forward kernel that can be resident at once on this device, -1: no answer (which is asked for again).
 int max_fwd_clusters(int dev, int size, int smem) {
   static PerDeviceValue<int> cache[kFastMaxCluster + 1];     // count + 1
   int n = cache[size].get(dev);
@@ -1484,7 +1487,7 @@ int max_fwd_clusters(int dev, int size, int smem) {
     int active = 0;
     if (cudaOccupancyMaxActiveClusters(&active, attn_fwd_fast_kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
-      active = 0;
+      return -1;
     }
     cache[size].set(dev, n = active + 1);
   }
@@ -1495,14 +1498,18 @@ int max_fwd_clusters(int dev, int size, int smem) {
 // The estimate, in us: a key tile 0.52, a part more 0.42 for those who join them, and 2.2 through the shared memory of a cluster or
 // 3.2 through the workspace.  (1041 rows, 10410 keys, 1 head, 93 tiles: 1 part 52.7 us, 2, 4 and 8 32.8, 22.4 and 17.6 through clusters, 4, 8, 12 and 16
 // 23.0, 18.3, 17.9 and 18.5 through the workspace.  Clusters of eight and four have room for 15 and 33 items only.)
-void fwd_parts(int dev, int items, int tiles, int n_sm, int smem, bool workspace, int* parts, int* cluster) {
+// Parts have references of their own, so their number decides the last bits of an output: it follows from the call's sizes alone.  What a
+// device reports depends on which of its SMs are in use (and the query may fail), so that only says who joins them (see attn_colsum_launch;
+// both ways add in one order).
+constexpr int kFastClusterRoom[kFastMaxCluster + 1] = {0, 0, 74, 45, 33, 26, 22, 15, 15};      // items, of 148 SMs
+void fwd_parts(int items, int tiles, int n_sm, bool workspace, int* parts, int* cluster) {
   *parts = 1;
   *cluster = 0;
   float best = kFastTileUs * tiles;
   for (int k = 2; k * items <= n_sm && k <= tiles; ++k) {
     const float loop = kFastTileUs * ((tiles + k - 1) / k) + kFastPartUs * k;
     if (loop + kFastClusterUs >= best) continue;
-    const bool fits = k <= kFastMaxCluster && items <= max_fwd_clusters(dev, k, smem);
+    const bool fits = k <= kFastMaxCluster && items <= kFastClusterRoom[k];
     const float us = loop + (fits ? kFastClusterUs : kFastWorkspaceUs);
     if (us < best && (fits || workspace)) {
       best = us;
@@ -1511,8 +1518,18 @@ void fwd_parts(int dev, int items, int tiles, int n_sm, int smem, bool workspace
     }
   }
 }
+int fwd_tiles(int T_hot, int T_ret) { return (T_hot + kFT - 1) / kFT + (T_ret + kFT - 1) / kFT; }
+bool fwd_evenly(int items, int tiles, int n_sm, bool workspace) {     // one CTA per SM, with equal shares of all units
+  return workspace && n_sm <= kFastMaxCtas && tiles >= kFastMinSplitTiles && items >= n_sm;
+}
 
 }  // namespace
+
+int attn_forward_plan(int M, int H, int T_hot, int T_ret, int n_sm, bool workspace, int* parts, int* cluster) {
+  const int items = (M + kBM - 1) / kBM * H, tiles = fwd_tiles(T_hot, T_ret);
+  fwd_parts(items, tiles, n_sm, workspace && n_sm <= kFastMaxCtas, parts, cluster);
+  return fwd_evenly(items, tiles, n_sm, workspace) ? n_sm : *parts * items;
+}
 
 void attn_subsample_plan(int M, float ratio, int* m_sub, int* stride, float* correction) {
   // attn-cuda/csrc/bindings.cpp:63-83
@@ -1630,10 +1647,11 @@ int attn_colsum_launch(const AttnArgs& a, int* ctl, bool ctl_zeroed, float* lse2
   // parts where that pays; else every CTA takes one item.
   fp.n_q_tiles = (a.M + kBM - 1) / kBM;
   fp.n_items = fp.n_q_tiles * a.H;
-  const int n_tiles_f = (a.T_hot + kFT - 1) / kFT + (a.T_ret + kFT - 1) / kFT;
-  int grid_split = 0;
-  if (part != nullptr && n_sm <= kFastMaxCtas && n_tiles_f >= kFastMinSplitTiles && fp.n_items >= n_sm) grid_split = n_sm;
-  fwd_parts(dev, fp.n_items, n_tiles_f, n_sm, fast_smem, part != nullptr && n_sm <= kFastMaxCtas, &fp.parts, &fp.cluster);
+  const int n_tiles_f = fwd_tiles(a.T_hot, a.T_ret);
+  const bool workspace = part != nullptr && n_sm <= kFastMaxCtas;
+  int grid_split = fwd_evenly(fp.n_items, n_tiles_f, n_sm, workspace) ? n_sm : 0;
+  fwd_parts(fp.n_items, n_tiles_f, n_sm, workspace, &fp.parts, &fp.cluster);
+  if (fp.cluster && workspace && max_fwd_clusters(dev, fp.parts, fast_smem) < fp.n_items) fp.cluster = 0;     // (would take turns)
   if (fp.parts > 1) grid_split = fp.parts * fp.n_items;
   fp.split = grid_split > 0 ? 1 : 0;
   fp.part = part;

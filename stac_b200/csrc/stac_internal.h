@@ -48,6 +48,7 @@ int current_device(int* dev);
 int device_sm_count(int dev, int* n_sm);
 
 void attn_subsample_plan(int M, float ratio, int* m_sub, int* stride, float* correction);
+int attn_forward_plan(int M, int H, int T_hot, int T_ret, int n_sm, bool workspace, int* parts, int* cluster);
 constexpr int kAttnCtlWords = 512;   // control words in front of the row log-sum-exps of a workspace
 size_t attn_lse2_elems(int M, int H);
 size_t attn_part_elems();

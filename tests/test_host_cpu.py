@@ -55,6 +55,34 @@ def test_every_thread_waits_for_the_kernel_before():
             assert waiting.get(launched, True), (name, launched)
 
 
+def _plan(M, H, T_hot, T_ret, n_sm=148, workspace=1):
+    import ctypes
+    from stac_b200 import _lib
+    parts, cluster = ctypes.c_int(-1), ctypes.c_int(-1)
+    grid = _lib.lib().stac_attn_forward_plan(M, H, T_hot, T_ret, n_sm, workspace, ctypes.byref(parts), ctypes.byref(cluster))
+    return grid, parts.value, cluster.value
+
+
+def test_forward_plan():
+    """In how many parts items are cut follows from the sizes (there is no device here to ask); the shapes of the attention tests take
+    the paths that they are there for; every part has at least one tile and a CTA of one wave."""
+    assert _plan(130, 3, 300, 0) == (6, 1, 0) and _plan(1041, 16, 2082, 0) == (144, 1, 0) and _plan(2600, 16, 800, 150) == (148, 1, 0)
+    for shape, parts, cluster in [((64, 1, 12 * 112, 0), 4, 1), ((130, 3, 150, 6000), 8, 1), ((128, 1, 40000, 0), 20, 0), ((257, 6, 9000, 100), 6, 1),
+                                  ((1100, 2, 2000, 100), 5, 1), ((700, 8, 2000, 0), 3, 0), ((4164, 2, 17697, 0), 2, 1), ((4164, 2, 3000, 300), 2, 1), ((128, 2, 40000, 0), 20, 0)]:
+        items = (shape[0] + 127) // 128 * shape[1]
+        assert _plan(*shape) == (parts * items, parts, cluster), (shape, _plan(*shape))
+    assert _plan(128, 1, 40000, 0, workspace=0)[1:] == (8, 1)       # nowhere to leave more parts
+    assert _plan(0, 1, 5, 0)[0] == 0 and _plan(1, 1, 0, 0)[0] == 0
+    rs = np.random.RandomState(0)
+    for _ in range(3000):
+        M, H, T_hot, T_ret = (int(np.exp(rs.uniform(0, np.log(n)))) for n in (4200, 16, 40000, 4000))
+        T_ret *= int(rs.randint(2))
+        grid, parts, cluster = _plan(M, H, T_hot, T_ret)
+        items, tiles = (M + 127) // 128 * H, -(-T_hot // 112) + -(-T_ret // 112)
+        assert 1 <= parts <= tiles and (parts == 1 or (grid == parts * items <= 148)) and (not cluster or 2 <= parts <= 8)
+        assert parts > 1 or grid == items or (grid == 148 <= items and tiles >= 8)
+
+
 def test_struct_layout_matches_header():
     import ctypes
     from stac_b200 import _lib
