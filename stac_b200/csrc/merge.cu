@@ -2027,7 +2027,8 @@ __device__ __forceinline__ void full_rows_by_warps(const MergeParams& p, const i
 // Many rows: eight lanes per row, each holding eight of the 64 values of a token (16-byte loads), so a warp
 // works on four rows at once.  Tokens are streamed (keys twice: once for the weights, once for
 // the weighted mean; the second read hits the cache) so that few registers are live and many
-// rows are in flight per SM.
+// rows are in flight per SM.  With more bf16 rows than are resident at once, theirs are asked for as soon as their places are known
+// (60 thousand rows 80, 116 -> 73, 107.5 us; fewer, or fp32, took up to 12 % longer with that).
 // (holding all eight key rows of a row in registers, at four CTAs per SM, measured 15 % slower for
 // the whole merge than streaming them at eight CTAs per SM: these per-row kernels want threads)
 template <typename T>
@@ -2036,6 +2037,7 @@ __device__ __forceinline__ void full_rows_by_groups(const MergeParams& p, const 
   const int gbase = lane & 24;                       // first lane of this group
   const unsigned gmask = 0xffu << gbase;
   const int groups = (gridDim.x * blockDim.x) >> 3;
+  const bool ahead = sizeof(T) == 2 && n_full > groups / 2;      // (half of the CTAs are resident at once, see launch_merge)
   for (int wi = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; wi < n_full; wi += groups) {
     const int2 hr = p.full_list[wi];
     const int h = hr.x, ri = hr.y;
@@ -2059,13 +2061,13 @@ __device__ __forceinline__ void full_rows_by_groups(const MergeParams& p, const 
     float ts = 0.f, pw_l = INFINITY;   // lane q < P of a saturated row: weight of pivot q
     if (sub < B) {
       ts = fmaxf(p.buf_S[my_seg], 1e-6f);
-      prefetch_row<T>(reinterpret_cast<uintptr_t>(bK + static_cast<long long>(my_seg) * D));
-      prefetch_row<T>(reinterpret_cast<uintptr_t>(bV + static_cast<long long>(my_seg) * D));
+      if (ahead) prefetch_row<T>(reinterpret_cast<uintptr_t>(bK + static_cast<long long>(my_seg) * D));
+      if (ahead) prefetch_row<T>(reinterpret_cast<uintptr_t>(bV + static_cast<long long>(my_seg) * D));
     }
     if (ps_l >= 0) {
       pw_l = p.piv_W[ps_l];
-      prefetch_row<T>(reinterpret_cast<uintptr_t>(pK + static_cast<long long>(ps_l) * D));
-      prefetch_row<T>(reinterpret_cast<uintptr_t>(pV + static_cast<long long>(ps_l) * D));
+      if (ahead) prefetch_row<T>(reinterpret_cast<uintptr_t>(pK + static_cast<long long>(ps_l) * D));
+      if (ahead) prefetch_row<T>(reinterpret_cast<uintptr_t>(pV + static_cast<long long>(ps_l) * D));
     }
     int seed = 0;
     float seed_s = -INFINITY, sumS = 0.f;
@@ -2227,9 +2229,11 @@ __device__ __forceinline__ void full_rows_by_groups(const MergeParams& p, const 
   }
 }
 
-// (us, eight lanes and a warp per row: 16 heads of 8328 tokens 23.2 and 9.6, 48 heads 25.6 and 10.3, 384 heads with 24 thousand full rows 25.6 and
-// 20.9, 64 thousand in fp32 51 and 55, 768 thousand 252 and 281.)
-constexpr int kManyFullRows = 40000;
+// A warp per row while those are two waves of warps at most (9472 on 148 SMs).  (us, eight lanes and a warp per row, rows with room for the pivot
+// and, behind the comma, without: 960 rows 15.5, 20.8 and 7.1, 10.0; 4800 16.3, 21.9 and 11.7, 17.7; 12000 17.5, 25.7 and 19.1, 30.3; 16000 19.5, 28.9
+// and 24.0, 39.4; 38400 52.8, 76.5 and 57.5, 90; fp32, 4800 16.5, 22.6 and 12.9, 19.5; 16000 24.5, 34.7 and 29.9, 45.6.  Rows that a stream
+// of 48 heads has left in DRAM: 8911 25.1 and 22.9, a stream of 384 heads: 27 thousand 49 and 44, 34 thousand 93 and 101.)
+constexpr int kManyFullRows = 9472;
 template <typename T>
 __global__ void __launch_bounds__(128, 8) rows_phase_b2_kernel(const MergeParams p) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
@@ -2353,6 +2357,7 @@ int launch_merge(MergeParams& mp, cudaStream_t st) {
   if (launch_behind(rows_phase_b1a_kernel, dim3(grid_a1), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(rows_phase_b1m_kernel<T, 2>, dim3(n_sm * 6), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   if (launch_behind(tokens_place_kernel<T>, grid_tok, dim3(kTokBlock), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
+  // (two waves: eight CTAs per SM are resident)
   if (launch_behind(rows_phase_b2_kernel<T>, dim3(n_sm * 16), dim3(128), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
   // (grid-stride over the freed ids, whose number only the device knows)
   if (launch_behind(finalize_kernel<T>, dim3(n_sm * 4), dim3(256), 0, st, mp) != cudaSuccess) return STAC_ERR_CUDA;
