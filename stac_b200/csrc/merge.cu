@@ -246,8 +246,10 @@ __device__ __forceinline__ int warp_scan_sum(int v, int lane) {      // inclusiv
 // 19.4 -> 14.1.  The lists in global memory cost a scattered 4-byte write per key, value and pass, and a round trip
 // to L2 around every block scan, one per 4 kThreads tokens.)
 // False, with nothing written, if a carried token's id does not fit: carried tokens may lie above this call's voxel count.
+// `known`: the items' voxel ids in shared memory (0xFFFF: none), which is written over, or nullptr.
 template <int kThreads, int kItems>
-__device__ __forceinline__ bool sort_tokens_shared(const MergeParams& p, int h, int os, int n_items, unsigned* buf, int* hist) {
+__device__ __forceinline__ bool sort_tokens_shared(const MergeParams& p, int h, int os, int n_items, unsigned* buf, int* hist,
+                                                   const unsigned short* known) {
   constexpr int kWarps = kThreads / 32, kHistRow = 257;
   constexpr unsigned kNone = 0xFFFFu;
   __shared__ int counts[kWarps];
@@ -259,22 +261,29 @@ __device__ __forceinline__ bool sort_tokens_shared(const MergeParams& p, int h, 
   if (threadIdx.x == 0) n_new_valid = n_valid = 0;
   const int n_it = (max(c1 - c0, 0) + 31) / 32;        // rounds of 32 items in which this warp has any
   unsigned item[kItems];
+  if (known != nullptr) {
 #pragma unroll
-  for (int t = 0; t < kItems; ++t) {       // positions first, so that all loads of a thread are in flight together
-    const int i = c0 + t * 32 + lane;
-    item[t] = i;
-    if (t < n_it && p.idx != nullptr && i < c1 && i < p.n_new) item[t] = p.idx[static_cast<long long>(h) * p.n_new + i];
-  }
+    for (int t = 0; t < kItems; ++t)
+      if (t < n_it) item[t] = c0 + t * 32 + lane < c1 ? known[c0 + t * 32 + lane] : kNone;
+    __syncthreads();
+  } else {
 #pragma unroll
-  for (int t = 0; t < kItems; ++t) {
-    if (t < n_it) {
+    for (int t = 0; t < kItems; ++t) {       // positions first, so that all loads of a thread are in flight together
       const int i = c0 + t * 32 + lane;
-      int vx = -1;
-      if (i < c1) {
-        vx = i < p.n_new ? p.vx_src[h * p.meta_head_stride + static_cast<int>(item[t])]
-                         : p.over_hv_in[2 * (os + i - p.n_new) + 1];
+      item[t] = i;
+      if (t < n_it && p.idx != nullptr && i < c1 && i < p.n_new) item[t] = p.idx[static_cast<long long>(h) * p.n_new + i];
+    }
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+      if (t < n_it) {
+        const int i = c0 + t * 32 + lane;
+        int vx = -1;
+        if (i < c1) {
+          vx = i < p.n_new ? p.vx_src[h * p.meta_head_stride + static_cast<int>(item[t])]
+                           : p.over_hv_in[2 * (os + i - p.n_new) + 1];
+        }
+        item[t] = vx;
       }
-      item[t] = vx;
     }
   }
   int* my_hist = hist + warp * kHistRow;
@@ -402,21 +411,29 @@ __device__ __forceinline__ bool sort_tokens_shared(const MergeParams& p, int h, 
 // place in its row is the number of the row's tokens before it.  Two 16-bit counters per word.
 // (The digits of sort_tokens_shared against counters: 16 heads of 8328 tokens, 4000 voxels 21.4 -> 12.8 us, 384 heads 64.5 -> 30.9, 384 heads of
 // 4164 44.1 -> 20.9, 100 heads of 1200 9.5 -> 7.4.)
-// False, with nothing written, if a carried token's id has no counter or a row has more than kMost tokens.
+// That takes the square of a row's tokens in comparisons: with too many in rows of more than kLong tokens the list is sorted by digits, from the
+// voxel ids that are in shared memory already.  (One voxel of 65, 300 and 1000 tokens among 4000: 16 heads of 8328 tokens 13.7, 18.5, 24.9 us, by digits
+// alone 21.1; 384 heads 30.8, 39, 67 and 68; 384 heads of 1041 tokens 12.6, 17.2, 17.4 and 14.4.  Sent back for any row above 64, and loaded
+// again, it was 25.1, 72 and 18 for all of them.  The rare ways out are marked as such: laid out in between, their code made calls that
+// do not take them up to 2 us longer.)
+// kWide, kCrowded: nothing is written; a carried token's id has no counter, or those rows are too long (`vox`: the voxel ids).
+enum { kCounted, kWide, kCrowded };
 template <int kThreads, int kItems>
-__device__ __forceinline__ bool sort_tokens_counted(const MergeParams& p, int h, int os, int n_items, unsigned* smem) {
-  constexpr int kWarps = kThreads / 32, kMost = 64;
+__device__ __forceinline__ int sort_tokens_counted(const MergeParams& p, int h, int os, int n_items, unsigned* smem,
+                                                   const unsigned short** ids) {
+  constexpr int kWarps = kThreads / 32, kLong = 64, kComparisons = 16;      // (of tokens of long rows, per token of the list)
   __shared__ int scan_sums[32];
-  __shared__ int scan_total, n_new_valid, n_valid;
+  __shared__ int scan_total, n_new_valid, n_valid, comparisons;
   const int V = p.voxel_used, words = (V + 1) / 2;
   unsigned* cnt = smem;                                                       // [words]
   unsigned short* row_of = reinterpret_cast<unsigned short*>(smem + words);   // [V]: rows before a voxel's
   unsigned short* vox = reinterpret_cast<unsigned short*>(smem + 2 * words);  // [n_items]: a token's voxel id, kNone: it has none
   unsigned short* buf = vox + kThreads * kItems;                              // [n_items]: tokens in the order of their voxels
+  *ids = vox;
   constexpr unsigned short kNone = 0xFFFFu;
   const int tid = threadIdx.x, lane = tid & 31;
   for (int w = tid; w < words; w += kThreads) cnt[w] = 0u;
-  if (tid == 0) n_new_valid = n_valid = 0;
+  if (tid == 0) n_new_valid = n_valid = comparisons = 0;
   int item[kItems];                  // voxel id, -1: none
 #pragma unroll
   for (int t = 0; t < kItems; ++t) {       // positions first, so that all loads of a thread are in flight together
@@ -449,7 +466,7 @@ __device__ __forceinline__ bool sort_tokens_counted(const MergeParams& p, int h,
     atomicAdd(&n_new_valid, new_valid);
     atomicAdd(&n_valid, valid);
   }
-  if (__syncthreads_or(wide)) return false;
+  if (__syncthreads_or(wide)) return kWide;
   // exclusive scan over the voxels of (rows << 16 | tokens); an odd number of words per thread: no bank conflicts
   const int per = ((words + kThreads - 1) / kThreads) | 1, w0 = min(words, tid * per), w1 = min(words, w0 + per);
   int sum = 0, most = 0;
@@ -458,8 +475,19 @@ __device__ __forceinline__ bool sort_tokens_counted(const MergeParams& p, int h,
     sum += lo + hi + ((lo > 0 ? 1 : 0) + (hi > 0 ? 1 : 0)) * 65536;
     most = max(most, max(lo, hi));
   }
+  if (__builtin_expect(__syncthreads_or(most > kLong), 0)) {
+    if (most > kLong) {
+      int squares = 0;                        // (9216 squared at most)
+      for (int w = w0; w < w1; ++w) {
+        const int lo = static_cast<int>(cnt[w] & 0xffffu), hi = static_cast<int>(cnt[w] >> 16);
+        squares += (lo > kLong ? lo * lo : 0) + (hi > kLong ? hi * hi : 0);
+      }
+      atomicAdd(&comparisons, squares);
+    }
+    __syncthreads();
+    if (comparisons > kComparisons * n_items) return kCrowded;
+  }
   int run = block_scan<kWarps>(sum, scan_sums, &scan_total);
-  if (__syncthreads_or(most > kMost)) return false;
   for (int w = w0; w < w1; ++w) {
     const int lo = static_cast<int>(cnt[w] & 0xffffu), hi = static_cast<int>(cnt[w] >> 16);
     const int run_hi = run + lo + (lo > 0 ? 65536 : 0);
@@ -509,11 +537,11 @@ __device__ __forceinline__ bool sort_tokens_counted(const MergeParams& p, int h,
     p.n_tok[h] = n;
     if (n_new_valid > 0) atomicOr(&p.plan[kPlanAnyValid], 1);
   }
-  return true;
+  return kCounted;
 }
 
 template <int kThreads, int kMinCtas, int kItems>
-__global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const MergeParams p) {
+__global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const __grid_constant__ MergeParams p) {
   constexpr int kWarps = kThreads / 32;
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel of the call
   // Digit counters, [warp][digit]: a warp's lanes count different digits of the same warp, so neighbouring
@@ -530,12 +558,15 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) sort_tokens_kernel(const M
   const int h = blockIdx.x;
   if constexpr (kItems > 0) {
     const int os = p.over_start_in[h], n_items = p.n_new + p.over_start_in[h + 1] - os;
+    const unsigned short* known = nullptr;
     if (p.counted && n_items <= min(p.ncap, kThreads * kItems)) {
-      if (sort_tokens_counted<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem))) return;
+      const int how = sort_tokens_counted<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem), &known);
+      if (__builtin_expect(how == kCounted, 1)) return;
+      if (how == kWide) known = nullptr;
       __syncthreads();
     }
     if (n_items <= min(p.ncap, kThreads * kItems) && p.voxel_used <= 0xFFFF &&
-        sort_tokens_shared<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem + kHistRow * kWarps), hist))
+        sort_tokens_shared<kThreads, kItems>(p, h, os, n_items, reinterpret_cast<unsigned*>(sort_smem + kHistRow * kWarps), hist, known))
       return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
