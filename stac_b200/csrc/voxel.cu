@@ -200,26 +200,34 @@ __global__ void resolve_pending_kernel(const long long* __restrict__ pt_keys, in
 // many tokens the probes and the flags that are set again and again decide, and many tokens lie in one voxel: where one CTA has
 // a token's whole cube and that is more than a warp's work (radius 2), and there are kMarkTokens, the first of a voxel's tokens
 // marks it and the others leave.
+// Cubes of up to 32 offsets (radius 0 and 1) are a thread's and a warp's work: with more than kManyTokens, CTAs of several tokens.  (Radius 0, 8328 tokens in 200
+// voxels and in voxels of their own, 20000 in 200: 6.2, 7.3, 7.4 us, with a CTA each 9.8, 10.9, 16.0; radius 1, 8328 tokens 8.6 and 10.2, with a CTA each
+// 10.3 and 12.0; up to 1041 tokens 0.3 us more than with one each.)
 // (A thread per token and offset, radius 2: four frames of 1041 tokens of a stream 16 -> 8.8 us, one 8.6 -> 7.0; 4164 tokens in
 // 900 voxels 29.7 -> 17.4, each in its own 25 -> 23.6.  32 tokens are a chain of latencies: 13.3 us, with marks 15.4.)
 constexpr unsigned kWantedFlag = 1u, kSeenFlag = 2u;    // of a voxel's byte: to be listed; a token in it has been here
-constexpr int kCtaOffsets = 128, kMarkTokens = 512;
-__global__ void neighbor_flag_kernel(const int* __restrict__ token_vx, int R, int mark,
+constexpr int kCtaOffsets = 128, kMarkTokens = 512, kManyTokens = 2048;
+static_assert(kCtaOffsets == 1 << 7, "lane_bits of a CTA");
+// kLaneBits: log2 of a token's threads (kCtaOffsets of them: the CTA is one token's)
+template <int kLaneBits>
+__global__ void neighbor_flag_kernel(const int* __restrict__ token_vx, int n_tokens, int R, int mark,
                                      const long long* __restrict__ table_keys, const int* __restrict__ n_voxels,
                                      const unsigned long long* __restrict__ hk, const int* __restrict__ hv, int hcap,
                                      unsigned* __restrict__ flags) {
   grid_dep_wait();   // launched with programmatic serialization behind the previous kernel in the stream
   __shared__ bool seen;
-  const int id = token_vx[blockIdx.x];
+  constexpr bool kOne = (1 << kLaneBits) == kCtaOffsets;
+  const int t = kOne ? blockIdx.x : blockIdx.x * (blockDim.x >> kLaneBits) + (threadIdx.x >> kLaneBits);
+  const int id = kOne || t < n_tokens ? token_vx[t] : -1;
   if (id < 0 || id >= *n_voxels) return;
   auto flag = [&](int v, unsigned bits) { return atomicOr(flags + (v >> 2), bits << (8 * (v & 3))) >> (8 * (v & 3)); };
   const long long center = table_keys[id];
-  if (mark) {
+  if (kOne && mark) {
     if (threadIdx.x == 0) seen = (flag(id, kSeenFlag) & kSeenFlag) != 0;
     __syncthreads();
     if (seen) return;
   }
-  const int side = 2 * R + 1, o = blockIdx.y * kCtaOffsets + threadIdx.x;
+  const int side = 2 * R + 1, o = blockIdx.y * kCtaOffsets + (threadIdx.x & ((1 << kLaneBits) - 1));
   const int xy = o / side, x = xy / side;
   if (x >= side) return;
   const long long dx = x - R, dy = xy - x * side - R, dz = o - xy * side - R;
@@ -452,10 +460,12 @@ int stac_voxel_neighbors(const int* token_voxel_ids, int n_tokens, int radius_ce
   if (!all_ids && n_tokens > 0) {
     if (token_voxel_ids == nullptr) return STAC_ERR_BAD_ARG;
     const int side = 2 * radius_cells + 1, chunks = (side * side * side + stac::kCtaOffsets - 1) / stac::kCtaOffsets;
-    const int threads = chunks > 1 ? stac::kCtaOffsets : (side * side * side + 31) / 32 * 32;
-    const int mark = chunks == 1 && threads > 32 && n_tokens >= stac::kMarkTokens ? 1 : 0;
-    if (stac::launch_behind(stac::neighbor_flag_kernel, dim3(n_tokens, chunks), dim3(threads), 0, st,
-                            token_voxel_ids, radius_cells, mark, reinterpret_cast<const long long*>(table_keys),
+    const int lane_bits = n_tokens <= stac::kManyTokens || radius_cells > 1 ? 7 : 5 * radius_cells;
+    const int threads = lane_bits < 7 ? 256 : chunks > 1 ? stac::kCtaOffsets : (side * side * side + 31) / 32 * 32;
+    const int tokens = lane_bits < 7 ? threads >> lane_bits : 1, mark = radius_cells == 2 && n_tokens >= stac::kMarkTokens ? 1 : 0;
+    auto* const kernel = lane_bits == 0 ? stac::neighbor_flag_kernel<0> : lane_bits == 5 ? stac::neighbor_flag_kernel<5> : stac::neighbor_flag_kernel<7>;
+    if (stac::launch_behind(kernel, dim3((n_tokens - 1) / tokens + 1, chunks), dim3(threads), 0, st,
+                            token_voxel_ids, n_tokens, radius_cells, mark, reinterpret_cast<const long long*>(table_keys),
                             n_voxels, static_cast<const unsigned long long*>(hash_keys), hash_vals,
                             static_cast<int>(hash_cap), reinterpret_cast<unsigned*>(flags)) != cudaSuccess)
       return STAC_ERR_CUDA;
