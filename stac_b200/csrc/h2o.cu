@@ -48,7 +48,10 @@ __device__ __forceinline__ unsigned int float_key(float f) {
 // keys lie in shared memory: from 18881 tokens only two fit an SM, from 28 thousand only one, and the larger CTAs have twice
 // the warps there (19500 tokens 43.9, 52.2, 33000 tokens 79, 111).
 constexpr int kSelectStaticSmem = 1280;      // counters and such, rounded up
-constexpr int kSelectFew = 256;              // keys that share a prefix and are ranked against one another: they fit the counters' memory
+// Keys that share a prefix and are ranked against one another, which takes the square of their number: they fit the counters' memory.  (Up to 256
+// of them: rows of 300 equal scores 9.7 against 5.6 us, 384 rows, and 7.0 with four passes before there was a ranking; 600 and 1041 small whole numbers 10.6, 11.2
+// against 7.0, 7.2; 4164 scores over many decades 17.3 against 11.2.  Up to 64 or 32: no better.)
+constexpr int kSelectFew = 128;
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads)
 h2o_select_kernel(const float* __restrict__ scores, long long row_stride, const unsigned char* __restrict__ is_base,
