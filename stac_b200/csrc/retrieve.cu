@@ -25,7 +25,7 @@ constexpr int kFineKeys = 128;    // keys in whose places 256 counters lie
 constexpr int kSelBins = 8192;    // counters of one radix digit (13 + 11 + 8 bits, most significant first)
 constexpr int kRankKeys = 3072;   // collected keys that are ranked by their places in the range of keys: two copies of them and
 constexpr int kRankBins = 4096;   // so many counters fill the buffer
-constexpr int kRankMost = 192;    // keys of one counter that are compared with one another
+constexpr int kRankPairs = 1 << 18;    // comparisons of keys of one counter with one another
 static_assert(2 * kRankKeys * 8 + kRankBins * 4 <= kSelCap * 8, "ranking in the candidate buffer");
 constexpr int kSelUnroll = 2;     // queried voxels per thread in flight
 // Threads of the selection kernel.  With more heads than SMs three CTAs of 512 share an SM and hide each
@@ -382,7 +382,9 @@ retrieve_select_kernel(const RetrieveParams p) {
     // scan of them), and a key's place among those of its piece is the number of larger ones.  Where weights crowd in one piece,
     // many equal ones or a few far above the others, the keys are sorted instead, below.
     // (us per retrieval with select and sort for all, and now: 16 heads, R = 2048 34.5 -> 22.8, 384 heads 60.3 -> 45.8, with 12.9 thousand queried
-    // voxels 119 -> 94, 48 heads, R = 2082 51 -> 39.)
+    // voxels 119 -> 94, 48 heads, R = 2082 51 -> 39.  About 2800 keys with 190, 400, 600 equal ones per head: 16 heads 16.1, 19.8, 27.1, sorted
+    // 26.9; 384 heads 111, 121, 130 and 130.  The sort behind an attempt takes 0.3 to 1.0 us more than without it.  Twice as many comparisons: 384 heads
+    // with 800 equal keys of 1200 75 against 56, sorted 53.)
     unsigned long long lo = ~0ull, hi = 0ull;
     for (int i = threadIdx.x; i < cnt; i += kSelThreads) {
       const unsigned long long x = cand[i];
@@ -401,6 +403,7 @@ retrieve_select_kernel(const RetrieveParams p) {
     }
     int* const piece = reinterpret_cast<int*>(cand + 2 * kRankKeys);
     for (int i = threadIdx.x; i < kRankBins; i += kSelThreads) piece[i] = 0;
+    if (threadIdx.x == 0) sh_above = 0;
     __syncthreads();
     lo = placed[lane % (kSelThreads / 32)];
     hi = placed[32 + lane % (kSelThreads / 32)];
@@ -416,12 +419,12 @@ retrieve_select_kernel(const RetrieveParams p) {
     for (int i = threadIdx.x; i < cnt; i += kSelThreads) atomicAdd(&piece[piece_of(cand[i])], 1);
     __syncthreads();
     constexpr int kPer = kRankBins / kSelThreads;
-    int c[kPer], sum = 0, most = 0;
+    int c[kPer], sum = 0, pairs = 0;
 #pragma unroll
     for (int e = 0; e < kPer; ++e) {
       c[e] = piece[threadIdx.x * kPer + e];
       sum += c[e];
-      most = max(most, c[e]);
+      pairs += c[e] * c[e];
     }
     int incl = sum;
 #pragma unroll
@@ -430,7 +433,10 @@ retrieve_select_kernel(const RetrieveParams p) {
       if (lane >= o) incl += t;
     }
     if (lane == 31) warp_sums[warp] = incl;
-    if (!__syncthreads_or(most > kRankMost)) {
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    if (lane == 0) atomicAdd(&sh_above, pairs);      // (the square of kRankKeys at most)
+    __syncthreads();
+    if (sh_above <= kRankPairs) {
       int run = lane < warp ? warp_sums[lane] : 0;     // (at most 32 warps)
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) run += __shfl_xor_sync(0xffffffffu, run, o);
