@@ -47,7 +47,8 @@ __device__ __forceinline__ unsigned int float_key(float f) {
 // (384 rows, 1024 against 512 threads: 8328 tokens 29.7, 25.6 us, 15615 tokens 38.3, 34.8, 18600 tokens 43.0, 41.5.)  A row's
 // keys lie in shared memory: from 18881 tokens only two fit an SM, from 28 thousand only one, and the larger CTAs have twice
 // the warps there (19500 tokens 43.9, 52.2, 33000 tokens 79, 111).
-constexpr int kSelectStaticSmem = 1280;      // counters and such, rounded up
+constexpr int kSelectStaticSmem = 1280;      // counters and such of a CTA of 512 threads, rounded up
+static_assert(kSelectStaticSmem >= (256 + 2 * 512 / 32 + 4) * 4, "static shared memory of the selection kernel");
 // Keys that share a prefix and are ranked against one another, which takes the square of their number: they fit the counters' memory.  (Up to 256
 // of them: rows of 300 equal scores 9.7 against 5.6 us, 384 rows, and 7.0 with four passes before there was a ranking; 600 and 1041 small whole numbers 10.6, 11.2
 // against 7.0, 7.2; 4164 scores over many decades 17.3 against 11.2.  Up to 64 or 32: no better.)

@@ -49,6 +49,16 @@ def _run_two_segment(M, H, T_hot, T_ret, seed, T_buf=None, subsample=1.0, spread
     return (out.float().cpu().numpy(), lse.cpu().numpy(), cs.cpu().numpy()), (o_ref, lse_ref, cs_ref)
 
 
+def _parts(M, H, T_hot, T_ret):
+    """In how many parts each item of the call is cut on this GPU, and whether by plan a cluster joins them."""
+    import ctypes
+    from stac_b200 import _lib
+    parts, cluster = ctypes.c_int(), ctypes.c_int()
+    n_sm = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _lib.lib().stac_attn_forward_plan(M, H, T_hot, T_ret, n_sm, 1, ctypes.byref(parts), ctypes.byref(cluster)) > 0
+    return parts.value, bool(cluster.value)
+
+
 def _assert_close(got, ref):
     (o, lse, cs), (o_ref, lse_ref, cs_ref) = got, ref
     assert np.isfinite(o).all() and np.isfinite(cs).all()
@@ -127,9 +137,9 @@ def test_forward_units_split_over_all_sms():
 @pytest.mark.parametrize("M,H,T_hot,T_ret,spread", [(700, 2, 2500, 140, 1.0), (4164, 2, 3000, 300, 1.0),
                                                      (300, 16, 3400, 140, 2.0), (520, 3, 1777, 0, 1.0)])
 def test_forward_items_cut_in_two_halves(M, H, T_hot, T_ret, spread):
-    """Few heads (a head-sharded stream): at most half as many (head, query tile) items as SMs
-    and long key ranges, so every item is computed by two CTAs, half of the key tiles each (an odd
-    tile count in the last case), and joined."""
+    """Few heads: at most half as many (head, query tile) items as SMs and long key ranges, so every item is computed by several
+    CTAs and joined: in five parts, in halves (a head-sharded stream of two heads), in three and in four."""
+    assert _parts(M, H, T_hot, T_ret) == {700: (5, True), 4164: (2, True), 300: (3, False), 520: (4, True)}[M]
     got, ref = _run_two_segment(M, H, T_hot, T_ret, seed=M + H, spread=spread)
     _assert_close(got, ref)
     again, _ = _run_two_segment(M, H, T_hot, T_ret, seed=M + H, spread=spread)
@@ -192,7 +202,8 @@ def test_one_key_far_above_the_first_keys():
     (130, 3, 300, 0),        # one CTA per item, a segment of three tiles
     (130, 2, 449, 130),      # a tile of one key, masked pivots
     (2600, 16, 800, 150),    # items cut over the SMs: parts of all lengths, several segments per CTA
-    (1100, 2, 2000, 100),    # items in halves
+    (1100, 2, 2000, 100),    # items in five parts
+    (4164, 2, 1200, 100),    # items in halves
 ])
 @pytest.mark.parametrize("first,last", [(0.4, 0.6), (0.97, 1.0), (0.2, 1.0)])       # where the keys are that are far from the others
 def test_some_segments_are_walked_twice(M, H, T_hot, T_ret, first, last):
@@ -232,8 +243,10 @@ def test_some_segments_are_walked_twice(M, H, T_hot, T_ret, first, last):
     (300, 2, 2500, 260),         # six items
     (130, 3, 150, 6000),         # mostly retrieved keys, a cluster of eight
     (128, 1, 40000, 0),          # more parts than a cluster has CTAs: through the workspace
-    (257, 6, 9000, 100),         # more items than clusters of the best size: through the workspace
-    (700, 8, 2000, 0),           # 48 items in halves
+    (257, 6, 9000, 100),         # clusters of six
+    (700, 8, 2000, 0),           # more items than clusters of the best size: through the workspace, 48 items in three parts
+    (128, 2, 40000, 0),          # two items of twenty parts through the workspace
+    (4164, 2, 3000, 300),        # 66 items in halves, a stream of two heads
 ])
 @pytest.mark.parametrize("kind", ["plain", "far", "masked"])
 def test_items_in_many_parts(M, H, T_hot, T_ret, kind):
@@ -253,6 +266,8 @@ def test_items_in_many_parts(M, H, T_hot, T_ret, kind):
     dev = torch.device("cuda:0")
     status = ops.DeviceStatus(dev)
     ret = (kr.to(dev), vr.to(dev), torch.from_numpy(bias).to(dev), T_ret) if T_ret else (None, None, None, 0)
+    assert _parts(M, H, T_hot, T_ret) == {(64, 1): (4, True), (1, 1): (5, True), (300, 2): (7, True), (130, 3): (8, True), (128, 1): (20, False),
+                                          (257, 6): (6, True), (700, 8): (3, False), (128, 2): (20, False), (4164, 2): (2, True)}[M, H]
     got, again = (ops.attn_colsum(q.to(dev), k.to(dev), v.to(dev), T_hot, *ret, want_lse=True, status=status) for _ in range(2))
     torch.cuda.synchronize()
     status.raise_if_set("attention")
