@@ -46,11 +46,11 @@ class LaggedInts:
         self.pin = torch.zeros(n, dtype=torch.int32).pin_memory()
         self.host, self.event, self.waiting = self.pin.data_ptr(), None, False      # one event, recorded again by every push
 
-    def push(self, *tensors):
+    def push(self, first, second=None, *more):
         """(Copies and event in one call of the library: 14 -> 5 us with two tensors against torch's.)"""
-        if len(tensors) not in (1, 2) or not all(t.is_cuda and t.dtype is torch.int32 and t.is_contiguous() for t in tensors):
-            tensors = (torch.cat([t.reshape(-1).to("cuda", torch.int32) for t in tensors]),)
-        first, second = tensors if len(tensors) == 2 else (tensors[0], None)
+        if more or not self._plain(first) or not (second is None or self._plain(second)):
+            tensors = (first, *((second,) if second is not None else ()), *more)
+            first, second = torch.cat([t.reshape(-1).to("cuda", torch.int32) for t in tensors]), None
         n, m = first.numel(), 0 if second is None else second.numel()
         assert n + m <= self.pin.numel()
         if self.event is None:
@@ -60,6 +60,10 @@ class LaggedInts:
         check(_lib.lib().stac_ints_to_host(self.host, first.data_ptr(), n, ptr(second), m, self.event, stream_ptr()),
               "stac_ints_to_host")
         self.waiting = True
+
+    @staticmethod
+    def _plain(t):
+        return t.is_cuda and t.dtype is torch.int32 and t.is_contiguous()
 
     def pending(self):
         return self.waiting

@@ -239,7 +239,9 @@ class KVManager:
         assert new_T % self.token_per_f == 0, "T_new must be a multiple of token_per_frame in append_kv()."
         slot = self._to_slot(layer_idx, strict=True)
         old_T = self._offset_hot[slot]
-        k, v = key_states.squeeze(0), value_states[0]      # (one batch of keys, see above; whatever values come, three dimensions go on)
+        k, v = key_states.squeeze(0), value_states.squeeze(0)
+        if v.dim() != 3 or value_states.dim() != 4:      # (only the keys are known to have one batch; indexing costs twice as much as squeezing)
+            v = value_states[0]
         if k.dtype != self.dtype or v.dtype != self.dtype or not k.is_cuda:
             k, v = k.to(self.device, self.dtype), v.to(self.device, self.dtype)
         # the GPU buffer takes the LAST tokens that fit, the host buffer the first ones
