@@ -407,21 +407,33 @@ __device__ __forceinline__ bool sort_tokens_shared(const MergeParams& p, int h, 
   return true;
 }
 
+// Comparisons that the rows of more than kLongCounted tokens take, of all threads (`comparisons`: zero before).  A function of its own: in line, its code
+// made calls without such rows up to 2 us longer.
+constexpr int kLongCounted = 64;
+__device__ __noinline__ int comparisons_of_long_rows(const unsigned* cnt, int w0, int w1, int* comparisons) {
+  int squares = 0;                        // (9216 squared at most)
+  for (int w = w0; w < w1; ++w) {
+    const int lo = static_cast<int>(cnt[w] & 0xffffu), hi = static_cast<int>(cnt[w] >> 16);
+    squares += (lo > kLongCounted ? lo * lo : 0) + (hi > kLongCounted ? hi * hi : 0);
+  }
+  if (squares > 0) atomicAdd(comparisons, squares);
+  __syncthreads();
+  return *comparisons;
+}
 // A counter per voxel id of the call instead of digits: tokens are scattered to the places of their voxel in any order, and a token's
 // place in its row is the number of the row's tokens before it.  Two 16-bit counters per word.
 // (The digits of sort_tokens_shared against counters: 16 heads of 8328 tokens, 4000 voxels 21.4 -> 12.8 us, 384 heads 64.5 -> 30.9, 384 heads of
 // 4164 44.1 -> 20.9, 100 heads of 1200 9.5 -> 7.4.)
-// That takes the square of a row's tokens in comparisons: with too many in rows of more than kLong tokens the list is sorted by digits, from the
-// voxel ids that are in shared memory already.  (One voxel of 65, 300 and 1000 tokens among 4000: 16 heads of 8328 tokens 13.7, 18.5, 24.9 us, by digits
-// alone 21.1; 384 heads 30.8, 39, 67 and 68; 384 heads of 1041 tokens 12.6, 17.2, 17.4 and 14.4.  Sent back for any row above 64, and loaded
-// again, it was 25.1, 72 and 18 for all of them.  The rare ways out are marked as such: laid out in between, their code made calls that
-// do not take them up to 2 us longer.)
+// That takes the square of a row's tokens in comparisons: with too many in rows of more than kLongCounted tokens the list is sorted by digits, from the
+// voxel ids that are in shared memory already.  (One voxel of 65, 300 and 1000 tokens among 4000: 16 heads of 8328 tokens 13.5, 18.3, 24.9 us, by digits
+// alone 21.1; 384 heads 31.0, 38, 67 and 68; 384 heads of 1041 tokens 13.7, 17.2, 17.4 and 14.4.  Sent back for any row above 64, and loaded
+// again, it was 25.1, 72 and 18 for all of them.)
 // kWide, kCrowded: nothing is written; a carried token's id has no counter, or those rows are too long (`vox`: the voxel ids).
 enum { kCounted, kWide, kCrowded };
 template <int kThreads, int kItems>
 __device__ __forceinline__ int sort_tokens_counted(const MergeParams& p, int h, int os, int n_items, unsigned* smem,
                                                    const unsigned short** ids) {
-  constexpr int kWarps = kThreads / 32, kLong = 64, kComparisons = 16;      // (of tokens of long rows, per token of the list)
+  constexpr int kWarps = kThreads / 32, kComparisons = 16;      // (of tokens of long rows, per token of the list)
   __shared__ int scan_sums[32];
   __shared__ int scan_total, n_new_valid, n_valid, comparisons;
   const int V = p.voxel_used, words = (V + 1) / 2;
@@ -475,18 +487,9 @@ __device__ __forceinline__ int sort_tokens_counted(const MergeParams& p, int h, 
     sum += lo + hi + ((lo > 0 ? 1 : 0) + (hi > 0 ? 1 : 0)) * 65536;
     most = max(most, max(lo, hi));
   }
-  if (__builtin_expect(__syncthreads_or(most > kLong), 0)) {
-    if (most > kLong) {
-      int squares = 0;                        // (9216 squared at most)
-      for (int w = w0; w < w1; ++w) {
-        const int lo = static_cast<int>(cnt[w] & 0xffffu), hi = static_cast<int>(cnt[w] >> 16);
-        squares += (lo > kLong ? lo * lo : 0) + (hi > kLong ? hi * hi : 0);
-      }
-      atomicAdd(&comparisons, squares);
-    }
-    __syncthreads();
-    if (comparisons > kComparisons * n_items) return kCrowded;
-  }
+  if (__builtin_expect(__syncthreads_or(most > kLongCounted), 0) &&
+      comparisons_of_long_rows(cnt, w0, w1, &comparisons) > kComparisons * n_items)
+    return kCrowded;
   int run = block_scan<kWarps>(sum, scan_sums, &scan_total);
   for (int w = w0; w < w1; ++w) {
     const int lo = static_cast<int>(cnt[w] & 0xffffu), hi = static_cast<int>(cnt[w] >> 16);
