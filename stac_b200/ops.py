@@ -108,6 +108,8 @@ _dropped = collections.deque()
 
 
 def _free_dropped():
+    if not _dropped or torch.cuda.is_current_stream_capturing():      # (an event must not be asked during a capture)
+        return
     for _ in range(len(_dropped)):
         try:
             pin, event = _dropped.popleft()

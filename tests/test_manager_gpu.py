@@ -454,7 +454,9 @@ def test_lagged_ints_are_dropped_without_a_wait():
     with torch.cuda.graph(g):
         x += 1
         del m
+        ops._free_dropped()      # (as a new mirror does)
         x += 1
+    assert len(ops._dropped) == 1
     g.replay()
     assert x.tolist() == [2, 2, 2]
     ops._free_dropped()
